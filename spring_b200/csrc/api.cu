@@ -338,7 +338,7 @@ int spring_ctx_destroy(spring_ctx* c) {
         dfree(c->d_scr_rep); dfree(c->d_tc_keys); dfree(c->d_tc_keys_s); dfree(c->d_tc_vals); dfree(c->d_tc_cnt);
         dfree(c->d_tc_seg); dfree(c->d_tc_ntl); dfree(c->d_tc_toff); dfree(c->d_tc_sort);
         dfree(c->d_scan_tmp); dfree(c->d_w); dfree(c->d_lw_all); dfree(c->d_lw_tmp); dfree(c->d_p3);
-        dfree(c->d_kappa); dfree(c->d_krn); dfree(c->d_rxyz); dfree(c->d_wiso);
+        dfree(c->d_kappa); dfree(c->d_krn); dfree(c->d_rxyz); dfree(c->d_wiso); dfree(c->d_tet_tab);
         free_enum4(c);
         dfree(c->d_v4_ph); dfree(c->d_v4_etab); dfree(c->d_v4_wf); dfree(c->d_v4_c); dfree(c->d_v4_map);
         dfree(c->d_v4_img); dfree(c->d_v4_cnt); dfree(c->d_v4_seg); dfree(c->d_v4_ntl); dfree(c->d_v4_toff);
@@ -792,6 +792,7 @@ int spring_compute_phonons(spring_ctx* c, const double* temps, double freq_cut) 
     SPRING_CHECK(set_temps(c, temps));
     SPRING_CHECK(alloc_phonons(c, c->ph_grid, c->nq));
     SPRING_CHECK(alloc_phonons(c, c->ph_irr, c->nq0));
+    SPRING_CHECK(alloc_tetra_tables(c));
     SPRING_CHECK(run_phonons_mesh(c));
     c->ph_grid.set = c->ph_irr.set = true;
     c->ph_gen += 1;
@@ -817,6 +818,7 @@ int spring_set_phonons(spring_ctx* c, int which, const double* temps, const doub
     Phonons& p = which == 0 ? c->ph_grid : c->ph_irr;
     const int n = which == 0 ? c->nq : c->nq0;
     SPRING_CHECK(alloc_phonons(c, p, n));
+    if (which == 0) SPRING_CHECK(alloc_tetra_tables(c));
     const size_t nd = c->ndof;
     SPRING_CHECK(h2d(c, p.evec.p, evec, sizeof(double2) * n * nd * nd, "eigenvectors"));
     SPRING_CHECK(h2d(c, p.omega.p, omega, sizeof(double) * n * nd, "omega"));
@@ -928,6 +930,7 @@ int spring_linewidth3(spring_ctx* c, int i0_first, int n_q0, int delta_mode, dou
         const int slots = w_slots(c, n_q0);
         const size_t slot = (size_t)c->nq * c->ndof * c->ndof * c->ndof;
         SPRING_CHECK(dalloc(c, c->d_w, slot * slots, "W buffer"));
+        SPRING_CHECK(run_tetra_tables(c));
         for (int b = 0; b < n_q0; b += slots) {
             const int nb = std::min(slots, n_q0 - b);
             SPRING_CHECK(run_v3_wgrid(c, c->ps_irr, irr_view(c), q0 + b, nb, c->d_w.p));

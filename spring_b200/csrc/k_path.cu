@@ -418,7 +418,7 @@ PathQ2Args path_q2_args(spring_ctx* c) {
 }  // namespace
 
 void path_release(PathPlan& p) {
-    dfree(p.q0v); dfree(p.q1v); dfree(p.q2v); dfree(p.w); dfree(p.lw); dfree(p.p3); dfree(p.zc); dfree(p.ex);
+    dfree(p.q0v); dfree(p.q1v); dfree(p.q2v); dfree(p.w); dfree(p.lw); dfree(p.p3); dfree(p.zc); dfree(p.ex); dfree(p.tab2);
     free_phonons(p.php);
     free_phonons(p.ph2);
     p.n_path = 0;
@@ -492,7 +492,7 @@ int path_enqueue(spring_ctx* c, PathPlan& p, int delta_mode, double sigma) {
             p.ph2.omega.p, p.w.p);
         SPRING_CHECK(launch_check(c, "k_v3_path"));
         if (delta_mode == SPRING_DELTA_TETRA) {
-            SPRING_CHECK(run_tetra3_path(c, p0, ns, n_path, p.w.p, p.php.omega.p, p.ph2.omega.p, p.ph2.nbe.p, rows,
+            SPRING_CHECK(run_tetra3_path(c, p0, ns, n_path, p.w.p, p.php.omega.p, p.ph2.omega.p, p.ph2.nbe.p, p.tab2.p,
                                          p.lw.p, p.p3.p));
         } else {
             const double os = 1.0 / sigma;
@@ -522,6 +522,8 @@ int run_path(spring_ctx* c, int n_path, const double* h_q0, const int* h_zc, int
              double* h_lw, double* h_omega) {
     PathPlan p;
     int rc = path_prepare(c, p, n_path, h_q0, h_zc);
+    if (rc == SPRING_OK && delta_mode == SPRING_DELTA_TETRA)
+        rc = dalloc(c, p.tab2, (size_t)p.slots * c->nq * tetra_table_doubles(c), "path tetrahedron tables");
     if (rc == SPRING_OK) rc = path_enqueue(c, p, delta_mode, sigma);
     if (rc == SPRING_OK) rc = path_fetch(c, p, h_lw, h_omega);
     cudaStreamSynchronize(c->stream);

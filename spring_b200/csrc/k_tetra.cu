@@ -6,172 +6,251 @@
 // Isotope: CalculateIsoW + CalculateIsoLwTetra (src/Kappa/Src/IsotopicScatter.f90:36-168),
 // and a Gaussian form delta(omega0 - omega1).
 //
-// One thread per (q0, tetrahedron, s1, s2).  The vertex energies of the three
-// channels (w1+w2, w2-w1, w1-w2) do not depend on s0, so each channel is sorted
-// once per thread (stable: ties keep the original vertex order, which is what
-// my_sort's first-uncovered search produces) and reused for every s0 and
-// temperature.  Case bounds, formulas and the order of the vertex sum follow
-// the reference; only the summation order over tetrahedra differs (partial
-// sums per thread, then warp/CTA reduction).
-// Roofline: FP64 ALU (about 60 flops and 10 divisions per tetrahedron, mode
-// triple and channel); W is read from the L2-resident W grid.
+// Nearly every (tetrahedron, s0, s1, s2) misses: at 16^3 about 2 % of the energies w0 lie inside a
+// tetrahedron's range.  So each warp screens 32 tetrahedra at a time in FP32 (range of the vertex
+// energies against the w0 of the pass, widened by far more than the rounding), queues the hits in
+// shared memory, and evaluates them 32 at a time in FP64 with the exact bounds: no lane idles through
+// another lane's divisions.  Screening reads single-precision frequencies and the evaluation reads mode
+// records (n(T), w), both laid out [s][q] so that a warp's neighbouring tetrahedra share cache lines.
+// With the same branch window on both legs the sums use the partner map's symmetry: p maps the
+// tetrahedra onto themselves and swaps the legs, W with them, so channel 3 equals channel 2 (weight 2)
+// and channel 1 needs s1 <= s2 only (weight 2 off the diagonal).
+// Case bounds and formulas follow the reference; the summation order differs (per-lane sums, then
+// warp/CTA reduction).
+// Roofline: issue (the screen) and the FP64 pipe (the evaluation); W is read from the L2-resident grid.
+// Two-atom cell, three temperatures, every irreducible q0: 16^3 140.7 -> 2.2 ms, 24^3 1135 -> 17.8 ms
+// against one thread per (tetrahedron, s1, s2) that ran every weight formula any lane of its warp needed.
+// Three blocks per SM (170 registers) beat four and five (17.8, 18.3, 19.3 ms at 24^3): the evaluation
+// waits on dependent loads, and more of them in flight per lane help more than more warps.
 #include "spring_internal.cuh"
 #include "tetra.cuh"
 
 namespace spring {
 namespace {
 
-constexpr int NS0 = 6;  // s0 values per pass (register accumulators)
+constexpr int NS0 = 6;   // s0 values per pass
+constexpr int BS2 = 6;   // s2 values of a unit, held in shared memory
+constexpr int TW = 4;    // warps per block
 
 struct TetArgs {
     int n, nq, nq0, nT, ntet;
-    long long ntab;  // rows of the q2 table (path mode)
     int q0_first;
-    int s0a, s0n;  // s0 pass: [s0a, s0a + s0n)
-    int lo1, n1, lo2, n2;
+    int lo0, hi0;        // s0 window
+    int lo1, hi1, lo2, hi2;
+    int per1;            // s1 values of a unit
+    int nb1, nb2;        // s1 and s2 blocks
+    long long units;     // (32-tetrahedron group, s1 block, s2 block) of one slot
+};
+
+// Doubles of a mode record: n(T), w, padded to an even number.
+__host__ __device__ constexpr int rec_size(int nt) { return (nt + 2) / 2 * 2; }
+
+// Table of `rows` grid (or path) points, [slot][s][q]: records of `rs` doubles (n(T), 0, w), and behind
+// them FP32 w.
+__global__ void k_tet_tables(int n, int nq, int nT, int rs, long long rows, const double* __restrict__ om,
+                             const double* __restrict__ nbe, double* __restrict__ rec) {
+    float* wf = reinterpret_cast<float*>(rec + rows * n * rs);
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < rows * n;
+         i += (long long)gridDim.x * blockDim.x) {
+        const long long row = i / n;
+        const int s = (int)(i % n);
+        const long long o = (row / nq * n + s) * nq + row % nq;
+        const double w = om[i];
+        wf[o] = (float)w;
+        double* r = rec + o * rs;
+        for (int t = 0; t < rs - 1; ++t) r[t] = t < nT ? nbe[(long long)t * rows * n + i] : 0.0;
+        r[rs - 1] = w;
+    }
+}
+
+template <int NT>
+struct TetSmem {
+    double acc[TW][NS0 * (NT + 1)][32];  // per-lane sums
+    unsigned queue[TW][32 * 24 + 32];
+    float o2[TW][BS2][4][32];  // second-leg frequencies of the unit
+    double w0[NS0];
 };
 
 // Q2TAB = false: kappa.x, the q2 of vertex q1 is the grid partner p(q1) of this q0.
-// Q2TAB = true: LineWidth.x path mode, the q2 phonons of vertex q1 come from a
-// per-q1 table (omega_q2All / nBE_q2All of Linewidth_m.f90:48-231), [slot][q1][s]
-// and [T][row][s] with row = slot * Nq + q1 of a table of `ntab` rows.
-template <int NTM, bool STRICT, bool Q2TAB>
-__global__ void __launch_bounds__(128) k_tetra3(TetArgs a, const int4* __restrict__ tet, const int* __restrict__ partner,
-                                                const double* __restrict__ wgrid, const double* __restrict__ om0,
-                                                const double* __restrict__ omg, const double* __restrict__ nbeg,
-                                                const double* __restrict__ om2t, const double* __restrict__ nbe2t,
-                                                double* __restrict__ out_lw, double* __restrict__ out_p3) {
-    __shared__ double sacc[NS0 * (NTM + 1)];
-    const int slot = blockIdx.y;
-    const int q0 = a.q0_first + slot;
-    const int n = a.n;
-    const size_t n3 = (size_t)n * n * n;
-    const int* part = Q2TAB ? nullptr : partner + (size_t)q0 * a.nq;
-    const size_t row0 = (size_t)slot * a.nq;  // first row of this slot in the q2 table
-    const double* W = wgrid + (size_t)slot * a.nq * n3;
-    for (int i = threadIdx.x; i < NS0 * (NTM + 1); i += blockDim.x) sacc[i] = 0.0;
+// Q2TAB = true: LineWidth.x path mode, the q2 phonons of vertex q1 come from a per-q1 table
+// (omega_q2All / nBE_q2All of Linewidth_m.f90:48-231) of this slot.
+// SYM: both legs have the same branch window (never in path mode).
+template <int NT, bool STRICT, bool Q2TAB, bool SYM>
+__global__ void __launch_bounds__(32 * TW, 3) k_tetra3(TetArgs a, const int4* __restrict__ tet,
+                                                    const int* __restrict__ partner, const double* __restrict__ wgrid,
+                                                    const double* __restrict__ om0, const double* __restrict__ rec1,
+                                                    const double* __restrict__ rec2, long long rows2,
+                                                    double* __restrict__ out_lw, double* __restrict__ out_p3) {
+    constexpr int RS = rec_size(NT), NCH = SYM ? 2 : 3, NP = SYM ? 2 : 1, PER = NCH * NS0, K = NP * PER;
+    constexpr int NPLANE = K < 16 ? 4 : 5;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TetSmem<NT>& S = *reinterpret_cast<TetSmem<NT>*>(smem_raw);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int slot = blockIdx.y, q0 = a.q0_first + slot;
+    const int s0a = a.lo0 + blockIdx.z * NS0, s0n = min(NS0, a.hi0 - s0a + 1);
+    const int n = a.n, nq = a.nq;
+    const int n3 = n * n * n;
+    const int* __restrict__ part = Q2TAB ? nullptr : partner + (size_t)q0 * nq;
+    const size_t off2 = Q2TAB ? (size_t)slot * n * nq : 0;
+    const float* __restrict__ wf1 = reinterpret_cast<const float*>(rec1 + (size_t)nq * n * RS);
+    const float* __restrict__ f2 = reinterpret_cast<const float*>(rec2 + rows2 * n * RS) + off2;
+    const double* __restrict__ r2 = rec2 + off2 * RS;
+    const double* __restrict__ W = wgrid + (size_t)slot * nq * n3 + (size_t)s0a * n * n;
+    for (int i = lane; i < NS0 * (NT + 1) * 32; i += 32) (&S.acc[warp][0][0])[i] = 0.0;
+    if (threadIdx.x < NS0) S.w0[threadIdx.x] = threadIdx.x < s0n ? om0[(size_t)q0 * n + s0a + threadIdx.x] : 0.0;
     __syncthreads();
-
-    double acc[NS0][NTM + 1];
+    float w0[NS0];
 #pragma unroll
-    for (int s = 0; s < NS0; ++s)
+    for (int i = 0; i < NS0; ++i) w0[i] = (float)S.w0[i];
+    unsigned live = 0;  // checks of existing s0
 #pragma unroll
-        for (int t = 0; t <= NTM; ++t) acc[s][t] = 0.0;
+    for (int k = 0; k < K; ++k)
+        if (k % NS0 < s0n) live |= 1u << (K - 1 - k);
+    double(*acc)[32] = S.acc[warp];
+    unsigned* queue = S.queue[warp];
+    float(*o2s)[4][32] = S.o2[warp];  // a lane reads back only what it wrote
 
-    const long long items = (long long)a.ntet * a.n1 * a.n2;
-    for (long long it = (long long)blockIdx.x * blockDim.x + threadIdx.x; it < items;
-         it += (long long)gridDim.x * blockDim.x) {
-        const int s2 = a.lo2 + (int)(it % a.n2);
-        const int s1 = a.lo1 + (int)((it / a.n2) % a.n1);
-        const int t = (int)(it / ((long long)a.n1 * a.n2));
-        const int4 tv = tet[t];
+    const long long stride = (long long)gridDim.x * TW;
+    for (long long u = (long long)blockIdx.x * TW + warp; u < a.units; u += stride) {
+        const int b2 = (int)(u % a.nb2), b1 = (int)(u / a.nb2 % a.nb1), g = (int)(u / ((long long)a.nb2 * a.nb1));
+        const int s1a = a.lo1 + b1 * a.per1, s1e = min(s1a + a.per1 - 1, a.hi1);
+        const int s2a = a.lo2 + b2 * BS2, s2n = min(BS2, a.hi2 - s2a + 1);
+        const bool on = g * 32 + lane < a.ntet;
+        const int4 tv = on ? tet[g * 32 + lane] : make_int4(0, 0, 0, 0);
         const int v1[4] = {tv.x, tv.y, tv.z, tv.w};
-        int v2[4];
-        double o1[4], o2[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-            v2[v] = Q2TAB ? v1[v] : part[v1[v]];
-            o1[v] = omg[(size_t)v1[v] * n + s1];
-            o2[v] = Q2TAB ? om2t[(row0 + v1[v]) * n + s2] : omg[(size_t)v2[v] * n + s2];
-        }
-        double M1[4], M2[4], M3[4];
+            const int v2 = Q2TAB ? v1[v] : part[v1[v]];
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            M1[v] = o1[v] + o2[v];
-            M2[v] = o2[v] - o1[v];
-            M3[v] = o1[v] - o2[v];
+            for (int k = 0; k < BS2; ++k) o2s[k][v][lane] = k < s2n ? f2[(size_t)(s2a + k) * nq + v2] : 0.0f;
         }
-        int p1[4], p2[4], p3[4];
-        tet::sort4(M1, p1);
-        tet::sort4(M2, p2);
-        tet::sort4(M3, p3);
-        double S1[4], S2[4], S3[4];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            S1[v] = M1[p1[v]];
-            S2[v] = M2[p2[v]];
-            S3[v] = M3[p3[v]];
-        }
-        // occupation factors per vertex and temperature
-        double fa[NTM][4], fb[NTM][4];  // n1+n2+1 and n1-n2
-#pragma unroll
-        for (int T = 0; T < NTM; ++T)
+
+        // FP64 evaluation of one queued hit: lane of the tetrahedron | s1 | s2 | check
+        auto evaluate = [&](unsigned code) {
+            const int tl = code & 31, s1 = (code >> 5) & 31, s2b = (code >> 10) & 31;
+            const int k = K - 1 - (int)(code >> 15);
+            const int s2 = s2b + k / PER, ch = k % PER / NS0, si = k % NS0;
+            const int4 t = tet[g * 32 + tl];
+            int x1[4] = {t.x, t.y, t.z, t.w}, x2[4];
+            const double* __restrict__ ra = rec1 + (size_t)s1 * nq * RS;
+            const double* __restrict__ rb = r2 + (size_t)s2 * nq * RS;
+            double M[4];
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
-                if (T < a.nT) {
-                    const double n1 = nbeg[((size_t)T * a.nq + v1[v]) * n + s1];
-                    const double n2 = Q2TAB ? nbe2t[((size_t)T * a.ntab + row0 + v1[v]) * n + s2]
-                                            : nbeg[((size_t)T * a.nq + v2[v]) * n + s2];
-                    fa[T][v] = n1 + n2 + 1.0;
-                    fb[T][v] = n1 - n2;
-                } else {
-                    fa[T][v] = fb[T][v] = 0.0;
-                }
+                x2[v] = Q2TAB ? x1[v] : part[x1[v]];
+                const double p = ra[(size_t)x1[v] * RS + RS - 1], q = rb[(size_t)x2[v] * RS + RS - 1];
+                M[v] = ch == 0 ? p + q : (ch == 1 ? q - p : p - q);
             }
+            tet::sort4_carry(M, x1, x2);
+            double gw, A[4];
+            if (!tet::g_weights<STRICT>(S.w0[si], M, gw, A)) return;
+            const double f = SYM ? (ch == 0 && s1 == s2 ? 1.0 : 2.0) : 1.0;
+            const double sg = !SYM && ch == 2 ? -1.0 : f;
+            const int col = (si * n + s1) * n + s2;
 #pragma unroll
-        for (int si = 0; si < NS0; ++si) {
-            if (si >= a.s0n) break;
-            const int s0 = a.s0a + si;
-            const double Mqs = om0[(size_t)q0 * n + s0];
-            double Wv[4];
+            for (int v = 0; v < 4; ++v) A[v] *= sg * W[(size_t)x1[v] * n3 + col];
+            double(*o)[32] = acc + si * (NT + 1);
+            o[NT][lane] += f * gw;
 #pragma unroll
-            for (int v = 0; v < 4; ++v) Wv[v] = W[(size_t)v1[v] * n3 + (s0 * n + s1) * n + s2];
-            double g, I[4];
-            // channel 1: F = W (n1 + n2 + 1), M = w1 + w2, added
-            bool e = tet::g_iver<STRICT>(Mqs, S1, g, I);
-            acc[si][NTM] += g;
-            if (e) {
+            for (int T0 = 0; T0 < NT; T0 += 2) {  // records are read two doubles at a time
+                if (T0 >= a.nT) break;
+                double sa = 0.0, sb = 0.0;
 #pragma unroll
-                for (int T = 0; T < NTM; ++T) {
-                    double s = 0.0;
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) s += I[v] * (Wv[p1[v]] * fa[T][p1[v]]);
-                    acc[si][T] += g * (ONEBYSIX * s);
+                for (int v = 0; v < 4; ++v) {
+                    const double2 na = *reinterpret_cast<const double2*>(ra + (size_t)x1[v] * RS + T0);
+                    const double2 nb = *reinterpret_cast<const double2*>(rb + (size_t)x2[v] * RS + T0);
+                    sa = fma(A[v], ch == 0 ? na.x + nb.x + 1.0 : na.x - nb.x, sa);
+                    if (T0 + 1 < NT) sb = fma(A[v], ch == 0 ? na.y + nb.y + 1.0 : na.y - nb.y, sb);
                 }
+                o[T0][lane] += sa;
+                if (T0 + 1 < NT) o[T0 + 1][lane] += sb;
             }
-            // channel 2: F = W (n1 - n2), M = w2 - w1, added
-            e = tet::g_iver<STRICT>(Mqs, S2, g, I);
-            acc[si][NTM] += g;
-            if (e) {
+        };
+
+        int qn = 0;
+        for (int s1 = s1a; s1 <= s1e; ++s1) {
+            float o1[4], e1 = 0.0f;
 #pragma unroll
-                for (int T = 0; T < NTM; ++T) {
-                    double s = 0.0;
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) s += I[v] * (Wv[p2[v]] * fb[T][p2[v]]);
-                    acc[si][T] += g * (ONEBYSIX * s);
-                }
+            for (int v = 0; v < 4; ++v) {
+                o1[v] = wf1[(size_t)s1 * nq + v1[v]];
+                e1 += fabsf(o1[v]);
             }
-            // channel 3: F = W (n1 - n2), M = w1 - w2, subtracted
-            e = tet::g_iver<STRICT>(Mqs, S3, g, I);
-            acc[si][NTM] += g;
-            if (e) {
+#pragma unroll 1
+            for (int kb = 0; kb < s2n; kb += NP) {
+                unsigned out = 0;  // one bit per check, set outside (the sign of half width - distance)
 #pragma unroll
-                for (int T = 0; T < NTM; ++T) {
-                    double s = 0.0;
+                for (int kk = 0; kk < NP; ++kk) {
+                    const int k = kb + kk;
+                    const float q0f = o2s[k][0][lane], q1f = o2s[k][1][lane], q2f = o2s[k][2][lane], q3f = o2s[k][3][lane];
+                    // FP32 rounding of the energies is below 4e-7 of the sum of magnitudes
+                    const float margin = 1e-6f * (e1 + (fabsf(q0f) + fabsf(q1f) + fabsf(q2f) + fabsf(q3f)));
+                    const float p0 = o1[0] + q0f, p1 = o1[1] + q1f, p2 = o1[2] + q2f, p3 = o1[3] + q3f;
+                    const float m0 = q0f - o1[0], m1 = q1f - o1[1], m2 = q2f - o1[2], m3 = q3f - o1[3];
+                    const float pl = fminf(fminf(p0, p1), fminf(p2, p3)), ph = fmaxf(fmaxf(p0, p1), fmaxf(p2, p3));
+                    const float ml = fminf(fminf(m0, m1), fminf(m2, m3)), mh = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+                    const float pm = 0.5f * (pl + ph), pr = fmaf(0.5f, ph - pl, margin);
+                    const float mm = 0.5f * (ml + mh), mr = fmaf(0.5f, mh - ml, margin);
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) s += I[v] * (Wv[p3[v]] * fb[T][p3[v]]);
-                    acc[si][T] -= g * (ONEBYSIX * s);
+                    for (int i = 0; i < NS0; ++i)
+                        out = __funnelshift_l(__float_as_uint(pr - fabsf(w0[i] - pm)), out, 1);
+#pragma unroll
+                    for (int i = 0; i < NS0; ++i)
+                        out = __funnelshift_l(__float_as_uint(mr - fabsf(w0[i] - mm)), out, 1);
+                    if (!SYM)
+#pragma unroll
+                        for (int i = 0; i < NS0; ++i)
+                            out = __funnelshift_l(__float_as_uint(mr - fabsf(w0[i] + mm)), out, 1);
                 }
+                unsigned in = on ? ~out & live : 0u;
+#pragma unroll
+                for (int kk = 0; kk < NP; ++kk) {
+                    unsigned drop = 0;
+                    if (kb + kk >= s2n) drop = (1u << PER) - 1;
+                    else if (SYM && s2a + kb + kk < s1) drop = ((1u << NS0) - 1) << NS0;  // channel 1: s1 <= s2
+                    in &= ~(drop << ((NP - 1 - kk) * PER));
+                }
+                const unsigned c = __popc(in);
+                unsigned pre = 0, tot = 0;
+                const unsigned lt = (1u << lane) - 1;
+#pragma unroll
+                for (int b = 0; b < NPLANE; ++b) {
+                    const unsigned m = __ballot_sync(0xffffffffu, (c >> b) & 1);
+                    pre += __popc(m & lt) << b;
+                    tot += __popc(m) << b;
+                }
+                if (tot == 0) continue;
+                const unsigned base = lane | s1 << 5 | (s2a + kb) << 10;
+                unsigned pos = qn + pre;
+                while (in) {
+                    const int b = __ffs(in) - 1;
+                    in &= in - 1;
+                    queue[pos++] = base | b << 15;
+                }
+                qn += tot;
+                __syncwarp();
+                while (qn >= 32) {
+                    qn -= 32;
+                    evaluate(queue[qn + lane]);
+                }
+                __syncwarp();
             }
         }
+        if (lane < qn) evaluate(queue[lane]);
+        __syncwarp();
     }
-    // reduce: warp, then CTA (shared), then global
-#pragma unroll
-    for (int s = 0; s < NS0; ++s)
-#pragma unroll
-        for (int T = 0; T <= NTM; ++T) {
-            const double v = tet::warp_sum(acc[s][T]);
-            if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(&sacc[s * (NTM + 1) + T], v);
-        }
+    // reduce: the block's warps and lanes, then global
     __syncthreads();
-    for (int i = threadIdx.x; i < NS0 * (NTM + 1); i += blockDim.x) {
-        const int s = i / (NTM + 1), T = i % (NTM + 1);
-        if (s >= a.s0n) continue;
-        const int s0 = a.s0a + s;
-        if (T < NTM) {
-            if (T < a.nT) atomicAdd(&out_lw[((size_t)T * a.nq0 + q0) * n + s0], sacc[i]);
+    for (int i = warp; i < NS0 * (NT + 1); i += TW) {
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < TW; ++w) v += S.acc[w][i][lane];
+        v = tet::warp_sum(v);
+        const int si = i / (NT + 1), T = i % (NT + 1);
+        if (lane != 0 || si >= s0n || v == 0.0) continue;
+        if (T < NT) {
+            if (T < a.nT) atomicAdd(&out_lw[((size_t)T * a.nq0 + q0) * n + s0a + si], v);
         } else {
-            atomicAdd(&out_p3[(size_t)q0 * n + s0], sacc[i]);
+            atomicAdd(&out_p3[(size_t)q0 * n + s0a + si], v);
         }
     }
 }
@@ -273,40 +352,76 @@ int grid_x(long long items, int threads, int slots) {
     return (int)(want < 1 ? 1 : want);
 }
 
+template <int NT, bool STRICT, bool Q2TAB, bool SYM>
+int launch_one(spring_ctx* c, const TetArgs& a, dim3 grid, const double* d_w, const int* part, const double* om0,
+               const double* rec2, long long rows2, double* d_lw, double* d_p3) {
+    const size_t smem = sizeof(TetSmem<NT>);
+    auto kern = k_tetra3<NT, STRICT, Q2TAB, SYM>;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "tetra3: injected launch failure");
+    kern<<<grid, 32 * TW, smem, c->stream>>>(a, reinterpret_cast<const int4*>(c->d_tetra.p), part, d_w, om0,
+                                             c->d_tet_tab.p, rec2, rows2, d_lw, d_p3);
+    return launch_check(c, Q2TAB ? "k_tetra3<path>" : "k_tetra3");
+}
+
 template <bool STRICT, bool Q2TAB>
 int launch_tetra3(spring_ctx* c, TetArgs a, int n_q0, const Pol& pol, const double* d_w, const int* part,
-                  const double* om0, const double* omg, const double* nbeg, const double* om2t, const double* nbe2t,
-                  double* d_lw, double* d_p3) {
+                  const double* om0, const double* rec2, long long rows2, double* d_lw, double* d_p3) {
+    if (c->nT > 9)
+        return fail(c, SPRING_ERR_UNSUPPORTED, "tetrahedron integration supports at most 9 temperatures per call");
+    a.lo0 = pol.lo[0];
+    a.hi0 = pol.hi[0];
     a.lo1 = pol.lo[1];
-    a.n1 = pol.hi[1] - pol.lo[1] + 1;
+    a.hi1 = pol.hi[1];
     a.lo2 = pol.lo[2];
-    a.n2 = pol.hi[2] - pol.lo[2] + 1;
-    const long long items = (long long)a.ntet * a.n1 * a.n2;
-    const int threads = 128;
-    dim3 grid(grid_x(items, threads, n_q0), n_q0);
-    const int4* tet = reinterpret_cast<const int4*>(c->d_tetra.p);
-    for (int s0a = pol.lo[0]; s0a <= pol.hi[0]; s0a += NS0) {
-        a.s0a = s0a;
-        a.s0n = std::min(NS0, pol.hi[0] - s0a + 1);
-        if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "tetra3: injected launch failure");
-        if (c->nT == 1) {
-            k_tetra3<1, STRICT, Q2TAB><<<grid, threads, 0, c->stream>>>(a, tet, part, d_w, om0, omg, nbeg, om2t, nbe2t,
-                                                                        d_lw, d_p3);
-        } else if (c->nT <= 3) {
-            k_tetra3<3, STRICT, Q2TAB><<<grid, threads, 0, c->stream>>>(a, tet, part, d_w, om0, omg, nbeg, om2t, nbe2t,
-                                                                        d_lw, d_p3);
-        } else if (c->nT <= 9) {
-            k_tetra3<9, STRICT, Q2TAB><<<grid, threads, 0, c->stream>>>(a, tet, part, d_w, om0, omg, nbeg, om2t, nbe2t,
-                                                                        d_lw, d_p3);
-        } else {
-            return fail(c, SPRING_ERR_UNSUPPORTED, "tetrahedron integration supports at most 9 temperatures per call");
-        }
-        SPRING_CHECK(launch_check(c, Q2TAB ? "k_tetra3<path>" : "k_tetra3"));
-    }
-    return SPRING_OK;
+    a.hi2 = pol.hi[2];
+    a.nb2 = (a.hi2 - a.lo2 + BS2) / BS2;
+    const int n1 = a.hi1 - a.lo1 + 1, groups = (a.ntet + 31) / 32, passes = (a.hi0 - a.lo0 + NS0) / NS0;
+    // Units are as long as the chip stays full (16 resident warps per SM): the s2 frequencies are
+    // loaded, and the queue's tail evaluated, once per unit.
+    a.per1 = 6;
+    while (a.per1 > 1 && (long long)groups * a.nb2 * ((n1 + a.per1 - 1) / a.per1) * n_q0 * passes < 148LL * 32) --a.per1;
+    a.nb1 = (n1 + a.per1 - 1) / a.per1;
+    a.units = (long long)groups * a.nb1 * a.nb2;
+    const long long cap = std::max<long long>(1, 148LL * 8 / ((long long)n_q0 * passes));
+    const dim3 grid((unsigned)std::max<long long>(1, std::min<long long>((a.units + TW - 1) / TW, cap)), n_q0, passes);
+    const bool sym = !Q2TAB && a.lo1 == a.lo2 && a.hi1 == a.hi2;
+#define SPRING_T3(NT)                                                                                                 \
+    return sym ? launch_one<NT, STRICT, Q2TAB, !Q2TAB>(c, a, grid, d_w, part, om0, rec2, rows2, d_lw, d_p3)             \
+               : launch_one<NT, STRICT, Q2TAB, false>(c, a, grid, d_w, part, om0, rec2, rows2, d_lw, d_p3)
+    if (c->nT == 1) SPRING_T3(1);
+    if (c->nT <= 3) SPRING_T3(3);
+    SPRING_T3(9);
+#undef SPRING_T3
+}
+
+// Record size of a context's tables: the kernel variant its temperature count selects.
+int tet_rs(const spring_ctx* c) { return rec_size(c->nT == 1 ? 1 : (c->nT <= 3 ? 3 : 9)); }
+
+int build_tables(spring_ctx* c, long long rows, const double* om, const double* nbe, double* rec) {
+    const int threads = 256;
+    const int blocks = (int)std::min<long long>((rows * c->ndof + threads - 1) / threads, 148LL * 16);
+    if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "tetra3: injected launch failure");
+    k_tet_tables<<<blocks, threads, 0, c->stream>>>(c->ndof, c->nq, c->nT, tet_rs(c), rows, om, nbe, rec);
+    return launch_check(c, "k_tet_tables");
 }
 
 }  // namespace
+
+// The grid's tables, allocated with the phonons (the no-allocation entry point fills them in place)
+// and filled by run_tetra_tables before run_tetra3 / run_tetra3_path.
+int alloc_tetra_tables(spring_ctx* c) {
+    if (c->nT > 9) return SPRING_OK;  // refused by run_tetra3
+    return dalloc(c, c->d_tet_tab, c->nq * tetra_table_doubles(c), "tetrahedron tables");
+}
+
+int run_tetra_tables(spring_ctx* c) {
+    if (c->nT > 9) return SPRING_OK;
+    return build_tables(c, c->nq, c->ph_grid.omega.p, c->ph_grid.nbe.p, c->d_tet_tab.p);
+}
+
+// Doubles per table row: ndof records and ndof floats.
+size_t tetra_table_doubles(const spring_ctx* c) { return (size_t)c->ndof * (tet_rs(c) + 1); }
 
 int run_tetra3(spring_ctx* c, int q0_first, int n_q0, const double* d_w, const Pol& pol, double* d_lw, double* d_p3) {
     TetArgs a{};
@@ -316,12 +431,12 @@ int run_tetra3(spring_ctx* c, int q0_first, int n_q0, const double* d_w, const P
     a.nT = c->nT;
     a.ntet = 6 * c->nq;
     a.q0_first = q0_first;
-    return launch_tetra3<false, false>(c, a, n_q0, pol, d_w, c->ps_irr.partner.p, c->ph_irr.omega.p,
-                                       c->ph_grid.omega.p, c->ph_grid.nbe.p, nullptr, nullptr, d_lw, d_p3);
+    return launch_tetra3<false, false>(c, a, n_q0, pol, d_w, c->ps_irr.partner.p, c->ph_irr.omega.p, c->d_tet_tab.p,
+                                       c->nq, d_lw, d_p3);
 }
 
 int run_tetra3_path(spring_ctx* c, int p_first, int n_slots, int n_path, const double* d_w, const double* om0,
-                    const double* om2t, const double* nbe2t, long long ntab, double* d_lw, double* d_scratch) {
+                    const double* om2t, const double* nbe2t, double* tab2, double* d_lw, double* d_scratch) {
     TetArgs a{};
     a.n = c->ndof;
     a.nq = c->nq;
@@ -329,14 +444,14 @@ int run_tetra3_path(spring_ctx* c, int p_first, int n_slots, int n_path, const d
     a.nT = c->nT;
     a.ntet = 6 * c->nq;
     a.q0_first = p_first;
-    a.ntab = ntab;
+    SPRING_CHECK(run_tetra_tables(c));
+    SPRING_CHECK(build_tables(c, (long long)n_slots * c->nq, om2t, nbe2t, tab2));
     Pol pol;
     for (int k = 0; k < 3; ++k) {
         pol.lo[k] = 0;
         pol.hi[k] = c->ndof - 1;
     }
-    return launch_tetra3<true, true>(c, a, n_slots, pol, d_w, nullptr, om0, c->ph_grid.omega.p, c->ph_grid.nbe.p,
-                                     om2t, nbe2t, d_lw, d_scratch);
+    return launch_tetra3<true, true>(c, a, n_slots, pol, d_w, nullptr, om0, tab2, (long long)n_slots * c->nq, d_lw, d_scratch);
 }
 
 int run_iso(spring_ctx* c, int q0_first, int n_q0, int delta_mode, double sigma, const double* g2, double* d_rate) {

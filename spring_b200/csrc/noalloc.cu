@@ -104,6 +104,7 @@ extern "C" int spring_linewidth3_tetra_noalloc(spring_ctx* c, int i0, const int*
         cudaError_t e = cudaMemsetAsync(lw, 0, sizeof(double) * (lsize + psize), c->stream);
         if (e != cudaSuccess) { rc = cuda_fail(c, e, "clear no-alloc slabs"); break; }
         if ((rc = run_v3_wgrid(c, c->ps_irr, irr_view(c), q0, 1, w)) != SPRING_OK) break;
+        if ((rc = run_tetra_tables(c)) != SPRING_OK) break;
         if ((rc = run_tetra3(c, q0, 1, w, pol, lw, p3)) != SPRING_OK) break;
         // lw slab [T][q0][s] -> caller's [T][s];  p3 [q0][s] -> caller's [s]
         e = cudaMemcpy2DAsync(d_lw, n * sizeof(double), lw + (size_t)q0 * n, (size_t)c->nq0 * n * sizeof(double),

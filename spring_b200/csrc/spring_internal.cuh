@@ -237,6 +237,7 @@ struct spring_ctx {
     spring::DBuf<double> d_krn;    // [q0][s][9]
     spring::DBuf<double> d_rxyz;
     spring::DBuf<double> d_wiso;   // [slot][q1][s0][s1]
+    spring::DBuf<double> d_tet_tab;  // tetrahedron tables of the grid: records (n(T), omega) [s][q], FP32 omega [s][q]
 
     // tensor-core V3 (spring_set_precision): operand tables and pair tiles grouped by q1
     spring::DBuf<uint16_t> d_tc_a;     // bf16 A operand images [q][hi, lo][mu]
@@ -380,6 +381,7 @@ int run_path(spring_ctx* c, int n_path, const double* h_q0, const int* h_zc, int
 struct PathPlan {
     int n_path = 0, slots = 0;
     DBuf<double> q0v, q1v, q2v, w, lw, p3;
+    DBuf<double> tab2;   // tetrahedron tables of the q2 points
     DBuf<int> zc, ex;
     Phonons php, ph2;
 };
@@ -400,10 +402,14 @@ void free_mlp(Mlp& m);
 // k_bte.cu
 int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* h_kappa_rta, int* h_iters);
 // k_tetra.cu
+int alloc_tetra_tables(spring_ctx* c);
+int run_tetra_tables(spring_ctx* c);  // before run_tetra3, after any change of the grid phonons
+size_t tetra_table_doubles(const spring_ctx* c);  // size of a table per row
 int run_tetra3(spring_ctx* c, int q0_first, int n_q0, const double* d_w, const Pol& pol, double* d_lw, double* d_p3);
-// LineWidth.x form: strict bounds, q2 phonons of vertex q1 from a table of `ntab` rows (row = slot * Nq + q1)
+// LineWidth.x form: strict bounds, q2 phonons of vertex q1 from a table (row = slot * Nq + q1) built in
+// tab2, tetra_table_doubles() doubles per row
 int run_tetra3_path(spring_ctx* c, int p_first, int n_slots, int n_path, const double* d_w, const double* om0,
-                    const double* om2t, const double* nbe2t, long long ntab, double* d_lw, double* d_scratch);
+                    const double* om2t, const double* nbe2t, double* tab2, double* d_lw, double* d_scratch);
 int run_iso(spring_ctx* c, int q0_first, int n_q0, int delta_mode, double sigma, const double* g2, double* d_rate);
 // k_kappa.cu
 int run_axpy_lw(spring_ctx* c, double a, const double* d_x, double* d_y, int q0_first, int n_q0);

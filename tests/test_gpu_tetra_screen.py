@@ -1,0 +1,51 @@
+"""The screened tetrahedron sums: every kernel variant at its edges, and the leg symmetry they use."""
+import numpy as np
+import pytest
+
+from oracle import driver as D
+from spring_b200 import synthetic as S
+from spring_b200.api import from_crystal
+
+
+@pytest.mark.parametrize("mesh", [(3, 3, 3), (4, 4, 4), (5, 4, 3), (1, 2, 6)])
+def test_partner_map_carries_the_tetrahedra_onto_themselves(mesh):
+    """q1 -> grid(-q0 - q1) is an involution that permutes the tetrahedra as vertex sets: channel 3 of
+    the sums equals channel 2, and channel 1 is symmetric in its legs."""
+    n = np.array(mesh)
+    q = np.stack(np.meshgrid(*[np.arange(m) for m in mesh], indexing="ij"), -1).reshape(-1, 3, order="F")
+    q = np.array([[g % n[0], g // n[0] % n[1], g // (n[0] * n[1])] for g in range(n.prod())])
+    cr = S.build("rocksalt2")
+    tet = D.make_tetrahedron(mesh, cr.G)[2] - 1
+    sets = sorted(tuple(sorted(t)) for t in tet)
+    for q0 in q:
+        p = (-(q0 + q)) % n
+        p = p[:, 0] + n[0] * (p[:, 1] + n[1] * p[:, 2])
+        assert np.array_equal(p[p], np.arange(n.prod()))
+        assert sorted(tuple(sorted(p[t])) for t in tet) == sets
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cell,N,nT,pol", [
+    ("rocksalt2", 3, 1, None),                               # 162 tetrahedra: a last group of two lanes
+    ("rocksalt2", 4, 2, None),                               # two of three temperature columns
+    ("rocksalt2", 4, 4, None),                               # four of nine
+    ("rocksalt2", 5, 9, [[1, 6], [2, 6], [2, 6]]),           # equal leg windows that start above 1
+    ("rocksalt2", 4, 3, [[2, 5], [1, 3], [1, 6]]),           # unequal leg windows: all three channels
+    ("rocksalt2", 4, 1, [[6, 6], [4, 4], [5, 6]]),
+    ("rocksalt8", 2, 3, None),                               # four passes over s0, four s2 blocks
+    ("rocksalt8", 2, 1, [[5, 21], [3, 19], [3, 19]]),        # s0 and s2 blocks with tails
+    ("rocksalt8", 2, 2, [[1, 7], [24, 24], [1, 13]]),
+])
+def test_screened_tetrahedron_sums_match_oracle(cell, N, nT, pol):
+    cr = S.build(cell)
+    temps = list(np.linspace(100.0, 900.0, nT))
+    st = D.Setup(cr, (N, N, N), temps)
+    ctx, _ = from_crystal(cr, (N, N, N), temps, phonons={"grid": st.ph, "irr": st.ph0})
+    p = None if pol is None else np.array(pol, np.int32)
+    lw, p3 = ctx.linewidth3(1, st.nq0, delta="tetra", pol3=p)
+    for i0 in range(st.nq0):
+        for it in range(nT):
+            r = D.linewidth3_q0(st, i0, delta="tetra", it=it, pol=p)
+            np.testing.assert_allclose(lw[it, i0], r["lw"], rtol=1e-9, atol=1e-14 * np.abs(lw).max())
+        np.testing.assert_allclose(p3[i0], r["p3_q0"], rtol=1e-9, atol=1e-14 * np.abs(p3).max())
+    ctx.close()
