@@ -393,6 +393,11 @@ int spring_batch_path_result(spring_batch* batch, int index, double* lw, double*
  * exp(-40) of its peak (the tensor-core path's pre-screen; the linewidths change below 1e-13
  * relative); 0 (default) evaluates every pair. */
 #define SPRING_OPT_FP64_PRESCREEN 3
+/* SPRING_OPT_BTE_ENTRIES = 4: most entries of the tetrahedron scattering operator spring_kappa_iter
+ * keeps in device memory (24 bytes each; a negative value restores the default, half the free memory
+ * and at most 40 GB).  A larger operator is not stored: every iteration then recomputes it, with the
+ * same result. */
+#define SPRING_OPT_BTE_ENTRIES 4
 int spring_set_option(spring_ctx* ctx, int option, int value);
 
 /* ---- diagnostics ------------------------------------------------------- */

@@ -325,7 +325,8 @@ int spring_ctx_destroy(spring_ctx* c) {
         free_phonons(c->ph_grid); free_phonons(c->ph_irr);
         free_pairs(c->ps_irr); free_pairs(c->ps_tr);
         dfree(c->d_tr_int); dfree(c->d_tr_grid); dfree(c->d_tr_pos); dfree(c->d_tr_sgn); dfree(c->d_tr_deg);
-        dfree(c->d_neg); dfree(c->d_wtr);
+        dfree(c->d_neg); dfree(c->d_bt_off); dfree(c->d_bt_kk); dfree(c->d_bt_pq);
+        dfree(c->bte.pq); dfree(c->bte.cf); dfree(c->bte.vec);
         dfree(c->d_bteg_row); dfree(c->d_bteg_kk); dfree(c->d_bteg_pq);
         dfree(c->ew.g); dfree(c->ew.r); dfree(c->ew.hz); dfree(c->ew.tau); dfree(c->ew.z); dfree(c->ew.cc);
         dfree(c->ew.dd); dfree(c->d_v4_rec);
@@ -426,6 +427,10 @@ int spring_set_option(spring_ctx* c, int option, int value) {
         case SPRING_OPT_GENERIC_V3: c->force_generic_v3 = value != 0; return SPRING_OK;
         case SPRING_OPT_WAIT_POLLS: c->tc_max_spins = value < 0 ? -1 : (long long)value; return SPRING_OK;
         case SPRING_OPT_FP64_PRESCREEN: c->fp64_prescreen = value != 0; return SPRING_OK;
+        case SPRING_OPT_BTE_ENTRIES:
+            c->bte_max_entries = value < 0 ? -1 : value;
+            c->bt_gen = -1;
+            return SPRING_OK;
         default: return fail(c, SPRING_ERR_ARG, "unknown option %d", option);
     }
 }
@@ -629,8 +634,8 @@ int spring_set_fc3(spring_ctx* c, int na3, const int* num, const int* idx, const
     SPRING_CHECK(h2d(c, c->d_fc3_btyp.p, btyp.data(), sizeof(int) * btyp.size(), "FC3 basis"));
     // no stream wait: h2d staged every byte in the context's pinned ring before queuing its copy
     c->fc3_set = true;
-    dfree(c->d_wtr);  // cached W grids depend on FC3
-    c->bteg_n = 0;    // and so does the Gaussian BTE operator
+    c->bt_gen = -1;   // the BTE operators depend on FC3
+    c->bteg_n = 0;
     return SPRING_OK;
 }
 
@@ -796,7 +801,6 @@ int spring_compute_phonons(spring_ctx* c, const double* temps, double freq_cut) 
     SPRING_CHECK(run_phonons_mesh(c));
     c->ph_grid.set = c->ph_irr.set = true;
     c->ph_gen += 1;
-    dfree(c->d_wtr);  // cached W grids depend on the phonons
     return SPRING_OK;
 }
 
@@ -827,7 +831,6 @@ int spring_set_phonons(spring_ctx* c, int which, const double* temps, const doub
     SPRING_CHECK(h2d(c, p.vel.p, vel, sizeof(double) * n * nd * 3, "group velocity"));
     p.set = true;
     c->ph_gen += 1;
-    if (which == 0) dfree(c->d_wtr);  // cached W grids depend on the grid phonons
     return SPRING_OK;
 }
 

@@ -18,11 +18,16 @@
 //   minus channel, vertex v:  partner u = -p(-v), M = w(v,s1) + w(u,s2),
 //                             W- = 4 W3(q0; -v s1; p(-v) s2) (1 + n(-v,s1) + n(p(-v),s2)),
 //                             dF term 0.5 (F(u,s2) + F(v,s1));
-// with p(x) = grid(-q0 - x).  One thread per (q0, tetrahedron, s1, s2) sorts each
-// channel's vertex energies once (stable) and loops over s0.  The W grids of
-// every q0 are computed once and kept in HBM when they fit a 40 GB budget, and
-// otherwise recomputed batch by batch on every pass.
-// Roofline: FP64 ALU (divisions of the tetrahedron weights), like k_tetra3.
+// with p(x) = grid(-q0 - x).  Because F(-q) = -F(q), both terms are -(F(x, s1) + F(p(x), s2)) times a
+// coefficient at the grid modes (x, s1), (p(x), s2) - x = -v for the minus channel - that depends on the
+// temperature only through n there.  So the tetrahedron weights are computed once: every (tetrahedron,
+// mode triple) whose energy range holds w0 adds its vertex weights to a dense (P, Q) grid of its q0, and
+// the non-zero entries, with 4 W folded in and the two orderings of a pair merged, go to HBM as rows of
+// the same operator the Gaussian form uses; an iteration is one pass over it.  When the operator does not
+// fit (half the free memory), the (P, Q) grids are rebuilt batch by batch on every pass instead.
+// Weights: FP32 screen and queued FP64 evaluation as in k_tetra3.  The former kernel evaluated the
+// weights of every tetrahedron again in every iteration.
+// Roofline: FP64 ALU for the weights, HBM / L2 (24 bytes and two gathers per entry) for the iterations.
 #include <algorithm>
 #include <cmath>
 #include <cub/cub.cuh>
@@ -34,196 +39,372 @@
 namespace spring {
 namespace {
 
-constexpr int NS0 = 6;
+constexpr int NS0 = 6, BS2 = 6, TW = 4;
 constexpr double ZERO_PREC = 5.0e-5;
 constexpr double FUNIT_E = 1.054571817 / 1.380649;  // FunitE_11m_K (Src_iterative/constants.f90:56)
 constexpr double KW_MK = 1.054571817 * 0.001;       // kW_mK (:58)
 
-struct PassArgs {
-    int n, nq, ntet, q0_first, s0a, s0n;
-    const int* tr_grid;   // [ntr]
-    const int* tr_pos;    // [nq]
-    const int* tr_sgn;    // [nq]
-    const int* neg;       // [nq]
-    const int* partner;   // [ntr][nq]
-    const double* wgrid;  // [slot][nq][n^3] for q0_first ..
-    const double* omega;  // [nq][n]
-    const double* nbe;    // [nq][n] at this temperature
-    const double* F;      // [ntr][n][3] (MODE 1)
-    double* out;          // MODE 0: inv_tau [ntr][n]; MODE 1: dF [ntr][n][3]
+__global__ void k_bte_wf(int nq, int n, const double* __restrict__ om, float* __restrict__ wf) {  // [s][q]
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nq * n; i += gridDim.x * blockDim.x)
+        wf[(size_t)(i % n) * nq + i / n] = (float)om[i];
+}
+
+struct WgtArgs {
+    int n, nq, ntet, q0_first;
+    int per1, nb1, nb2;         // s1 values of a unit; s1 and s2 blocks
+    long long units;
+    const int* tr_grid;         // [ntr]
+    const int* neg;             // [nq]
+    const int* partner;         // [ntr][nq]
+    const float* wf;            // [n][nq]
+    const double* omega;        // [nq][n]
+    double2* pq;                // [slot][s0][s1][s2][x] (P, Q), zeroed
 };
 
-template <int MODE>
-__global__ void __launch_bounds__(128) k_bte_pass(PassArgs a, const int4* __restrict__ tet) {
-    constexpr int NC = MODE == 0 ? 1 : 3;
-    __shared__ double sacc[NS0 * 3];
-    const int slot = blockIdx.y;
-    const int q0 = a.q0_first + slot;
-    const int n = a.n;
-    const size_t n3 = (size_t)n * n * n;
-    const int g0 = a.tr_grid[q0];
-    const int* p = a.partner + (size_t)q0 * a.nq;
-    const double* W3 = a.wgrid + (size_t)slot * a.nq * n3;
-    for (int i = threadIdx.x; i < NS0 * 3; i += blockDim.x) sacc[i] = 0.0;
+// Tetrahedron weights of the plus (P) and minus (Q, half weight) channel of every q0 of a batch: warps
+// screen 32 tetrahedra at a time in FP32, queue the (tetrahedron, s1, s2, s0, channel) whose range holds
+// w0, and evaluate 32 of them at a time (k_tetra.cu has the reasons).
+__global__ void __launch_bounds__(32 * TW, 4) k_bte_weights(WgtArgs a, const int4* __restrict__ tet) {
+    constexpr int K = 2 * NS0;
+    __shared__ unsigned queue_[TW][32 * K + 32];
+    __shared__ float o2_[TW][BS2][8][32];
+    __shared__ double w0d[NS0];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int slot = blockIdx.y, q0 = a.q0_first + slot;
+    const int n = a.n, nq = a.nq;
+    const int s0a = blockIdx.z * NS0, s0n = min(NS0, n - s0a);
+    const int* __restrict__ p = a.partner + (size_t)q0 * nq;
+    const int* __restrict__ neg = a.neg;
+    double* pq = reinterpret_cast<double*>(a.pq) + ((size_t)slot * n + s0a) * n * n * nq * 2;
+    if (threadIdx.x < NS0)
+        w0d[threadIdx.x] = threadIdx.x < s0n ? a.omega[(size_t)a.tr_grid[q0] * n + s0a + threadIdx.x] : 0.0;
     __syncthreads();
-    double acc[NS0][NC];
+    float w0[NS0];
+    unsigned live = 0;
 #pragma unroll
-    for (int s = 0; s < NS0; ++s)
-#pragma unroll
-        for (int k = 0; k < NC; ++k) acc[s][k] = 0.0;
-
-    const long long items = (long long)a.ntet * n * n;
-    for (long long it = (long long)blockIdx.x * blockDim.x + threadIdx.x; it < items;
-         it += (long long)gridDim.x * blockDim.x) {
-        const int s2 = (int)(it % n), s1 = (int)((it / n) % n), t = (int)(it / ((long long)n * n));
-        const int4 tv = tet[t];
+    for (int i = 0; i < NS0; ++i) {
+        w0[i] = (float)w0d[i];
+        if (i < s0n) live |= (1u << (K - 1 - i)) | (1u << (NS0 - 1 - i));
+    }
+    unsigned* queue = queue_[warp];
+    float(*o2)[8][32] = o2_[warp];
+    const long long stride = (long long)gridDim.x * TW;
+    for (long long u = (long long)blockIdx.x * TW + warp; u < a.units; u += stride) {
+        const int b2 = (int)(u % a.nb2), b1 = (int)(u / a.nb2 % a.nb1), g = (int)(u / ((long long)a.nb2 * a.nb1));
+        const int s1a = b1 * a.per1, s1e = min(s1a + a.per1, n);
+        const int s2a = b2 * BS2, s2n = min(BS2, n - s2a);
+        const bool on = g * 32 + lane < a.ntet;
+        const int4 tv = on ? tet[g * 32 + lane] : make_int4(0, 0, 0, 0);
         const int x[4] = {tv.x, tv.y, tv.z, tv.w};
 #pragma unroll
-        for (int ch = 0; ch < 2; ++ch) {
-            int part[4], wrow[4];
-            double M[4], Wf[4];  // Wf: the occupation factor; W3 is read per s0
+        for (int v = 0; v < 4; ++v) {
+            const int pp = neg[p[x[v]]], pm = neg[p[neg[x[v]]]];
+            for (int k = 0; k < s2n; ++k) {
+                o2[k][v][lane] = a.wf[(size_t)(s2a + k) * nq + pp];
+                o2[k][4 + v][lane] = a.wf[(size_t)(s2a + k) * nq + pm];
+            }
+        }
+        auto evaluate = [&](unsigned code) {
+            const int tl = code & 31, s1 = (code >> 5) & 31, s2 = (code >> 10) & 31;
+            const int k = K - 1 - (int)(code >> 15), ch = k / NS0, si = k % NS0;
+            const int4 t = tet[g * 32 + tl];
+            int at[4] = {t.x, t.y, t.z, t.w}, row[4];
+            double M[4];
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
-                if (ch == 0) {
-                    const int px = p[x[v]];
-                    part[v] = a.neg[px];
-                    wrow[v] = x[v];
-                    M[v] = a.omega[(size_t)part[v] * n + s2] - a.omega[(size_t)x[v] * n + s1];
-                    Wf[v] = a.nbe[(size_t)x[v] * n + s1] - a.nbe[(size_t)px * n + s2];
-                } else {
-                    const int y = a.neg[x[v]];
-                    const int py = p[y];
-                    part[v] = a.neg[py];
-                    wrow[v] = y;
-                    M[v] = a.omega[(size_t)x[v] * n + s1] + a.omega[(size_t)part[v] * n + s2];
-                    Wf[v] = 1.0 + a.nbe[(size_t)y * n + s1] + a.nbe[(size_t)py * n + s2];
-                }
+                row[v] = ch == 0 ? at[v] : neg[at[v]];
+                const double w1 = a.omega[(size_t)at[v] * n + s1], w2 = a.omega[(size_t)neg[p[row[v]]] * n + s2];
+                M[v] = ch == 0 ? w2 - w1 : w1 + w2;
             }
-            int pm[4];
-            tet::sort4(M, pm);
-            double S[4];
+            tet::sort4_carry(M, row, at);
+            double gw, A[4];
+            if (!tet::g_weights<true>(w0d[si], M, gw, A)) return;
+            const double f = ch == 0 ? 1.0 : 0.5;
+            double* o = pq + ((size_t)(si * n + s1) * n + s2) * nq * 2 + ch;
 #pragma unroll
-            for (int v = 0; v < 4; ++v) S[v] = M[pm[v]];
-            // F terms per vertex (MODE 1): plus F(part,s2) - F(x,s1); minus F(part,s2) + F(x,s1)
-            double Fc[4][NC];
-            if (MODE == 1) {
+            for (int v = 0; v < 4; ++v) atomicAdd(o + 2 * (size_t)row[v], f * A[v]);
+        };
+        int qn = 0;
+        for (int s1 = s1a; s1 < s1e; ++s1) {
+            float o1[4], e1 = 0.0f;
 #pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const int xv = x[pm[v]], pv = part[pm[v]];
-                    const double sx = a.tr_sgn[xv], sp = a.tr_sgn[pv];
-                    const double* f1 = a.F + ((size_t)a.tr_pos[xv] * n + s1) * 3;
-                    const double* f2 = a.F + ((size_t)a.tr_pos[pv] * n + s2) * 3;
-#pragma unroll
-                    for (int k = 0; k < NC; ++k)
-                        Fc[v][k] = ch == 0 ? (sp * f2[k] - sx * f1[k]) : (sp * f2[k] + sx * f1[k]);
-                }
+            for (int v = 0; v < 4; ++v) {
+                o1[v] = a.wf[(size_t)s1 * nq + x[v]];
+                e1 += fabsf(o1[v]);
             }
+#pragma unroll 1
+            for (int k = 0; k < s2n; ++k) {
+                unsigned out = 0;  // one bit per check, set outside
 #pragma unroll
-            for (int si = 0; si < NS0; ++si) {
-                if (si >= a.s0n) break;
-                const int s0 = a.s0a + si;
-                const double Mqs = a.omega[(size_t)g0 * n + s0];
-                double g, I[4];
-                if (!tet::g_iver<true>(Mqs, S, g, I)) continue;
-                if (!(fabs(I[0] + I[1] + I[2] + I[3] - 1.0) < ZERO_PREC)) continue;
-                const double pre = ch == 0 ? ONEBYSIX * g : 0.5 * ONEBYSIX * g;
-                double tv[NC];
+                for (int ch = 0; ch < 2; ++ch) {
+                    const float a0 = o2[k][4 * ch][lane], a1 = o2[k][4 * ch + 1][lane], a2 = o2[k][4 * ch + 2][lane],
+                                a3 = o2[k][4 * ch + 3][lane];
+                    const float margin = 1e-6f * (e1 + (fabsf(a0) + fabsf(a1) + fabsf(a2) + fabsf(a3)));
+                    const float sg = ch == 0 ? -1.0f : 1.0f;
+                    const float m0 = fmaf(sg, o1[0], a0), m1 = fmaf(sg, o1[1], a1), m2 = fmaf(sg, o1[2], a2),
+                                m3 = fmaf(sg, o1[3], a3);
+                    const float lo = fminf(fminf(m0, m1), fminf(m2, m3)), hi = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+                    const float mid = 0.5f * (lo + hi), half = fmaf(0.5f, hi - lo, margin);
 #pragma unroll
-                for (int k = 0; k < NC; ++k) tv[k] = 0.0;
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const int q = pm[v];
-                    const double Wv = 4.0 * W3[(size_t)wrow[q] * n3 + (s0 * n + s1) * n + s2] * Wf[q];
-                    if (MODE == 0) {
-                        tv[0] += I[v] * Wv;
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < NC; ++k) tv[k] += (I[v] * Wv) * Fc[v][k];
-                    }
+                    for (int i = 0; i < NS0; ++i)
+                        out = __funnelshift_l(__float_as_uint(half - fabsf(w0[i] - mid)), out, 1);
                 }
+                unsigned in = on ? ~out & live : 0u;
+                const unsigned c = __popc(in);
+                unsigned pre = 0, tot = 0;
+                const unsigned lt = (1u << lane) - 1;
 #pragma unroll
-                for (int k = 0; k < NC; ++k) acc[si][k] += pre * tv[k];
+                for (int b = 0; b < 4; ++b) {
+                    const unsigned m = __ballot_sync(0xffffffffu, (c >> b) & 1);
+                    pre += __popc(m & lt) << b;
+                    tot += __popc(m) << b;
+                }
+                if (tot == 0) continue;
+                const unsigned base = lane | s1 << 5 | (s2a + k) << 10;
+                unsigned pos = qn + pre;
+                while (in) {
+                    const int b = __ffs(in) - 1;
+                    in &= in - 1;
+                    queue[pos++] = base | b << 15;
+                }
+                qn += tot;
+                __syncwarp();
+                while (qn >= 32) {
+                    qn -= 32;
+                    evaluate(queue[qn + lane]);
+                }
+                __syncwarp();
             }
         }
-    }
-#pragma unroll
-    for (int s = 0; s < NS0; ++s)
-#pragma unroll
-        for (int k = 0; k < NC; ++k) {
-            const double v = tet::warp_sum(acc[s][k]);
-            if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(&sacc[s * 3 + k], v);
-        }
-    __syncthreads();
-    for (int i = threadIdx.x; i < NS0 * NC; i += blockDim.x) {
-        const int s = i / NC, k = i % NC;
-        if (s >= a.s0n || sacc[s * 3 + k] == 0.0) continue;
-        const int s0 = a.s0a + s;
-        if (MODE == 0) atomicAdd(&a.out[(size_t)q0 * n + s0], sacc[s * 3]);
-        else atomicAdd(&a.out[((size_t)q0 * n + s0) * 3 + k], sacc[s * 3 + k]);
+        if (lane < qn) evaluate(queue[lane]);
+        __syncwarp();
     }
 }
 
-// F0 = FunitE w v / (1/tau T^2) where |1/tau| > zero_prec (CreateFzero).
-__global__ void k_bte_f0(int ntr, int n, const int* tr_grid, const double* omega, const double* vel,
-                         const double* inv_tau, double T, double* F0) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntr * n; i += gridDim.x * blockDim.x) {
-        const int q = i / n, s = i % n, g0 = tr_grid[q];
-        const double it = inv_tau[i];
-        for (int k = 0; k < 3; ++k) {
-            double f = 0.0;
-            if (!(g0 == 0 && s < 3) && fabs(it) > ZERO_PREC)
-                f = FUNIT_E * omega[(size_t)g0 * n + s] * vel[((size_t)g0 * n + s) * 3 + k] / (it * (T * T));
-            F0[(size_t)i * 3 + k] = f;
-        }
+// The merged entry of grid modes (x, s1), (p(x), s2) of one row, element j = (s1 n + s2) nq + x of its
+// (P, Q) block: both orderings of the pair share W and F(x, s1) + F(p(x), s2).  False when another
+// element stands for it or it is zero.
+__device__ __forceinline__ bool bte_entry(int j, int n, int nq, int s0, const int* __restrict__ p,
+                                          const double2* __restrict__ pq, const double* __restrict__ W, int2& kk,
+                                          double2& e) {
+    const int x = j % nq, s12 = j / nq, s1 = s12 / n, s2 = s12 % n, px = p[x];
+    if (px < x || (px == x && s2 < s1)) return false;
+    const double2 u = pq[j];
+    if (px == x && s1 == s2) {
+        e = make_double2(0.0, u.y);
+    } else {
+        const double2 v = pq[(s2 * n + s1) * nq + px];
+        e = make_double2(u.x - v.x, u.y + v.y);
     }
+    if (e.x == 0.0 && e.y == 0.0) return false;
+    const double w = 4.0 * W[(size_t)x * n * n * n + (s0 * n + s1) * n + s2];
+    if (w == 0.0) return false;
+    e.x *= w;
+    e.y *= w;
+    kk = make_int2(x * n + s1, px * n + s2);
+    return true;
 }
 
-// multiplyTaudFnew then F = F0 + dF.
-__global__ void k_bte_update(int ntr, int n, const int* tr_grid, const double* inv_tau, const double* F0,
-                             double* dF, double* F) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntr * n; i += gridDim.x * blockDim.x) {
-        const int q = i / n, s = i % n;
-        const double it = inv_tau[i];
-        const bool scale = !(tr_grid[q] == 0 && s < 3) && fabs(it) > ZERO_PREC;
-        for (int k = 0; k < 3; ++k) {
-            double d = dF[(size_t)i * 3 + k];
-            if (scale) d /= it;
-            F[(size_t)i * 3 + k] = F0[(size_t)i * 3 + k] + d;
-        }
-    }
-}
+struct RowArgs {
+    int n, nq, q0_first;
+    const int* partner;    // [ntr][nq]
+    const double2* pq;     // [slot][s0][s1][s2][x]
+    const double* wgrid;   // [slot][x][s0][s1][s2]
+};
 
-// kappa = kW_mK / (Nq V) sum_{q, s} deg w n (n+1) v (x) F   (one CTA, tree reduction)
-__global__ void __launch_bounds__(256) k_bte_kappa(int ntr, int n, int nq, double vol, const int* tr_grid,
-                                                   const int* deg, const double* omega, const double* nbe,
-                                                   const double* vel, const double* F, double* kappa) {
-    __shared__ double red[256][9];
-    double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int i = threadIdx.x; i < ntr * n; i += blockDim.x) {
-        const int q = i / n, s = i % n, g0 = tr_grid[q];
-        if (g0 == 0 && s < 3) continue;
-        const double w = omega[(size_t)g0 * n + s], nb = nbe[(size_t)g0 * n + s];
-        const double pre = double(deg[q]) * w * nb * (nb + 1.0);
-        const double* v = vel + ((size_t)g0 * n + s) * 3;
-        const double* f = F + (size_t)i * 3;
-        for (int x = 0; x < 3; ++x)
-            for (int y = 0; y < 3; ++y) acc[3 * x + y] += pre * (v[x] * f[y]);
+// One block per segment of a row: blockIdx.x = (slot n + s0) nseg + segment, [seg, seg + 1) / nseg of the
+// row's elements.  COUNT: its entries to cnt.  Otherwise they are written in element order from base + boff
+// on, and that offset to off.
+template <bool COUNT>
+__global__ void __launch_bounds__(256) k_bte_entries(RowArgs a, int nseg, int* __restrict__ cnt,
+                                                     const int* __restrict__ boff, long long base0, int last,
+                                                     int* __restrict__ off, int2* __restrict__ kk,
+                                                     double2* __restrict__ pqo) {
+    __shared__ int wsum[8];
+    const int n = a.n, nq = a.nq, row = blockIdx.x / nseg, seg = blockIdx.x % nseg;
+    const int slot = row / n, s0 = row % n, len = n * n * nq;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int step = ((len + nseg - 1) / nseg + 255) / 256 * 256;
+    const int j1 = min(len, (seg + 1) * step);
+    const int* p = a.partner + (size_t)(a.q0_first + slot) * nq;
+    const double2* pq = a.pq + (size_t)row * len;
+    const double* W = a.wgrid + (size_t)slot * nq * n * n * n;
+    int total = 0;
+    long long base = 0;
+    if (!COUNT) {
+        const size_t g = (size_t)a.q0_first * n * nseg + blockIdx.x;
+        base = base0 + boff[blockIdx.x];
+        if (threadIdx.x == 0) off[g] = (int)base;
+        if (threadIdx.x == 0 && last && blockIdx.x == gridDim.x - 1) off[g + 1] = (int)(base0 + boff[blockIdx.x + 1]);
     }
-    for (int k = 0; k < 9; ++k) red[threadIdx.x][k] = acc[k];
-    __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-        if (threadIdx.x < h)
-            for (int k = 0; k < 9; ++k) red[threadIdx.x][k] += red[threadIdx.x + h][k];
+    for (int j0 = seg * step; j0 < j1; j0 += 256) {
+        const int j = j0 + (int)threadIdx.x;
+        int2 k;
+        double2 e;
+        const bool on = j < j1 && bte_entry(j, n, nq, s0, p, pq, W, k, e);
+        if (COUNT) {
+            total += on;
+            continue;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (lane == 0) wsum[warp] = __popc(m);
+        __syncthreads();
+        int before = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            before += w < warp ? wsum[w] : 0;
+            all += wsum[w];
+        }
+        if (on) {
+            const long long o = base + before + __popc(m & ((1u << lane) - 1));
+            kk[o] = k;
+            pqo[o] = e;
+        }
+        base += all;
         __syncthreads();
     }
-    if (threadIdx.x < 9) kappa[threadIdx.x] = KW_MK * (1.0 / (double(nq) * vol)) * red[0][threadIdx.x];
+    if (COUNT) {
+        for (int o = 16; o > 0; o >>= 1) total += __shfl_down_sync(0xffffffffu, total, o);
+        if (lane == 0) wsum[warp] = total;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int t = 0;
+            for (int w = 0; w < 8; ++w) t += wsum[w];
+            cnt[blockIdx.x] = t;
+        }
+    }
 }
 
-int grid_x(long long items, int threads, int slots) {
-    long long want = (items + (long long)threads * 4 - 1) / ((long long)threads * 4);
-    long long cap = (148LL * 16 + slots - 1) / slots;
-    if (want > cap) want = cap;
-    return (int)(want < 1 ? 1 : want);
+// Sums of one block's 256 threads, valid in thread 0.
+template <int NV>
+__device__ __forceinline__ void block_sum(double* v, double (*red)[8]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        v[k] = tet::warp_sum(v[k]);
+        if (lane == 0) red[k][warp] = v[k];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            double t = 0.0;
+            for (int w = 0; w < 8; ++w) t += red[k][w];
+            v[k] = t;
+        }
+    __syncthreads();
+}
+
+// Row sums straight from the (P, Q) blocks of a batch (the operator did not fit): MODE 0 1/tau, MODE 1
+// dF = -sum c (F(k1) + F(k2)).
+template <int MODE>
+__global__ void __launch_bounds__(256) k_bte_dense(RowArgs a, const double* __restrict__ nbe,
+                                                   const double* __restrict__ Fg, double* __restrict__ out) {
+    __shared__ double red[3][8];
+    const int n = a.n, nq = a.nq, slot = blockIdx.x / n, s0 = blockIdx.x % n, len = n * n * nq;
+    const int* p = a.partner + (size_t)(a.q0_first + slot) * nq;
+    const double2* pq = a.pq + (size_t)blockIdx.x * len;
+    const double* W = a.wgrid + (size_t)slot * nq * n * n * n;
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int j = threadIdx.x; j < len; j += 256) {
+        int2 k;
+        double2 e;
+        if (!bte_entry(j, n, nq, s0, p, pq, W, k, e)) continue;
+        const double n1 = nbe[k.x], n2 = nbe[k.y];
+        const double c = (n1 - n2) * e.x + (1.0 + n1 + n2) * e.y;
+        if (MODE == 0) {
+            v[0] += c;
+        } else {
+            for (int d = 0; d < 3; ++d) v[d] -= c * (Fg[4 * (size_t)k.x + d] + Fg[4 * (size_t)k.y + d]);
+        }
+    }
+    constexpr int NV = MODE == 0 ? 1 : 3;
+    block_sum<NV>(v, red);
+    if (threadIdx.x == 0)
+        for (int d = 0; d < NV; ++d) out[((size_t)a.q0_first * n + blockIdx.x) * NV + d] = v[d];
+}
+
+struct StepArgs {
+    int ntr, n, nq;
+    double vol, T;
+    const int* tr_grid;
+    const int* neg;
+    const int* deg;
+    const double* omega;
+    const double* nbe;      // at this temperature
+    const double* vel;
+    const double* inv_tau;
+    const double* dF;
+    double* F0;
+    double* Fg;             // [g][s][4] F at every grid mode, padded to one 32-byte sector
+    double* part;           // [blocks][9] kappa partial sums
+    unsigned* ticket;       // zero between launches
+    double* kappa;          // [9] of this iteration
+};
+
+// One iteration's end for every mode of the time-reversal set: F = F0 (INIT, CreateFzero:
+// F0 = FunitE w v / (1/tau T^2) where |1/tau| > zero_prec) or F0 + dF tau (multiplyTaudFnew); F at both
+// grid points of the pair (F(-q) = -F(q)); and kappa = kW_mK / (Nq V) sum deg w n (n+1) v (x) F, block
+// sums added in block order by the last block to finish.
+template <bool INIT>
+__global__ void __launch_bounds__(256) k_bte_step(StepArgs a) {
+    __shared__ double red[9][8];
+    __shared__ bool last;
+    const int n = a.n;
+    double acc[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) acc[k] = 0.0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.ntr * n; i += gridDim.x * blockDim.x) {
+        const int q = i / n, s = i % n, g0 = a.tr_grid[q], gn = a.neg[g0];
+        const double it = a.inv_tau[i];
+        const bool zero = g0 == 0 && s < 3;
+        const bool scale = !zero && fabs(it) > ZERO_PREC;
+        const double w = a.omega[(size_t)g0 * n + s];
+        const double* v = a.vel + ((size_t)g0 * n + s) * 3;
+        double f[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            if (INIT) {
+                f[k] = scale ? FUNIT_E * w * v[k] / (it * (a.T * a.T)) : 0.0;
+                a.F0[(size_t)i * 3 + k] = f[k];
+            } else {
+                double d = a.dF[(size_t)i * 3 + k];
+                if (scale) d /= it;
+                f[k] = a.F0[(size_t)i * 3 + k] + d;
+            }
+        }
+        double2* o = reinterpret_cast<double2*>(a.Fg + 4 * ((size_t)g0 * n + s));
+        o[0] = make_double2(f[0], f[1]);
+        o[1] = make_double2(f[2], 0.0);
+        if (gn != g0) {
+            o = reinterpret_cast<double2*>(a.Fg + 4 * ((size_t)gn * n + s));
+            o[0] = make_double2(-f[0], -f[1]);
+            o[1] = make_double2(-f[2], 0.0);
+        }
+        if (zero) continue;
+        const double nb = a.nbe[(size_t)g0 * n + s];
+        const double pre = double(a.deg[q]) * w * nb * (nb + 1.0);
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+#pragma unroll
+            for (int y = 0; y < 3; ++y) acc[3 * x + y] += pre * (v[x] * f[y]);
+    }
+    block_sum<9>(acc, red);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) a.part[9 * (size_t)blockIdx.x + k] = acc[k];
+        __threadfence();
+        last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    if (threadIdx.x < 9) {
+        __threadfence();
+        double t = 0.0;
+        for (unsigned b = 0; b < gridDim.x; ++b) t += __ldcg(a.part + 9 * (size_t)b + threadIdx.x);
+        a.kappa[threadIdx.x] = KW_MK * (1.0 / (double(a.nq) * a.vol)) * t;
+    }
+    if (threadIdx.x == 0) *a.ticket = 0;
 }
 
 // Time-reversal set on the host from the grid addresses.
@@ -271,7 +452,6 @@ int build_tr_set(spring_ctx* c) {
     c->ps_tr.q0_int = c->d_tr_int.p;
     c->ps_tr.q0_grid = c->d_tr_grid.p;
     c->ps_tr.done = false;
-    dfree(c->d_wtr);
     return SPRING_OK;
 }
 
@@ -302,67 +482,141 @@ __global__ void k_bteg_gather(long long n, const s3::BteEntry* __restrict__ e, c
         pq[i] = make_double2(x.P, x.Q);
     }
 }
-// c = (n1 - n2) P + (1 + n1 + n2) Q at one temperature
-__global__ void k_bteg_coef(long long n, const int2* __restrict__ kk, const double2* __restrict__ pq,
-                            const double* __restrict__ nbe, double* __restrict__ cf) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+// Row r holds the entries off[r nseg] .. off[(r + 1) nseg].  One block per row: c = (n1 - n2) P + (1 + n1 + n2) Q of its entries at one temperature, and their sum,
+// 1/tau.
+__global__ void __launch_bounds__(256) k_bteg_coef(int nseg, const int* __restrict__ off, const int2* __restrict__ kk,
+                                                  const double2* __restrict__ pq, const double* __restrict__ nbe,
+                                                  double* __restrict__ cf, double* __restrict__ inv_tau) {
+    __shared__ double red[1][8];
+    double v[1] = {0.0};
+    const int end = off[((size_t)blockIdx.x + 1) * nseg];
+    for (int i = off[(size_t)blockIdx.x * nseg] + threadIdx.x; i < end; i += 256) {
         const int2 k = kk[i];
-        const double2 v = pq[i];
+        const double2 e = pq[i];
         const double n1 = nbe[k.x], n2 = nbe[k.y];
-        cf[i] = (n1 - n2) * v.x + (1.0 + n1 + n2) * v.y;
+        const double c = (n1 - n2) * e.x + (1.0 + n1 + n2) * e.y;
+        cf[i] = c;
+        v[0] += c;
     }
+    block_sum<1>(v, red);
+    if (threadIdx.x == 0) inv_tau[blockIdx.x] = v[0];
 }
-// F at every grid mode from the time-reversal slots: Fg[g][s] = sgn(g) F[pos(g)][s], padded to four
-// doubles (32 bytes, one L2 sector) per mode for the row pass's gathers.
-__global__ void k_bteg_expand(int nq, int n, const int* __restrict__ pos, const int* __restrict__ sgn,
-                              const double* __restrict__ F, double* __restrict__ Fg) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nq * n; i += gridDim.x * blockDim.x) {
-        const int g = i / n, sx = i % n;
-        const double sg = sgn[g];
-        const double* f = F + ((size_t)pos[g] * n + sx) * 3;
-        double2* o = reinterpret_cast<double2*>(Fg + 4 * (size_t)i);
-        o[0] = make_double2(sg * f[0], sg * f[1]);
-        o[1] = make_double2(sg * f[2], 0.0);
-    }
-}
-// One warp per row: MODE 0 inv_tau[r] = sum c; MODE 1 dF[r] = -sum c (Fg[k1] + Fg[k2]) (Fg: four
-// doubles per mode, the fourth zero).
-template <int MODE>
-__global__ void __launch_bounds__(256) k_bteg_rows(int rows, const int* __restrict__ rowoff, const int2* __restrict__ kk,
+
+// dF[r] = -sum c (Fg[k1] + Fg[k2]), one block per row (Fg: four doubles per mode, the fourth zero).
+__global__ void __launch_bounds__(256) k_bteg_rows(int nseg, const int* __restrict__ off, const int2* __restrict__ kk,
                                                   const double* __restrict__ cf, const double* __restrict__ Fg,
-                                                  double* __restrict__ out) {
-    const int lane = threadIdx.x & 31;
-    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += (gridDim.x * blockDim.x) >> 5) {
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-        for (int i = rowoff[r] + lane; i < rowoff[r + 1]; i += 32) {
-            const double c = cf[i];
-            if (MODE == 0) {
-                a0 += c;
-            } else {
-                const int2 k = kk[i];
-                const double2* f1 = reinterpret_cast<const double2*>(Fg + 4 * (size_t)k.x);
-                const double2* f2 = reinterpret_cast<const double2*>(Fg + 4 * (size_t)k.y);
-                const double2 u1 = f1[0], v1 = f1[1], u2 = f2[0], v2 = f2[1];
-                a0 -= c * (u1.x + u2.x);
-                a1 -= c * (u1.y + u2.y);
-                a2 -= c * (v1.x + v2.x);
-            }
-        }
-        a0 = tet::warp_sum(a0);
-        if (MODE == 1) {
-            a1 = tet::warp_sum(a1);
-            a2 = tet::warp_sum(a2);
-        }
-        if (lane == 0) {
-            if (MODE == 0) {
-                out[r] = a0;
-            } else {
-                out[3 * (size_t)r] = a0;
-                out[3 * (size_t)r + 1] = a1;
-                out[3 * (size_t)r + 2] = a2;
-            }
-        }
+                                                  double* __restrict__ dF) {
+    __shared__ double red[3][8];
+    double v[3] = {0.0, 0.0, 0.0};
+    const int end = off[((size_t)blockIdx.x + 1) * nseg];
+    for (int i = off[(size_t)blockIdx.x * nseg] + threadIdx.x; i < end; i += 256) {
+        const double c = cf[i];
+        const int2 k = kk[i];
+        const double2* f1 = reinterpret_cast<const double2*>(Fg + 4 * (size_t)k.x);
+        const double2* f2 = reinterpret_cast<const double2*>(Fg + 4 * (size_t)k.y);
+        const double2 u1 = f1[0], v1 = f1[1], u2 = f2[0], v2 = f2[1];
+        v[0] -= c * (u1.x + u2.x);
+        v[1] -= c * (u1.y + u2.y);
+        v[2] -= c * (v1.x + v2.x);
     }
+    block_sum<3>(v, red);
+    if (threadIdx.x == 0)
+        for (int d = 0; d < 3; ++d) dF[3 * (size_t)blockIdx.x + d] = v[d];
+}
+
+}  // namespace
+
+namespace {
+
+// The loop of main.f90:295-361 at every temperature: tau(T) fills w.inv_tau, df(T) fills w.dF from w.Fg.
+// `ahead`: iterations queued before kappa is read back and the convergence test made (iterations past
+// the converged one change no output).
+template <class Tau, class DF>
+int bte_iterate(spring_ctx* c, double eps_k, int max_iter, int ahead, Tau tau, DF df, double* h_kappa,
+                double* h_kappa_rta, int* h_iters) {
+    const int n = c->ndof, ntr = c->ntr, nq = c->nq, rows = ntr * n;
+    constexpr int MAX_AHEAD = 16;
+    const int blocks = std::max(1, std::min((rows + 255) / 256, 148));
+    BteWork& w = c->bte;
+    // one buffer: Fg | F0 | dF | 1/tau | kappa partial sums | kappa of the queued iterations | ticket
+    const size_t nFg = (size_t)nq * n * 4, nF = (size_t)rows * 3;
+    SPRING_CHECK(dalloc(c, w.vec, nFg + 2 * nF + rows + (size_t)blocks * 9 + 9 * (MAX_AHEAD + 1) + 1, "BTE vectors"));
+    w.Fg = w.vec.p;
+    w.F0 = w.Fg + nFg;
+    w.dF = w.F0 + nF;
+    w.inv_tau = w.dF + nF;
+    double* part = w.inv_tau + rows;
+    double* hist = part + (size_t)blocks * 9;
+    unsigned* ticket = reinterpret_cast<unsigned*>(hist + 9 * (MAX_AHEAD + 1));
+    SPRING_CHECK(zero(c, ticket, sizeof(double), "BTE ticket"));
+    auto step = [&](bool init, int T, int at) -> int {
+        const StepArgs a{ntr, n, nq, c->vol, c->temps[T], c->d_tr_grid.p, c->d_neg.p, c->d_tr_deg.p, c->ph_grid.omega.p,
+                         c->ph_grid.nbe.p + (size_t)T * nq * n, c->ph_grid.vel.p, w.inv_tau, w.dF, w.F0, w.Fg, part,
+                         ticket, hist + 9 * at};
+        if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
+        if (init) k_bte_step<true><<<blocks, 256, 0, c->stream>>>(a);
+        else k_bte_step<false><<<blocks, 256, 0, c->stream>>>(a);
+        return launch_check(c, init ? "k_bte_step<init>" : "k_bte_step");
+    };
+    for (int T = 0; T < c->nT; ++T) {
+        SPRING_CHECK(tau(T));
+        SPRING_CHECK(step(true, T, 0));
+        double kap[(MAX_AHEAD + 1) * 9], k0[9], kold[9], knew[9];
+        int iter = 0, chunk = std::min(ahead, MAX_AHEAD);
+        double dprev = 0.0, d = 0.0;
+        for (bool done = false, first = true; !done; first = false) {
+            chunk = std::max(1, std::min(chunk, max_iter + 1 - iter));
+            for (int k = 1; k <= chunk; ++k) {
+                SPRING_CHECK(df(T));
+                SPRING_CHECK(step(false, T, k));
+            }
+            SPRING_CHECK(d2h(c, kap, hist, sizeof(double) * 9 * (chunk + 1), "kappa"));
+            if (first) {
+                std::copy(kap, kap + 9, k0);
+                std::copy(kap, kap + 9, kold);
+            }
+            for (int k = 1; k <= chunk && !done; ++k) {
+                ++iter;
+                std::copy(kap + 9 * k, kap + 9 * k + 9, knew);
+                dprev = d;
+                d = 0.0;
+                for (int x = 0; x < 9; ++x) d = std::max(d, std::fabs(knew[x] - kold[x]));
+                done = d < eps_k || iter > max_iter;
+                if (!done) std::copy(knew, knew + 9, kold);
+            }
+            if (ahead > 1) {  // the rest at the present rate of convergence
+                chunk = ahead;
+                if (d > 0.0 && dprev > d) chunk = (int)std::min(double(MAX_AHEAD), std::ceil(std::log(d / eps_k) / std::log(dprev / d)));
+            }
+        }
+        if (h_kappa) std::copy(knew, knew + 9, h_kappa + 9 * T);
+        if (h_kappa_rta) std::copy(k0, k0 + 9, h_kappa_rta + 9 * T);
+        if (h_iters) h_iters[T] = iter;
+    }
+    return SPRING_OK;
+}
+
+// The iterations over an operator in HBM: `cnt` entries, row r at off[r nseg] .. off[(r + 1) nseg].
+int bte_operator_run(spring_ctx* c, int rows, int nseg, const int* off, const int2* kk, const double2* pq, long long cnt,
+                     double eps_k, int max_iter, double* h_kappa, double* h_kappa_rta, int* h_iters) {
+    BteWork& w = c->bte;
+    SPRING_CHECK(dalloc(c, w.cf, std::max<long long>(cnt, 1), "operator coefficients"));
+    auto tau = [&](int T) -> int {
+        if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
+        k_bteg_coef<<<rows, 256, 0, c->stream>>>(nseg, off, kk, pq, c->ph_grid.nbe.p + (size_t)T * c->nq * c->ndof, w.cf.p,
+                                                w.inv_tau);
+        return launch_check(c, "k_bteg_coef");
+    };
+    auto df = [&](int) -> int {
+        if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
+        k_bteg_rows<<<rows, 256, 0, c->stream>>>(nseg, off, kk, w.cf.p, w.Fg, w.dF);
+        return launch_check(c, "k_bteg_rows<dF>");
+    };
+    // A pass over few entries is shorter than the wait for kappa: several are queued per readback.
+    const int rc = bte_iterate(c, eps_k, max_iter, cnt < (4 << 20) ? 8 : 1, tau, df, h_kappa, h_kappa_rta, h_iters);
+    cudaStreamSynchronize(c->stream);
+    if (w.cf.n > (8u << 20)) dfree(w.cf);  // large ones are given back
+    return rc;
 }
 
 }  // namespace
@@ -455,181 +709,151 @@ int run_bte_gauss(spring_ctx* c, double sigma, double eps_k, int max_iter, doubl
         h_stats[0] = (double)cnt;
         h_stats[1] = (double)npairs;
     }
-    // ---- iterations per temperature
-    DBuf<double> inv_tau, F0, F, dF, kap, cf, Fg;
-    int rc = dalloc(c, inv_tau, (size_t)rows, "1/tau");
-    if (rc == SPRING_OK) rc = dalloc(c, F0, (size_t)rows * 3, "F0");
-    if (rc == SPRING_OK) rc = dalloc(c, F, (size_t)rows * 3, "F");
-    if (rc == SPRING_OK) rc = dalloc(c, dF, (size_t)rows * 3, "dF");
-    if (rc == SPRING_OK) rc = dalloc(c, kap, 9, "kappa");
-    if (rc == SPRING_OK) rc = dalloc(c, cf, std::max<long long>(cnt, 1), "operator coefficients");
-    if (rc == SPRING_OK) rc = dalloc(c, Fg, (size_t)nq * n * 4, "F on the grid");
-    const int rblocks = std::max(1, std::min((rows + 7) / 8, 148 * 16));
-    const int eblocks = std::max(1, std::min((rows + threads - 1) / threads, 148 * 8));
-    auto kappa_of = [&](int T, const double* Fv, double* out9) -> int {
-        if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
-        k_bte_kappa<<<1, 256, 0, c->stream>>>(ntr, n, nq, c->vol, c->d_tr_grid.p, c->d_tr_deg.p, c->ph_grid.omega.p,
-                                              c->ph_grid.nbe.p + (size_t)T * nq * n, c->ph_grid.vel.p, Fv, kap.p);
-        SPRING_CHECK(launch_check(c, "k_bte_kappa"));
-        return d2h(c, out9, kap.p, sizeof(double) * 9, "kappa");
-    };
-    for (int T = 0; rc == SPRING_OK && T < c->nT; ++T) {
-        const double* nbeT = c->ph_grid.nbe.p + (size_t)T * nq * n;
-        if (cnt > 0) {
-            if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure"); break; }
-            k_bteg_coef<<<blocks_for(cnt), threads, 0, c->stream>>>(cnt, c->d_bteg_kk.p, c->d_bteg_pq.p, nbeT, cf.p);
-            if ((rc = launch_check(c, "k_bteg_coef")) != SPRING_OK) break;
-        }
-        if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure"); break; }
-        k_bteg_rows<0><<<rblocks, 256, 0, c->stream>>>(rows, c->d_bteg_row.p, c->d_bteg_kk.p, cf.p, nullptr, inv_tau.p);
-        if ((rc = launch_check(c, "k_bteg_rows<tau>")) != SPRING_OK) break;
-        if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure"); break; }
-        k_bte_f0<<<eblocks, threads, 0, c->stream>>>(ntr, n, c->d_tr_grid.p, c->ph_grid.omega.p, c->ph_grid.vel.p,
-                                                    inv_tau.p, c->temps[T], F0.p);
-        if ((rc = launch_check(c, "k_bte_f0")) != SPRING_OK) break;
-        if (cudaMemcpyAsync(F.p, F0.p, sizeof(double) * rows * 3, cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess) {
-            rc = fail(c, SPRING_ERR_CUDA, "F copy");
-            break;
-        }
-        double k0[9], kold[9], knew[9];
-        if ((rc = kappa_of(T, F.p, k0)) != SPRING_OK) break;
-        std::copy(k0, k0 + 9, kold);
-        std::copy(k0, k0 + 9, knew);
-        int iter = 0;
-        for (;;) {
-            ++iter;
-            if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure"); break; }
-            k_bteg_expand<<<blocks_for((long long)nq * n), threads, 0, c->stream>>>(nq, n, c->d_tr_pos.p, c->d_tr_sgn.p,
-                                                                                     F.p, Fg.p);
-            if ((rc = launch_check(c, "k_bteg_expand")) != SPRING_OK) break;
-            if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure"); break; }
-            k_bteg_rows<1><<<rblocks, 256, 0, c->stream>>>(rows, c->d_bteg_row.p, c->d_bteg_kk.p, cf.p, Fg.p, dF.p);
-            if ((rc = launch_check(c, "k_bteg_rows<dF>")) != SPRING_OK) break;
-            if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure"); break; }
-            k_bte_update<<<eblocks, threads, 0, c->stream>>>(ntr, n, c->d_tr_grid.p, inv_tau.p, F0.p, dF.p, F.p);
-            if ((rc = launch_check(c, "k_bte_update")) != SPRING_OK) break;
-            if ((rc = kappa_of(T, F.p, knew)) != SPRING_OK) break;
-            double d = 0.0;
-            for (int k = 0; k < 9; ++k) d = std::max(d, std::fabs(knew[k] - kold[k]));
-            if (d < eps_k || iter > max_iter) break;
-            std::copy(knew, knew + 9, kold);
-        }
-        if (rc != SPRING_OK) break;
-        if (h_kappa) std::copy(knew, knew + 9, h_kappa + 9 * T);
-        if (h_kappa_rta) std::copy(k0, k0 + 9, h_kappa_rta + 9 * T);
-        if (h_iters) h_iters[T] = iter;
-    }
-    dfree(inv_tau); dfree(F0); dfree(F); dfree(dF); dfree(kap); dfree(cf); dfree(Fg);
-    return rc;
+    return bte_operator_run(c, rows, 1, c->d_bteg_row.p, c->d_bteg_kk.p, c->d_bteg_pq.p, cnt, eps_k, max_iter, h_kappa,
+                            h_kappa_rta, h_iters);
 }
 
 int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* h_kappa_rta, int* h_iters) {
     if (c->ntr == 0) SPRING_CHECK(build_tr_set(c));
     if (!c->ps_tr.done) SPRING_CHECK(run_enumerate3(c, c->ps_tr));
-    const int n = c->ndof, ntr = c->ntr, nq = c->nq;
+    const int n = c->ndof, ntr = c->ntr, nq = c->nq, rows = ntr * n;
     const size_t slot = (size_t)nq * n * n * n;
     const Q0View view{c->d_tr_int.p, c->d_tr_grid.p, c->ph_grid.evec.p, c->ph_grid.omega.p, c->ph_grid.oneby.p};
-    // W grids: all of them resident when they fit the budget, else batches recomputed per pass
-    const size_t budget = (size_t)40 << 30;
-    size_t free_b = 0, total_b = 0;
-    cudaMemGetInfo(&free_b, &total_b);
-    const bool cache_all = slot * ntr * sizeof(double) <= std::min(budget, free_b / 2);
-    int batch = ntr;
-    if (cache_all) {
-        if (!c->d_wtr.p || c->d_wtr.n < slot * ntr) {
-            SPRING_CHECK(dalloc(c, c->d_wtr, slot * ntr, "time-reversal W grids"));
-            SPRING_CHECK(run_v3_wgrid(c, c->ps_tr, view, 0, ntr, c->d_wtr.p));
-        }
-    } else {
-        batch = (int)std::max<size_t>(1, ((size_t)96 << 20) / (slot * sizeof(double)));
-        batch = std::min(batch, ntr);
-        SPRING_CHECK(dalloc(c, c->d_w, slot * batch, "W buffer"));
-    }
-    DBuf<double> inv_tau, F0, F, dF, kap;
-    int rc = dalloc(c, inv_tau, (size_t)ntr * n, "1/tau");
-    if (rc == SPRING_OK) rc = dalloc(c, F0, (size_t)ntr * n * 3, "F0");
-    if (rc == SPRING_OK) rc = dalloc(c, F, (size_t)ntr * n * 3, "F");
-    if (rc == SPRING_OK) rc = dalloc(c, dF, (size_t)ntr * n * 3, "dF");
-    if (rc == SPRING_OK) rc = dalloc(c, kap, 9, "kappa");
-
-    auto pass = [&](int mode, int T) -> int {
-        PassArgs pa;
-        pa.n = n;
-        pa.nq = nq;
-        pa.ntet = 6 * nq;
-        pa.tr_grid = c->d_tr_grid.p;
-        pa.tr_pos = c->d_tr_pos.p;
-        pa.tr_sgn = c->d_tr_sgn.p;
-        pa.neg = c->d_neg.p;
-        pa.partner = c->ps_tr.partner.p;
-        pa.omega = c->ph_grid.omega.p;
-        pa.nbe = c->ph_grid.nbe.p + (size_t)T * nq * n;
-        pa.F = F.p;
-        pa.out = mode == 0 ? inv_tau.p : dF.p;
-        const long long items = (long long)pa.ntet * n * n;
-        for (int b = 0; b < ntr; b += batch) {
-            const int nb = std::min(batch, ntr - b);
-            if (!cache_all) SPRING_CHECK(run_v3_wgrid(c, c->ps_tr, view, b, nb, c->d_w.p));
-            pa.q0_first = b;
-            pa.wgrid = cache_all ? c->d_wtr.p + slot * b : c->d_w.p;
-            dim3 grid(grid_x(items, 128, nb), nb);
-            for (int s0a = 0; s0a < n; s0a += NS0) {
-                pa.s0a = s0a;
-                pa.s0n = std::min(NS0, n - s0a);
-                if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
-                if (mode == 0) k_bte_pass<0><<<grid, 128, 0, c->stream>>>(pa, reinterpret_cast<const int4*>(c->d_tetra.p));
-                else k_bte_pass<1><<<grid, 128, 0, c->stream>>>(pa, reinterpret_cast<const int4*>(c->d_tetra.p));
-                SPRING_CHECK(launch_check(c, mode == 0 ? "k_bte_pass<tau>" : "k_bte_pass<dF>"));
-            }
-        }
-        return SPRING_OK;
-    };
-    auto kappa_of = [&](int T, const double* Fv, double* out9) -> int {
+    // q0 per batch: their (P, Q) and W grids stay around the L2 size
+    const int batch = (int)std::max<size_t>(1, std::min<size_t>(ntr, ((size_t)96 << 20) / (slot * sizeof(double2))));
+    DBuf<float> wf;
+    DBuf<int> cnt, boff;
+    BteWork& w = c->bte;
+    // W and the tetrahedron weights of q0 b .. b + nb - 1 into d_w and w.pq
+    auto build = [&](int b, int nb) -> int {
+        SPRING_CHECK(run_v3_wgrid(c, c->ps_tr, view, b, nb, c->d_w.p));
+        SPRING_CHECK(zero(c, w.pq.p, sizeof(double2) * slot * nb, "tetrahedron weights"));
+        WgtArgs a{};
+        a.n = n;
+        a.nq = nq;
+        a.ntet = 6 * nq;
+        a.q0_first = b;
+        a.tr_grid = c->d_tr_grid.p;
+        a.neg = c->d_neg.p;
+        a.partner = c->ps_tr.partner.p;
+        a.wf = wf.p;
+        a.omega = c->ph_grid.omega.p;
+        a.pq = w.pq.p;
+        const int groups = (a.ntet + 31) / 32, passes = (n + NS0 - 1) / NS0;
+        a.nb2 = (n + BS2 - 1) / BS2;
+        a.per1 = 6;  // as in k_tetra3: shorter units while the chip is not full
+        while (a.per1 > 1 && (long long)groups * a.nb2 * ((n + a.per1 - 1) / a.per1) * nb * passes < 148LL * 32) --a.per1;
+        a.nb1 = (n + a.per1 - 1) / a.per1;
+        a.units = (long long)groups * a.nb1 * a.nb2;
+        const long long cap = std::max<long long>(1, 148LL * 8 / ((long long)nb * passes));
+        const dim3 grid((unsigned)std::max<long long>(1, std::min<long long>((a.units + TW - 1) / TW, cap)), nb, passes);
         if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
-        k_bte_kappa<<<1, 256, 0, c->stream>>>(ntr, n, nq, c->vol, c->d_tr_grid.p, c->d_tr_deg.p, c->ph_grid.omega.p,
-                                              c->ph_grid.nbe.p + (size_t)T * nq * n, c->ph_grid.vel.p, Fv, kap.p);
-        SPRING_CHECK(launch_check(c, "k_bte_kappa"));
-        return d2h(c, out9, kap.p, sizeof(double) * 9, "kappa");
+        k_bte_weights<<<grid, 32 * TW, 0, c->stream>>>(a, reinterpret_cast<const int4*>(c->d_tetra.p));
+        return launch_check(c, "k_bte_weights");
     };
-    const int threads = 256, blocks = std::max(1, std::min((ntr * n + threads - 1) / threads, 148 * 8));
-    for (int T = 0; rc == SPRING_OK && T < c->nT; ++T) {
-        rc = zero(c, inv_tau.p, sizeof(double) * ntr * n, "1/tau");
-        if (rc == SPRING_OK) rc = pass(0, T);
-        if (rc == SPRING_OK && !launch_injected(c)) {
-            k_bte_f0<<<blocks, threads, 0, c->stream>>>(ntr, n, c->d_tr_grid.p, c->ph_grid.omega.p, c->ph_grid.vel.p,
-                                                        inv_tau.p, c->temps[T], F0.p);
-            rc = launch_check(c, "k_bte_f0");
+    auto row_args = [&](int b) { return RowArgs{n, nq, b, c->ps_tr.partner.p, w.pq.p, c->d_w.p}; };
+    bool stored = c->bt_gen == c->ph_gen && c->bt_pairs == c->ps_tr.gen && c->bt_n >= 0;
+    const int len = n * n * nq;
+    const int nseg = std::max(1, std::min(16, len / 4096));
+    int rc = SPRING_OK;
+    if (!stored) {
+        c->bt_gen = -1;
+        rc = dalloc(c, wf, (size_t)nq * n, "FP32 frequencies");
+        if (rc == SPRING_OK) rc = dalloc(c, c->d_w, slot * batch, "W buffer");
+        if (rc == SPRING_OK) rc = dalloc(c, w.pq, slot * batch, "tetrahedron weights");
+        if (rc == SPRING_OK) rc = dalloc(c, cnt, (size_t)batch * n * nseg + 1, "operator counts");
+        if (rc == SPRING_OK) rc = dalloc(c, boff, (size_t)batch * n * nseg + 1, "operator counts");
+        if (rc == SPRING_OK) rc = dalloc(c, c->d_bt_off, (size_t)rows * nseg + 1, "operator rows");
+        if (rc == SPRING_OK && launch_injected(c)) rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
+        if (rc == SPRING_OK) {
+            k_bte_wf<<<std::min((nq * n + 255) / 256, 148 * 8), 256, 0, c->stream>>>(nq, n, c->ph_grid.omega.p, wf.p);
+            rc = launch_check(c, "k_bte_wf");
         }
-        if (rc == SPRING_OK)
-            rc = cudaMemcpyAsync(F.p, F0.p, sizeof(double) * ntr * n * 3, cudaMemcpyDeviceToDevice, c->stream) ==
-                         cudaSuccess ? SPRING_OK : fail(c, SPRING_ERR_CUDA, "F copy");
-        double k0[9], kold[9], knew[9];
-        if (rc == SPRING_OK) rc = kappa_of(T, F.p, k0);
-        if (rc != SPRING_OK) break;
-        std::copy(k0, k0 + 9, kold);
-        std::copy(k0, k0 + 9, knew);
-        int iter = 0;
-        for (;;) {
-            ++iter;
-            rc = zero(c, dF.p, sizeof(double) * ntr * n * 3, "dF");
-            if (rc == SPRING_OK) rc = pass(1, T);
-            if (rc == SPRING_OK && !launch_injected(c)) {
-                k_bte_update<<<blocks, threads, 0, c->stream>>>(ntr, n, c->d_tr_grid.p, inv_tau.p, F0.p, dF.p, F.p);
-                rc = launch_check(c, "k_bte_update");
+        size_t free_b = 0, total_b = 0;
+        cudaMemGetInfo(&free_b, &total_b);
+        const long long per = sizeof(int2) + sizeof(double2);
+        const long long held = (long long)std::min(c->d_bt_kk.n, c->d_bt_pq.n);
+        long long most = std::max<long long>(held, (long long)(std::min((size_t)40 << 30, free_b / 2) / per));
+        most = std::min<long long>(most, c->bte_max_entries < 0 ? 0x7fffffffLL : c->bte_max_entries);
+        long long total = 0;
+        stored = true;
+        for (int b = 0; rc == SPRING_OK && stored && b < ntr; b += batch) {
+            const int nb = std::min(batch, ntr - b), segs = nb * n * nseg;
+            if ((rc = build(b, nb)) != SPRING_OK) break;
+            if ((rc = zero(c, cnt.p + segs, sizeof(int), "operator counts")) != SPRING_OK) break;
+            if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure"); break; }
+            k_bte_entries<true><<<segs, 256, 0, c->stream>>>(row_args(b), nseg, cnt.p, nullptr, 0, 0, nullptr, nullptr, nullptr);
+            if ((rc = launch_check(c, "k_bte_entries<count>")) != SPRING_OK) break;
+            if ((rc = run_exclusive_scan(c, cnt.p, boff.p, segs + 1)) != SPRING_OK) break;
+            int here = 0;
+            if ((rc = d2h(c, &here, boff.p + segs, sizeof here, "operator count")) != SPRING_OK) break;
+            const long long need = total + here;
+            if (need > most) { stored = false; break; }
+            if (need > (long long)std::min(c->d_bt_kk.n, c->d_bt_pq.n)) {
+                // room for the remaining rows at the fill seen so far
+                const long long done_rows = (long long)(b + nb);
+                long long cap = (long long)((double)need * ntr / done_rows * 1.1) + 1024;
+                cap = std::max(need, std::min(cap, most));
+                DBuf<int2> kk;
+                DBuf<double2> pq;
+                rc = dalloc(c, kk, cap, "BTE operator");
+                if (rc == SPRING_OK) rc = dalloc(c, pq, cap, "BTE operator");
+                if (rc == SPRING_OK && total > 0 &&
+                    (cudaMemcpyAsync(kk.p, c->d_bt_kk.p, sizeof(int2) * total, cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess ||
+                     cudaMemcpyAsync(pq.p, c->d_bt_pq.p, sizeof(double2) * total, cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess))
+                    rc = fail(c, SPRING_ERR_CUDA, "BTE operator copy");
+                cudaStreamSynchronize(c->stream);
+                if (rc == SPRING_ERR_ALLOC) {  // it does not fit after all
+                    dfree(kk);
+                    dfree(pq);
+                    rc = SPRING_OK;
+                    stored = false;
+                    break;
+                }
+                std::swap(kk, c->d_bt_kk);
+                std::swap(pq, c->d_bt_pq);
+                dfree(kk);
+                dfree(pq);
+                if (rc != SPRING_OK) break;
             }
-            if (rc == SPRING_OK) rc = kappa_of(T, F.p, knew);
-            if (rc != SPRING_OK) break;
-            double d = 0.0;
-            for (int k = 0; k < 9; ++k) d = std::max(d, std::fabs(knew[k] - kold[k]));
-            if (d < eps_k || iter > max_iter) break;
-            std::copy(knew, knew + 9, kold);
+            if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure"); break; }
+            k_bte_entries<false><<<segs, 256, 0, c->stream>>>(row_args(b), nseg, nullptr, boff.p, total, b + nb == ntr,
+                                                             c->d_bt_off.p, c->d_bt_kk.p, c->d_bt_pq.p);
+            rc = launch_check(c, "k_bte_entries");
+            total = need;
         }
-        if (rc != SPRING_OK) break;
-        if (h_kappa) std::copy(knew, knew + 9, h_kappa + 9 * T);
-        if (h_kappa_rta) std::copy(k0, k0 + 9, h_kappa_rta + 9 * T);
-        if (h_iters) h_iters[T] = iter;
+        if (rc == SPRING_OK && stored) {
+            c->bt_n = total;
+            c->bt_gen = c->ph_gen;
+            c->bt_pairs = c->ps_tr.gen;
+        }
     }
-    dfree(inv_tau); dfree(F0); dfree(F); dfree(dF); dfree(kap);
+    if (rc == SPRING_OK && stored) {
+        rc = bte_operator_run(c, rows, nseg, c->d_bt_off.p, c->d_bt_kk.p, c->d_bt_pq.p, c->bt_n, eps_k, max_iter, h_kappa,
+                              h_kappa_rta, h_iters);
+    } else if (rc == SPRING_OK) {
+        dfree(c->d_bt_kk);
+        dfree(c->d_bt_pq);
+        c->bt_n = -1;
+        auto pass = [&](int mode, int T) -> int {
+            for (int b = 0; b < ntr; b += batch) {
+                const int nb = std::min(batch, ntr - b);
+                SPRING_CHECK(build(b, nb));
+                if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
+                const double* nbe = c->ph_grid.nbe.p + (size_t)T * nq * n;
+                if (mode == 0) k_bte_dense<0><<<nb * n, 256, 0, c->stream>>>(row_args(b), nbe, nullptr, w.inv_tau);
+                else k_bte_dense<1><<<nb * n, 256, 0, c->stream>>>(row_args(b), nbe, w.Fg, w.dF);
+                SPRING_CHECK(launch_check(c, mode == 0 ? "k_bte_dense<tau>" : "k_bte_dense<dF>"));
+            }
+            return SPRING_OK;
+        };
+        rc = bte_iterate(c, eps_k, max_iter, 1, [&](int T) { return pass(0, T); }, [&](int T) { return pass(1, T); },
+                         h_kappa, h_kappa_rta, h_iters);
+    }
+    cudaStreamSynchronize(c->stream);
+    dfree(wf);
+    dfree(cnt);
+    dfree(boff);
     return rc;
 }
 

@@ -86,6 +86,13 @@ struct EwaldDev {
     DBuf<double2> cc, dd;
 };
 
+// Workspace of the iterative BTE (k_bte.cu), kept between calls.
+struct BteWork {
+    DBuf<double2> pq;          // (P, Q) grids of a batch
+    DBuf<double> cf, vec;      // operator coefficients of one temperature; the vectors below
+    double *Fg = nullptr, *F0 = nullptr, *dF = nullptr, *inv_tau = nullptr;
+};
+
 // Point-defect scattering (spring_set_point_defect, k_pdef.cu).
 struct PointDefectDev {
     bool on = false, mat_inv_full = true, optc_therm = true;
@@ -125,6 +132,7 @@ struct spring_ctx {
     bool force_generic_v3 = false;  // spring_set_option(SPRING_OPT_GENERIC_V3): use the any-cell V3 kernel
     long long tc_max_spins = -1;    // spring_set_option(SPRING_OPT_WAIT_POLLS); -1: the kernels' default
     bool fp64_prescreen = false;    // spring_set_option(SPRING_OPT_FP64_PRESCREEN)
+    int bte_max_entries = -1;       // spring_set_option(SPRING_OPT_BTE_ENTRIES); -1: what the memory allows
 
     // per-launch CUDA-event records (spring_set_profiling)
     struct ProfRec {
@@ -201,7 +209,14 @@ struct spring_ctx {
     spring::DBuf<int> d_tr_sgn;    // [q] +1 representative, -1 its inverse
     spring::DBuf<int> d_tr_deg;    // [ntr]
     spring::DBuf<int> d_neg;       // [q] grid index of -q
-    spring::DBuf<double> d_wtr;    // cached W grids of the time-reversal set
+    // tetrahedron BTE operator (k_bte.cu run_bte), rows of bt_off; kept until FC3, the phonons or the pairs
+    // change (bt_n < 0: it did not fit)
+    spring::DBuf<int> d_bt_off;
+    spring::DBuf<int2> d_bt_kk;
+    spring::DBuf<double2> d_bt_pq;
+    long long bt_n = 0;
+    int bt_gen = -1, bt_pairs = -1;
+    spring::BteWork bte;
     spring::DBuf<double> d_v4_rec;  // V4 tensor-core mode records (omega, 1/omega, n(T))
     spring::EwaldDev ew;
     spring::PointDefectDev pd;

@@ -1,0 +1,48 @@
+"""The stored tetrahedron operator of the iterative kappa: rows in segments, several batches of q0,
+the form that is not stored, and cells with more than one pass over s0."""
+import numpy as np
+import pytest
+
+from oracle import driver as D
+from spring_b200 import _lib as L
+from spring_b200 import synthetic as S
+from spring_b200.api import from_crystal
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("cell,N,nT", [("rocksalt2", 3, 1), ("rocksalt2", 6, 2), ("rocksalt8", 3, 1)])
+def test_kappa_iter_operator_matches_oracle(cell, N, nT):
+    cr = S.build(cell)
+    temps = [300.0, 700.0][:nT]
+    st = D.Setup(cr, (N, N, N), temps)
+    ctx, _ = from_crystal(cr, (N, N, N), temps, phonons={"grid": st.ph, "irr": st.ph0})
+    out = ctx.kappa_iter(eps_k=1e-6)
+    for it in range(nT):
+        ref = D.bte_iter(st, it=it, eps_k=1e-6)
+        scale = np.abs(ref["kappa_rta"]).max()
+        np.testing.assert_allclose(out["kappa_rta"][it], ref["kappa_rta"], rtol=1e-9, atol=1e-9 * scale)
+        assert abs(int(out["iters"][it]) - ref["iters"]) <= 1
+        np.testing.assert_allclose(out["kappa"][it], ref["kappa"], rtol=1e-6, atol=1e-6 * np.abs(ref["kappa"]).max())
+    ctx.close()
+
+
+@pytest.mark.parametrize("N", [4, 9])
+def test_kappa_iter_same_without_the_stored_operator(N):
+    """9^3: several batches of q0, rows in several segments."""
+    cr = S.build("rocksalt2")
+    ctx, _ = from_crystal(cr, (N, N, N), [300.0, 700.0])
+    a = ctx.kappa_iter(eps_k=1e-6, max_iter=12)
+    again = ctx.kappa_iter(eps_k=1e-6, max_iter=12)          # the kept operator
+    np.testing.assert_array_equal(again["kappa"], a["kappa"])
+    ctx.set_option(L.SPRING_OPT_BTE_ENTRIES, 1000)
+    b = ctx.kappa_iter(eps_k=1e-6, max_iter=12)
+    assert np.array_equal(a["iters"], b["iters"])
+    for key in ("kappa", "kappa_rta"):
+        # the same terms in another order: rows of about 1e4 terms, FP64
+        np.testing.assert_allclose(b[key], a[key], rtol=1e-10, atol=1e-10 * np.abs(a[key]).max())
+    ctx.set_option(L.SPRING_OPT_BTE_ENTRIES, -1)
+    one = ctx.kappa_iter(eps_k=1e-6, max_iter=0)             # a limit inside the first queued block
+    assert np.all(one["iters"] == 1)
+    np.testing.assert_allclose(one["kappa_rta"], a["kappa_rta"], rtol=1e-10, atol=1e-10 * np.abs(a["kappa_rta"]).max())
+    ctx.close()
