@@ -326,7 +326,8 @@ int spring_ctx_destroy(spring_ctx* c) {
         free_pairs(c->ps_irr); free_pairs(c->ps_tr);
         dfree(c->d_tr_int); dfree(c->d_tr_grid); dfree(c->d_tr_pos); dfree(c->d_tr_sgn); dfree(c->d_tr_deg);
         dfree(c->d_neg); dfree(c->d_bt_off); dfree(c->d_bt_kk); dfree(c->d_bt_pq);
-        dfree(c->bte.pq); dfree(c->bte.cf); dfree(c->bte.vec);
+        dfree(c->bte.pq); dfree(c->bte.cf); dfree(c->bte.vec); dfree(c->bte.ent);
+        dfree(c->bte.ctr); dfree(c->bte.cnt); dfree(c->bte.wf); dfree(c->bte.boff);
         dfree(c->d_bteg_row); dfree(c->d_bteg_kk); dfree(c->d_bteg_pq);
         dfree(c->ew.g); dfree(c->ew.r); dfree(c->ew.hz); dfree(c->ew.tau); dfree(c->ew.z); dfree(c->ew.cc);
         dfree(c->ew.dd); dfree(c->d_v4_rec);

@@ -30,7 +30,6 @@
 // Roofline: FP64 ALU for the weights, HBM / L2 (24 bytes and two gathers per entry) for the iterations.
 #include <algorithm>
 #include <cmath>
-#include <cub/cub.cuh>
 
 #include "spring_internal.cuh"
 #include "tetra.cuh"
@@ -466,22 +465,21 @@ int build_tr_set(spring_ctx* c) {
 // and the minus channel at -q1 and -q2 gives (1 + n1 + n2) d(w0 - w1 - w2), each times 4 W3 and -(F1 + F2)
 // because F(-q) = -F(q).  The entries are sorted by row once and kept in HBM (CSR); an iteration is one
 // pass over them.
-__global__ void k_bteg_keys(long long n, const s3::BteEntry* __restrict__ e, int* __restrict__ key,
-                            int* __restrict__ idx, int* __restrict__ rowcnt) {
+// Rank of every entry within its row, in its pad word, and the entries per row.
+__global__ void k_bteg_count(long long n, s3::BteEntry* __restrict__ e, int* __restrict__ rowcnt) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        e[i].pad = atomicAdd(&rowcnt[e[i].r0], 1);
+}
+__global__ void k_bteg_scatter(long long n, const s3::BteEntry* __restrict__ e, const int* __restrict__ rowoff,
+                               int2* __restrict__ kk, double2* __restrict__ pq) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        key[i] = e[i].r0;
-        idx[i] = (int)i;
-        atomicAdd(&rowcnt[e[i].r0], 1);
+        const s3::BteEntry x = e[i];
+        const int o = rowoff[x.r0] + x.pad;
+        kk[o] = make_int2(x.k1, x.k2);
+        pq[o] = make_double2(x.P, x.Q);
     }
 }
-__global__ void k_bteg_gather(long long n, const s3::BteEntry* __restrict__ e, const int* __restrict__ idx,
-                              int2* __restrict__ kk, double2* __restrict__ pq) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const s3::BteEntry x = e[idx[i]];
-        kk[i] = make_int2(x.k1, x.k2);
-        pq[i] = make_double2(x.P, x.Q);
-    }
-}
+
 // Row r holds the entries off[r nseg] .. off[(r + 1) nseg].  One block per row: c = (n1 - n2) P + (1 + n1 + n2) Q of its entries at one temperature, and their sum,
 // 1/tau.
 __global__ void __launch_bounds__(256) k_bteg_coef(int nseg, const int* __restrict__ off, const int2* __restrict__ kk,
@@ -636,67 +634,55 @@ int run_bte_gauss(spring_ctx* c, double sigma, double eps_k, int max_iter, doubl
     if (!(c->bteg_sigma == sigma && c->bteg_gen == c->ph_gen && c->bteg_pairs == c->ps_tr.gen && c->bteg_n > 0 &&
           c->bteg_prec == c->precision)) {
         c->bteg_n = 0;
-        DBuf<s3::BteEntry> ent;
-        DBuf<unsigned long long> ctr;
-        SPRING_CHECK(dalloc(c, ctr, 1, "operator count"));
+        BteWork& w = c->bte;
+        SPRING_CHECK(dalloc(c, w.ctr, 1, "operator count"));
+        SPRING_CHECK(dalloc(c, w.cnt, rows + 1, "operator rows"));
+        SPRING_CHECK(dalloc(c, c->d_bteg_row, rows + 1, "operator rows"));
+        constexpr long long EB = sizeof(s3::BteEntry);
         long long cap = std::max<long long>(1 << 20, npairs * 216 / 40);  // the window passes ~1-2% of the triples
+        cap = std::max<long long>(cap, w.ent.n / EB);
         long long cnt = 0;
-        for (int attempt = 0; attempt < 2; ++attempt) {
-            int rc = dalloc(c, ent, (size_t)cap, "BTE operator entries");
-            if (rc == SPRING_OK) rc = zero(c, ctr.p, sizeof(unsigned long long), "operator count");
+        int rc = SPRING_OK;
+        for (int attempt = 0; rc == SPRING_OK && attempt < 2; ++attempt) {
+            rc = dalloc(c, w.ent, (size_t)(cap * EB), "BTE operator entries");
+            if (rc == SPRING_OK) rc = zero(c, w.ctr.p, sizeof(unsigned long long), "operator count");
             bool handled = false;
             // BF16 / BF16x3 contexts: the tensor-core pass writes the entries; FP64: the FP64 pass
-            if (rc == SPRING_OK) rc = run_v3tc_bte(c, 0, ntr, sigma, ent.p, ctr.p, cap, &handled);
+            if (rc == SPRING_OK) rc = run_v3tc_bte(c, 0, ntr, sigma, w.ent.p, w.ctr.p, cap, &handled);
             if (rc == SPRING_OK && !handled)
-                rc = launch_v3s_bte(c, c->ps_tr, view, 0, ntr, sigma, ent.p, ctr.p, cap, &handled);
+                rc = launch_v3s_bte(c, c->ps_tr, view, 0, ntr, sigma, w.ent.p, w.ctr.p, cap, &handled);
             unsigned long long h = 0;
-            if (rc == SPRING_OK) rc = d2h(c, &h, ctr.p, sizeof h, "operator count");
-            if (rc != SPRING_OK) { dfree(ent); dfree(ctr); return rc; }
+            if (rc == SPRING_OK) rc = d2h(c, &h, w.ctr.p, sizeof h, "operator count");
             cnt = (long long)h;
             if (cnt <= cap) break;
-            dfree(ent);
             cap = cnt + cnt / 16 + 1024;
         }
-        dfree(ctr);
-        if (cnt > cap) { dfree(ent); return fail(c, SPRING_ERR_CUDA, "BTE operator: entry count changed between runs"); }
-        if (cnt > 0x7fffffffLL) { dfree(ent); return fail(c, SPRING_ERR_UNSUPPORTED, "BTE operator above 2^31 entries"); }
-        DBuf<int> key, keys, idx, idxs, cntr;
-        int rc = dalloc(c, key, std::max<long long>(cnt, 1), "operator keys");
-        if (rc == SPRING_OK) rc = dalloc(c, keys, std::max<long long>(cnt, 1), "operator keys");
-        if (rc == SPRING_OK) rc = dalloc(c, idx, std::max<long long>(cnt, 1), "operator keys");
-        if (rc == SPRING_OK) rc = dalloc(c, idxs, std::max<long long>(cnt, 1), "operator keys");
-        if (rc == SPRING_OK) rc = dalloc(c, cntr, rows + 1, "operator rows");
-        if (rc == SPRING_OK) rc = dalloc(c, c->d_bteg_row, rows + 1, "operator rows");
-        if (rc == SPRING_OK) rc = zero(c, cntr.p, sizeof(int) * (rows + 1), "operator rows");
+        if (rc == SPRING_OK && cnt > cap) rc = fail(c, SPRING_ERR_CUDA, "BTE operator: entry count changed between runs");
+        if (rc == SPRING_OK && cnt > 0x7fffffffLL) rc = fail(c, SPRING_ERR_UNSUPPORTED, "BTE operator above 2^31 entries");
+        if (rc == SPRING_OK) rc = dalloc(c, c->d_bteg_kk, cnt, "BTE operator");
+        if (rc == SPRING_OK) rc = dalloc(c, c->d_bteg_pq, cnt, "BTE operator");
+        if (rc == SPRING_OK) rc = zero(c, w.cnt.p, sizeof(int) * (rows + 1), "operator rows");
+        auto* ent = reinterpret_cast<s3::BteEntry*>(w.ent.p);
         if (rc == SPRING_OK && cnt > 0) {
-            k_bteg_keys<<<blocks_for(cnt), threads, 0, c->stream>>>(cnt, ent.p, key.p, idx.p, cntr.p);
-            rc = launch_check(c, "k_bteg_keys");
+            if (launch_injected(c)) rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
+            if (rc == SPRING_OK) {
+                k_bteg_count<<<blocks_for(cnt), threads, 0, c->stream>>>(cnt, ent, w.cnt.p);
+                rc = launch_check(c, "k_bteg_count");
+            }
         }
-        if (rc == SPRING_OK) rc = run_exclusive_scan(c, cntr.p, c->d_bteg_row.p, rows + 1);
+        if (rc == SPRING_OK) rc = run_exclusive_scan(c, w.cnt.p, c->d_bteg_row.p, rows + 1);
         if (rc == SPRING_OK && cnt > 0) {
-            int bits = 1;
-            while ((1 << bits) <= rows) ++bits;
-            size_t tb = 0;
-            cub::DeviceRadixSort::SortPairs(nullptr, tb, key.p, keys.p, idx.p, idxs.p, (int)cnt, 0, bits, c->stream);
-            DBuf<uint8_t> tmp;
-            rc = dalloc(c, tmp, std::max<size_t>(tb, 1), "operator sort");
+            if (launch_injected(c)) rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
             if (rc == SPRING_OK) {
-                const cudaError_t e = cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.p, keys.p, idx.p, idxs.p, (int)cnt,
-                                                                      0, bits, c->stream);
-                c->launches += 1;
-                if (e != cudaSuccess) rc = cuda_fail(c, e, "operator sort");
+                k_bteg_scatter<<<blocks_for(cnt), threads, 0, c->stream>>>(cnt, ent, c->d_bteg_row.p, c->d_bteg_kk.p,
+                                                                          c->d_bteg_pq.p);
+                rc = launch_check(c, "k_bteg_scatter");
             }
-            if (rc == SPRING_OK) rc = dalloc(c, c->d_bteg_kk, cnt, "BTE operator");
-            if (rc == SPRING_OK) rc = dalloc(c, c->d_bteg_pq, cnt, "BTE operator");
-            if (rc == SPRING_OK) {
-                k_bteg_gather<<<blocks_for(cnt), threads, 0, c->stream>>>(cnt, ent.p, idxs.p, c->d_bteg_kk.p, c->d_bteg_pq.p);
-                rc = launch_check(c, "k_bteg_gather");
-            }
+        }
+        if (w.ent.n > ((size_t)256 << 20)) {  // large ones are given back
             cudaStreamSynchronize(c->stream);
-            dfree(tmp);
+            dfree(w.ent);
         }
-        cudaStreamSynchronize(c->stream);
-        dfree(ent); dfree(key); dfree(keys); dfree(idx); dfree(idxs); dfree(cntr);
         if (rc != SPRING_OK) return rc;
         c->bteg_n = cnt;
         c->bteg_sigma = sigma;
@@ -721,8 +707,6 @@ int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* 
     const Q0View view{c->d_tr_int.p, c->d_tr_grid.p, c->ph_grid.evec.p, c->ph_grid.omega.p, c->ph_grid.oneby.p};
     // q0 per batch: their (P, Q) and W grids stay around the L2 size
     const int batch = (int)std::max<size_t>(1, std::min<size_t>(ntr, ((size_t)96 << 20) / (slot * sizeof(double2))));
-    DBuf<float> wf;
-    DBuf<int> cnt, boff;
     BteWork& w = c->bte;
     // W and the tetrahedron weights of q0 b .. b + nb - 1 into d_w and w.pq
     auto build = [&](int b, int nb) -> int {
@@ -736,7 +720,7 @@ int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* 
         a.tr_grid = c->d_tr_grid.p;
         a.neg = c->d_neg.p;
         a.partner = c->ps_tr.partner.p;
-        a.wf = wf.p;
+        a.wf = w.wf.p;
         a.omega = c->ph_grid.omega.p;
         a.pq = w.pq.p;
         const int groups = (a.ntet + 31) / 32, passes = (n + NS0 - 1) / NS0;
@@ -758,15 +742,15 @@ int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* 
     int rc = SPRING_OK;
     if (!stored) {
         c->bt_gen = -1;
-        rc = dalloc(c, wf, (size_t)nq * n, "FP32 frequencies");
+        rc = dalloc(c, w.wf, (size_t)nq * n, "FP32 frequencies");
         if (rc == SPRING_OK) rc = dalloc(c, c->d_w, slot * batch, "W buffer");
         if (rc == SPRING_OK) rc = dalloc(c, w.pq, slot * batch, "tetrahedron weights");
-        if (rc == SPRING_OK) rc = dalloc(c, cnt, (size_t)batch * n * nseg + 1, "operator counts");
-        if (rc == SPRING_OK) rc = dalloc(c, boff, (size_t)batch * n * nseg + 1, "operator counts");
+        if (rc == SPRING_OK) rc = dalloc(c, w.cnt, (size_t)batch * n * nseg + 1, "operator counts");
+        if (rc == SPRING_OK) rc = dalloc(c, w.boff, (size_t)batch * n * nseg + 1, "operator counts");
         if (rc == SPRING_OK) rc = dalloc(c, c->d_bt_off, (size_t)rows * nseg + 1, "operator rows");
         if (rc == SPRING_OK && launch_injected(c)) rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
         if (rc == SPRING_OK) {
-            k_bte_wf<<<std::min((nq * n + 255) / 256, 148 * 8), 256, 0, c->stream>>>(nq, n, c->ph_grid.omega.p, wf.p);
+            k_bte_wf<<<std::min((nq * n + 255) / 256, 148 * 8), 256, 0, c->stream>>>(nq, n, c->ph_grid.omega.p, w.wf.p);
             rc = launch_check(c, "k_bte_wf");
         }
         size_t free_b = 0, total_b = 0;
@@ -780,13 +764,13 @@ int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* 
         for (int b = 0; rc == SPRING_OK && stored && b < ntr; b += batch) {
             const int nb = std::min(batch, ntr - b), segs = nb * n * nseg;
             if ((rc = build(b, nb)) != SPRING_OK) break;
-            if ((rc = zero(c, cnt.p + segs, sizeof(int), "operator counts")) != SPRING_OK) break;
+            if ((rc = zero(c, w.cnt.p + segs, sizeof(int), "operator counts")) != SPRING_OK) break;
             if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure"); break; }
-            k_bte_entries<true><<<segs, 256, 0, c->stream>>>(row_args(b), nseg, cnt.p, nullptr, 0, 0, nullptr, nullptr, nullptr);
+            k_bte_entries<true><<<segs, 256, 0, c->stream>>>(row_args(b), nseg, w.cnt.p, nullptr, 0, 0, nullptr, nullptr, nullptr);
             if ((rc = launch_check(c, "k_bte_entries<count>")) != SPRING_OK) break;
-            if ((rc = run_exclusive_scan(c, cnt.p, boff.p, segs + 1)) != SPRING_OK) break;
+            if ((rc = run_exclusive_scan(c, w.cnt.p, w.boff.p, segs + 1)) != SPRING_OK) break;
             int here = 0;
-            if ((rc = d2h(c, &here, boff.p + segs, sizeof here, "operator count")) != SPRING_OK) break;
+            if ((rc = d2h(c, &here, w.boff.p + segs, sizeof here, "operator count")) != SPRING_OK) break;
             const long long need = total + here;
             if (need > most) { stored = false; break; }
             if (need > (long long)std::min(c->d_bt_kk.n, c->d_bt_pq.n)) {
@@ -817,7 +801,7 @@ int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* 
                 if (rc != SPRING_OK) break;
             }
             if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure"); break; }
-            k_bte_entries<false><<<segs, 256, 0, c->stream>>>(row_args(b), nseg, nullptr, boff.p, total, b + nb == ntr,
+            k_bte_entries<false><<<segs, 256, 0, c->stream>>>(row_args(b), nseg, nullptr, w.boff.p, total, b + nb == ntr,
                                                              c->d_bt_off.p, c->d_bt_kk.p, c->d_bt_pq.p);
             rc = launch_check(c, "k_bte_entries");
             total = need;
@@ -850,10 +834,6 @@ int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* 
         rc = bte_iterate(c, eps_k, max_iter, 1, [&](int T) { return pass(0, T); }, [&](int T) { return pass(1, T); },
                          h_kappa, h_kappa_rta, h_iters);
     }
-    cudaStreamSynchronize(c->stream);
-    dfree(wf);
-    dfree(cnt);
-    dfree(boff);
     return rc;
 }
 

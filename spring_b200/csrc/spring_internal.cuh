@@ -90,6 +90,11 @@ struct EwaldDev {
 struct BteWork {
     DBuf<double2> pq;          // (P, Q) grids of a batch
     DBuf<double> cf, vec;      // operator coefficients of one temperature; the vectors below
+    DBuf<unsigned char> ent;   // unsorted entries of the Gaussian operator
+    DBuf<unsigned long long> ctr;
+    DBuf<int> cnt;
+    DBuf<float> wf;
+    DBuf<int> boff;
     double *Fg = nullptr, *F0 = nullptr, *dF = nullptr, *inv_tau = nullptr;
 };
 
