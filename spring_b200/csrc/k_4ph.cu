@@ -408,116 +408,224 @@ struct T4Args {
     int pol_lo[4], pol_hi[4];
 };
 
-// one thread per (q1, tetrahedron of q2, s1, s2, s3); all s0 and temperatures in the thread
-__global__ void __launch_bounds__(128) k_tetra4(T4Args a, const int4* __restrict__ tet, const int* __restrict__ all,
-                                                const double* __restrict__ Wq, const int* __restrict__ q0int,
-                                                const double* __restrict__ om0, const double* __restrict__ nbe0,
-                                                const double* __restrict__ omg, const double* __restrict__ nbeg,
-                                                double* __restrict__ out) {
-    __shared__ double sacc[N * 10];
-    const int per[5][3] = {{0, 2, 1}, {1, 0, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}};
-    for (int i = threadIdx.x; i < N * 10; i += blockDim.x) sacc[i] = 0.0;
-    __syncthreads();
+// Warps screen 32 tetrahedra over q2 at a time for one q1, queue the hits (tetrahedron, s1, s2, s3, channel,
+// s0) and evaluate 32 of them at a time, as in k_tetra3 (k_tetra.cu has the reasons).  The FP32 ranges of
+// w2 + w3 and w3 - w2 over a tetrahedron serve every s1: the channels shift them by w1.  The legs are not
+// folded: the reference's reading of the stored W is not symmetric in them.
+// One thread per (q1, tetrahedron, s1, s2, s3) ran every weight formula any lane of its warp needed, with 17
+// divisions per evaluation: 116.6 -> 15.3 ms at 5^3 (ten q0, one temperature).
+constexpr int T4W = 4;  // warps per block
+
+template <int NT>
+struct T4Smem {
+    double acc[T4W][N * NT][32];           // per-lane sums [s0][T]
+    unsigned queue[T4W][32 * 18 + 32];
+    float w23[T4W][2][N][4][32];           // w(q2, s2), w(q3, s3) of the lane's tetrahedron
+    int v2[T4W][4][32], v3[T4W][4][32], pos[T4W][4][32], typ[T4W][32];  // its vertices and their quartets
+    float w0m[N][8], w0p[N][8];            // w0 - w1, w0 + w1 by s1 ([..][s0], two values of padding)
+    double w0[N];
+};
+
+template <int NT>
+__global__ void __launch_bounds__(32 * T4W, 3) k_tetra4(T4Args a, int per1, int nb1, const int4* __restrict__ tet,
+                                                        const int* __restrict__ all, const double* __restrict__ Wq,
+                                                        const int* __restrict__ q0int, const double* __restrict__ om0,
+                                                        const double* __restrict__ nbe0, const double* __restrict__ omg,
+                                                        const double* __restrict__ nbeg, double* __restrict__ out) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T4Smem<NT>& S = *reinterpret_cast<T4Smem<NT>*>(smem_raw);
+    constexpr int K = 3 * N;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool gq0 = q0int[0] == 0 && q0int[1] == 0 && q0int[2] == 0;
-    const int s0a = gq0 ? 3 : a.pol_lo[0];
-    const int n1r = a.pol_hi[1] - a.pol_lo[1] + 1, n2r = a.pol_hi[2] - a.pol_lo[2] + 1, n3r = a.pol_hi[3] - a.pol_lo[3] + 1;
-    const long long items = (long long)a.nq * a.ntet * n1r * n2r * n3r;
-    double acc[N][9];
+    const int s0a = gq0 ? 3 : a.pol_lo[0], s0e = a.pol_hi[0];
+    for (int i = lane; i < N * NT * 32; i += 32) (&S.acc[warp][0][0])[i] = 0.0;
+    if (threadIdx.x < N) S.w0[threadIdx.x] = om0[threadIdx.x];
+    unsigned live = 0;
 #pragma unroll
-    for (int s = 0; s < N; ++s)
-#pragma unroll
-        for (int t = 0; t < 9; ++t) acc[s][t] = 0.0;
-    for (long long it = (long long)blockIdx.x * blockDim.x + threadIdx.x; it < items;
-         it += (long long)gridDim.x * blockDim.x) {
-        const int s3 = a.pol_lo[3] + (int)(it % n3r);
-        const int s2 = a.pol_lo[2] + (int)((it / n3r) % n2r);
-        const int s1 = a.pol_lo[1] + (int)((it / ((long long)n3r * n2r)) % n1r);
-        const long long r = it / ((long long)n3r * n2r * n1r);
-        const int t = (int)(r % a.ntet), q1 = (int)(r / a.ntet);
-        const int4 tv = tet[t];
-        const int v2[4] = {tv.x, tv.y, tv.z, tv.w};
-        int v3[4], typ[4], pos[4];
-        double M[3][4];
-        const double w1 = omg[(size_t)q1 * N + s1];
-        bool ok = true;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int* e = all + 3 * ((size_t)q1 * a.nq + v2[v]);
-            typ[v] = e[0];
-            pos[v] = e[1] - 1;
-            v3[v] = e[2] - 1;
-            ok = ok && typ[v] >= 0 && typ[v] <= 5 && pos[v] >= 0 && pos[v] < a.nquart && v3[v] >= 0 && v3[v] < a.nq;
+    for (int k = 0; k < K; ++k)
+        if (k % N >= s0a && k % N <= s0e) live |= 1u << (K - 1 - k);
+    const int groups = (a.ntet + 31) / 32;
+    unsigned* queue = S.queue[warp];
+    double(*acc)[32] = S.acc[warp];
+    // blockIdx.y: q1 (strided); the block's warps share it
+    for (int q1 = blockIdx.y; q1 < a.nq; q1 += gridDim.y) {
+        __syncthreads();
+        if (threadIdx.x < N * N) {
+            const int s1 = threadIdx.x / N, s0 = threadIdx.x % N;
+            const float w0 = (float)S.w0[s0], w1 = (float)omg[(size_t)q1 * N + s1];
+            S.w0m[s1][s0] = w0 - w1;
+            S.w0p[s1][s0] = w0 + w1;
         }
-        if (!ok) continue;  // every cell is written by the enumeration; an unwritten one is skipped, not read
+        __syncthreads();
+        for (int u = blockIdx.x * T4W + warp; u < groups * nb1; u += gridDim.x * T4W) {
+            const int g = u / nb1;
+            const int s1a = a.pol_lo[1] + u % nb1 * per1, s1e = min(s1a + per1 - 1, a.pol_hi[1]);
+            const int t = g * 32 + lane;
+            bool on = t < a.ntet;
+            __syncwarp();
+            if (on) {
+                const int4 tv = tet[t];
+                const int v2[4] = {tv.x, tv.y, tv.z, tv.w};
+                int typ = 0;
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const double w2 = omg[(size_t)v2[v] * N + s2], w3 = omg[(size_t)v3[v] * N + s3];
-            M[0][v] = (w1 + w2 + w3);
-            M[1][v] = (w2 + w3 - w1);
-            M[2][v] = (w3 - w1 - w2);
-        }
-        int pm[3][4];
-        double Sm[3][4];
+                for (int v = 0; v < 4; ++v) {
+                    const int* e = all + 3 * ((size_t)q1 * a.nq + v2[v]);
+                    const int ty = e[0], ps = e[1] - 1, v3 = e[2] - 1;
+                    // every cell is written by the enumeration; an unwritten one is skipped, not read
+                    const bool ok = ty >= 0 && ty <= 5 && ps >= 0 && ps < a.nquart && v3 >= 0 && v3 < a.nq;
+                    on = on && ok;
+                    S.v2[warp][v][lane] = v2[v];
+                    S.v3[warp][v][lane] = ok ? v3 : 0;
+                    S.pos[warp][v][lane] = ps;
+                    typ |= ty << (4 * v);
 #pragma unroll
-        for (int ch = 0; ch < 3; ++ch) {
-            tet::sort4(M[ch], pm[ch]);
+                    for (int s = 0; s < N; ++s) {
+                        S.w23[warp][0][s][v][lane] = (float)omg[(size_t)v2[v] * N + s];
+                        S.w23[warp][1][s][v][lane] = (float)omg[(size_t)(ok ? v3 : 0) * N + s];
+                    }
+                }
+                S.typ[warp][lane] = typ;
+            }
+            __syncwarp();
+            // FP64 evaluation of a hit: lane of the tetrahedron | s1 | s2 | s3 | check
+            auto evaluate = [&](unsigned code) {
+                const int tl = code & 31, s1 = (code >> 5) & 7, s2 = (code >> 8) & 7, s3 = (code >> 11) & 7;
+                const int k = K - 1 - (int)(code >> 14), ch = k / N, s0 = k % N;
+                const double w1 = omg[(size_t)q1 * N + s1];
+                double M[4];
+                int vs[4] = {0, 1, 2, 3}, unused[4] = {0, 0, 0, 0};
 #pragma unroll
-            for (int v = 0; v < 4; ++v) Sm[ch][v] = M[ch][pm[ch][v]];
-        }
-        int wofs[4];  // mode offset of (s1,s2,s3) read through the reference's permutation
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int before[3] = {s1, s2, s3};
-            int af[3];
-            for (int k = 0; k < 3; ++k) af[k] = typ[v] == 0 ? before[k] : before[per[typ[v] - 1][k]];
-            wofs[v] = (af[0] * N + af[1]) * N + af[2];
-        }
-        for (int s0 = s0a; s0 <= a.pol_hi[0]; ++s0) {
-            const double Mqs = om0[s0];
-            double Wv[4];
-#pragma unroll
-            for (int v = 0; v < 4; ++v) Wv[v] = Wq[(size_t)pos[v] * 1296 + s0 * 216 + wofs[v]];
-#pragma unroll
-            for (int ch = 0; ch < 3; ++ch) {
-                double g, I[4];
-                const bool e = tet::g_iver<false>(Mqs, Sm[ch], g, I);
-#pragma unroll
-                for (int v = 0; v < 4; ++v) if (isnan(I[v])) I[v] = 0.0;
-                if (isnan(g)) g = 0.0;
-                if (!e) continue;
+                for (int v = 0; v < 4; ++v) {
+                    const double w2 = omg[(size_t)S.v2[warp][v][tl] * N + s2], w3 = omg[(size_t)S.v3[warp][v][tl] * N + s3];
+                    M[v] = ch == 0 ? w1 + w2 + w3 : (ch == 1 ? w2 + w3 - w1 : w3 - w1 - w2);
+                }
+                tet::sort4_carry(M, vs, unused);
+                double gw, A[4];
+                if (!tet::g_weights<false>(S.w0[s0], M, gw, A)) return;
                 const double wt = ch == 0 ? ONEBYSIX : 0.5;
+                const int typ = S.typ[warp][tl];
+                size_t o2[4], o3[4];
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    const int q = vs[v], ty = (typ >> (4 * q)) & 7;
+                    // modes of the stored quartet read through the reference's permutation
+                    // 0: 123, 1: 132, 2: 213, 3: 231, 4: 312, 5: 321
+                    const int m1 = ty < 2 ? s1 : (ty < 4 ? s2 : s3);
+                    const int m2 = ty == 0 || ty == 5 ? s2 : (ty == 1 || ty == 3 ? s3 : s1);
+                    const int m3 = s1 + s2 + s3 - m1 - m2;
+                    const double W = Wq[(size_t)S.pos[warp][q][tl] * 1296 + s0 * 216 + (m1 * N + m2) * N + m3];
+                    A[v] = isnan(A[v]) ? 0.0 : wt * A[v] * W;
+                    o2[v] = (size_t)S.v2[warp][q][tl] * N + s2;
+                    o3[v] = (size_t)S.v3[warp][q][tl] * N + s3;
+                }
                 for (int T = 0; T < a.nT; ++T) {
                     const double* nb = nbeg + (size_t)T * a.nq * N;
-                    const double n0 = nbe0[(size_t)T * a.nq0 * N + s0];
-                    const double n1 = nb[(size_t)q1 * N + s1];
+                    const double n1 = nb[(size_t)q1 * N + s1], n0 = nbe0[(size_t)T * a.nq0 * N + s0];
+                    const double f1 = ch == 0 ? n1 : 1.0 + n1, one = ch == 2 ? 1.0 : 0.0;
                     double sum = 0.0;
 #pragma unroll
+                    for (int v = 0; v < 4; ++v) sum = fma(A[v], f1 * (one + nb[o2[v]]) * nb[o3[v]], sum);
+                    acc[s0 * NT + T][lane] += sum / n0;
+                }
+            };
+            int qn = 0;
+            for (int s2 = a.pol_lo[2]; s2 <= a.pol_hi[2]; ++s2) {
+                float b2[4], e2 = 0.0f;
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    b2[v] = S.w23[warp][0][s2][v][lane];
+                    e2 += fabsf(b2[v]);
+                }
+                for (int s3 = a.pol_lo[3]; s3 <= a.pol_hi[3]; ++s3) {
+                    float pl = 0.0f, ph = 0.0f, ml = 0.0f, mh = 0.0f, e3 = e2;
+#pragma unroll
                     for (int v = 0; v < 4; ++v) {
-                        const int q = pm[ch][v];
-                        const double n2 = nb[(size_t)v2[q] * N + s2], n3 = nb[(size_t)v3[q] * N + s3];
-                        const double f = ch == 0 ? (n1 * n2 * n3 / n0)
-                                                 : (ch == 1 ? ((1.0 + n1) * n2 * n3 / n0)
-                                                            : ((1.0 + n1) * (1.0 + n2) * n3 / n0));
-                        sum += I[v] * (Wv[q] * f);
+                        const float c = S.w23[warp][1][s3][v][lane], p = b2[v] + c, m = c - b2[v];
+                        e3 += fabsf(c);
+                        pl = v ? fminf(pl, p) : p;
+                        ph = v ? fmaxf(ph, p) : p;
+                        ml = v ? fminf(ml, m) : m;
+                        mh = v ? fmaxf(mh, m) : m;
                     }
-                    acc[s0][T] += wt * g * (ONEBYSIX * sum);
+                    const float pm = 0.5f * (pl + ph), mm = 0.5f * (ml + mh);
+                    const float pr = 0.5f * (ph - pl), mr = 0.5f * (mh - ml);
+#pragma unroll 1
+                    for (int s1 = s1a; s1 <= s1e; ++s1) {
+                        unsigned o = 0;  // one bit per check, set outside
+                        // FP32 rounding of the energies is below 4e-7 of the sum of magnitudes
+                        // (|w1| and |w0| are at most |w0 - w1| + |w0 + w1|)
+                        const float marg = 1e-6f * (e3 + fabsf(S.w0m[s1][0]) + fabsf(S.w0p[s1][0]));
+                        const float hp = pr + marg, hm = mr + marg;
+                        float wm[N], wp[N];
+#pragma unroll
+                        for (int i = 0; i < N; ++i) {
+                            wm[i] = S.w0m[s1][i];
+                            wp[i] = S.w0p[s1][i];
+                        }
+#pragma unroll
+                        for (int i = 0; i < N; ++i) o = __funnelshift_l(__float_as_uint(hp - fabsf(wm[i] - pm)), o, 1);
+#pragma unroll
+                        for (int i = 0; i < N; ++i) o = __funnelshift_l(__float_as_uint(hp - fabsf(wp[i] - pm)), o, 1);
+#pragma unroll
+                        for (int i = 0; i < N; ++i) o = __funnelshift_l(__float_as_uint(hm - fabsf(wp[i] - mm)), o, 1);
+                        unsigned in = on ? ~o & live : 0u;
+                        const unsigned c = __popc(in);
+                        unsigned pre = 0, tot = 0;
+                        const unsigned lt = (1u << lane) - 1;
+#pragma unroll
+                        for (int b = 0; b < 5; ++b) {
+                            const unsigned m = __ballot_sync(0xffffffffu, (c >> b) & 1);
+                            pre += __popc(m & lt) << b;
+                            tot += __popc(m) << b;
+                        }
+                        if (tot == 0) continue;
+                        const unsigned base = lane | s1 << 5 | s2 << 8 | s3 << 11;
+                        unsigned pos = qn + pre;
+                        while (in) {
+                            const int b = __ffs(in) - 1;
+                            in &= in - 1;
+                            queue[pos++] = base | b << 14;
+                        }
+                        qn += tot;
+                        __syncwarp();
+                        while (qn >= 32) {
+                            qn -= 32;
+                            evaluate(queue[qn + lane]);
+                        }
+                        __syncwarp();
+                    }
                 }
             }
+            if (lane < qn) evaluate(queue[lane]);
+            __syncwarp();
         }
     }
-#pragma unroll
-    for (int s = 0; s < N; ++s)
-#pragma unroll
-        for (int T = 0; T < 9; ++T) {
-            double v = acc[s][T];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(&sacc[s * 10 + T], v);
-        }
     __syncthreads();
-    for (int i = threadIdx.x; i < N * a.nT; i += blockDim.x) {
-        const int s = i / a.nT, T = i % a.nT;
-        if (sacc[s * 10 + T] != 0.0) atomicAdd(&out[((size_t)T * a.nq0 + a.q0) * N + s], sacc[s * 10 + T]);
+    for (int i = warp; i < N * NT; i += T4W) {
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < T4W; ++w) v += S.acc[w][i][lane];
+        v = tet::warp_sum(v);
+        const int s0 = i / NT, T = i % NT;
+        if (lane == 0 && T < a.nT && v != 0.0) atomicAdd(&out[((size_t)T * a.nq0 + a.q0) * N + s0], v);
     }
+}
+
+template <int NT>
+int launch_tetra4(spring_ctx* c, const T4Args& t, const int* all, const double* wq, const int* q0i, const double* om0,
+                  const double* nbe0, double* d_rate) {
+    const int n1 = t.pol_hi[1] - t.pol_lo[1] + 1, groups = (t.ntet + 31) / 32;
+    int per1 = 6;  // as in k_tetra3: shorter units while the chip is not full
+    while (per1 > 1 && (long long)t.nq * groups * ((n1 + per1 - 1) / per1) < 148LL * 24) --per1;
+    const int nb1 = (n1 + per1 - 1) / per1;
+    const int gy = std::min(t.nq, 148 * 3), gx = std::max(1, std::min((groups * nb1 + T4W - 1) / T4W, (148 * 6 + gy - 1) / gy));
+    const size_t smem = sizeof(T4Smem<NT>);
+    cudaFuncSetAttribute(k_tetra4<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "tetra4: injected launch failure");
+    k_tetra4<NT><<<dim3(gx, gy), 32 * T4W, smem, c->stream>>>(t, per1, nb1, reinterpret_cast<const int4*>(c->d_tetra.p), all,
+                                                              wq, q0i, om0, nbe0, c->ph_grid.omega.p, c->ph_grid.nbe.p,
+                                                              d_rate);
+    return launch_check(c, "k_tetra4");
 }
 
 // Enumerate the quartets of q0 into device buffers (grid-pair scratch owned by the caller).
@@ -665,13 +773,9 @@ int run_lw4(spring_ctx* c, int q0_first, int n_q0, int delta_mode, double sigma,
                 t.pol_lo[k] = a.pol_lo[k];
                 t.pol_hi[k] = a.pol_hi[k];
             }
-            const long long items = (long long)c->nq * t.ntet * (t.pol_hi[1] - t.pol_lo[1] + 1) *
-                                    (t.pol_hi[2] - t.pol_lo[2] + 1) * (t.pol_hi[3] - t.pol_lo[3] + 1);
-            const int tb = (int)std::max<long long>(1, std::min<long long>((items + 511) / 512, 148LL * 16));
-            if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "tetra4: injected launch failure"); break; }
-            k_tetra4<<<tb, 128, 0, c->stream>>>(t, reinterpret_cast<const int4*>(c->d_tetra.p), b.all.p, wq.p, q0i, om0,
-                                                nbe0, c->ph_grid.omega.p, c->ph_grid.nbe.p, d_rate);
-            rc = launch_check(c, "k_tetra4");
+            rc = c->nT == 1 ? launch_tetra4<1>(c, t, b.all.p, wq.p, q0i, om0, nbe0, d_rate)
+                 : c->nT <= 3 ? launch_tetra4<3>(c, t, b.all.p, wq.p, q0i, om0, nbe0, d_rate)
+                              : launch_tetra4<9>(c, t, b.all.p, wq.p, q0i, om0, nbe0, d_rate);
         }
     }
     cudaStreamSynchronize(c->stream);

@@ -49,3 +49,27 @@ def test_screened_tetrahedron_sums_match_oracle(cell, N, nT, pol):
             np.testing.assert_allclose(lw[it, i0], r["lw"], rtol=1e-9, atol=1e-14 * np.abs(lw).max())
         np.testing.assert_allclose(p3[i0], r["p3_q0"], rtol=1e-9, atol=1e-14 * np.abs(p3).max())
     ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mesh,nT,pol", [
+    ((3, 3, 3), 1, None),                                    # a last group of two lanes
+    ((2, 5, 3), 9, None),
+    ((3, 4, 2), 2, [[3, 5], [2, 4], [1, 6], [5, 6]]),
+    ((4, 4, 4), 4, [[1, 6], [6, 6], [2, 2], [1, 6]]),
+])
+def test_screened_four_phonon_sums_match_oracle(mesh, nT, pol):
+    cr = S.build("rocksalt2", fc4=True)
+    temps = list(np.linspace(100.0, 900.0, nT))
+    W = np.eye(3, dtype=np.int32)[None]
+    st = D.Setup(cr, mesh, temps, W=W, Rxyz=np.eye(3)[None])
+    ctx, _ = from_crystal(cr, mesh, temps, phonons={"grid": st.ph, "irr": st.ph0}, W=W, Rxyz=np.eye(3)[None],
+                          with_fc4=True)
+    p = None if pol is None else np.array(pol, np.int32)
+    first = st.nq0 // 2
+    rate = ctx.linewidth4(first, 3, delta="tetra", pol4=p)
+    for k in range(3):
+        for it in range(nT):
+            ro, _ = D.lw4_tetra(st, first - 1 + k, it, pol=p)
+            np.testing.assert_allclose(rate[it, k], ro, rtol=1e-9, atol=1e-12 * max(np.abs(ro).max(), 1e-30))
+    ctx.close()
