@@ -256,100 +256,194 @@ __global__ void __launch_bounds__(32 * TW, 3) k_tetra3(TetArgs a, const int4* __
 }
 
 // ---- isotope ------------------------------------------------------------
-// W_iso(s1,s0,q1) = pi w0(s0)^2 / 2 / Nq * sum_b g2(b) |e1(b,s1)^H e0(b,s0)|^2  -> [slot][q1][s0][s1]
-__global__ void k_iso_w(int n, int nb, int nq, int q0_first, int nslot, double scale, const double* __restrict__ g2,
-                        const double2* __restrict__ ev0, const double* __restrict__ om0, const double2* __restrict__ evg,
-                        double* __restrict__ wiso) {
-    const long long total = (long long)nslot * nq * n * n;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int s1 = (int)(i % n), s0 = (int)((i / n) % n);
-        const int q1 = (int)((i / ((long long)n * n)) % nq);
-        const int slot = (int)(i / ((long long)n * n * nq));
-        const int q0 = q0_first + slot;
-        const double2* a0 = ev0 + ((size_t)q0 * n + s0) * n;
-        const double2* a1 = evg + ((size_t)q1 * n + s1) * n;
-        double acc = 0.0;
-        for (int b = 0; b < nb; ++b) {
-            double dr = 0.0, di = 0.0;
-            for (int c = 0; c < 3; ++c) {  // conj(e1) * e0
-                const double2 x = a1[3 * b + c], y = a0[3 * b + c];
-                dr += x.x * y.x + x.y * y.y;
-                di += x.x * y.y - x.y * y.x;
+// W_iso(s1,s0,q1) = pi w0(s0)^2 / 2 / Nq * sum_b g2(b) |e1(b,s1)^H e0(b,s0)|^2.  One thread per (s1, q1) with
+// q1 along the warp forms it for NS0 values of s0, e0 in shared memory.  The Gaussian form weights it with
+// the delta at once; most (s0, s1) bands are further apart than the delta reaches for all 32 points, and the
+// warp skips them.  The tetrahedron form stores it as [slot][s0][s1][q1], where the vertices of neighbouring
+// tetrahedra share cache lines (forming it per vertex in the evaluation gathered 96 bytes a vertex: 5.7 ms).
+// Sums stay in registers or per-lane words until the block's end; one shared atomic per term had made the
+// kernels 26 ms (tetrahedron) and 4.2 ms (Gaussian) per call at 24^3, two-atom cell.  Now 4.3 ms and
+// 1.0 ms; 16^3: 3.4 -> 0.53 ms and 0.47 -> 0.12 ms.
+struct IsoArgs {
+    int n, nb, nq, nq0, nT, ntet;
+    int q0_first, per;  // per: 32-tetrahedron groups of a unit (at most 8)
+    double scale, os, os2;
+    double g2[MAX_NB];
+};
+constexpr int ISW = 4;  // warps per block
+
+__device__ __forceinline__ double iso_pref(const IsoArgs& a, double acc, double w0) {
+    return acc * a.scale * (w0 * w0) * 0.5 / double(a.nq);
+}
+
+// GAUSS: out is the rate; else the W grid of the slots.
+template <bool GAUSS>
+__global__ void __launch_bounds__(32 * ISW) k_iso_w(IsoArgs a, const double2* __restrict__ ev0,
+                                                    const double* __restrict__ om0, const double2* __restrict__ evg,
+                                                    const double* __restrict__ omg, double* __restrict__ out) {
+    __shared__ double2 e0[NS0 * MAX_NDOF];
+    __shared__ double red[ISW][NS0], w0s[NS0];
+    const int n = a.n, q0 = a.q0_first + blockIdx.y, s0a = blockIdx.z * NS0, s0n = min(NS0, n - s0a);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < NS0 * n; i += blockDim.x)
+        e0[i] = i < s0n * n ? ev0[((size_t)q0 * n + s0a) * n + i] : make_double2(0.0, 0.0);
+    if (threadIdx.x < NS0) w0s[threadIdx.x] = threadIdx.x < s0n ? om0[(size_t)q0 * n + s0a + threadIdx.x] : 0.0;
+    __syncthreads();
+    double sum[NS0];
+#pragma unroll
+    for (int i = 0; i < NS0; ++i) sum[i] = 0.0;
+    const int chunks = (a.nq + 31) / 32;
+    for (int u = blockIdx.x * ISW + warp; u < chunks * n; u += gridDim.x * ISW) {
+        const int s1 = u / chunks, q1 = u % chunks * 32 + lane;
+        const bool on = q1 < a.nq;
+        const size_t it = (size_t)(on ? q1 : 0) * n + s1;
+        const double w1 = omg[it];
+        const double2* e1 = evg + it * n;
+        double W[NS0], x[NS0];
+        unsigned near = 0;  // s0 with a lane whose exp does not underflow to 0 (a NaN counts)
+#pragma unroll
+        for (int i = 0; i < NS0; ++i) {
+            W[i] = 0.0;
+            const double d = w0s[i] - w1;
+            x[i] = -0.5 * a.os2 * d * d;
+            if (!GAUSS || __any_sync(0xffffffffu, on && !(x[i] <= -745.2))) near |= 1u << i;
+        }
+        if (near == 0) continue;
+        for (int b = 0; b < a.nb; ++b) {
+            const double2 p0 = e1[3 * b], p1 = e1[3 * b + 1], p2 = e1[3 * b + 2];
+            const double g = a.g2[b];
+#pragma unroll
+            for (int i = 0; i < NS0; ++i) {
+                if (!(near >> i & 1)) continue;
+                const double2* y = e0 + i * n + 3 * b;
+                double dr = 0.0, di = 0.0;  // conj(e1) * e0
+                dr += p0.x * y[0].x + p0.y * y[0].y;
+                di += p0.x * y[0].y - p0.y * y[0].x;
+                dr += p1.x * y[1].x + p1.y * y[1].y;
+                di += p1.x * y[1].y - p1.y * y[1].x;
+                dr += p2.x * y[2].x + p2.y * y[2].y;
+                di += p2.x * y[2].y - p2.y * y[2].x;
+                W[i] += g * (dr * dr + di * di);
             }
-            acc += g2[b] * (dr * dr + di * di);
         }
-        const double M = om0[(size_t)q0 * n + s0];
-        wiso[i] = acc * scale * (M * M) * 0.5 / double(nq);
+#pragma unroll
+        for (int i = 0; i < NS0; ++i)
+            if (GAUSS) {
+                if ((near >> i & 1) && on) sum[i] += iso_pref(a, W[i], w0s[i]) * a.os * ONEBYSQRT2PI * exp(x[i]);
+            } else if (on && i < s0n) {
+                out[(((size_t)blockIdx.y * n + s0a + i) * n + s1) * a.nq + q1] = iso_pref(a, W[i], w0s[i]);
+            }
+    }
+    if (!GAUSS) return;
+#pragma unroll
+    for (int i = 0; i < NS0; ++i) {
+        const double v = tet::warp_sum(sum[i]);
+        if (lane == 0) red[warp][i] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < s0n) {
+        double v = 0.0;
+        for (int w = 0; w < ISW; ++w) v += red[w][threadIdx.x];
+        if (v != 0.0)
+            for (int T = 0; T < a.nT; ++T) atomicAdd(&out[((size_t)T * a.nq0 + q0) * n + s0a + threadIdx.x], v);
     }
 }
 
-__global__ void __launch_bounds__(128) k_iso_tetra(int n, int nq, int nq0, int ntet, int q0_first, int nT,
-                                                   const int4* __restrict__ tet, const double* __restrict__ wiso,
-                                                   const double* __restrict__ om0, const double* __restrict__ omg,
-                                                   double* __restrict__ out) {
-    __shared__ double sacc[MAX_NDOF];
-    const int slot = blockIdx.y, q0 = q0_first + slot;
-    for (int i = threadIdx.x; i < MAX_NDOF; i += blockDim.x) sacc[i] = 0.0;
+// Tetrahedron: warps screen 32 tetrahedra for four s1 at a time and evaluate the queued hits, as k_tetra3.
+__global__ void __launch_bounds__(32 * ISW, 4) k_iso_tetra(IsoArgs a, const int4* __restrict__ tet,
+                                                           const double* __restrict__ wiso,
+                                                           const double* __restrict__ om0,
+                                                           const double* __restrict__ omg, double* __restrict__ out) {
+    constexpr int S1B = 4, K = S1B * NS0;
+    __shared__ double acc_[ISW][NS0][32], w0s[NS0];
+    __shared__ unsigned queue_[ISW][32 * K + 32];
+    const int n = a.n, q0 = a.q0_first + blockIdx.y, s0a = blockIdx.z * NS0, s0n = min(NS0, n - s0a);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double(*acc)[32] = acc_[warp];
+    unsigned* queue = queue_[warp];
+    const double* __restrict__ Wi = wiso + ((size_t)blockIdx.y * n + s0a) * n * a.nq;
+    if (threadIdx.x < NS0) w0s[threadIdx.x] = threadIdx.x < s0n ? om0[(size_t)q0 * n + s0a + threadIdx.x] : 0.0;
+#pragma unroll
+    for (int i = 0; i < NS0; ++i) acc[i][lane] = 0.0;
     __syncthreads();
-    const double* Wi = wiso + (size_t)slot * nq * n * n;
-    const long long items = (long long)ntet * n;
-    for (long long it = (long long)blockIdx.x * blockDim.x + threadIdx.x; it < items;
-         it += (long long)gridDim.x * blockDim.x) {
-        const int s1 = (int)(it % n), t = (int)(it / n);
-        const int4 tv = tet[t];
-        const int v1[4] = {tv.x, tv.y, tv.z, tv.w};
-        double M[4];
-        for (int v = 0; v < 4; ++v) M[v] = omg[(size_t)v1[v] * n + s1];
-        int p[4];
-        tet::sort4(M, p);
-        double S[4];
-        for (int v = 0; v < 4; ++v) S[v] = M[p[v]];
-        for (int s0 = 0; s0 < n; ++s0) {
-            double g, I[4];
-            const bool e = tet::g_iver<false>(om0[(size_t)q0 * n + s0], S, g, I);
-            for (int v = 0; v < 4; ++v) if (isnan(I[v])) I[v] = 0.0;
-            if (isnan(g)) g = 0.0;
-            double s = 0.0;
-            if (e)
-                for (int v = 0; v < 4; ++v) s += I[v] * Wi[((size_t)v1[p[v]] * n + s0) * n + s1];
-            const double c = g * (ONEBYSIX * s);
-            if (c != 0.0) atomicAdd(&sacc[s0], c);
+    float w0[NS0];
+#pragma unroll
+    for (int i = 0; i < NS0; ++i) w0[i] = (float)w0s[i];
+    const int groups = (a.ntet + 31) / 32, nb1 = (n + S1B - 1) / S1B, blocks = (groups + a.per - 1) / a.per;
+    const long long units = (long long)blocks * nb1;
+    for (long long u = (long long)blockIdx.x * ISW + warp; u < units; u += (long long)gridDim.x * ISW) {
+        const int t0 = (int)(u / nb1) * a.per * 32, s1a = (int)(u % nb1) * S1B;
+        auto evaluate = [&](unsigned code) {
+            const int k = K - 1 - (int)(code >> 8), s1 = s1a + k / NS0, si = k % NS0;
+            const int4 t = tet[t0 + (code & 255)];
+            int x[4] = {t.x, t.y, t.z, t.w}, unused[4] = {0, 0, 0, 0};
+            double M[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) M[v] = omg[(size_t)x[v] * n + s1];
+            tet::sort4_carry(M, x, unused);
+            double gw, A[4], s = 0.0;
+            if (!tet::g_weights<false>(w0s[si], M, gw, A)) return;
+            const double* w = Wi + ((size_t)si * n + s1) * a.nq;
+#pragma unroll
+            for (int v = 0; v < 4; ++v)
+                if (!isnan(A[v])) s += A[v] * w[x[v]];  // undefined weights count as zero
+            acc[si][lane] += s;
+        };
+        unsigned qn = 0;
+        for (int gi = 0; gi < a.per && t0 + gi * 32 < a.ntet; ++gi) {
+            const bool on = t0 + gi * 32 + lane < a.ntet;
+            const int4 tv = on ? tet[t0 + gi * 32 + lane] : make_int4(0, 0, 0, 0);
+            unsigned out_bits = 0;  // one bit per check, set outside
+#pragma unroll
+            for (int k = 0; k < S1B; ++k) {
+                const bool have = on && s1a + k < n;
+                const int s1 = have ? s1a + k : 0;
+                const float m0 = (float)omg[(size_t)tv.x * n + s1], m1 = (float)omg[(size_t)tv.y * n + s1],
+                            m2 = (float)omg[(size_t)tv.z * n + s1], m3 = (float)omg[(size_t)tv.w * n + s1];
+                const float lo = fminf(fminf(m0, m1), fminf(m2, m3)), hi = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+                const float mid = 0.5f * (lo + hi);
+                const float half = fmaf(0.5f, hi - lo, 1e-6f * (fabsf(m0) + fabsf(m1) + fabsf(m2) + fabsf(m3)));
+#pragma unroll
+                for (int i = 0; i < NS0; ++i)
+                    out_bits = __funnelshift_l(have && i < s0n ? __float_as_uint(half - fabsf(w0[i] - mid)) : 0x80000000u,
+                                               out_bits, 1);
+            }
+            unsigned in = ~out_bits & ((1u << K) - 1);
+            const unsigned c = __popc(in);
+            unsigned pos = 0, tot = 0;
+            const unsigned lt = (1u << lane) - 1;
+#pragma unroll
+            for (int b = 0; b < 5; ++b) {
+                const unsigned m = __ballot_sync(0xffffffffu, (c >> b) & 1);
+                pos += __popc(m & lt) << b;
+                tot += __popc(m) << b;
+            }
+            pos += qn;
+            while (in) {
+                const int b = __ffs(in) - 1;
+                in &= in - 1;
+                queue[pos++] = lane | gi << 5 | b << 8;
+            }
+            qn += tot;
+            __syncwarp();
+            while (qn >= 32) {
+                qn -= 32;
+                evaluate(queue[qn + lane]);
+            }
+            __syncwarp();
         }
+        if (lane < qn) evaluate(queue[lane]);
+        __syncwarp();
     }
     __syncthreads();
-    for (int s0 = threadIdx.x; s0 < n; s0 += blockDim.x)
-        for (int T = 0; T < nT; ++T) atomicAdd(&out[((size_t)T * nq0 + q0) * n + s0], sacc[s0]);
-}
-
-__global__ void __launch_bounds__(128) k_iso_gauss(int n, int nq, int nq0, int q0_first, int nT, double os, double os2,
-                                                   const double* __restrict__ wiso, const double* __restrict__ om0,
-                                                   const double* __restrict__ omg, double* __restrict__ out) {
-    __shared__ double sacc[MAX_NDOF];
-    const int slot = blockIdx.y, q0 = q0_first + slot;
-    for (int i = threadIdx.x; i < MAX_NDOF; i += blockDim.x) sacc[i] = 0.0;
-    __syncthreads();
-    const double* Wi = wiso + (size_t)slot * nq * n * n;
-    const long long items = (long long)nq * n;
-    for (long long it = (long long)blockIdx.x * blockDim.x + threadIdx.x; it < items;
-         it += (long long)gridDim.x * blockDim.x) {
-        const int s1 = (int)(it % n), q1 = (int)(it / n);
-        const double w1 = omg[(size_t)q1 * n + s1];
-        for (int s0 = 0; s0 < n; ++s0) {
-            const double d = om0[(size_t)q0 * n + s0] - w1;
-            const double c = Wi[((size_t)q1 * n + s0) * n + s1] * os * ONEBYSQRT2PI * exp(-0.5 * os2 * d * d);
-            if (c != 0.0) atomicAdd(&sacc[s0], c);
-        }
+    for (int i = warp; i < s0n; i += ISW) {
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < ISW; ++w) v += acc_[w][i][lane];
+        v = tet::warp_sum(v);
+        if (lane == 0 && v != 0.0)
+            for (int T = 0; T < a.nT; ++T) atomicAdd(&out[((size_t)T * a.nq0 + q0) * n + s0a + i], v);
     }
-    __syncthreads();
-    for (int s0 = threadIdx.x; s0 < n; s0 += blockDim.x)
-        for (int T = 0; T < nT; ++T) atomicAdd(&out[((size_t)T * nq0 + q0) * n + s0], sacc[s0]);
-}
-
-int grid_x(long long items, int threads, int slots) {
-    long long want = (items + (long long)threads * 4 - 1) / ((long long)threads * 4);
-    long long cap = (148LL * 16 + slots - 1) / slots;
-    if (want > cap) want = cap;
-    return (int)(want < 1 ? 1 : want);
 }
 
 template <int NT, bool STRICT, bool Q2TAB, bool SYM>
@@ -455,44 +549,56 @@ int run_tetra3_path(spring_ctx* c, int p_first, int n_slots, int n_path, const d
 }
 
 int run_iso(spring_ctx* c, int q0_first, int n_q0, int delta_mode, double sigma, const double* g2, double* d_rate) {
-    const size_t per = (size_t)c->nq * c->ndof * c->ndof;
-    size_t budget = (size_t)64 << 20;
-    int slots = (int)std::max<size_t>(1, budget / (per * sizeof(double)));
-    slots = std::min(slots, n_q0);
-    SPRING_CHECK(dalloc(c, c->d_wiso, per * slots, "isotope W"));
-    DBuf<double> dg2;
-    SPRING_CHECK(dalloc(c, dg2, c->nb, "g2"));
-    int rc = h2d(c, dg2.p, g2, sizeof(double) * c->nb, "g2");
-    const int threads = 128;
-    for (int b = 0; rc == SPRING_OK && b < n_q0; b += slots) {
-        const int ns = std::min(slots, n_q0 - b);
-        const long long tot = (long long)ns * per;
-        const int blocks = (int)std::min<long long>((tot + threads - 1) / threads, 148LL * 64);
-        if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "iso: injected launch failure"); break; }
-        k_iso_w<<<blocks, threads, 0, c->stream>>>(c->ndof, c->nb, c->nq, q0_first + b, ns, PI, dg2.p,
-                                                   c->ph_irr.evec.p, c->ph_irr.omega.p, c->ph_grid.evec.p, c->d_wiso.p);
-        rc = launch_check(c, "k_iso_w");
-        if (rc != SPRING_OK) break;
-        if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "iso: injected launch failure"); break; }
-        if (delta_mode == SPRING_DELTA_TETRA) {
-            const long long items = 6LL * c->nq * c->ndof;
-            dim3 grid(grid_x(items, threads, ns), ns);
-            k_iso_tetra<<<grid, threads, 0, c->stream>>>(c->ndof, c->nq, c->nq0, 6 * c->nq, q0_first + b, c->nT,
-                                                         reinterpret_cast<const int4*>(c->d_tetra.p), c->d_wiso.p,
-                                                         c->ph_irr.omega.p, c->ph_grid.omega.p, d_rate);
-            rc = launch_check(c, "k_iso_tetra");
-        } else {
-            const long long items = (long long)c->nq * c->ndof;
-            dim3 grid(grid_x(items, threads, ns), ns);
-            k_iso_gauss<<<grid, threads, 0, c->stream>>>(c->ndof, c->nq, c->nq0, q0_first + b, c->nT, 1.0 / sigma,
-                                                         1.0 / (sigma * sigma), c->d_wiso.p, c->ph_irr.omega.p,
-                                                         c->ph_grid.omega.p, d_rate);
-            rc = launch_check(c, "k_iso_gauss");
-        }
+    IsoArgs a{};
+    a.n = c->ndof;
+    a.nb = c->nb;
+    a.nq = c->nq;
+    a.nq0 = c->nq0;
+    a.nT = c->nT;
+    a.ntet = 6 * c->nq;
+    a.scale = PI;
+    for (int b = 0; b < c->nb; ++b) a.g2[b] = g2[b];
+    const bool tetra = delta_mode == SPRING_DELTA_TETRA;
+    if (!tetra) {
+        a.os = 1.0 / sigma;
+        a.os2 = 1.0 / (sigma * sigma);
     }
-    cudaStreamSynchronize(c->stream);
-    dfree(dg2);
-    return rc;
+    const int passes = (c->ndof + NS0 - 1) / NS0;
+    const int groups = (a.ntet + 31) / 32, nb1 = (c->ndof + 3) / 4;
+    const long long wunits = (long long)((c->nq + 31) / 32) * c->ndof;
+    const size_t per = (size_t)c->nq * c->ndof * c->ndof;
+    // q0 per launch: the grid's y extent; tetrahedron: a W grid around the L2 size
+    int slots = 32768;
+    if (tetra) {
+        slots = (int)std::max<size_t>(1, std::min<size_t>(slots, ((size_t)64 << 20) / (per * sizeof(double))));
+        slots = std::min(slots, n_q0);
+        SPRING_CHECK(dalloc(c, c->d_wiso, per * slots, "isotope W"));
+    }
+    for (int b = 0; b < n_q0; b += slots) {
+        const int ns = std::min(slots, n_q0 - b);
+        a.q0_first = q0_first + b;
+        // one unit a warp until the chip is full, then as few blocks as fill it
+        const long long cap = std::max<long long>(1, 148LL * 16 / ((long long)ns * passes));
+        const dim3 wgrid((unsigned)std::min((wunits + ISW - 1) / ISW, cap), ns, passes);
+        if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "iso: injected launch failure");
+        if (!tetra) {
+            k_iso_w<true><<<wgrid, 32 * ISW, 0, c->stream>>>(a, c->ph_irr.evec.p, c->ph_irr.omega.p, c->ph_grid.evec.p,
+                                                             c->ph_grid.omega.p, d_rate);
+            SPRING_CHECK(launch_check(c, "k_iso_gauss"));
+            continue;
+        }
+        k_iso_w<false><<<wgrid, 32 * ISW, 0, c->stream>>>(a, c->ph_irr.evec.p, c->ph_irr.omega.p, c->ph_grid.evec.p,
+                                                          c->ph_grid.omega.p, c->d_wiso.p);
+        SPRING_CHECK(launch_check(c, "k_iso_w"));
+        a.per = 8;  // long units keep the evaluations full; shorter while the chip is not
+        while (a.per > 1 && (long long)(groups + a.per - 1) / a.per * nb1 * ns * passes < 148LL * 32) --a.per;
+        const long long units = (long long)((groups + a.per - 1) / a.per) * nb1;
+        if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "iso: injected launch failure");
+        k_iso_tetra<<<dim3((unsigned)std::min((units + ISW - 1) / ISW, cap), ns, passes), 32 * ISW, 0, c->stream>>>(
+            a, reinterpret_cast<const int4*>(c->d_tetra.p), c->d_wiso.p, c->ph_irr.omega.p, c->ph_grid.omega.p, d_rate);
+        SPRING_CHECK(launch_check(c, "k_iso_tetra"));
+    }
+    return SPRING_OK;
 }
 
 }  // namespace spring

@@ -256,7 +256,7 @@ struct spring_ctx {
     spring::DBuf<double> d_kap_part;  // per-block partial sums of the kappa kernel
     spring::DBuf<double> d_krn;    // [q0][s][9]
     spring::DBuf<double> d_rxyz;
-    spring::DBuf<double> d_wiso;   // [slot][q1][s0][s1]
+    spring::DBuf<double> d_wiso;   // isotope W [slot][s0][s1][q1]
     spring::DBuf<double> d_tet_tab;  // tetrahedron tables of the grid: records (n(T), omega) [s][q], FP32 omega [s][q]
 
     // tensor-core V3 (spring_set_precision): operand tables and pair tiles grouped by q1

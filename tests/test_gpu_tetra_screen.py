@@ -73,3 +73,24 @@ def test_screened_four_phonon_sums_match_oracle(mesh, nT, pol):
             ro, _ = D.lw4_tetra(st, first - 1 + k, it, pol=p)
             np.testing.assert_allclose(rate[it, k], ro, rtol=1e-9, atol=1e-12 * max(np.abs(ro).max(), 1e-30))
     ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("delta", ["tetra", "gauss"])
+@pytest.mark.parametrize("cell,N,nT", [("rocksalt2", 3, 1), ("rocksalt2", 4, 11), ("rocksalt8", 2, 2)])
+def test_isotope_rate_matches_oracle(cell, N, nT, delta):
+    """Six and 24 branches (one and four passes over s0), a last group of two tetrahedra, and more
+    temperatures than the 3-phonon sums take."""
+    cr = S.build(cell)
+    temps = list(np.linspace(100.0, 900.0, nT))
+    st = D.Setup(cr, (N, N, N), temps)
+    ctx, _ = from_crystal(cr, (N, N, N), temps, phonons={"grid": st.ph, "irr": st.ph0})
+    g2 = np.linspace(1e-3, 3e-3, cr.nbasis)
+    rate = ctx.linewidth_iso(1, st.nq0, g2, delta=delta, sigma=0.3767)
+    for i0 in range(st.nq0):
+        wi = D.iso_w(cr.nbasis, st.ph0["evec"][i0], st.ph0["omega"][i0], st.ph["evec"], g2)
+        ref = (D.iso_lw_gauss(st.ph0["omega"][i0], st.ph["omega"], wi, 0.3767) if delta == "gauss"
+               else D.iso_lw_tetra(st.ph0["omega"][i0], st.ph["omega"], wi, st.tetra))
+        for it in range(nT):
+            np.testing.assert_allclose(rate[it, i0], ref, rtol=1e-9, atol=1e-14 * max(1.0, np.abs(rate).max()))
+    ctx.close()
