@@ -625,6 +625,12 @@ int spring_set_fc3(spring_ctx* c, int na3, const int* num, const int* idx, const
                 }
     }
     c->na3 = na3;
+    c->fc3_types = 0;
+    for (int mu = 0; mu < nb; ++mu) {
+        int types = 0;
+        for (int nu = 0; nu < nb; ++nu) types += off[(size_t)mu * (nb + 1) + nu + 1] > off[(size_t)mu * (nb + 1) + nu];
+        c->fc3_types = std::max(c->fc3_types, types);
+    }
     SPRING_CHECK(dalloc(c, c->d_fc3_off, off.size(), "FC3 slot offsets"));
     SPRING_CHECK(h2d(c, c->d_fc3_off.p, off.data(), sizeof(int) * off.size(), "FC3 slot offsets"));
     SPRING_CHECK(dalloc(c, c->d_fc3, t.size(), "FC3"));

@@ -115,6 +115,8 @@ int run_v3_gauss(spring_ctx* c, int q0_first, int n_q0, double sigma, const Pol&
                                 &handled, plist, nlist));
     }
     if (handled) return SPRING_OK;
+    SPRING_CHECK(launch_v3m(c, c->ps_irr, irr_view(c), q0_first, n_q0, 0, sigma, &pol, d_lw, d_p3, nullptr, &handled));
+    if (handled) return SPRING_OK;
     V3Args a{};
     a.onebysigma = 1.0 / sigma;
     a.onebysigma2 = a.onebysigma * a.onebysigma;
@@ -129,6 +131,8 @@ int run_v3_wgrid(spring_ctx* c, const PairSet& ps, const Q0View& v, int q0_first
     bool handled = false;
     if (!c->force_generic_v3)
         SPRING_CHECK(launch_v3s(c, ps, v, q0_first, n_q0, 1, 0.0, nullptr, nullptr, nullptr, d_w, &handled));
+    if (handled) return SPRING_OK;
+    SPRING_CHECK(launch_v3m(c, ps, v, q0_first, n_q0, 1, 0.0, nullptr, nullptr, nullptr, d_w, &handled));
     if (handled) return SPRING_OK;
     V3Args a{};
     return launch_v3<1>(c, ps, v, q0_first, n_q0, a, nullptr, nullptr, d_w);

@@ -168,6 +168,7 @@ struct spring_ctx {
     // FC3: [mu][N1][N2][alpha][beta][gamma] (Fortran memory order), zero beyond atm_num
     bool fc3_set = false;
     int na3 = 0;
+    int fc3_types = 0;                // most basis atoms among one atom's neighbour slots
     spring::DBuf<double> d_fc3;
     spring::DBuf<double> d_fc3_posr;  // [mu][N][3]  Cartesian cell vector
     spring::DBuf<int> d_fc3_btyp;     // [mu][N] 0-based basis index
@@ -362,6 +363,9 @@ struct Pol { int lo[3], hi[3]; };
 Q0View irr_view(spring_ctx* c);
 int run_v3_gauss(spring_ctx* c, int q0_first, int n_q0, double sigma, const Pol& pol, double* d_lw, double* d_p3);
 int run_v3_wgrid(spring_ctx* c, const PairSet& ps, const Q0View& v, int q0_first, int n_q0, double* d_w);
+// k_v3m.cu: V3 on the FP64 matrix instructions; *handled is false when the cell does not fit it
+int launch_v3m(spring_ctx* c, const PairSet& ps, const Q0View& v, int q0_first, int n_q0, int epi, double sigma,
+               const Pol* pol, double* lw, double* p3, double* w, bool* handled);
 // k_v3s.cu: specialised V3 for two-atom cells; *handled is false when the cell does not fit it
 int launch_v3s(spring_ctx* c, const PairSet& ps, const Q0View& v, int q0_first, int n_q0, int epi, double sigma,
                const Pol* pol, double* lw, double* p3, double* w, bool* handled, const int* plist = nullptr,
