@@ -15,8 +15,10 @@
 // lanes read distinct banks.
 // Gaussian epilogue: W of the block goes to shared memory; warps screen (s1, s2, channel) of one s0 against
 // the underflow point of exp and evaluate 32 hits at a time, one accumulator per temperature.
-// Bound: FP64 tensor pipe (9216 m8n8k4 per pair of the 8-atom cell, 37k cycles of one SM) and the barriers
-// between the steps.  V3M_TIMES
+// 8-atom cell: 6^3, nine temperatures 12.7 -> 0.85 ms, 8^3, three 52.1 -> 3.1 ms (14 TFLOP/s); W grids of
+// 6^3 12.6 -> 0.75 ms.  Bound: of the 100k cycles a pair takes, 37k are the FP64 tensor pipe (9216 m8n8k4;
+// Phi, H and T1 take 23k, 16k and 9k), 31k the latency of the Gaussian epilogue and 15k that of the inputs
+// and D, which three warps per scheduler do not hide.
 #include <algorithm>
 
 #include "v3item.cuh"
@@ -26,6 +28,7 @@ namespace spring {
 namespace {
 
 constexpr int MW = 12, MT_ = 9;  // warps per CTA; temperatures per epilogue pass
+constexpr int QCAP = 576;        // hits of one epilogue unit: 8 x 24 (s1, s2), three channels
 
 // Shared-memory layout (in double2 unless noted) and sizes of one launch.
 struct V3mLayout {
@@ -76,15 +79,22 @@ __global__ void __launch_bounds__(32 * MW, 1) k_v3m(V3Args a_, V3mLayout L, V3Pt
     int* sKh = sNt + MAX_NB;                              // [nu] rows (mu, a) of H's sum, a multiple of 4
     int* sKo = sKh + MAX_NB;                              // [nu][24] T1 offset of row (mu, a), nu b = 0
     int* sKr = sKo + MAX_NB * MAX_NDOF;                   // [nu][24] row of e0 (n: a zero column)
-    unsigned* sQ = reinterpret_cast<unsigned*>(sX + L.oQ);  // [MW][128] hit queues, behind W
+    int* sKe = sKr + MAX_NB * MAX_NDOF;                   // [mu][24] e2 offset of D's columns (0 beyond them: D is zero)
+    unsigned short* sQ = reinterpret_cast<unsigned short*>(sX + L.oQ);  // [MW][QCAP] hit queues, behind W
+    int* sSl = sKe + MAX_NB * MAX_NDOF;                   // [mu][8] first slot | slots << 8 of each type
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lr = lane >> 2, lc = lane & 3;
     constexpr int TH = 32 * MW;
 
     if (tid < nb) {  // the types of mu = tid
         int cnt = 0;
         for (int nu = 0; nu < nb; ++nu)
-            if (off[tid * (nb + 1) + nu + 1] > off[tid * (nb + 1) + nu]) sTy[tid * MAX_NB + cnt++] = nu;
+            if (off[tid * (nb + 1) + nu + 1] > off[tid * (nb + 1) + nu]) {
+                sSl[tid * MAX_NB + cnt] = off[tid * (nb + 1) + nu] | (off[tid * (nb + 1) + nu + 1] - off[tid * (nb + 1) + nu]) << 8;
+                sTy[tid * MAX_NB + cnt++] = nu;
+            }
         sNt[tid] = cnt;
+        for (int k = 0; k < MAX_NDOF; ++k)
+            sKe[tid * MAX_NDOF + k] = k < 3 * cnt ? (3 * sTy[tid * MAX_NB + k / 3] + k % 3) * L.S2 : 0;
     }
     __syncthreads();
     if (tid < nb) {  // the mu that have type nu = tid
@@ -158,41 +168,51 @@ __global__ void __launch_bounds__(32 * MW, 1) k_v3m(V3Args a_, V3mLayout L, V3Pt
                 sPP[i] = make_double2(m * (p1.x * p2.x - p1.y * p2.y), m * (p1.x * p2.y + p1.y * p2.x));
             }
             __syncthreads();
-            for (int i = tid; i < gm * 3 * L.KT * L.KT; i += TH) {
-                const int k = i % L.KT, r = i / L.KT % L.KT, ma = i / (L.KT * L.KT), ml = ma / 3, mu = mg + ml;
-                double2 acc = make_double2(0.0, 0.0);
-                const int K = 3 * sNt[mu];
-                if (r < K && k < K) {
-                    const int nu = sTy[mu * MAX_NB + r / 3], eta = sTy[mu * MAX_NB + k / 3];
-                    const int abc = (ma % 3 * 3 + r % 3) * 3 + k % 3;
-                    const int* o = off + mu * (nb + 1);
-                    const double* f = P.fc3 + (size_t)mu * na * na * 27 + abc;
-                    for (int N1 = o[nu]; N1 < o[nu + 1]; ++N1)
-                        for (int N2 = o[eta]; N2 < o[eta + 1]; ++N2) {
-                            const double fv = f[(N1 * na + N2) * 27];
-                            const double2 pp = sPP[(ml * na + N1) * na + N2];
-                            acc.x = fma(fv, pp.x, acc.x);
-                            acc.y = fma(fv, pp.y, acc.y);
+            // D: one thread per (mu, a, row, eta), three columns each (their FC3 values are adjacent); the
+            // terms are independent loads
+            const int kt = L.KT / 3 + (L.KT % 3 != 0);  // column triples, the last possibly cut
+            for (int i = tid; i < gm * 3 * L.KT * kt; i += TH) {
+                const int kp = i % kt, j = i / kt, r = j % L.KT, ma = j / L.KT, ml = ma / 3, mu = mg + ml;
+                double2 acc[3];
+#pragma unroll
+                for (int g = 0; g < 3; ++g) acc[g] = make_double2(0.0, 0.0);
+                if (r < 3 * sNt[mu] && kp < sNt[mu]) {
+                    const int l1 = sSl[mu * MAX_NB + r / 3], l2 = sSl[mu * MAX_NB + kp];
+                    const int a1 = l1 & 255, a2 = l2 & 255, c1 = l1 >> 8, cnt = c1 * (l2 >> 8);
+                    const double* f = P.fc3 + (size_t)mu * na * na * 27 + (ma % 3 * 3 + r % 3) * 3;
+#pragma unroll 4
+                    for (int t = 0, N1 = a1, N2 = a2; t < cnt; ++t) {
+                        const double* fv = f + (N1 * na + N2) * 27;
+                        const double2 pp = sPP[(ml * na + N1) * na + N2];
+#pragma unroll
+                        for (int g = 0; g < 3; ++g) {
+                            acc[g].x = fma(fv[g], pp.x, acc[g].x);
+                            acc[g].y = fma(fv[g], pp.y, acc[g].y);
                         }
+                        if (++N1 == a1 + c1) {
+                            N1 = a1;
+                            ++N2;
+                        }
+                    }
                 }
-                sD[(ma * L.KT + r) * L.DS + k] = acc;
+#pragma unroll
+                for (int g = 0; g < 3; ++g)
+                    if (3 * kp + g < L.KT) sD[j * L.DS + 3 * kp + g] = acc[g];
             }
             __syncthreads();
             // T1 of (mu, a): one warp each
             for (int u = warp; u < gm * 3; u += MW) {
-                const int mu = mg + u / 3;
+                const int mu = mg + u / 3, K = 3 * sNt[mu];
                 const double2* D = sD + u * L.KT * L.DS;
                 double2* T1 = sT1 + (mu * 3 + u % 3) * L.TB;
-                for (int mt = 0; mt * 8 < L.KT; ++mt) {
+                for (int mt = 0; mt * 8 < K; ++mt) {
                     const double2* A = D + min(mt * 8 + lr, L.KT - 1) * L.DS + lc;
                     double c[NT][2][2];
 #pragma unroll
                     for (int t = 0; t < NT; ++t) c[t][0][0] = c[t][0][1] = c[t][1][0] = c[t][1][1] = 0.0;
-                    for (int k0 = 0; k0 < L.KT; k0 += 4) {
+                    for (int k0 = 0; k0 < K; k0 += 4) {
                         const double2 av = A[k0];
-                        const int kk = k0 + lc;  // D is zero beyond mu's rows: any row of e2 does there
-                        const int row = kk < 3 * sNt[mu] ? 3 * sTy[mu * MAX_NB + kk / 3] + kk % 3 : 0;
-                        const double2* B = sE2 + row * L.S2 + lr;
+                        const double2* B = sE2 + sKe[mu * MAX_NDOF + k0 + lc] + lr;
 #pragma unroll
                         for (int t = 0; t < NT; ++t) cmma(c[t], av, B[8 * t]);
                     }
@@ -207,17 +227,23 @@ __global__ void __launch_bounds__(32 * MW, 1) k_v3m(V3Args a_, V3mLayout L, V3Pt
         const bool gq1 = g1 == 0, gq2 = g2 == 0;
         for (int sb = 0; sb < n; sb += 8) {
             // H of s0 = sb .. sb + 7
-            for (int t = warp; t < L.NR * NT; t += MW) {
-                const int r = t / NT, nt = t % NT;
-                double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+            for (int r = warp; r < L.NR; r += MW) {
+                double c[NT][2][2];
+#pragma unroll
+                for (int t = 0; t < NT; ++t) c[t][0][0] = c[t][0][1] = c[t][1][0] = c[t][1][1] = 0.0;
                 if (r < n) {
                     const int nu = r / 3, K = sKh[nu];
                     const double2* A = sE0 + (sb + lr) * L.RS;
-                    const double2* B = sT1 + (r % 3) * L.S2 + 8 * nt + lr;
-                    for (int k0 = 0; k0 < K; k0 += 4)
-                        cmma(c, A[sKr[nu * MAX_NDOF + k0 + lc]], B[sKo[nu * MAX_NDOF + k0 + lc]]);
+                    const double2* B = sT1 + (r % 3) * L.S2 + lr;
+                    for (int k0 = 0; k0 < K; k0 += 4) {
+                        const double2 av = A[sKr[nu * MAX_NDOF + k0 + lc]];
+                        const double2* Bk = B + sKo[nu * MAX_NDOF + k0 + lc];
+#pragma unroll
+                        for (int t = 0; t < NT; ++t) cmma(c[t], av, Bk[8 * t]);
+                    }
                 }
-                put2(sH + lr * L.HS + r * L.S2 + 8 * nt + 2 * lc, c);
+#pragma unroll
+                for (int t = 0; t < NT; ++t) put2(sH + lr * L.HS + r * L.S2 + 8 * t + 2 * lc, c[t]);
             }
             __syncthreads();
             // Phi of (s0, eight s1): up to two units per warp, written once every warp has read its H
@@ -267,7 +293,7 @@ __global__ void __launch_bounds__(32 * MW, 1) k_v3m(V3Args a_, V3mLayout L, V3Pt
                 }
             } else {
                 const double pre = a.onebysigma * ONEBYSQRT2PI, mult = g1 != g2 ? 2.0 : 1.0;
-                unsigned* queue = sQ + warp * 128;
+                unsigned short* queue = sQ + warp * QCAP;
                 for (int t0 = 0; t0 < a.nT; t0 += MT_) {
                     const int nt = min(MT_, a.nT - t0);
                     if (a.nT > MT_) {
@@ -278,66 +304,85 @@ __global__ void __launch_bounds__(32 * MW, 1) k_v3m(V3Args a_, V3mLayout L, V3Pt
                         }
                         __syncthreads();
                     }
-                    // (s0, a third of the (s1, s2)): two units per warp at 24 branches
+                    // (s0, a third of the s1): two units per warp at 24 branches; a step takes rp rows of s1
+                    const int rp = 32 / n, lrow = lane / n, s2 = lane % n;
+                    const bool lane_on = lrow < rp && s2 >= a.pol_lo[2] && s2 <= a.pol_hi[2] && !(gq2 && s2 < 3);
+                    const double w2 = sc[2 * MAX_NDOF + s2];
                     for (int u = warp; u < 24; u += MW) {
                         const int s0l = u & 7, s0 = sb + s0l;
                         if (s0 >= n || s0 < a.pol_lo[0] || s0 > a.pol_hi[0]) continue;
                         const double w0 = sc[s0];
-                        const int step = (n * n + 2) / 3, j0 = (u >> 3) * step, j1 = min(j0 + step, n * n);
+                        const int step = (n + 2) / 3, i0 = (u >> 3) * step, i1 = min(i0 + step, n);
                         double acc[MT_], accp = 0.0;
 #pragma unroll
                         for (int t = 0; t < MT_; ++t) acc[t] = 0.0;
-                        auto evaluate = [&](unsigned code) {
-                            const int j = code & 1023, ch = code >> 10, s1 = j / n, s2 = j % n;
-                            const double w1 = sc[MAX_NDOF + s1], w2 = sc[2 * MAX_NDOF + s2];
-                            const double d = ch == 0 ? w0 - w1 - w2 : (ch == 1 ? w0 + w1 - w2 : w0 - w1 + w2);
-                            const double e = pre * exp(-(0.5 * a.onebysigma2 * (d * d)));
-                            accp += e;
-                            const double v = sW[(s0l * n + s1) * (n + 1) + s2] * (ch == 2 ? -e : e);
-                            const double *n1 = sN + s1, *n2 = sN + MT_ * MAX_NDOF + s2;
-#pragma unroll
-                            for (int t = 0; t < MT_; ++t) {
-                                if (t >= nt) break;
-                                const double x = n1[t * MAX_NDOF], y = n2[t * MAX_NDOF];
-                                acc[t] = fma(v, ch == 0 ? x + y + 1.0 : x - y, acc[t]);
-                            }
-                        };
                         int qn = 0;
-                        for (int jb = j0; jb < j1; jb += 32) {
-                            const int j = jb + lane, s1 = j / n, s2 = j % n;
+#pragma unroll 4
+                        for (int ib = i0; ib < i1; ib += rp) {
+                            const int s1 = ib + lrow;
                             unsigned in = 0;
-                            if (j < j1 && s1 >= a.pol_lo[1] && s1 <= a.pol_hi[1] && s2 >= a.pol_lo[2] && s2 <= a.pol_hi[2] &&
-                                !(gq1 && s1 < 3) && !(gq2 && s2 < 3)) {
-                                const double w1 = sc[MAX_NDOF + s1], w2 = sc[2 * MAX_NDOF + s2];
+                            if (lane_on && s1 < i1 && s1 >= a.pol_lo[1] && s1 <= a.pol_hi[1] && !(gq1 && s1 < 3)) {
+                                const double w1 = sc[MAX_NDOF + s1];
                                 const double d1 = w0 - w1 - w2, d2 = w0 + w1 - w2, d3 = w0 - w1 + w2;
                                 in = (0.5 * a.onebysigma2 * (d1 * d1) < EXP_UNDERFLOW ? 1 : 0) |
                                      (0.5 * a.onebysigma2 * (d2 * d2) < EXP_UNDERFLOW ? 2 : 0) |
                                      (0.5 * a.onebysigma2 * (d3 * d3) < EXP_UNDERFLOW ? 4 : 0);
                             }
+                            const unsigned code = s1 | s2 << 5, lt = (1u << lane) - 1;
 #pragma unroll
                             for (int ch = 0; ch < 3; ++ch) {
                                 const unsigned m = __ballot_sync(0xffffffffu, in >> ch & 1);
-                                if (in >> ch & 1) queue[qn + __popc(m & ((1u << lane) - 1))] = j | ch << 10;
+                                if (in >> ch & 1) queue[qn + __popc(m & lt)] = code | ch << 10;
                                 qn += __popc(m);
                             }
-                            __syncwarp();
-                            while (qn >= 32) {
-                                qn -= 32;
-                                evaluate(queue[qn + lane]);
-                            }
-                            __syncwarp();
                         }
-                        if (lane < qn) evaluate(queue[lane]);
                         __syncwarp();
+                        // two hits per lane at a time: their exponentials overlap
+                        for (int i = lane; i < qn; i += 64) {
+                            double v[2];
+                            const double *n1[2], *n2[2];
+                            bool sum[2];
 #pragma unroll
-                        for (int t = 0; t < MT_; ++t) {
-                            if (t >= nt) break;
-                            const double v = tet::warp_sum(acc[t]);
-                            if (lane == 0 && v != 0.0)
-                                atomicAdd(&P.out_lw[((size_t)(t0 + t) * a.nq0 + q0) * n + s0], mult * v);
+                            for (int h = 0; h < 2; ++h) {
+                                const bool have = i + 32 * h < qn;
+                                const unsigned code = have ? queue[i + 32 * h] : 0;
+                                const int t1 = code & 31, t2 = code >> 5 & 31, ch = code >> 10;
+                                const double v1 = sc[MAX_NDOF + t1], v2 = sc[2 * MAX_NDOF + t2];
+                                const double d = ch == 0 ? w0 - v1 - v2 : (ch == 1 ? w0 + v1 - v2 : w0 - v1 + v2);
+                                const double e = have ? pre * exp(-(0.5 * a.onebysigma2 * (d * d))) : 0.0;
+                                accp += e;
+                                v[h] = sW[(s0l * n + t1) * (n + 1) + t2] * (ch == 2 ? -e : e);
+                                if (!have) v[h] = 0.0;
+                                n1[h] = sN + t1;
+                                n2[h] = sN + MT_ * MAX_NDOF + t2;
+                                sum[h] = ch == 0;
+                            }
+#pragma unroll
+                            for (int t = 0; t < MT_; ++t) {
+                                if (t >= nt) break;
+#pragma unroll
+                                for (int h = 0; h < 2; ++h) {
+                                    const double x = n1[h][t * MAX_NDOF], y = n2[h][t * MAX_NDOF];
+                                    acc[t] = fma(v[h], sum[h] ? x + y + 1.0 : x - y, acc[t]);
+                                }
+                            }
                         }
-                        const double v = tet::warp_sum(accp);
-                        if (lane == 0 && v != 0.0 && t0 == 0) atomicAdd(&P.out_p3[(size_t)q0 * n + s0], mult * v);
+                        __syncwarp();
+                        // the sums of three temperatures and the phase space run side by side
+#pragma unroll
+                        for (int t = 0; t < MT_; t += 3) {
+                            if (t >= nt) break;
+                            double x[4] = {acc[t], acc[t + 1], acc[t + 2], accp};
+                            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                                for (int h = 0; h < 4; ++h) x[h] += __shfl_down_sync(0xffffffffu, x[h], o);
+                            if (lane != 0) continue;
+#pragma unroll
+                            for (int h = 0; h < 3; ++h)
+                                if (t + h < nt && x[h] != 0.0)
+                                    atomicAdd(&P.out_lw[((size_t)(t0 + t + h) * a.nq0 + q0) * n + s0], mult * x[h]);
+                            if (t == 0 && t0 == 0 && x[3] != 0.0) atomicAdd(&P.out_p3[(size_t)q0 * n + s0], mult * x[3]);
+                        }
                     }
                 }
             }
@@ -365,14 +410,14 @@ V3mLayout v3m_layout(int nb, int n, int na, int types) {
     L.oPh = n * L.S2;
     L.oPP = L.oPh + nb * 2 * na;
     L.oQ = (8 * n * (n + 1) + 1) / 2;
-    const int h = std::max(8 * L.HS, L.oQ + MW * 128 * (int)sizeof(unsigned) / (int)sizeof(double2));
+    const int h = std::max(8 * L.HS, L.oQ + MW * QCAP * (int)sizeof(unsigned short) / (int)sizeof(double2));
     const auto x_of = [&](int gm) { return L.oPP + gm * na * na + gm * 3 * L.KT * L.DS; };
     L.GM = nb;  // as many mu per group as H's place holds, at least one
     while (L.GM > 1 && x_of(L.GM) > h) --L.GM;
     L.oD = L.oPP + L.GM * na * na;
     L.oI = (L.oX + std::max(h, x_of(L.GM))) * (int)sizeof(double2);
     L.bytes = L.oI + (6 + 2 * MT_) * MAX_NDOF * (int)sizeof(double) +
-              (MAX_NB * MAX_NB + 2 * MAX_NB + 2 * MAX_NB * MAX_NDOF) * (int)sizeof(int);
+              (2 * MAX_NB * MAX_NB + 2 * MAX_NB + 3 * MAX_NB * MAX_NDOF) * (int)sizeof(int);
     return L;
 }
 
