@@ -336,7 +336,8 @@ int spring_kappa_iter_gauss(spring_ctx* ctx, double sigma, double eps_k, int max
  * process.  Requests on one context must not overlap in q0.  A request on a
  * two-atom context set to SPRING_BF16 / SPRING_BF16X3 runs through the
  * tensor-core pass of spring_linewidth3 (same kernel, same results) right
- * after the graph, inside the same spring_batch_run; path requests
+ * after the graph, inside the same spring_batch_run, and a request on a cell of
+ * four or more atoms through the FP64 matrix kernel there; path requests
  * (spring_batch_add_path) are launched inside the graph. */
 typedef struct spring_batch spring_batch;
 int spring_batch_create(spring_batch** batch);

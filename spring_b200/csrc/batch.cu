@@ -9,7 +9,9 @@
 // (`chunk` at a time), so uneven workloads (Ndof 6 and 24, 12^3 to 20^3 meshes,
 // 1 to 9 temperatures) share one launch without tail effects.  Each item runs
 // the any-cell FP64 V3 work item of k_v3.cu against its workload's
-// descriptor (staged in shared memory when the workload changes).  The zero
+// descriptor (staged in shared memory when the workload changes); cells of 12
+// and more branches that k_v3m.cu takes, and tensor-core requests, run their own
+// kernel right after the graph.  The zero
 // fills, the kernel and the LW_Allq0 updates are captured in one CUDA graph.
 //
 // Autotuner: threads per CTA, CTAs per SM, the s0 block of large cells and the
@@ -130,7 +132,7 @@ struct spring_batch {
         double sigma;
         spring::Pol pol;
         long long pairs = 0, items = 0;
-        int kind = 1;       // 0: two-atom groups, 1: any cell, 2: tensor-core pass (outside the kernel)
+        int kind = 1;       // 0: two-atom groups, 1: any cell, 2: a pass of its own (outside the kernel)
         double cost = 0.0;  // per item, for the heaviest-first order
     };
     std::vector<Work> work;
@@ -208,6 +210,10 @@ std::string shape_key(const spring_batch* b) {
 // persistent FP64 kernel.
 bool tc_request(const spring_ctx* c) { return c->precision != SPRING_FP64 && c->nb == 2 && c->na3 <= 8; }
 
+// Requests that run by themselves after the graph: the tensor-core ones, and cells whose V3 the FP64 matrix
+// kernel takes (one CTA of 227 KB per SM; an item of the persistent kernel costs 15 times its work there).
+bool own_pass(const spring_ctx* c) { return tc_request(c) || spring::v3m_takes(c); }
+
 // Device descriptors of every request for the configuration in b->cfg, in heaviest-first order;
 // returns the shared-memory size, the item offsets and the fold total on the host too.
 int build_desc(spring_batch* b, std::vector<BatchDesc>& D, std::vector<long long>& off, size_t* smem,
@@ -223,9 +229,9 @@ int build_desc(spring_batch* b, std::vector<BatchDesc>& D, std::vector<long long
         if (spring::pairoff_host(c, ps) != SPRING_OK) return bfail(b, SPRING_ERR_CUDA, "%s", c->err.c_str());
         w.pairs = ps.h_pairoff[w.q0 + w.n_q0] - ps.h_pairoff[w.q0];
         w.kind = (b->cfg[0] && c->nb == spring::s3::NB && c->na3 == spring::s3::NA && c->nT <= spring::s3::MAXT) ? 0 : 1;
-        if (tc_request(c)) w.kind = 2;
+        if (own_pass(c)) w.kind = 2;
         if (w.kind == 2) {
-            w.items = 0;  // the tensor-core pass runs it, beside the persistent kernel
+            w.items = 0;  // its own pass runs it, after the persistent kernel
             w.cost = 0.0;
         } else if (w.kind == 0) {
             w.items = (w.pairs + spring::s3::PP - 1) / spring::s3::PP;
@@ -291,7 +297,11 @@ int build_desc(spring_batch* b, std::vector<BatchDesc>& D, std::vector<long long
                                  c->ph_grid.oneby.p, c->ph_grid.nbe.p, c->d_lw_tmp.p, c->d_p3.p, nullptr};
             *smem = std::max(*smem, sizeof(spring::s3::Smem));
         } else {
-            *smem = std::max(*smem, spring::v3_smem(n, c->na3, sb, c->nT));
+            const size_t need = spring::v3_smem(n, c->na3, sb, c->nT);
+            // a configuration is refused by its items' size, also where the request runs by itself
+            if (need > 227 * 1024)
+                return bfail(b, SPRING_ERR_UNSUPPORTED, "batch work item needs %zu bytes of shared memory", need);
+            if (w.kind == 1) *smem = std::max(*smem, need);
         }
         D[k].lw_all = c->d_lw_all.p;
         D[k].fold0 = fold;
@@ -427,17 +437,17 @@ int enqueue_paths(spring_batch* b) {
     return SPRING_OK;
 }
 
-// The tensor-core requests after the graph (which zeroed their scratch): the pass of
+// The requests with a pass of their own after the graph (which zeroed their scratch): the pass of
 // spring_linewidth3 on each context's stream, then its LW_Allq0 update; the batch stream waits for
 // them.
-int run_tc_requests(spring_batch* b) {
+int run_own_passes(spring_batch* b) {
     for (const auto& w : b->work) {
         if (w.kind != 2) continue;
         spring_ctx* c = w.c;
         BCHECK(join_ctx_out(b, c));
         int rc = spring::run_v3_gauss(c, w.q0, w.n_q0, w.sigma, w.pol, c->d_lw_tmp.p, c->d_p3.p);
         if (rc == SPRING_OK) rc = spring::run_axpy_lw(c, 1.0, c->d_lw_tmp.p, c->d_lw_all.p, w.q0, w.n_q0);
-        if (rc != SPRING_OK) return bfail(b, rc, "tensor-core request: %s", c->err.c_str());
+        if (rc != SPRING_OK) return bfail(b, rc, "request: %s", c->err.c_str());
         BCHECK(join_ctx_in(b, c));
     }
     return SPRING_OK;
@@ -693,7 +703,7 @@ int spring_batch_run(spring_batch* b) {
     BCHECK(bcuda(b, cudaEventRecord(b->ev0, b->stream), "batch timing"));
     BCHECK(bcuda(b, cudaGraphLaunch(b->exec, b->stream), "batch graph launch"));
     b->work[0].c->launches += 2;
-    BCHECK(run_tc_requests(b));
+    BCHECK(run_own_passes(b));
     BCHECK(bcuda(b, cudaEventRecord(b->ev1, b->stream), "batch timing"));
     BCHECK(join_out(b));
     BCHECK(bcuda(b, cudaEventSynchronize(b->ev1), "batch run"));

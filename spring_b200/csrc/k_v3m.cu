@@ -423,16 +423,20 @@ V3mLayout v3m_layout(int nb, int n, int na, int types) {
 
 }  // namespace
 
+// Whether launch_v3m takes the context's cell.  Fewer branches leave the 8-wide tiles half empty and a step
+// too short for its barriers: at 3 to 9 branches the kernel in k_v3.cu takes 0.24 - 0.33 ms where this one
+// takes 0.50 - 1.3; from 12 on this one is ahead (12: 0.93 -> 0.50 ms, 15: 3.0 -> 0.36, 18: 2.2 -> 0.40,
+// 24: 10.1 -> 0.55; W grids of 16 q0).
+bool v3m_takes(const spring_ctx* c) {
+    return c->ndof >= 12 && v3m_layout(c->nb, c->ndof, c->na3, c->fc3_types).bytes <= 227 * 1024;
+}
+
 // Launch for pair set ps, q0 block [q0_first, +n_q0); *handled is false when the layout does not fit.
 int launch_v3m(spring_ctx* c, const PairSet& ps, const Q0View& v, int q0_first, int n_q0, int epi, double sigma,
                const Pol* pol, double* lw, double* p3, double* w, bool* handled) {
     *handled = false;
-    // Fewer branches leave the 8-wide tiles half empty and a step too short for its barriers: at 3 to 9
-    // branches the kernel in k_v3.cu takes 0.24 - 0.33 ms where this one takes 0.50 - 1.3; from 12 on this
-    // one is ahead (12: 0.93 -> 0.75 ms, 15: 3.0 -> 0.46, 18: 2.2 -> 0.49, 24: 10.1 -> 0.67; W grids of 16 q0).
-    if (c->ndof < 12) return SPRING_OK;
+    if (!v3m_takes(c)) return SPRING_OK;
     const V3mLayout L = v3m_layout(c->nb, c->ndof, c->na3, c->fc3_types);
-    if (L.bytes > 227 * 1024) return SPRING_OK;
     *handled = true;
     V3Args a{};
     a.nb = c->nb;

@@ -364,6 +364,7 @@ Q0View irr_view(spring_ctx* c);
 int run_v3_gauss(spring_ctx* c, int q0_first, int n_q0, double sigma, const Pol& pol, double* d_lw, double* d_p3);
 int run_v3_wgrid(spring_ctx* c, const PairSet& ps, const Q0View& v, int q0_first, int n_q0, double* d_w);
 // k_v3m.cu: V3 on the FP64 matrix instructions; *handled is false when the cell does not fit it
+bool v3m_takes(const spring_ctx* c);
 int launch_v3m(spring_ctx* c, const PairSet& ps, const Q0View& v, int q0_first, int n_q0, int epi, double sigma,
                const Pol* pol, double* lw, double* p3, double* w, bool* handled);
 // k_v3s.cu: specialised V3 for two-atom cells; *handled is false when the cell does not fit it
