@@ -9,9 +9,9 @@
 // (`chunk` at a time), so uneven workloads (Ndof 6 and 24, 12^3 to 20^3 meshes,
 // 1 to 9 temperatures) share one launch without tail effects.  Each item runs
 // the any-cell FP64 V3 work item of k_v3.cu against its workload's
-// descriptor (staged in shared memory when the workload changes); cells of 12
-// and more branches that k_v3m.cu takes, and tensor-core requests, run their own
-// kernel right after the graph.  The zero
+// descriptor (staged in shared memory when the workload changes); requests that
+// the tensor-core pass or an FP64 matrix kernel takes (two-atom cells, k_v3s.cu;
+// 12 and more branches, k_v3m.cu) run it right after the graph.  The zero
 // fills, the kernel and the LW_Allq0 updates are captured in one CUDA graph.
 //
 // Autotuner: threads per CTA, CTAs per SM, the s0 block of large cells and the
@@ -28,19 +28,15 @@
 #include <vector>
 
 #include "v3item.cuh"
-#include "v3sitem.cuh"
 
 namespace spring {
 namespace {
 
-constexpr int BT = s3::THREADS;  // threads per CTA: the two-atom group layout needs exactly 288
+constexpr int BT = 288;  // threads per CTA
 
 struct BatchDesc {
-    int kind;        // 0: two-atom groups of s3::PP pairs (k_v3s layout), 1: any cell, (pair, s0 block)
-    V3Args a;        // kind 1 (and the fold's sizes for both kinds)
-    V3Ptrs P;        // kind 1 (out_lw also read by the fold)
-    s3::S3Args a3;   // kind 0
-    s3::S3Ptrs P3;   // kind 0
+    V3Args a;        // (pair, s0 block) items, and the fold's sizes
+    V3Ptrs P;        // out_lw also read by the fold
     double* lw_all;  // LW_Allq0 of the context
     long long fold0, fold_n;  // this request's slab [T][q0 range][s] in the fold kernel's index space
 };
@@ -48,9 +44,8 @@ struct BatchDesc {
 __global__ void __launch_bounds__(BT, 2) k_v3_batch(const BatchDesc* __restrict__ desc, const long long* __restrict__ off,
                                                     int nw, int chunk, unsigned long long* __restrict__ ctr) {
     extern __shared__ __align__(16) double2 smem2[];
-    s3::Smem& S = *reinterpret_cast<s3::Smem*>(smem2);
     __shared__ long long s_it;
-    __shared__ int s_w, s_new;
+    __shared__ int s_w;
     __shared__ BatchDesc s_d;
     if (threadIdx.x == 0) s_w = -1;
     const long long total = off[nw];
@@ -65,23 +60,15 @@ __global__ void __launch_bounds__(BT, 2) k_v3_batch(const BatchDesc* __restrict_
             int w = 0;
             while (w + 1 < nw && off[w + 1] <= it) ++w;
             __syncthreads();
-            if (threadIdx.x == 0) {
-                s_new = w != s_w;
-                if (s_new) {
-                    s_d = desc[w];
-                    s_w = w;
-                }
+            if (threadIdx.x == 0 && w != s_w) {
+                s_d = desc[w];
+                s_w = w;
             }
             __syncthreads();
             const long long local = it - off[w];
-            if (s_d.kind == 0) {
-                if (s_new) s3::v3s_stage(S, s_d.P3);  // v3s_group syncs before reading the constants
-                s3::v3s_group<0>(S, s_d.a3, s_d.P3, (int)local);
-            } else {
-                const int pr = s_d.a.pair_first + (int)(local / s_d.a.nsb);
-                const int s0b = (int)(local % s_d.a.nsb) * s_d.a.sb;
-                v3_item<0>(s_d.a, s_d.P, pr, s0b, smem2);
-            }
+            const int pr = s_d.a.pair_first + (int)(local / s_d.a.nsb);
+            const int s0b = (int)(local % s_d.a.nsb) * s_d.a.sb;
+            v3_item<0>(s_d.a, s_d.P, pr, s0b, smem2);
         }
     }
 }
@@ -132,7 +119,7 @@ struct spring_batch {
         double sigma;
         spring::Pol pol;
         long long pairs = 0, items = 0;
-        int kind = 1;       // 0: two-atom groups, 1: any cell, 2: a pass of its own (outside the kernel)
+        bool own = false;   // a pass of its own, outside the persistent kernel
         double cost = 0.0;  // per item, for the heaviest-first order
     };
     std::vector<Work> work;
@@ -149,7 +136,7 @@ struct spring_batch {
     };
     std::vector<PathReq> paths;
     std::string err;
-    // two-atom group path (1: where the cell fits), CTAs per SM (0: occupancy limit), s0 block for
+    // two-atom cells by their own kernel (1: where the cell fits), CTAs per SM (0: occupancy limit), s0 block for
     // Ndof > 12 (0: 6), work items per scheduler step
     int cfg[4] = {1, 0, 0, 1};
     int device = -1;
@@ -210,9 +197,12 @@ std::string shape_key(const spring_batch* b) {
 // persistent FP64 kernel.
 bool tc_request(const spring_ctx* c) { return c->precision != SPRING_FP64 && c->nb == 2 && c->na3 <= 8; }
 
-// Requests that run by themselves after the graph: the tensor-core ones, and cells whose V3 the FP64 matrix
-// kernel takes (one CTA of 227 KB per SM; an item of the persistent kernel costs 15 times its work there).
-bool own_pass(const spring_ctx* c) { return tc_request(c) || spring::v3m_takes(c); }
+// Requests that run by themselves after the graph: the tensor-core ones, and cells whose V3 an FP64 matrix
+// kernel takes (one CTA per SM with most of its shared memory; an item of the persistent kernel costs 15 times
+// the work there for 24 branches, 5 times for a two-atom cell).
+bool own_pass(const spring_batch* b, const spring_ctx* c) {
+    return tc_request(c) || spring::v3m_takes(c) || (b->cfg[0] && !c->force_generic_v3 && spring::v3s_takes(c));
+}
 
 // Device descriptors of every request for the configuration in b->cfg, in heaviest-first order;
 // returns the shared-memory size, the item offsets and the fold total on the host too.
@@ -228,14 +218,10 @@ int build_desc(spring_batch* b, std::vector<BatchDesc>& D, std::vector<long long
         const spring::PairSet& ps = c->ps_irr;
         if (spring::pairoff_host(c, ps) != SPRING_OK) return bfail(b, SPRING_ERR_CUDA, "%s", c->err.c_str());
         w.pairs = ps.h_pairoff[w.q0 + w.n_q0] - ps.h_pairoff[w.q0];
-        w.kind = (b->cfg[0] && c->nb == spring::s3::NB && c->na3 == spring::s3::NA && c->nT <= spring::s3::MAXT) ? 0 : 1;
-        if (own_pass(c)) w.kind = 2;
-        if (w.kind == 2) {
+        w.own = own_pass(b, c);
+        if (w.own) {
             w.items = 0;  // its own pass runs it, after the persistent kernel
             w.cost = 0.0;
-        } else if (w.kind == 0) {
-            w.items = (w.pairs + spring::s3::PP - 1) / spring::s3::PP;
-            w.cost = spring::s3::PP * (27.0 * 4 * c->na3 * c->na3 + 8.0 * n * n * n * n);
         } else {
             w.items = w.pairs * ((n + sb - 1) / sb);
             w.cost = (double)n * n * n * sb + 27.0 * c->na3 * c->na3 * n * n;
@@ -273,39 +259,14 @@ int build_desc(spring_batch* b, std::vector<BatchDesc>& D, std::vector<long long
                                 c->d_fc3_btyp.p, c->d_mass_rs.p, c->d_qpnt.p, v.q0_int, v.q0_grid, v.evec, v.omega,
                                 v.oneby, c->ph_grid.evec.p, c->ph_grid.omega.p, c->ph_grid.oneby.p,
                                 c->ph_grid.nbe.p, c->d_lw_tmp.p, c->d_p3.p, nullptr};
-        D[k].kind = w.kind;
-        if (w.kind == 0) {
-            spring::s3::S3Args& a3 = D[k].a3;
-            a3.nq = c->nq;
-            a3.nT = c->nT;
-            a3.nq0 = c->ps_irr.n0;
-            a3.q0_first = w.q0;
-            a3.pair_first = c->ps_irr.h_pairoff[w.q0];
-            a3.pair_end = c->ps_irr.h_pairoff[w.q0 + w.n_q0];
-            a3.plist = nullptr;
-            a3.ngroups = (int)w.items;
-            a3.mfac = a.mfac;
-            a3.onebysigma = a.onebysigma;
-            a3.onebysigma2 = a.onebysigma2;
-            for (int i = 0; i < 3; ++i) {
-                a3.pol_lo[i] = w.pol.lo[i];
-                a3.pol_hi[i] = w.pol.hi[i];
-            }
-            D[k].P3 = spring::s3::S3Ptrs{c->ps_irr.pairs.p, c->ps_irr.pair_q0.p, c->d_fc3.p, c->d_fc3_posr.p,
-                                 c->d_fc3_btyp.p, c->d_fc3_off.p, c->d_mass_rs.p, c->d_qpnt.p, v.q0_int, v.q0_grid,
-                                 v.evec, v.omega, v.oneby, c->ph_grid.evec.p, c->ph_grid.omega.p,
-                                 c->ph_grid.oneby.p, c->ph_grid.nbe.p, c->d_lw_tmp.p, c->d_p3.p, nullptr};
-            *smem = std::max(*smem, sizeof(spring::s3::Smem));
-        } else {
-            const size_t need = spring::v3_smem(n, c->na3, sb, c->nT);
-            // a configuration is refused by its items' size, also where the request runs by itself
-            if (need > 227 * 1024)
-                return bfail(b, SPRING_ERR_UNSUPPORTED, "batch work item needs %zu bytes of shared memory", need);
-            if (w.kind == 1) *smem = std::max(*smem, need);
-        }
+        const size_t need = spring::v3_smem(n, c->na3, sb, c->nT);
+        // a configuration is refused by its items' size, also where the request runs by itself
+        if (need > 227 * 1024)
+            return bfail(b, SPRING_ERR_UNSUPPORTED, "batch work item needs %zu bytes of shared memory", need);
+        if (!w.own) *smem = std::max(*smem, need);
         D[k].lw_all = c->d_lw_all.p;
         D[k].fold0 = fold;
-        D[k].fold_n = w.kind == 2 ? 0 : (long long)c->nT * w.n_q0 * n;  // kind 2 folds after its own pass
+        D[k].fold_n = w.own ? 0 : (long long)c->nT * w.n_q0 * n;  // an own pass folds by itself
         fold += D[k].fold_n;
         off[k + 1] = off[k] + w.items;
     }
@@ -442,7 +403,7 @@ int enqueue_paths(spring_batch* b) {
 // them.
 int run_own_passes(spring_batch* b) {
     for (const auto& w : b->work) {
-        if (w.kind != 2) continue;
+        if (!w.own) continue;
         spring_ctx* c = w.c;
         BCHECK(join_ctx_out(b, c));
         int rc = spring::run_v3_gauss(c, w.q0, w.n_q0, w.sigma, w.pol, c->d_lw_tmp.p, c->d_p3.p);

@@ -33,7 +33,7 @@
 
 #include "spring_internal.cuh"
 #include "tetra.cuh"
-#include "v3sitem.cuh"
+#include "v3s.cuh"
 
 namespace spring {
 namespace {

@@ -368,6 +368,7 @@ bool v3m_takes(const spring_ctx* c);
 int launch_v3m(spring_ctx* c, const PairSet& ps, const Q0View& v, int q0_first, int n_q0, int epi, double sigma,
                const Pol* pol, double* lw, double* p3, double* w, bool* handled);
 // k_v3s.cu: specialised V3 for two-atom cells; *handled is false when the cell does not fit it
+bool v3s_takes(const spring_ctx* c);
 int launch_v3s(spring_ctx* c, const PairSet& ps, const Q0View& v, int q0_first, int n_q0, int epi, double sigma,
                const Pol* pol, double* lw, double* p3, double* w, bool* handled, const int* plist = nullptr,
                int nlist = 0);
