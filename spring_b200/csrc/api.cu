@@ -342,6 +342,7 @@ int spring_ctx_destroy(spring_ctx* c) {
         dfree(c->d_scan_tmp); dfree(c->d_w); dfree(c->d_lw_all); dfree(c->d_lw_tmp); dfree(c->d_p3);
         dfree(c->d_kappa); dfree(c->d_krn); dfree(c->d_rxyz); dfree(c->d_wiso); dfree(c->d_tet_tab);
         free_enum4(c);
+        free_path_ws(c);
         dfree(c->d_v4_ph); dfree(c->d_v4_etab); dfree(c->d_v4_wf); dfree(c->d_v4_c); dfree(c->d_v4_map);
         dfree(c->d_v4_img); dfree(c->d_v4_cnt); dfree(c->d_v4_seg); dfree(c->d_v4_ntl); dfree(c->d_v4_toff);
         dfree(c->d_v4_stat); dfree(c->d_v4_tiles);

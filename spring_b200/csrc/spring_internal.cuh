@@ -247,6 +247,8 @@ struct spring_ctx {
     spring::DBuf<int> d_v4_cnt, d_v4_seg, d_v4_ntl, d_v4_toff, d_v4_stat;
     spring::DBuf<int4> d_v4_tiles;
 
+    void* path_ws = nullptr;       // buffers of spring_linewidth_path (k_path.cu)
+
     // scratch
     spring::DBuf<int> d_scan_tmp;
     spring::DBuf<double> d_w;      // W buffer for tetrahedron integration [slot][q1][s0][s1][s2]
@@ -415,6 +417,7 @@ int path_prepare(spring_ctx* c, PathPlan& p, int n_path, const double* h_q0, con
 int path_enqueue(spring_ctx* c, PathPlan& p, int delta_mode, double sigma);
 int path_fetch(spring_ctx* c, PathPlan& p, double* h_lw, double* h_omega);
 void path_release(PathPlan& p);
+void free_path_ws(spring_ctx* c);
 int path_points(const double* G, int n_nodes, const double* q_high_sym, double* qpoints, double* dist, int* zc);
 // k_mlp.cu: the surrogate network (row-major X[n][SPRING_MLP_INPUTS], y[n])
 int mlp_num_params();
