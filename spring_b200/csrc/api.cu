@@ -327,7 +327,12 @@ int spring_ctx_destroy(spring_ctx* c) {
         dfree(c->d_tr_int); dfree(c->d_tr_grid); dfree(c->d_tr_pos); dfree(c->d_tr_sgn); dfree(c->d_tr_deg);
         dfree(c->d_neg); dfree(c->d_bt_off); dfree(c->d_bt_kk); dfree(c->d_bt_pq);
         dfree(c->bte.pq); dfree(c->bte.cf); dfree(c->bte.vec); dfree(c->bte.ent);
-        dfree(c->bte.ctr); dfree(c->bte.cnt); dfree(c->bte.wf); dfree(c->bte.boff);
+        dfree(c->bte.ctr); dfree(c->bte.cnt); dfree(c->bte.wf); dfree(c->bte.ke); dfree(c->bte.tmp);
+        for (int k = 0; k < 2; ++k) {
+            dfree(c->bte.key[k]);
+            dfree(c->bte.idx[k]);
+        }
+        dfree(c->bte.boff);
         dfree(c->d_bteg_row); dfree(c->d_bteg_kk); dfree(c->d_bteg_pq);
         dfree(c->ew.g); dfree(c->ew.r); dfree(c->ew.hz); dfree(c->ew.tau); dfree(c->ew.z); dfree(c->ew.cc);
         dfree(c->ew.dd); dfree(c->d_v4_rec);

@@ -30,6 +30,7 @@
 // Roofline: FP64 ALU for the weights, HBM / L2 (24 bytes and two gathers per entry) for the iterations.
 #include <algorithm>
 #include <cmath>
+#include <cub/cub.cuh>
 
 #include "spring_internal.cuh"
 #include "tetra.cuh"
@@ -274,24 +275,25 @@ __global__ void __launch_bounds__(256) k_bte_entries(RowArgs a, int nseg, int* _
     }
 }
 
-// Sums of one block's 256 threads, valid in thread 0.
+// Sums of one block's 256 threads: thread k < NV gets v[k] summed.
 template <int NV>
-__device__ __forceinline__ void block_sum(double* v, double (*red)[8]) {
+__device__ __forceinline__ double block_sum(const double* v, double (*red)[8]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double x[NV];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        v[k] = tet::warp_sum(v[k]);
-        if (lane == 0) red[k][warp] = v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
+    for (int k = 0; k < NV; ++k) x[k] = v[k];
+    for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            double t = 0.0;
-            for (int w = 0; w < 8; ++w) t += red[k][w];
-            v[k] = t;
-        }
+        for (int k = 0; k < NV; ++k) x[k] += __shfl_down_sync(0xffffffffu, x[k], o);
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) red[k][warp] = x[k];
     __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x < NV)
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += red[threadIdx.x][w];
+    return t;
 }
 
 // Row sums straight from the (P, Q) blocks of a batch (the operator did not fit): MODE 0 1/tau, MODE 1
@@ -318,9 +320,8 @@ __global__ void __launch_bounds__(256) k_bte_dense(RowArgs a, const double* __re
         }
     }
     constexpr int NV = MODE == 0 ? 1 : 3;
-    block_sum<NV>(v, red);
-    if (threadIdx.x == 0)
-        for (int d = 0; d < NV; ++d) out[((size_t)a.q0_first * n + blockIdx.x) * NV + d] = v[d];
+    const double t = block_sum<NV>(v, red);
+    if (threadIdx.x < NV) out[((size_t)a.q0_first * n + blockIdx.x) * NV + threadIdx.x] = t;
 }
 
 struct StepArgs {
@@ -333,9 +334,11 @@ struct StepArgs {
     const double* nbe;      // at this temperature
     const double* vel;
     const double* inv_tau;
-    const double* dF;
+    const double* dF;       // [row][parts][3]
+    int parts;
     double* F0;
-    double* Fg;             // [g][s][4] F at every grid mode, padded to one 32-byte sector
+    double* F;              // [row][3], or null
+    double* Fg;             // [g][s][4] F at every grid mode, padded to one 32-byte sector, or null
     double* part;           // [blocks][9] kappa partial sums
     unsigned* ticket;       // zero between launches
     double* kappa;          // [9] of this iteration
@@ -344,7 +347,7 @@ struct StepArgs {
 // One iteration's end for every mode of the time-reversal set: F = F0 (INIT, CreateFzero:
 // F0 = FunitE w v / (1/tau T^2) where |1/tau| > zero_prec) or F0 + dF tau (multiplyTaudFnew); F at both
 // grid points of the pair (F(-q) = -F(q)); and kappa = kW_mK / (Nq V) sum deg w n (n+1) v (x) F, block
-// sums added in block order by the last block to finish.
+// sums added in a fixed order by the last block to finish.
 template <bool INIT>
 __global__ void __launch_bounds__(256) k_bte_step(StepArgs a) {
     __shared__ double red[9][8];
@@ -367,16 +370,21 @@ __global__ void __launch_bounds__(256) k_bte_step(StepArgs a) {
                 f[k] = scale ? FUNIT_E * w * v[k] / (it * (a.T * a.T)) : 0.0;
                 a.F0[(size_t)i * 3 + k] = f[k];
             } else {
-                double d = a.dF[(size_t)i * 3 + k];
+                double d = 0.0;
+                for (int h = 0; h < a.parts; ++h) d += a.dF[((size_t)i * a.parts + h) * 3 + k];
                 if (scale) d /= it;
                 f[k] = a.F0[(size_t)i * 3 + k] + d;
             }
         }
-        double2* o = reinterpret_cast<double2*>(a.Fg + 4 * ((size_t)g0 * n + s));
-        o[0] = make_double2(f[0], f[1]);
-        o[1] = make_double2(f[2], 0.0);
-        if (gn != g0) {
-            o = reinterpret_cast<double2*>(a.Fg + 4 * ((size_t)gn * n + s));
+        if (a.F)
+            for (int k = 0; k < 3; ++k) a.F[(size_t)i * 3 + k] = f[k];
+        if (a.Fg) {
+            double2* o = reinterpret_cast<double2*>(a.Fg + 4 * ((size_t)g0 * n + s));
+            o[0] = make_double2(f[0], f[1]);
+            o[1] = make_double2(f[2], 0.0);
+        }
+        if (a.Fg && gn != g0) {
+            double2* o = reinterpret_cast<double2*>(a.Fg + 4 * ((size_t)gn * n + s));
             o[0] = make_double2(-f[0], -f[1]);
             o[1] = make_double2(-f[2], 0.0);
         }
@@ -388,20 +396,22 @@ __global__ void __launch_bounds__(256) k_bte_step(StepArgs a) {
 #pragma unroll
             for (int y = 0; y < 3; ++y) acc[3 * x + y] += pre * (v[x] * f[y]);
     }
-    block_sum<9>(acc, red);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < 9; ++k) a.part[9 * (size_t)blockIdx.x + k] = acc[k];
+    const double part = block_sum<9>(acc, red);
+    if (threadIdx.x < 9) {
+        a.part[9 * (size_t)blockIdx.x + threadIdx.x] = part;
         __threadfence();
-        last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
     if (!last) return;
-    if (threadIdx.x < 9) {
-        __threadfence();
+    // at most 148 block sums: a warp per component, in a fixed order (components 0..7, then 8)
+    __threadfence();
+    for (int k = threadIdx.x >> 5; k < 9; k += 8) {
         double t = 0.0;
-        for (unsigned b = 0; b < gridDim.x; ++b) t += __ldcg(a.part + 9 * (size_t)b + threadIdx.x);
-        a.kappa[threadIdx.x] = KW_MK * (1.0 / (double(a.nq) * a.vol)) * t;
+        for (unsigned b = threadIdx.x & 31; b < gridDim.x; b += 32) t += __ldcg(a.part + 9 * (size_t)b + k);
+        t = tet::warp_sum(t);
+        if ((threadIdx.x & 31) == 0) a.kappa[k] = KW_MK * (1.0 / (double(a.nq) * a.vol)) * t;
     }
     if (threadIdx.x == 0) *a.ticket = 0;
 }
@@ -465,18 +475,27 @@ int build_tr_set(spring_ctx* c) {
 // and the minus channel at -q1 and -q2 gives (1 + n1 + n2) d(w0 - w1 - w2), each times 4 W3 and -(F1 + F2)
 // because F(-q) = -F(q).  The entries are sorted by row once and kept in HBM (CSR); an iteration is one
 // pass over them.
-// Rank of every entry within its row, in its pad word, and the entries per row.
-__global__ void k_bteg_count(long long n, s3::BteEntry* __restrict__ e, int* __restrict__ rowcnt) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        e[i].pad = atomicAdd(&rowcnt[e[i].r0], 1);
-}
-__global__ void k_bteg_scatter(long long n, const s3::BteEntry* __restrict__ e, const int* __restrict__ rowoff,
-                               int2* __restrict__ kk, double2* __restrict__ pq) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+// Sort keys (row, k1, s2): unique within an operator, so that a rebuilt one has the same order and sums to the
+// same bits however its entries were appended.
+__global__ void k_bteg_keys(long long cnt, int n, int bits, const s3::BteEntry* __restrict__ e,
+                            unsigned long long* __restrict__ key, int* __restrict__ idx) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (long long)gridDim.x * blockDim.x) {
         const s3::BteEntry x = e[i];
-        const int o = rowoff[x.r0] + x.pad;
-        kk[o] = make_int2(x.k1, x.k2);
-        pq[o] = make_double2(x.P, x.Q);
+        key[i] = ((unsigned long long)x.r0 << bits | (unsigned)x.k1) << 3 | (unsigned)(x.k2 % n);
+        idx[i] = (int)i;
+    }
+}
+// The sorted operator, and the first entry of every row (rows without entries included).
+__global__ void k_bteg_gather(long long cnt, int rows, int shift, const s3::BteEntry* __restrict__ e,
+                              const unsigned long long* __restrict__ key, const int* __restrict__ idx,
+                              int* __restrict__ rowoff, int2* __restrict__ kk, double2* __restrict__ pq) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i <= cnt; i += (long long)gridDim.x * blockDim.x) {
+        const int r = i < cnt ? (int)(key[i] >> shift) : rows, before = i > 0 ? (int)(key[i - 1] >> shift) : -1;
+        for (int k = before + 1; k <= r; ++k) rowoff[k] = (int)i;
+        if (i == cnt) continue;
+        const s3::BteEntry x = e[idx[i]];
+        kk[i] = make_int2(x.k1, x.k2);
+        pq[i] = make_double2(x.P, x.Q);
     }
 }
 
@@ -496,8 +515,8 @@ __global__ void __launch_bounds__(256) k_bteg_coef(int nseg, const int* __restri
         cf[i] = c;
         v[0] += c;
     }
-    block_sum<1>(v, red);
-    if (threadIdx.x == 0) inv_tau[blockIdx.x] = v[0];
+    const double t = block_sum<1>(v, red);
+    if (threadIdx.x == 0) inv_tau[blockIdx.x] = t;
 }
 
 // dF[r] = -sum c (Fg[k1] + Fg[k2]), one block per row (Fg: four doubles per mode, the fourth zero).
@@ -517,40 +536,93 @@ __global__ void __launch_bounds__(256) k_bteg_rows(int nseg, const int* __restri
         v[1] -= c * (u1.y + u2.y);
         v[2] -= c * (v1.x + v2.x);
     }
-    block_sum<3>(v, red);
-    if (threadIdx.x == 0)
-        for (int d = 0; d < 3; ++d) dF[3 * (size_t)blockIdx.x + d] = v[d];
+    const double t = block_sum<3>(v, red);
+    if (threadIdx.x < 3) dF[3 * (size_t)blockIdx.x + threadIdx.x] = t;
+}
+
+// (k1, k2) of every entry as modes of the time-reversal set in 16 bits each (at most 8533 rows fit the shared
+// memory), the top bit set where F changes sign.
+__global__ void k_bteg_encode(long long cnt, int n, const int2* __restrict__ kk, const int* __restrict__ pos,
+                              const int* __restrict__ sgn, unsigned* __restrict__ ke) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (long long)gridDim.x * blockDim.x) {
+        const int2 k = kk[i];
+        const int a = k.x / n, b = k.y / n;
+        const unsigned x = (pos[a] * n + k.x % n) | (sgn[a] < 0 ? 0x8000 : 0), y = (pos[b] * n + k.y % n) | (sgn[b] < 0 ? 0x8000 : 0);
+        ke[i] = x | y << 16;
+    }
+}
+
+// The same sums with F of the whole time-reversal set in shared memory (24 bytes a mode).  The two gathers of
+// an entry are what bounds k_bteg_rows - 64 bytes of L2 traffic beside 16 of operator, about 5 TB/s - and F is
+// small: 125 KB at 12^3.  One CTA per SM; a warp takes a quarter of a row, so that uneven rows spread, and
+// k_bte_step adds the quarters in order.  12^3 (3.5e6 entries): 45.7 -> 27 us per pass,
+// now bound by the bank conflicts of six random 8-byte reads an entry (more unrolling, smaller parts or blocks
+// change nothing; entries in k1 order rather than as appended: 31 -> 27).
+constexpr int ROW_PARTS = 4, RSM = 1024;
+__global__ void __launch_bounds__(RSM, 1) k_bteg_rows_sm(int rows, int nseg, const int* __restrict__ off,
+                                                          const unsigned* __restrict__ ke, const double* __restrict__ cf,
+                                                          const double* __restrict__ F, double* __restrict__ dF) {
+    extern __shared__ double sF[];
+    for (int i = threadIdx.x; i < 3 * rows; i += RSM) sF[i] = F[i];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warps = gridDim.x * (RSM / 32);
+    for (int u = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; u < rows * ROW_PARTS; u += warps) {
+        const int r = u / ROW_PARTS, part = u % ROW_PARTS;
+        const int b = off[(size_t)r * nseg], e = off[((size_t)r + 1) * nseg];
+        const int step = ((e - b + ROW_PARTS - 1) / ROW_PARTS + 31) & ~31;
+        const int i1 = min(b + (part + 1) * step, e);
+        double v0 = 0.0, v1 = 0.0, v2 = 0.0;
+#pragma unroll 4
+        for (int i = b + part * step + lane; i < i1; i += 32) {
+            const double c = cf[i];
+            const unsigned k = ke[i];
+            const double c1 = k & 0x8000u ? c : -c, c2 = k & 0x80000000u ? c : -c;
+            const double* f1 = sF + 3 * (k & 0x7fffu);
+            const double* f2 = sF + 3 * (k >> 16 & 0x7fffu);
+            v0 += c1 * f1[0] + c2 * f2[0];
+            v1 += c1 * f1[1] + c2 * f2[1];
+            v2 += c1 * f1[2] + c2 * f2[2];
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+            v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+            v2 += __shfl_xor_sync(0xffffffffu, v2, o);
+        }
+        if (lane < 3) dF[3 * (size_t)u + lane] = lane == 0 ? v0 : (lane == 1 ? v1 : v2);
+    }
 }
 
 }  // namespace
 
 namespace {
 
-// The loop of main.f90:295-361 at every temperature: tau(T) fills w.inv_tau, df(T) fills w.dF from w.Fg.
+// The loop of main.f90:295-361 at every temperature: tau(T) fills w.inv_tau, df(T) fills w.dF from w.Fg
+// (F at the grid modes) or, with several partial sums per row (`parts`), from w.F (F by rows).
 // `ahead`: iterations queued before kappa is read back and the convergence test made (iterations past
 // the converged one change no output).
 template <class Tau, class DF>
-int bte_iterate(spring_ctx* c, double eps_k, int max_iter, int ahead, Tau tau, DF df, double* h_kappa,
+int bte_iterate(spring_ctx* c, double eps_k, int max_iter, int ahead, int parts, Tau tau, DF df, double* h_kappa,
                 double* h_kappa_rta, int* h_iters) {
     const int n = c->ndof, ntr = c->ntr, nq = c->nq, rows = ntr * n;
     constexpr int MAX_AHEAD = 16;
     const int blocks = std::max(1, std::min((rows + 255) / 256, 148));
     BteWork& w = c->bte;
-    // one buffer: Fg | F0 | dF | 1/tau | kappa partial sums | kappa of the queued iterations | ticket
+    // one buffer: Fg | F0 | F | dF | 1/tau | kappa partial sums | kappa of the queued iterations | ticket
     const size_t nFg = (size_t)nq * n * 4, nF = (size_t)rows * 3;
-    SPRING_CHECK(dalloc(c, w.vec, nFg + 2 * nF + rows + (size_t)blocks * 9 + 9 * (MAX_AHEAD + 1) + 1, "BTE vectors"));
+    SPRING_CHECK(dalloc(c, w.vec, nFg + (2 + parts) * nF + rows + (size_t)blocks * 9 + 9 * (MAX_AHEAD + 1) + 1, "BTE vectors"));
     w.Fg = w.vec.p;
     w.F0 = w.Fg + nFg;
-    w.dF = w.F0 + nF;
-    w.inv_tau = w.dF + nF;
+    w.F = w.F0 + nF;
+    w.dF = w.F + nF;
+    w.inv_tau = w.dF + parts * nF;
     double* part = w.inv_tau + rows;
     double* hist = part + (size_t)blocks * 9;
     unsigned* ticket = reinterpret_cast<unsigned*>(hist + 9 * (MAX_AHEAD + 1));
     SPRING_CHECK(zero(c, ticket, sizeof(double), "BTE ticket"));
     auto step = [&](bool init, int T, int at) -> int {
         const StepArgs a{ntr, n, nq, c->vol, c->temps[T], c->d_tr_grid.p, c->d_neg.p, c->d_tr_deg.p, c->ph_grid.omega.p,
-                         c->ph_grid.nbe.p + (size_t)T * nq * n, c->ph_grid.vel.p, w.inv_tau, w.dF, w.F0, w.Fg, part,
-                         ticket, hist + 9 * at};
+                         c->ph_grid.nbe.p + (size_t)T * nq * n, c->ph_grid.vel.p, w.inv_tau, w.dF, parts, w.F0, parts > 1 ? w.F : nullptr,
+                         parts > 1 ? nullptr : w.Fg, part, ticket, hist + 9 * at};
         if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
         if (init) k_bte_step<true><<<blocks, 256, 0, c->stream>>>(a);
         else k_bte_step<false><<<blocks, 256, 0, c->stream>>>(a);
@@ -605,15 +677,34 @@ int bte_operator_run(spring_ctx* c, int rows, int nseg, const int* off, const in
                                                 w.inv_tau);
         return launch_check(c, "k_bteg_coef");
     };
+    // F in shared memory where it fits beside the block (about 14^3 for a two-atom cell) and the operator is
+    // long enough to pay for loading it into every SM
+    const size_t smem = sizeof(double) * 3 * rows;
+    const bool in_smem = smem <= 200 * 1024 && cnt >= 16 * (long long)rows;
+    int sms = 148;
+    if (in_smem) {
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+        cudaFuncSetAttribute(k_bteg_rows_sm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        SPRING_CHECK(dalloc(c, w.ke, cnt, "operator modes"));
+        if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
+        k_bteg_encode<<<(int)std::min<long long>((cnt + 255) / 256, 148LL * 16), 256, 0, c->stream>>>(
+            cnt, c->ndof, kk, c->d_tr_pos.p, c->d_tr_sgn.p, w.ke.p);
+        SPRING_CHECK(launch_check(c, "k_bteg_encode"));
+    }
     auto df = [&](int) -> int {
         if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
-        k_bteg_rows<<<rows, 256, 0, c->stream>>>(nseg, off, kk, w.cf.p, w.Fg, w.dF);
+        if (in_smem)
+            k_bteg_rows_sm<<<std::min(sms, (rows * ROW_PARTS + RSM / 32 - 1) / (RSM / 32)), RSM, smem, c->stream>>>(rows, nseg, off, w.ke.p,
+                                                                                                w.cf.p, w.F, w.dF);
+        else
+            k_bteg_rows<<<rows, 256, 0, c->stream>>>(nseg, off, kk, w.cf.p, w.Fg, w.dF);
         return launch_check(c, "k_bteg_rows<dF>");
     };
     // A pass over few entries is shorter than the wait for kappa: several are queued per readback.
-    const int rc = bte_iterate(c, eps_k, max_iter, cnt < (4 << 20) ? 8 : 1, tau, df, h_kappa, h_kappa_rta, h_iters);
+    const int rc = bte_iterate(c, eps_k, max_iter, cnt < (4 << 20) ? 8 : 1, in_smem ? ROW_PARTS : 1, tau, df, h_kappa, h_kappa_rta, h_iters);
     cudaStreamSynchronize(c->stream);
     if (w.cf.n > (8u << 20)) dfree(w.cf);  // large ones are given back
+    if (w.ke.n > (8u << 20)) dfree(w.ke);
     return rc;
 }
 
@@ -636,7 +727,6 @@ int run_bte_gauss(spring_ctx* c, double sigma, double eps_k, int max_iter, doubl
         c->bteg_n = 0;
         BteWork& w = c->bte;
         SPRING_CHECK(dalloc(c, w.ctr, 1, "operator count"));
-        SPRING_CHECK(dalloc(c, w.cnt, rows + 1, "operator rows"));
         SPRING_CHECK(dalloc(c, c->d_bteg_row, rows + 1, "operator rows"));
         constexpr long long EB = sizeof(s3::BteEntry);
         long long cap = std::max<long long>(1 << 20, npairs * 216 / 40);  // the window passes ~1-2% of the triples
@@ -661,27 +751,45 @@ int run_bte_gauss(spring_ctx* c, double sigma, double eps_k, int max_iter, doubl
         if (rc == SPRING_OK && cnt > 0x7fffffffLL) rc = fail(c, SPRING_ERR_UNSUPPORTED, "BTE operator above 2^31 entries");
         if (rc == SPRING_OK) rc = dalloc(c, c->d_bteg_kk, cnt, "BTE operator");
         if (rc == SPRING_OK) rc = dalloc(c, c->d_bteg_pq, cnt, "BTE operator");
-        if (rc == SPRING_OK) rc = zero(c, w.cnt.p, sizeof(int) * (rows + 1), "operator rows");
-        auto* ent = reinterpret_cast<s3::BteEntry*>(w.ent.p);
+        const auto* ent = reinterpret_cast<const s3::BteEntry*>(w.ent.p);
+        int bits = 1;
+        while ((1LL << bits) < (long long)nq * n) ++bits;
+        int rbits = 1;
+        while ((1 << rbits) < rows) ++rbits;
+        const int top = bits + 3 + rbits;
+        size_t tb = 0;
+        cub::DeviceRadixSort::SortPairs(nullptr, tb, (unsigned long long*)nullptr, (unsigned long long*)nullptr, (int*)nullptr,
+                                        (int*)nullptr, (int)cnt, 0, top, c->stream);
+        for (int k = 0; k < 2; ++k) {
+            if (rc == SPRING_OK) rc = dalloc(c, w.key[k], cnt, "operator keys");
+            if (rc == SPRING_OK) rc = dalloc(c, w.idx[k], cnt, "operator keys");
+        }
+        if (rc == SPRING_OK) rc = dalloc(c, w.tmp, std::max<size_t>(tb, 1), "operator sort");
+        if (rc == SPRING_OK && launch_injected(c)) rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
         if (rc == SPRING_OK && cnt > 0) {
-            if (launch_injected(c)) rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
+            k_bteg_keys<<<blocks_for(cnt), threads, 0, c->stream>>>(cnt, n, bits, ent, w.key[0].p, w.idx[0].p);
+            rc = launch_check(c, "k_bteg_keys");
             if (rc == SPRING_OK) {
-                k_bteg_count<<<blocks_for(cnt), threads, 0, c->stream>>>(cnt, ent, w.cnt.p);
-                rc = launch_check(c, "k_bteg_count");
+                const cudaError_t e = cub::DeviceRadixSort::SortPairs(w.tmp.p, tb, w.key[0].p, w.key[1].p, w.idx[0].p,
+                                                                      w.idx[1].p, (int)cnt, 0, top, c->stream);
+                c->launches += 1;
+                if (e != cudaSuccess) rc = cuda_fail(c, e, "operator sort");
             }
         }
-        if (rc == SPRING_OK) rc = run_exclusive_scan(c, w.cnt.p, c->d_bteg_row.p, rows + 1);
-        if (rc == SPRING_OK && cnt > 0) {
-            if (launch_injected(c)) rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
-            if (rc == SPRING_OK) {
-                k_bteg_scatter<<<blocks_for(cnt), threads, 0, c->stream>>>(cnt, ent, c->d_bteg_row.p, c->d_bteg_kk.p,
-                                                                          c->d_bteg_pq.p);
-                rc = launch_check(c, "k_bteg_scatter");
-            }
+        if (rc == SPRING_OK && launch_injected(c)) rc = fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
+        if (rc == SPRING_OK) {
+            k_bteg_gather<<<blocks_for(cnt + 1), threads, 0, c->stream>>>(cnt, rows, bits + 3, ent, w.key[1].p, w.idx[1].p,
+                                                                         c->d_bteg_row.p, c->d_bteg_kk.p, c->d_bteg_pq.p);
+            rc = launch_check(c, "k_bteg_gather");
         }
         if (w.ent.n > ((size_t)256 << 20)) {  // large ones are given back
             cudaStreamSynchronize(c->stream);
             dfree(w.ent);
+            for (int k = 0; k < 2; ++k) {
+                dfree(w.key[k]);
+                dfree(w.idx[k]);
+            }
+            dfree(w.tmp);
         }
         if (rc != SPRING_OK) return rc;
         c->bteg_n = cnt;
@@ -831,7 +939,7 @@ int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* 
             }
             return SPRING_OK;
         };
-        rc = bte_iterate(c, eps_k, max_iter, 1, [&](int T) { return pass(0, T); }, [&](int T) { return pass(1, T); },
+        rc = bte_iterate(c, eps_k, max_iter, 1, 1, [&](int T) { return pass(0, T); }, [&](int T) { return pass(1, T); },
                          h_kappa, h_kappa_rta, h_iters);
     }
     return rc;

@@ -91,11 +91,15 @@ struct BteWork {
     DBuf<double2> pq;          // (P, Q) grids of a batch
     DBuf<double> cf, vec;      // operator coefficients of one temperature; the vectors below
     DBuf<unsigned char> ent;   // unsorted entries of the Gaussian operator
+    DBuf<unsigned long long> key[2];  // their sort: keys, indices, scratch
+    DBuf<int> idx[2];
+    DBuf<unsigned char> tmp;
     DBuf<unsigned long long> ctr;
     DBuf<int> cnt;
     DBuf<float> wf;
     DBuf<int> boff;
-    double *Fg = nullptr, *F0 = nullptr, *dF = nullptr, *inv_tau = nullptr;
+    DBuf<unsigned> ke;             // operator modes of the time-reversal set
+    double *Fg = nullptr, *F0 = nullptr, *F = nullptr, *dF = nullptr, *inv_tau = nullptr;
 };
 
 // Point-defect scattering (spring_set_point_defect, k_pdef.cu).

@@ -46,3 +46,27 @@ def test_kappa_iter_same_without_the_stored_operator(N):
     assert np.all(one["iters"] == 1)
     np.testing.assert_allclose(one["kappa_rta"], a["kappa_rta"], rtol=1e-10, atol=1e-10 * np.abs(a["kappa_rta"]).max())
     ctx.close()
+
+
+@pytest.mark.parametrize("N", [3, 7])
+def test_kappa_iter_small_sets_without_the_stored_operator(N):
+    """F in shared memory against the sums that are not stored."""
+    cr = S.build("rocksalt2")
+    ctx, _ = from_crystal(cr, (N, N, N), [300.0])
+    a = ctx.kappa_iter(eps_k=1e-9, max_iter=5)
+    ctx.set_option(L.SPRING_OPT_BTE_ENTRIES, 10)
+    b = ctx.kappa_iter(eps_k=1e-9, max_iter=5)
+    np.testing.assert_allclose(b["kappa"], a["kappa"], rtol=1e-10, atol=1e-10 * np.abs(a["kappa"]).max())
+    ctx.close()
+
+
+def test_kappa_iter_gauss_rebuilt_operator_gives_the_same_bits():
+    """16^3: F (295 KB) does not fit shared memory, and the entries are appended in another order each time."""
+    cr = S.build("rocksalt2")
+    ctx, _ = from_crystal(cr, (16, 16, 16), [300.0])
+    a = ctx.kappa_iter_gauss(0.7534, eps_k=1e-9, max_iter=3)
+    ctx.compute_phonons([300.0])
+    b = ctx.kappa_iter_gauss(0.7534, eps_k=1e-9, max_iter=3)
+    assert a["entries"] == b["entries"] and a["iters"][0] == 4
+    np.testing.assert_array_equal(b["kappa"], a["kappa"])
+    ctx.close()
