@@ -408,33 +408,46 @@ struct T4Args {
     int pol_lo[4], pol_hi[4];
 };
 
-// Warps screen 32 tetrahedra over q2 at a time for one q1, queue the hits (tetrahedron, s1, s2, s3, channel,
-// s0) and evaluate 32 of them at a time, as in k_tetra3 (k_tetra.cu has the reasons).  The FP32 ranges of
-// w2 + w3 and w3 - w2 over a tetrahedron serve every s1: the channels shift them by w1.  The legs are not
-// folded: the reference's reading of the stored W is not symmetric in them.
-// One thread per (q1, tetrahedron, s1, s2, s3) ran every weight formula any lane of its warp needed, with 17
-// divisions per evaluation: 116.6 -> 15.3 ms at 5^3 (ten q0, one temperature).
+// One lane per tetrahedron over q2, one q1 per block.  The channels' energies are w1 + p, p - w1 and m - w1 with
+// p = w2 + w3 and m = w3 - w2, so for every (s2, s3) the lane sorts p and m once, screens the 18 (s0, channel)
+// of every s1 in FP32 against their ranges (widened by far more than the rounding) into a mask of up to 108
+// bits, and, when the warp has a hit, forms the six reciprocals of each set once: about 7 % of the checks hit
+// (6^3), 7 per (tetrahedron, s2, s3), all of which use them.  The hits of the 32 tetrahedra are queued and
+// evaluated 32 at a time (each lane working off its own mask instead idles behind the busiest one: 16.6 ms);
+// what an evaluation reads of its tetrahedron (sorted energies, reciprocals, occupation products, W offsets)
+// lies in that lane's shared-memory column.
+// Vertex energies closer than 1e-5 of their magnitude (a tetrahedron that holds both legs of a pair, the
+// resonances w0 + w1 -> w0 + w1) are the exception: there the rounding of (w1 + w2) + w3 decides between the
+// cases, so such hits form, sort and weight the channel's own energies.
+// The legs are not folded: the reference's reading of the stored W is not symmetric in them.
+// One temperature: 5^3, ten q0 116.6 -> 5.8 ms, 6^3, sixteen 546 -> 25 ms against one thread per (q1, tetrahedron,
+// s1, s2, s3) that ran every formula any lane of its warp needed; 15.3 and 45 ms with each hit sorting its own
+// energies and taking its own reciprocals.  Bound by issue (IPC 1.75) and the latency of the W reads.
 constexpr int T4W = 4;  // warps per block
 
 template <int NT>
 struct T4Smem {
-    double acc[T4W][N * NT][32];           // per-lane sums [s0][T]
-    unsigned queue[T4W][32 * 18 + 32];
-    float w23[T4W][2][N][4][32];           // w(q2, s2), w(q3, s3) of the lane's tetrahedron
-    int v2[T4W][4][32], v3[T4W][4][32], pos[T4W][4][32], typ[T4W][32];  // its vertices and their quartets
-    float w0m[N][8], w0p[N][8];            // w0 - w1, w0 + w1 by s1 ([..][s0], two values of padding)
+    double acc[T4W][N * NT][32];        // per-lane sums [s0][T]
+    double val[T4W][2][10][32];         // p, m sets: sorted energies; 1/(30), (10), (21), (32), (20), (31)
+    double nf[T4W][2][NT][4][32];       // n2 n3 and (1 + n2) n3 by vertex
+    int off[T4W][4][32];                // by vertex: W offset of (s2, s3) | stride of s1 << 8
+    int pos[T4W][4][32], v2[T4W][4][32], v3[T4W][4][32];  // quartet and points of each vertex
+    int rank[T4W][2][32];               // vertices by rank, two bits each; 256: well separated
+    unsigned short queue[T4W][32 * 6 * 3 * N];  // lane | check << 5
+    double w0m[N][N], w0p[N][N];        // w0 - w1, w0 + w1 [s1][s0]
+    float f0m[N][8], f0p[N][8];         // the same in FP32 (two values of padding)
+    double fac[NT][2][N][N];            // n1 / n0 / 6, (1 + n1) / n0 / 2 [T][.][s1][s0]
     double w0[N];
 };
 
 template <int NT>
-__global__ void __launch_bounds__(32 * T4W, 3) k_tetra4(T4Args a, int per1, int nb1, const int4* __restrict__ tet,
+__global__ void __launch_bounds__(32 * T4W, 3) k_tetra4(T4Args a, int per2, int nb2, const int4* __restrict__ tet,
                                                         const int* __restrict__ all, const double* __restrict__ Wq,
                                                         const int* __restrict__ q0int, const double* __restrict__ om0,
                                                         const double* __restrict__ nbe0, const double* __restrict__ omg,
                                                         const double* __restrict__ nbeg, double* __restrict__ out) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T4Smem<NT>& S = *reinterpret_cast<T4Smem<NT>*>(smem_raw);
-    constexpr int K = 3 * N;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool gq0 = q0int[0] == 0 && q0int[1] == 0 && q0int[2] == 0;
     const int s0a = gq0 ? 3 : a.pol_lo[0], s0e = a.pol_hi[0];
@@ -442,125 +455,86 @@ __global__ void __launch_bounds__(32 * T4W, 3) k_tetra4(T4Args a, int per1, int 
     if (threadIdx.x < N) S.w0[threadIdx.x] = om0[threadIdx.x];
     unsigned live = 0;
 #pragma unroll
-    for (int k = 0; k < K; ++k)
-        if (k % N >= s0a && k % N <= s0e) live |= 1u << (K - 1 - k);
+    for (int k = 0; k < 3 * N; ++k)
+        if (k % N >= s0a && k % N <= s0e) live |= 1u << (3 * N - 1 - k);
     const int groups = (a.ntet + 31) / 32;
-    unsigned* queue = S.queue[warp];
     double(*acc)[32] = S.acc[warp];
-    // blockIdx.y: q1 (strided); the block's warps share it
     for (int q1 = blockIdx.y; q1 < a.nq; q1 += gridDim.y) {
         __syncthreads();
-        if (threadIdx.x < N * N) {
-            const int s1 = threadIdx.x / N, s0 = threadIdx.x % N;
-            const float w0 = (float)S.w0[s0], w1 = (float)omg[(size_t)q1 * N + s1];
+        for (int i = threadIdx.x; i < N * N; i += blockDim.x) {
+            const int s1 = i / N, s0 = i % N;
+            const double w0 = S.w0[s0], w1 = omg[(size_t)q1 * N + s1];
             S.w0m[s1][s0] = w0 - w1;
             S.w0p[s1][s0] = w0 + w1;
+            S.f0m[s1][s0] = (float)(w0 - w1);
+            S.f0p[s1][s0] = (float)(w0 + w1);
+            for (int T = 0; T < a.nT; ++T) {
+                const double n1 = nbeg[((size_t)T * a.nq + q1) * N + s1], n0 = nbe0[(size_t)T * a.nq0 * N + s0];
+                S.fac[T][0][s1][s0] = ONEBYSIX * (n1 / n0);
+                S.fac[T][1][s1][s0] = 0.5 * ((1.0 + n1) / n0);
+            }
         }
         __syncthreads();
-        for (int u = blockIdx.x * T4W + warp; u < groups * nb1; u += gridDim.x * T4W) {
-            const int g = u / nb1;
-            const int s1a = a.pol_lo[1] + u % nb1 * per1, s1e = min(s1a + per1 - 1, a.pol_hi[1]);
-            const int t = g * 32 + lane;
+        for (int u = blockIdx.x * T4W + warp; u < groups * nb2; u += gridDim.x * T4W) {
+            const int t = u / nb2 * 32 + lane;
+            const int s2a = a.pol_lo[2] + u % nb2 * per2, s2e = min(s2a + per2 - 1, a.pol_hi[2]);
             bool on = t < a.ntet;
-            __syncwarp();
-            if (on) {
-                const int4 tv = tet[t];
-                const int v2[4] = {tv.x, tv.y, tv.z, tv.w};
-                int typ = 0;
+            const int4 tv = on ? tet[t] : make_int4(0, 0, 0, 0);
+            const int v2[4] = {tv.x, tv.y, tv.z, tv.w};
+            int v3[4], cst[4];  // cst: strides of s1, s2, s3 in W
 #pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const int* e = all + 3 * ((size_t)q1 * a.nq + v2[v]);
-                    const int ty = e[0], ps = e[1] - 1, v3 = e[2] - 1;
-                    // every cell is written by the enumeration; an unwritten one is skipped, not read
-                    const bool ok = ty >= 0 && ty <= 5 && ps >= 0 && ps < a.nquart && v3 >= 0 && v3 < a.nq;
-                    on = on && ok;
-                    S.v2[warp][v][lane] = v2[v];
-                    S.v3[warp][v][lane] = ok ? v3 : 0;
-                    S.pos[warp][v][lane] = ps;
-                    typ |= ty << (4 * v);
-#pragma unroll
-                    for (int s = 0; s < N; ++s) {
-                        S.w23[warp][0][s][v][lane] = (float)omg[(size_t)v2[v] * N + s];
-                        S.w23[warp][1][s][v][lane] = (float)omg[(size_t)(ok ? v3 : 0) * N + s];
-                    }
-                }
-                S.typ[warp][lane] = typ;
+            for (int v = 0; v < 4; ++v) {
+                const int* e = all + 3 * ((size_t)q1 * a.nq + v2[v]);
+                const int ty = on ? e[0] : 0, ps = on ? e[1] - 1 : 0;
+                v3[v] = on ? e[2] - 1 : 0;
+                // every cell is written by the enumeration; an unwritten one is skipped, not read
+                const bool ok = ty >= 0 && ty <= 5 && ps >= 0 && ps < a.nquart && v3[v] >= 0 && v3[v] < a.nq;
+                on = on && ok;
+                if (!ok) v3[v] = 0;
+                S.pos[warp][v][lane] = ps;
+                S.v2[warp][v][lane] = v2[v];
+                S.v3[warp][v][lane] = v3[v];
+                // modes of the stored quartet read through the reference's permutation
+                // 0: 123, 1: 132, 2: 213, 3: 231, 4: 312, 5: 321
+                const int c1 = ty < 2 ? 36 : (ty == 2 || ty == 4 ? 6 : 1);
+                const int c2 = ty == 2 || ty == 3 ? 36 : (ty == 0 || ty == 5 ? 6 : 1);
+                cst[v] = c1 | c2 << 8 | (43 - c1 - c2) << 16;
             }
-            __syncwarp();
-            // FP64 evaluation of a hit: lane of the tetrahedron | s1 | s2 | s3 | check
-            auto evaluate = [&](unsigned code) {
-                const int tl = code & 31, s1 = (code >> 5) & 7, s2 = (code >> 8) & 7, s3 = (code >> 11) & 7;
-                const int k = K - 1 - (int)(code >> 14), ch = k / N, s0 = k % N;
-                const double w1 = omg[(size_t)q1 * N + s1];
-                double M[4];
-                int vs[4] = {0, 1, 2, 3}, unused[4] = {0, 0, 0, 0};
+            for (int s2 = s2a; s2 <= s2e; ++s2) {
+                double w2[4];
 #pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const double w2 = omg[(size_t)S.v2[warp][v][tl] * N + s2], w3 = omg[(size_t)S.v3[warp][v][tl] * N + s3];
-                    M[v] = ch == 0 ? w1 + w2 + w3 : (ch == 1 ? w2 + w3 - w1 : w3 - w1 - w2);
-                }
-                tet::sort4_carry(M, vs, unused);
-                double gw, A[4];
-                if (!tet::g_weights<false>(S.w0[s0], M, gw, A)) return;
-                const double wt = ch == 0 ? ONEBYSIX : 0.5;
-                const int typ = S.typ[warp][tl];
-                size_t o2[4], o3[4];
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const int q = vs[v], ty = (typ >> (4 * q)) & 7;
-                    // modes of the stored quartet read through the reference's permutation
-                    // 0: 123, 1: 132, 2: 213, 3: 231, 4: 312, 5: 321
-                    const int m1 = ty < 2 ? s1 : (ty < 4 ? s2 : s3);
-                    const int m2 = ty == 0 || ty == 5 ? s2 : (ty == 1 || ty == 3 ? s3 : s1);
-                    const int m3 = s1 + s2 + s3 - m1 - m2;
-                    const double W = Wq[(size_t)S.pos[warp][q][tl] * 1296 + s0 * 216 + (m1 * N + m2) * N + m3];
-                    A[v] = isnan(A[v]) ? 0.0 : wt * A[v] * W;
-                    o2[v] = (size_t)S.v2[warp][q][tl] * N + s2;
-                    o3[v] = (size_t)S.v3[warp][q][tl] * N + s3;
-                }
-                for (int T = 0; T < a.nT; ++T) {
-                    const double* nb = nbeg + (size_t)T * a.nq * N;
-                    const double n1 = nb[(size_t)q1 * N + s1], n0 = nbe0[(size_t)T * a.nq0 * N + s0];
-                    const double f1 = ch == 0 ? n1 : 1.0 + n1, one = ch == 2 ? 1.0 : 0.0;
-                    double sum = 0.0;
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) sum = fma(A[v], f1 * (one + nb[o2[v]]) * nb[o3[v]], sum);
-                    acc[s0 * NT + T][lane] += sum / n0;
-                }
-            };
-            int qn = 0;
-            for (int s2 = a.pol_lo[2]; s2 <= a.pol_hi[2]; ++s2) {
-                float b2[4], e2 = 0.0f;
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    b2[v] = S.w23[warp][0][s2][v][lane];
-                    e2 += fabsf(b2[v]);
-                }
+                for (int v = 0; v < 4; ++v) w2[v] = omg[(size_t)v2[v] * N + s2];
                 for (int s3 = a.pol_lo[3]; s3 <= a.pol_hi[3]; ++s3) {
-                    float pl = 0.0f, ph = 0.0f, ml = 0.0f, mh = 0.0f, e3 = e2;
+                    double p[4], m[4];
+                    int ip[4] = {0, 1, 2, 3}, im[4] = {0, 1, 2, 3}, unused[4] = {0, 0, 0, 0};
+                    float mag = 0.0f;
 #pragma unroll
                     for (int v = 0; v < 4; ++v) {
-                        const float c = S.w23[warp][1][s3][v][lane], p = b2[v] + c, m = c - b2[v];
-                        e3 += fabsf(c);
-                        pl = v ? fminf(pl, p) : p;
-                        ph = v ? fmaxf(ph, p) : p;
-                        ml = v ? fminf(ml, m) : m;
-                        mh = v ? fmaxf(mh, m) : m;
+                        const double w3 = omg[(size_t)v3[v] * N + s3];
+                        p[v] = w2[v] + w3;
+                        m[v] = w3 - w2[v];
+                        mag += (float)fmax(fabs(p[v]), fabs(m[v]));
                     }
+                    tet::sort4_carry(p, ip, unused);
+                    tet::sort4_carry(m, im, unused);
+                    // screen: one bit per check, set outside
+                    const float pl = (float)p[0], ph = (float)p[3], ml = (float)m[0], mh = (float)m[3];
                     const float pm = 0.5f * (pl + ph), mm = 0.5f * (ml + mh);
                     const float pr = 0.5f * (ph - pl), mr = 0.5f * (mh - ml);
-#pragma unroll 1
-                    for (int s1 = s1a; s1 <= s1e; ++s1) {
-                        unsigned o = 0;  // one bit per check, set outside
+                    unsigned long long hit[2] = {0, 0};
+#pragma unroll
+                    for (int s1 = 0; s1 < N; ++s1) {
+                        if (s1 < a.pol_lo[1] || s1 > a.pol_hi[1]) continue;
+                        unsigned o = 0;
                         // FP32 rounding of the energies is below 4e-7 of the sum of magnitudes
-                        // (|w1| and |w0| are at most |w0 - w1| + |w0 + w1|)
-                        const float marg = 1e-6f * (e3 + fabsf(S.w0m[s1][0]) + fabsf(S.w0p[s1][0]));
+                        // (|w1| and |w0| are at most |w0 - w1| + |w0 + w1|; a NaN leaves every check open)
+                        const float marg = 1e-6f * (mag + fabsf(S.f0m[s1][0]) + fabsf(S.f0p[s1][0]));
                         const float hp = pr + marg, hm = mr + marg;
                         float wm[N], wp[N];
 #pragma unroll
                         for (int i = 0; i < N; ++i) {
-                            wm[i] = S.w0m[s1][i];
-                            wp[i] = S.w0p[s1][i];
+                            wm[i] = S.f0m[s1][i];
+                            wp[i] = S.f0p[s1][i];
                         }
 #pragma unroll
                         for (int i = 0; i < N; ++i) o = __funnelshift_l(__float_as_uint(hp - fabsf(wm[i] - pm)), o, 1);
@@ -568,36 +542,125 @@ __global__ void __launch_bounds__(32 * T4W, 3) k_tetra4(T4Args a, int per1, int 
                         for (int i = 0; i < N; ++i) o = __funnelshift_l(__float_as_uint(hp - fabsf(wp[i] - pm)), o, 1);
 #pragma unroll
                         for (int i = 0; i < N; ++i) o = __funnelshift_l(__float_as_uint(hm - fabsf(wp[i] - mm)), o, 1);
-                        unsigned in = on ? ~o & live : 0u;
-                        const unsigned c = __popc(in);
-                        unsigned pre = 0, tot = 0;
-                        const unsigned lt = (1u << lane) - 1;
-#pragma unroll
-                        for (int b = 0; b < 5; ++b) {
-                            const unsigned m = __ballot_sync(0xffffffffu, (c >> b) & 1);
-                            pre += __popc(m & lt) << b;
-                            tot += __popc(m) << b;
-                        }
-                        if (tot == 0) continue;
-                        const unsigned base = lane | s1 << 5 | s2 << 8 | s3 << 11;
-                        unsigned pos = qn + pre;
-                        while (in) {
-                            const int b = __ffs(in) - 1;
-                            in &= in - 1;
-                            queue[pos++] = base | b << 14;
-                        }
-                        qn += tot;
-                        __syncwarp();
-                        while (qn >= 32) {
-                            qn -= 32;
-                            evaluate(queue[qn + lane]);
-                        }
-                        __syncwarp();
+                        if (on) hit[s1 / 3] |= (unsigned long long)(~o & live) << (18 * (s1 % 3));
                     }
+                    if (!__any_sync(0xffffffffu, (hit[0] | hit[1]) != 0)) continue;
+                    const double gap = 1e-5 * (double)mag;  // false for a NaN too
+                    const bool sp = p[1] - p[0] > gap && p[2] - p[1] > gap && p[3] - p[2] > gap;
+                    const bool sm = m[1] - m[0] > gap && m[2] - m[1] > gap && m[3] - m[2] > gap;
+                    S.rank[warp][0][lane] = ip[0] | ip[1] << 2 | ip[2] << 4 | ip[3] << 6 | sp << 8;
+                    S.rank[warp][1][lane] = im[0] | im[1] << 2 | im[2] << 4 | im[3] << 6 | sm << 8;
+#pragma unroll
+                    for (int v = 0; v < 4; ++v)
+                        S.off[warp][v][lane] = (s2 * (cst[v] >> 8 & 255) + s3 * (cst[v] >> 16)) | (cst[v] & 255) << 8;
+#pragma unroll
+                    for (int set = 0; set < 2; ++set) {
+                        const double* e = set ? m : p;
+                        double(*V)[32] = S.val[warp][set];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) V[k][lane] = e[k];
+                        V[4][lane] = 1.0 / (e[3] - e[0]);
+                        V[5][lane] = 1.0 / (e[1] - e[0]);
+                        V[6][lane] = 1.0 / (e[2] - e[1]);
+                        V[7][lane] = 1.0 / (e[3] - e[2]);
+                        V[8][lane] = 1.0 / (e[2] - e[0]);
+                        V[9][lane] = 1.0 / (e[3] - e[1]);
+                    }
+#pragma unroll 1
+                    for (int T = 0; T < a.nT; ++T) {
+                        const double* nb = nbeg + (size_t)T * a.nq * N;
+#pragma unroll
+                        for (int v = 0; v < 4; ++v) {
+                            const double n2 = nb[(size_t)v2[v] * N + s2], n3 = nb[(size_t)v3[v] * N + s3];
+                            S.nf[warp][0][T][v][lane] = n2 * n3;
+                            S.nf[warp][1][T][v][lane] = (1.0 + n2) * n3;
+                        }
+                    }
+                    const int c = __popcll(hit[0]) + __popcll(hit[1]);
+                    int before = 0, tot = 0;
+                    const unsigned lt = (1u << lane) - 1;
+#pragma unroll
+                    for (int b = 0; b < 7; ++b) {
+                        const unsigned bal = __ballot_sync(0xffffffffu, (c >> b) & 1);
+                        before += __popc(bal & lt) << b;
+                        tot += __popc(bal) << b;
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        for (unsigned long long in = hit[h]; in; in &= in - 1)
+                            S.queue[warp][before++] = (unsigned short)(lane | (54 * h + __ffsll((long long)in) - 1) << 5);
+                    __syncwarp();
+                    for (int i = lane; i < tot; i += 32) {
+                        const unsigned code = S.queue[warp][i];
+                        const int tl = code & 31, bit = code >> 5, s1 = bit / 18, k = 17 - (bit - 18 * s1);
+                        const int ch = k >= 12 ? 2 : (k >= 6 ? 1 : 0), s0 = k - 6 * ch, set = ch >> 1;
+                        const int rk = S.rank[warp][set][tl];
+                        double A[4];
+                        int vs[4];  // vertex of each weight
+                        if (!(rk & 256)) {
+                            double M[4];
+                            const double w1 = omg[(size_t)q1 * N + s1];
+                            int none[4] = {0, 0, 0, 0};
+#pragma unroll
+                            for (int v = 0; v < 4; ++v) {
+                                const double y = omg[(size_t)S.v2[warp][v][tl] * N + s2], w3 = omg[(size_t)S.v3[warp][v][tl] * N + s3];
+                                M[v] = ch == 0 ? w1 + y + w3 : (ch == 1 ? y + w3 - w1 : w3 - w1 - y);
+                                vs[v] = v;
+                            }
+                            tet::sort4_carry(M, vs, none);
+                            double gw;
+                            if (!tet::g_weights<false>(S.w0[s0], M, gw, A)) continue;
+                        } else {
+                            const double(*V)[32] = S.val[warp][set];
+                            const double x = ch == 0 ? S.w0m[s1][s0] : S.w0p[s1][s0];
+                            const double e0 = V[0][tl], e1 = V[1][tl], e2 = V[2][tl], e3 = V[3][tl];
+                            const double t0 = x - e0, t1 = x - e1, t2 = x - e2, t3 = x - e3;
+                            const bool c1 = x >= e0 && x < e1, c2 = x >= e1 && x < e2, c3 = x >= e2 && x <= e3;
+                            if (!(c1 || c2 || c3)) continue;
+                            // the weights of tet::g_weights from the set's reciprocals
+                            const double r30 = V[4][tl], ra = V[c1 ? 5 : (c2 ? 6 : 7)][tl], rb = V[c3 ? 9 : 8][tl];
+                            if (c2) {
+                                const double rc = V[9][tl];
+                                const double uu = t0 * rb, ww = t2 * rb, y = t1 * rc, z = t3 * rc;
+                                const double hh = -(uu * t2 + y * t3), hr = hh * r30, ha = hh * ra;
+                                const double kf = ra * r30 * ONEBYSIX;
+                                A[0] = kf * (t0 * (ww * ww) - t3 * hr);
+                                A[1] = kf * (t1 * (z * z) - t2 * ha);
+                                A[2] = kf * (t1 * ha - t2 * (uu * uu));
+                                A[3] = kf * (t0 * hr - t3 * (y * y));
+                            } else {
+                                const double tt = c1 ? t0 : t3;
+                                const double kf = (tt * tt) * (ra * rb * r30) * ONEBYSIX;
+                                const double far = (c1 ? t3 : t0) * r30;
+                                const double kt = c1 ? kf * tt : -kf * tt;
+                                const double near = c1 ? -kf * (t1 * ra + t2 * rb + far) : kf * (far + t1 * rb + t2 * ra);
+                                A[0] = c1 ? near : kt * r30;
+                                A[1] = c1 ? kt * ra : kt * rb;
+                                A[2] = c1 ? kt * rb : kt * ra;
+                                A[3] = c1 ? kt * r30 : near;
+                            }
+#pragma unroll
+                            for (int r = 0; r < 4; ++r) vs[r] = rk >> (2 * r) & 3;
+                        }
+                        const double* Ws = Wq + s0 * 216;
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            const int o = S.off[warp][vs[r]][tl];
+                            const double W = Ws[(size_t)S.pos[warp][vs[r]][tl] * 1296 + (o & 255) + s1 * (o >> 8)];
+                            A[r] = isnan(A[r]) ? 0.0 : A[r] * W;  // undefined weights count as zero
+                        }
+#pragma unroll
+                        for (int T = 0; T < NT; ++T) {
+                            if (T >= a.nT) break;
+                            double sum = 0.0;
+#pragma unroll
+                            for (int r = 0; r < 4; ++r) sum = fma(A[r], S.nf[warp][set][T][vs[r]][tl], sum);
+                            acc[s0 * NT + T][lane] += sum * S.fac[T][ch ? 1 : 0][s1][s0];
+                        }
+                    }
+                    __syncwarp();
                 }
             }
-            if (lane < qn) evaluate(queue[lane]);
-            __syncwarp();
         }
     }
     __syncthreads();
@@ -614,15 +677,16 @@ __global__ void __launch_bounds__(32 * T4W, 3) k_tetra4(T4Args a, int per1, int 
 template <int NT>
 int launch_tetra4(spring_ctx* c, const T4Args& t, const int* all, const double* wq, const int* q0i, const double* om0,
                   const double* nbe0, double* d_rate) {
-    const int n1 = t.pol_hi[1] - t.pol_lo[1] + 1, groups = (t.ntet + 31) / 32;
-    int per1 = 6;  // as in k_tetra3: shorter units while the chip is not full
-    while (per1 > 1 && (long long)t.nq * groups * ((n1 + per1 - 1) / per1) < 148LL * 24) --per1;
-    const int nb1 = (n1 + per1 - 1) / per1;
-    const int gy = std::min(t.nq, 148 * 3), gx = std::max(1, std::min((groups * nb1 + T4W - 1) / T4W, (148 * 6 + gy - 1) / gy));
+    const int n2 = t.pol_hi[2] - t.pol_lo[2] + 1, groups = (t.ntet + 31) / 32;
+    int per2 = 6;  // shorter units (of s2) while the chip is not full
+    while (per2 > 1 && (long long)t.nq * groups * ((n2 + per2 - 1) / per2) < 148LL * 192) --per2;
+    const int nb2 = (n2 + per2 - 1) / per2;
+    // one unit a warp: the blocks of a q1 end together and the scheduler evens out the rest
+    const int gy = std::min(t.nq, 65535), gx = (groups * nb2 + T4W - 1) / T4W;
     const size_t smem = sizeof(T4Smem<NT>);
     cudaFuncSetAttribute(k_tetra4<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "tetra4: injected launch failure");
-    k_tetra4<NT><<<dim3(gx, gy), 32 * T4W, smem, c->stream>>>(t, per1, nb1, reinterpret_cast<const int4*>(c->d_tetra.p), all,
+    k_tetra4<NT><<<dim3(gx, gy), 32 * T4W, smem, c->stream>>>(t, per2, nb2, reinterpret_cast<const int4*>(c->d_tetra.p), all,
                                                               wq, q0i, om0, nbe0, c->ph_grid.omega.p, c->ph_grid.nbe.p,
                                                               d_rate);
     return launch_check(c, "k_tetra4");
@@ -650,20 +714,16 @@ int enumerate4(spring_ctx* c, int q0, Enum4Bufs& b, bool want_all, int* d_perm, 
     k_enum4_flags<<<blocks, threads, 0, c->stream>>>(c->nq, m, q0v, c->d_qint.p, b.g3.p, b.rep.p);
     SPRING_CHECK(launch_check(c, "k_enum4_flags"));
     SPRING_CHECK(run_exclusive_scan(c, b.rep.p, b.pos.p, (int)tot));
-    int last[2];
-    SPRING_CHECK(d2h(c, &last[0], b.pos.p + tot - 1, sizeof(int), "quartet count"));
-    SPRING_CHECK(d2h(c, &last[1], b.rep.p + tot - 1, sizeof(int), "quartet count"));
-    const long long nquart = (long long)last[0] + last[1];
+    int last = 0;
+    SPRING_CHECK(d2h_sum2(c, b.pos.p + tot - 1, b.rep.p + tot - 1, &last, "quartet count"));
+    const long long nquart = last;
     SPRING_CHECK(dalloc(c, b.quart, std::max<long long>(nquart, 1), "quartet list"));
     SPRING_CHECK(zero(c, b.total.p, sizeof(unsigned long long), "quartet count"));
     if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "enumerate4: injected launch failure");
     k_enum4_write<<<blocks, threads, 0, c->stream>>>(c->nq, m, q0v, c->d_qint.p, b.g3.p, b.rep.p, b.pos.p,
                                                      want_all ? b.all.p : nullptr, d_perm, cap, b.quart.p, b.total.p);
     SPRING_CHECK(launch_check(c, "k_enum4_write"));
-    unsigned long long total = 0;
-    SPRING_CHECK(d2h(c, &total, b.total.p, sizeof total, "quartet total"));
     h_counts[0] = nquart;
-    h_counts[1] = (long long)total;
     return SPRING_OK;
 }
 
@@ -676,6 +736,9 @@ void free4(Enum4Bufs& b) {
 int run_enumerate4_fortran(spring_ctx* c, int q0, int* d_all, int* d_perm, long long cap, long long* h_counts) {
     Enum4Bufs b;
     int rc = enumerate4(c, q0, b, d_all != nullptr, d_perm, cap, h_counts);
+    unsigned long long total = 0;
+    if (rc == SPRING_OK) rc = d2h(c, &total, b.total.p, sizeof total, "quartet total");
+    h_counts[1] = (long long)total;
     if (rc == SPRING_OK && d_all) {
         const size_t bytes = sizeof(int) * 3 * (size_t)c->nq * c->nq;
         cudaError_t e = cudaMemcpyAsync(d_all, b.all.p, bytes, cudaMemcpyDeviceToDevice, c->stream);
@@ -724,8 +787,10 @@ int run_lw4(spring_ctx* c, int q0_first, int n_q0, int delta_mode, double sigma,
     const size_t smem = sizeof(V4Smem);
     cudaFuncSetAttribute(k_v4<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaFuncSetAttribute(k_v4<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    Enum4Bufs b;
-    DBuf<double> wq;
+    // quartet lists and (up to 512 MB) their W stay with the context
+    if (!c->e4) c->e4 = new Enum4Bufs();
+    Enum4Bufs& b = *static_cast<Enum4Bufs*>(c->e4);
+    DBuf<double>& wq = c->d_w4;
     int rc = SPRING_OK;
     for (int q0 = q0_first; rc == SPRING_OK && q0 < q0_first + n_q0; ++q0) {
         long long cnt[2];
@@ -751,7 +816,7 @@ int run_lw4(spring_ctx* c, int q0_first, int n_q0, int delta_mode, double sigma,
             size_t free_b = 0, total_b = 0;
             cudaMemGetInfo(&free_b, &total_b);
             const size_t need = (size_t)a.nquart * 1296 * sizeof(double);
-            if (need > free_b / 2) {
+            if (need > (free_b + wq.n * sizeof(double)) / 2) {
                 rc = fail(c, SPRING_ERR_UNSUPPORTED, "tetrahedron four-phonon W of one q0 needs %zu bytes", need);
                 break;
             }
@@ -779,8 +844,8 @@ int run_lw4(spring_ctx* c, int q0_first, int n_q0, int delta_mode, double sigma,
         }
     }
     cudaStreamSynchronize(c->stream);
-    free4(b);
-    dfree(wq);
+    if (wq.n * sizeof(double) > ((size_t)512 << 20)) dfree(wq);
+    if ((size_t)c->nq * c->nq > ((size_t)64 << 20)) free4(b);
     return rc;
 }
 

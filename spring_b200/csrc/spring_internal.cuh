@@ -227,6 +227,7 @@ struct spring_ctx {
     long long bt_n = 0;
     int bt_gen = -1, bt_pairs = -1;
     spring::BteWork bte;
+    spring::DBuf<double> d_w4;      // four-phonon W of one q0's quartets (tetrahedron form)
     spring::DBuf<double> d_v4_rec;  // V4 tensor-core mode records (omega, 1/omega, n(T))
     spring::EwaldDev ew;
     spring::PointDefectDev pd;
