@@ -15,9 +15,12 @@
 // phase, so its Born-charge-folded terms HZ_R are precomputed on the host (host/ewald.hpp) and the
 // kernel forms sum_R e^{iqR} HZ_R and sum_R iR e^{iqR} HZ_R.  The reciprocal-space sum is staged in
 // shared memory 64 G-vectors at a time (K = G + q, exp(-K.eps.K / 4 Lmb^2) / K.eps.K, the
-// derivative factors and e^{iK.tau_mu} per atom), and each thread accumulates one (nu, mu, a, b)
+// derivative factors and e^{iK.tau_mu} per atom), and each thread accumulates one (nu, mu, a <= b)
 // entry and its three derivatives over its share of the chunk; the Born charges are applied once
 // per q after the sum (CombineZStar is linear).  FP64 throughout.
+// FP64 ALU bound: about 38 operations per (G, nu, mu, a <= b), 8 per (R, entry) with the phases' products
+// staged and two of D and its derivatives per thread.  Eight atoms, 295 points, 125 G and 125 R: 648 -> 150
+// us (two atoms 92 -> 46) against 128 threads, all nine (a, b) and one output at a time.
 // Output dd[item][0][row][col] = D_ew, dd[item][1 + k][row][col] = dD_ew/dq_k.
 #include <algorithm>
 #include <string>
@@ -28,7 +31,8 @@
 namespace spring {
 namespace {
 
-constexpr int EW_THREADS = 128;
+constexpr int EW_THREADS = 384;  // at most; two CTAs of them per SM
+constexpr int EW_SPLIT = 128;    // small cells: the G sum in EW_SPLIT / E shares
 constexpr int GC = 64;   // G-vectors per staged chunk
 constexpr int RC = 128;  // R-points per staged chunk
 
@@ -49,9 +53,9 @@ struct EwArgs {
 struct EwSmem {
     double2* raw;   // [J][4][E]
     double2* comb;  // [4][E]
-    double* gs;     // [GC][8]: K, KG, KpLmb, epsK
+    double* gs;     // [GC][8]: K, KG, epsK KpLmb
     double2* ph;    // [GC][nb]: e^{i K.tau_mu}
-    double2* rph;   // [RC]: e^{i q.R}
+    double2* rph;   // [RC][4]: e^{i q.R}, i R_k e^{i q.R}
 };
 
 __device__ __forceinline__ void decode(int e, int nb, int& b, int& al, int& nu, int& mu) {
@@ -64,7 +68,7 @@ __device__ __forceinline__ void decode(int e, int nb, int& b, int& al, int& nu, 
 // D_ew(q) (and, with grad, its three derivatives) into comb[k][e], e in the (b, a, nu, mu) order,
 // already scaled: comb = eV_A2 (CqZ) / sqrt(m m).  Every thread of the CTA calls it.
 __device__ void ew_eval(const EwArgs& a, const double q[3], bool grad, const EwSmem& S) {
-    const int tid = threadIdx.x, T = blockDim.x, E = a.E, J = a.J, nc = grad ? 4 : 1;
+    const int tid = threadIdx.x, T = blockDim.x, E = a.E, J = a.J, nb2 = a.nb * a.nb, nc = grad ? 4 : 1;
     for (int w = tid; w < J * 4 * E; w += T) S.raw[w] = make_double2(0.0, 0.0);
     const bool qnz = fabs(q[0]) > CMP_PREC || fabs(q[1]) > CMP_PREC || fabs(q[2]) > CMP_PREC;
     for (int g0 = 0; g0 < a.ng; g0 += GC) {
@@ -76,7 +80,6 @@ __device__ void ew_eval(const EwArgs& a, const double q[3], bool grad, const EwS
             const bool use = qnz || fabs(G[0]) > CMP_PREC || fabs(G[1]) > CMP_PREC || fabs(G[2]) > CMP_PREC;
             if (!use) {
                 for (int k = 0; k < 8; ++k) s[k] = 0.0;
-                for (int mu = 0; mu < a.nb; ++mu) S.ph[i * a.nb + mu] = make_double2(0.0, 0.0);
                 continue;
             }
             const double K[3] = {G[0] + q[0], G[1] + q[1], G[2] + q[2]};
@@ -87,77 +90,93 @@ __device__ void ew_eval(const EwArgs& a, const double q[3], bool grad, const EwS
             s[1] = K[1];
             s[2] = K[2];
             s[3] = exp(-KeK * a.inv4l2) / KeK;
-            s[4] = 1.0 / KeK + a.q4;
-            for (int ii = 0; ii < 3; ++ii)  // dot(eps(:, ii), K) + dot(K, eps(ii, :))
-                s[5 + ii] = (a.eps[3 * ii] * K[0] + a.eps[1 + 3 * ii] * K[1] + a.eps[2 + 3 * ii] * K[2]) +
-                            (K[0] * a.eps[ii] + K[1] * a.eps[ii + 3] + K[2] * a.eps[ii + 6]);
-            for (int mu = 0; mu < a.nb; ++mu) {
-                double sn, cs;
-                sincos(K[0] * a.tau[3 * mu] + K[1] * a.tau[3 * mu + 1] + K[2] * a.tau[3 * mu + 2], &sn, &cs);
-                S.ph[i * a.nb + mu] = make_double2(cs, sn);
+            const double kpl = 1.0 / KeK + a.q4;
+            for (int ii = 0; ii < 3; ++ii) {  // dot(eps(:, ii), K) + dot(K, eps(ii, :))
+                const double ek = (a.eps[3 * ii] * K[0] + a.eps[1 + 3 * ii] * K[1] + a.eps[2 + 3 * ii] * K[2]) +
+                                  (K[0] * a.eps[ii] + K[1] * a.eps[ii + 3] + K[2] * a.eps[ii + 6]);
+                s[5 + ii] = ek * kpl;
             }
         }
+        for (int w = tid; w < gn * a.nb; w += T) {
+            const int i = w / a.nb, mu = w % a.nb;
+            const double* G = a.g + 3 * (g0 + i);
+            double sn = 0.0, cs = 0.0;
+            if (qnz || fabs(G[0]) > CMP_PREC || fabs(G[1]) > CMP_PREC || fabs(G[2]) > CMP_PREC) {
+                const double K[3] = {G[0] + q[0], G[1] + q[1], G[2] + q[2]};
+                sincos(K[0] * a.tau[3 * mu] + K[1] * a.tau[3 * mu + 1] + K[2] * a.tau[3 * mu + 2], &sn, &cs);
+            }
+            S.ph[w] = make_double2(cs, sn);
+        }
         __syncthreads();
-        const bool one = E * J <= T;
-        for (int w = tid; one ? w < E * J : w < E; w += T) {
-            const int j = one ? w / E : 0, e = one ? w % E : w;
-            const int step = one ? J : 1;
-            int b, al, nu, mu;
-            decode(e, a.nb, b, al, nu, mu);
+        // the sum is symmetric in (a, b), so six of the nine
+        for (int w = tid; w < 6 * nb2 * J; w += T) {
+            const int c6 = w % 6, pair = w / 6 % nb2, j = w / (6 * nb2);
+            const int b = c6 < 3 ? 0 : c6 < 5 ? 1 : 2, al = c6 < 3 ? c6 : c6 < 5 ? c6 - 2 : 2;
+            const int nu = pair % a.nb, mu = pair / a.nb;
             double tmn[3];
             for (int k = 0; k < 3; ++k) tmn[k] = a.tau[3 * mu + k] - a.tau[3 * nu + k];
             double2 acc[4] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0),
                               make_double2(0.0, 0.0)};
-            for (int i = j; i < gn; i += step) {
+            for (int i = j; i < gn; i += J) {
                 const double* s = S.gs + 8 * i;
                 const double2 pm = S.ph[i * a.nb + mu], pn = S.ph[i * a.nb + nu];
                 // e^{iK.(tau_mu - tau_nu)} = pm conj(pn)
                 const double2 ph = make_double2(pm.x * pn.x + pm.y * pn.y, pm.y * pn.x - pm.x * pn.y);
                 const double2 Kmn = make_double2(s[3] * ph.x, s[3] * ph.y);
-                const double kk = s[al] * s[b];
+                const double sa = s[al], sb = s[b];
+                const double kk = sa * sb;
                 const double2 Kab = make_double2(kk * Kmn.x, kk * Kmn.y);
                 acc[0].x += Kab.x;
                 acc[0].y += Kab.y;
                 if (grad)
                     for (int d = 0; d < 3; ++d) {
                         // Kab (i tmn_d - epsK_d KpLmb) + Kmn d(K_a K_b)/dK_d
-                        const double f = s[5 + d] * s[4];
-                        const double km = (al == d ? s[b] : 0.0) + (b == d ? s[al] : 0.0);
+                        const double f = s[5 + d];
+                        const double km = (al == d ? sb : 0.0) + (b == d ? sa : 0.0);
                         acc[1 + d].x += -Kab.y * tmn[d] - Kab.x * f + Kmn.x * km;
                         acc[1 + d].y += Kab.x * tmn[d] - Kab.y * f + Kmn.y * km;
                     }
             }
+            const int e = b + 3 * al + 9 * pair, et = al + 3 * b + 9 * pair;
             for (int k = 0; k < nc; ++k) {
-                double2& r = S.raw[(j * 4 + k) * E + e];
+                double2* raw = S.raw + (j * 4 + k) * E;
+                double2 r = raw[e];
                 r.x += acc[k].x;
                 r.y += acc[k].y;
+                raw[e] = r;
+                raw[et] = r;
             }
         }
     }
     __syncthreads();
-    // CombineZStar of the reciprocal part, times 4 pi / vol
+    // CombineZStar of the reciprocal part, times 4 pi / vol; two of D and its derivatives per thread
     const double ks = 4.0 * 3.141592653589793 / a.vol;
-    for (int w = tid; w < nc * E; w += T) {
-        const int k = w / E, e = w % E;
+    const int nh = grad ? 2 : 1;  // halves: D and d/dq_x, d/dq_y and d/dq_z
+    for (int w = tid; w < nh * E; w += T) {
+        const int h = w / E, e = w % E;
         int b, al, nu, mu;
         decode(e, a.nb, b, al, nu, mu);
         const double* Zm = a.z + 9 * mu;
         const double* Zn = a.z + 9 * nu;
-        double2 s = make_double2(0.0, 0.0);
+        double2 s[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
         for (int ap = 0; ap < 3; ++ap)
             for (int bp = 0; bp < 3; ++bp) {
                 const int src = bp + 3 * ap + 9 * nu + 9 * a.nb * mu;
-                double2 v = make_double2(0.0, 0.0);
-                for (int j = 0; j < J; ++j) {
-                    const double2 x = S.raw[(j * 4 + k) * E + src];
-                    v.x += x.x;
-                    v.y += x.y;
-                }
                 const double zz = Zm[ap + 3 * al] * Zn[bp + 3 * b];
-                s.x += zz * v.x;
-                s.y += zz * v.y;
+                for (int k = 0; k < 2; ++k) {
+                    if (k == 1 && !grad) continue;
+                    double2 v = make_double2(0.0, 0.0);
+                    for (int j = 0; j < J; ++j) {
+                        const double2 x = S.raw[(j * 4 + 2 * h + k) * E + src];
+                        v.x += x.x;
+                        v.y += x.y;
+                    }
+                    s[k].x += zz * v.x;
+                    s[k].y += zz * v.y;
+                }
             }
-        S.comb[k * E + e] = make_double2(ks * s.x, ks * s.y);
+        S.comb[2 * h * E + e] = make_double2(ks * s[0].x, ks * s[0].y);
+        if (grad) S.comb[(2 * h + 1) * E + e] = make_double2(ks * s[1].x, ks * s[1].y);
     }
     // minus the real-space part: sum_R e^{iqR} HZ_R (and i R_k e^{iqR} HZ_R)
     for (int r0 = 0; r0 < a.nr; r0 += RC) {
@@ -167,27 +186,28 @@ __device__ void ew_eval(const EwArgs& a, const double q[3], bool grad, const EwS
             const double* R = a.r + 3 * (r0 + i);
             double sn, cs;
             sincos(q[0] * R[0] + q[1] * R[1] + q[2] * R[2], &sn, &cs);
-            S.rph[i] = make_double2(cs, sn);
+            S.rph[4 * i] = make_double2(cs, sn);
+            for (int k = 0; k < 3; ++k) S.rph[4 * i + 1 + k] = make_double2(-(R[k] * sn), R[k] * cs);  // i R_k e^{iqR}
         }
         __syncthreads();
-        for (int w = tid; w < nc * E; w += T) {
-            const int k = w / E, e = w % E;
-            double2 acc = make_double2(0.0, 0.0);
+        for (int w = tid; w < nh * E; w += T) {
+            const int h = w / E, e = w % E;
+            const double* hz = a.hz + (size_t)r0 * E + e;
+            double2 acc[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+#pragma unroll 8
             for (int i = 0; i < rn; ++i) {
-                const double h = a.hz[(size_t)(r0 + i) * E + e];
-                const double2 p = S.rph[i];
-                if (k == 0) {
-                    acc.x += p.x * h;
-                    acc.y += p.y * h;
-                } else {
-                    const double Rk = a.r[3 * (r0 + i) + k - 1];
-                    acc.x -= Rk * p.y * h;  // i R_k e^{iqR} h
-                    acc.y += Rk * p.x * h;
-                }
+                const double x = hz[(size_t)i * E];
+                const double2 p = S.rph[4 * i + 2 * h], p1 = S.rph[4 * i + 2 * h + 1];
+                acc[0].x += p.x * x;
+                acc[0].y += p.y * x;
+                acc[1].x += p1.x * x;
+                acc[1].y += p1.y * x;
             }
-            double2& c = S.comb[k * E + e];
-            c.x -= acc.x;
-            c.y -= acc.y;
+            for (int k = 0; k < nh; ++k) {
+                double2& c = S.comb[(2 * h + k) * E + e];
+                c.x -= acc[k].x;
+                c.y -= acc[k].y;
+            }
         }
     }
     __syncthreads();
@@ -217,7 +237,7 @@ __device__ __forceinline__ void put(const EwArgs& a, const EwSmem& S, int src, i
 }
 
 // Work item i < n_a: point list_a[i] (or i) of list A (nqa points), else point i - n_a of list B.
-__global__ void __launch_bounds__(EW_THREADS) k_ewald(EwArgs a, const double* __restrict__ qa, int nqa,
+__global__ void __launch_bounds__(EW_THREADS, 2) k_ewald(EwArgs a, const double* __restrict__ qa, int nqa,
                                                       const int* __restrict__ list_a, int n_a,
                                                       const double* __restrict__ qb, int nqb, int n_b,
                                                       double2* __restrict__ dd) {
@@ -229,7 +249,7 @@ __global__ void __launch_bounds__(EW_THREADS) k_ewald(EwArgs a, const double* __
     S.ph = reinterpret_cast<double2*>(S.gs + 8 * GC);
     S.rph = S.ph + GC * a.nb;
     const int n = a.n;
-    for (int item = blockIdx.x; item < n_a + n_b; item += gridDim.x) {
+    for (int item = blockIdx.y; item < n_a + n_b; item += gridDim.y) {
         const bool in_a = item < n_a;
         const double* Q = in_a ? qa : qb;
         const int nq = in_a ? nqa : nqb;
@@ -237,6 +257,10 @@ __global__ void __launch_bounds__(EW_THREADS) k_ewald(EwArgs a, const double* __
         const double q[3] = {Q[3 * qi], Q[3 * qi + 1], Q[3 * qi + 2]};
         double2* out = dd + (size_t)item * 4 * n * n;
         const bool gamma = fabs(q[0]) < CMP_PREC && fabs(q[1]) < CMP_PREC && fabs(q[2]) < CMP_PREC;
+        // Gamma takes seven evaluations: with four parts (blockIdx.x) D(0) and each derivative have their own
+        // CTA, and they start first
+        const int part = blockIdx.x, parts = gridDim.x;
+        if (!gamma && part > 0) continue;
         if (!gamma) {
             ew_eval(a, q, true, S);
             for (int k = 0; k < 4; ++k) put(a, S, k, k, out);
@@ -250,27 +274,30 @@ __global__ void __launch_bounds__(EW_THREADS) k_ewald(EwArgs a, const double* __
             else qh[k] = q[k] - Q[3 * (qi - 1) + k];
         }
         const double h = sqrt(qh[0] * qh[0] + qh[1] * qh[1] + qh[2] * qh[2]) / 8.0;
-        // DynMat_NA: D_ew(0) plus 4 pi eV_A2 (qh.Z_mu)_a (qh.Z_nu)_b / (vol qh.eps.qh sqrt(m m))
-        const double zero[3] = {0.0, 0.0, 0.0};
-        ew_eval(a, zero, false, S);
-        double den = 0.0;
-        for (int j = 0; j < 3; ++j)
-            den += (qh[0] * a.eps[3 * j] + qh[1] * a.eps[1 + 3 * j] + qh[2] * a.eps[2 + 3 * j]) * qh[j];
-        const double fna = 4.0 * 3.141592653589793 * a.ev_a2 / (a.vol * den);
-        for (int e = threadIdx.x; e < a.E; e += blockDim.x) {
-            int b, al, nu, mu;
-            decode(e, a.nb, b, al, nu, mu);
-            double t1 = 0.0, t2 = 0.0;
-            for (int j = 0; j < 3; ++j) {
-                t1 += qh[j] * a.z[al + 3 * j + 9 * mu];  // dot_product(q, Zstar(alpha, :, mu))
-                t2 += qh[j] * a.z[b + 3 * j + 9 * nu];
+        if (part == 0) {
+            // DynMat_NA: D_ew(0) plus 4 pi eV_A2 (qh.Z_mu)_a (qh.Z_nu)_b / (vol qh.eps.qh sqrt(m m))
+            const double zero[3] = {0.0, 0.0, 0.0};
+            ew_eval(a, zero, false, S);
+            double den = 0.0;
+            for (int j = 0; j < 3; ++j)
+                den += (qh[0] * a.eps[3 * j] + qh[1] * a.eps[1 + 3 * j] + qh[2] * a.eps[2 + 3 * j]) * qh[j];
+            const double fna = 4.0 * 3.141592653589793 * a.ev_a2 / (a.vol * den);
+            for (int e = threadIdx.x; e < a.E; e += blockDim.x) {
+                int b, al, nu, mu;
+                decode(e, a.nb, b, al, nu, mu);
+                double t1 = 0.0, t2 = 0.0;
+                for (int j = 0; j < 3; ++j) {
+                    t1 += qh[j] * a.z[al + 3 * j + 9 * mu];  // dot_product(q, Zstar(alpha, :, mu))
+                    t2 += qh[j] * a.z[b + 3 * j + 9 * nu];
+                }
+                const double na = (t1 * t2) * (a.mrs[mu] * a.mrs[nu]) * fna;
+                const double2 d0 = S.comb[e];
+                out[(3 * mu + al) * n + 3 * nu + b] = make_double2(d0.x + na, d0.y);
             }
-            const double na = (t1 * t2) * (a.mrs[mu] * a.mrs[nu]) * fna;
-            const double2 d0 = S.comb[e];
-            out[(3 * mu + al) * n + 3 * nu + b] = make_double2(d0.x + na, d0.y);
         }
         __syncthreads();
         for (int k = 0; k < 3; ++k) {  // (DynEw(q + h/2 e_k) - DynEw(q - h/2 e_k)) / h
+            if (parts > 1 && part != k + 1) continue;
             double qp[3] = {q[0], q[1], q[2]};
             qp[k] += 0.5 * h;
             ew_eval(a, qp, false, S);
@@ -293,7 +320,7 @@ __global__ void __launch_bounds__(EW_THREADS) k_ewald(EwArgs a, const double* __
 
 size_t ew_smem_bytes(int nb, int J) {
     const int E = 9 * nb * nb;
-    return sizeof(double2) * ((size_t)J * 4 * E + 4 * E) + sizeof(double) * 8 * GC + sizeof(double2) * (GC * nb + RC);
+    return sizeof(double2) * ((size_t)J * 4 * E + 4 * E) + sizeof(double) * 8 * GC + sizeof(double2) * (GC * nb + 4 * RC);
 }
 
 }  // namespace
@@ -358,7 +385,7 @@ int launch_ewald(spring_ctx* c, const double* qa, int nqa, const int* list_a, in
     a.nb = c->nb;
     a.n = n;
     a.E = 9 * c->nb * c->nb;
-    a.J = std::max(1, EW_THREADS / a.E);
+    a.J = std::max(1, EW_SPLIT / a.E);
     a.ng = D.ng;
     a.nr = D.nr;
     a.gamma_mode = gamma_mode;
@@ -380,8 +407,11 @@ int launch_ewald(spring_ctx* c, const double* qa, int nqa, const int* list_a, in
     const size_t smem = ew_smem_bytes(a.nb, a.J);
     if (smem > 48 * 1024) cudaFuncSetAttribute(k_ewald, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "ewald: injected launch failure");
-    const int blocks = std::min(items, 148 * 8);
-    k_ewald<<<blocks, EW_THREADS, smem, c->stream>>>(a, qa, nqa, list_a, n_a, qb, nqb, n_b, D.dd.p);
+    const int threads = std::min(EW_THREADS, std::max(64, (std::max(6 * a.nb * a.nb * a.J, 2 * a.E) + 31) / 32 * 32));
+    // Parts where one CTA's seven evaluations at Gamma would be the critical path (2 atoms, 286 points: 92 us
+    // in one CTA, 42 in four; 8 atoms: 648, 483); a long list hides them, and its empty parts are not free.
+    k_ewald<<<dim3(items <= 2048 ? 4 : 1, std::min(items, 148 * 8)), threads, smem, c->stream>>>(
+        a, qa, nqa, list_a, n_a, qb, nqb, n_b, D.dd.p);
     SPRING_CHECK(launch_check(c, "k_ewald"));
     *dd_out = D.dd.p;
     return SPRING_OK;
