@@ -17,9 +17,9 @@
 // (s0 s1 c d)), M = 128 quartets, N = 64 per block, one chunk (s0, three s1) at a time into one of
 // two tensor-memory buffers.  The complex product is written as a real one:
 //   A[q][k] = [Re P | Im P],  B[(re, r)][k] = [Re X | -Im X],  B[(im, r)][k] = [Im X | Re X].
-// The epilogue (FP32, two threads per quartet, three s3 each) contracts E_q3 and E_q2, screens every
-// mode quad in FP32 against the windows of its seven delta terms, and evaluates the terms inside
-// them in FP64: W = |Phi|^2 (1/w0)(1/w1)(1/w2)(1/w3) Sctr4THz2/Nq^2 and
+// The epilogue (FP32, three threads per quartet, two s3 each) contracts E_q3 and E_q2, screens every
+// delta term of every mode quad in FP32 against its window, lists the terms inside, and evaluates the
+// listed ones in FP64, two per lane: W = |Phi|^2 (1/w0)(1/w1)(1/w2)(1/w3) Sctr4THz2/Nq^2 and
 //   rate(s0) += W [ w1 n1 n2 n3 d(w0 - w1 - w2 - w3)
 //                 + sum_k w2_k (1 + n_k) n_i n_j d(w0 + w_k - w_i - w_j)
 //                 + sum_k w3_k (1 + n_i)(1 + n_j) n_k d(w0 + w_i + w_j - w_k) ] / n0,
@@ -27,9 +27,13 @@
 // gathered by which point plays the first (channel 2) or last (channel 3) role; for three distinct
 // points all seven weights are 1.  Precision: SPRING_BF16 rounds A and B to BF16 once;
 // SPRING_BF16X3 splits both into hi + lo parts and accumulates hi*hi + hi*lo + lo*hi.
-// Roofline: the FP32 epilogue (about 62 kflop of contraction per quartet) bounds the kernel; the
-// tensor pipe carries the X' GEMM (about 0.25 Mflop algorithmic per quartet, issued three times
-// for BF16x3).
+// Bound by the epilogue's instruction issue: about 290 FP32 operations per lane and (s0, s1) for the contraction
+// by E_q3, 230 for E_q2 and 210 for the screen (the last two as packed pairs), 47% of the issue slots used by
+// three warps per scheduler (128 registers each; four would spill); the tensor pipe carries the X' GEMM (about
+// 0.25 Mflop algorithmic per quartet, issued three times for BF16x3).  6 q0 at 8^3: 9.88 -> 5.16 ms, by steps:
+// listed terms instead of a loop per quad in the lane that owns it (a third of the lanes active, one serial
+// exp at a time) 7.02, quartets dealt to the warps in turn and three threads per row instead of two 6.26, Z by
+// blocks and accumulators by the number of temperatures (fewer spills) 5.76, packed FP32 5.16.
 #include <algorithm>
 #include <vector>
 #include <cub/cub.cuh>
@@ -49,12 +53,41 @@ constexpr int NBLK = 4;         // (nu2, nu3) blocks
 constexpr int CROWS = 64;       // B rows of one (chunk, block): 3 s1 x 3 c x (re, im) x 3 d = 54, padded
 constexpr int NCHUNK = 12;      // chunks of a tile: (s0, s1 in {0,1,2} or {3,4,5})
 constexpr int KLIST = 128;      // entries of one block's K list
-constexpr int EPI_WARPS = 8;    // two threads per quartet row
-constexpr int V4_THREADS = EPI_WARPS * 32 + 64;  // + copy warp (8) + MMA warp (9)
+constexpr int S3 = 2;           // s3 per epilogue thread
+constexpr int EPI_WARPS = 4 * NM / S3;  // three threads per quartet row
+constexpr int V4_THREADS = EPI_WARPS * 32 + 64;  // + copy warp + MMA warp
 constexpr int TCOLS = 512;      // two buffers of 4 blocks x 64 columns
 constexpr double EXP_CUT = 40.0;
 constexpr long long MAX_SPINS = 1LL << 26;  // drains of work already issued
-constexpr int E2S = 37;         // float2 stride of one quartet's E_q2 in shared memory (36 used)
+constexpr int E2S = 76;         // float stride of one quartet's E_q2 in shared memory (72 used)
+constexpr int HITS = 768;       // entries of a warp's list of delta terms to evaluate
+// E_q2 of the tile, then each epilogue warp's |Phi|^2 of one (s0, s1) and its list
+constexpr size_t E2_BYTES = (size_t)QT * E2S * 4, SCR_BYTES = (size_t)EPI_WARPS * (NM * S3 * 32 * 4 + HITS * 2);
+constexpr size_t WORK_BYTES = 75776;
+static_assert(E2_BYTES + SCR_BYTES <= WORK_BYTES, "work area");
+
+// Two FP32 values in one register pair (each rounded as its scalar form)
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pack2(float x, float y) {
+    f2 v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
+    return v;
+}
+__device__ __forceinline__ float2 unpack2(f2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 
 // Row of the B image (= accumulator column inside a block's 64) of value i = c*6 + ri*3 + d
 // (ri = 0 Re, 1 Im) of s1 slot j: the first 16 values of each j at 16 j, the last two at 48 + 2 j,
@@ -251,6 +284,21 @@ __global__ void k4_total(int nq, const int* __restrict__ toff, const int* __rest
 }
 
 // ------------------------------------------------------------------ the tensor-core pass
+// e^-x for 0 <= x <= 40 (within 2.3e-16 of exp), without branches so that several run side by side: Cody and Waite's two-step reduction
+// by ln 2, the Taylor polynomial to r^13 (remainder below 5e-18 for |r| <= ln 2 / 2) in Estrin's order.
+__device__ __forceinline__ double exp_neg(double x) {
+    constexpr double SHIFT = 6755399441055744.0;  // 1.5 2^52: the sum's low word is the rounded integer
+    const double t = fma(-x, 1.4426950408889634, SHIFT), k = t - SHIFT;
+    const double r = fma(-k, 2.3190468138462996e-17, fma(-k, 0.6931471805599453, -x));
+    const double r2 = r * r, r4 = r2 * r2;
+    const double a = fma(r, 1.0 / 6, 1.0 / 2), b = fma(r, 1.0 / 120, 1.0 / 24), c = fma(r, 1.0 / 5040, 1.0 / 720);
+    const double d = fma(r, 1.0 / 362880, 1.0 / 40320), e = fma(r, 1.0 / 39916800, 1.0 / 3628800);
+    const double f = fma(r, 1.0 / 6227020800.0, 1.0 / 479001600);
+    const double lo = fma(r2, b, a), mid = fma(r2, d, c), hi = fma(r2, f, e);
+    const double y = 1.0 + fma(r2, fma(r4, fma(r4, hi, mid), lo), r);
+    return __hiloint2double(__double2hiint(y) + __double2loint(t) * (1 << 20), __double2loint(y));
+}
+
 struct V4Args {
     int nq, nT, nq0, q0, ntiles, tiles_per_cta, H, gq0;
     int rs;                      // doubles per mode record (omega, 1/omega, n(T)), even
@@ -261,10 +309,10 @@ struct V4Args {
     long long max_spins;
 };
 
-// Shared memory: A (H parts x QT x ktot bf16), one B part (CROWS x ktot bf16), E_q2 of every quartet
-// (a private copy for each of its two threads), then this tail.
+// Shared memory: A (H parts x QT x ktot bf16), one B part (CROWS x ktot bf16), the work area (E_q2 of every
+// quartet, the epilogue warps' scratch), then this tail.
 struct V4Sm {
-    alignas(8) uint64_t afull, afree, bfull, bfree, tfull[2], tempty[2];
+    alignas(8) uint64_t afull, afree, bfull, bfree, tfull[2], tempty[2], e2[4];
     uint32_t tslot;
     int abort;
     double w0[NM], ob0[NM], n0inv[9][NM];
@@ -272,6 +320,8 @@ struct V4Sm {
     double rate[NM][9];  // this CTA's sums for q0, flushed once at the end
 };
 
+// NT: at least the number of temperatures
+template <int NT>
 __global__ void __launch_bounds__(V4_THREADS, 1)
 k_v4tc(V4Args a, Blk4 bk, const int4* __restrict__ tiles, const int4* __restrict__ quart,
        const __nv_bfloat16* __restrict__ img, const double2* __restrict__ ph, const float2* __restrict__ etab,
@@ -283,8 +333,8 @@ k_v4tc(V4Args a, Blk4 bk, const int4* __restrict__ tiles, const int4* __restrict
     const size_t abytes = (size_t)H * QT * bk.ktot * 2, bbytes = (size_t)CROWS * bk.ktot * 2;
     uint8_t* sA = smraw;
     uint8_t* sB = smraw + abytes;
-    float2* sE2 = reinterpret_cast<float2*>(smraw + abytes + bbytes);
-    V4Sm& S = *reinterpret_cast<V4Sm*>(smraw + abytes + bbytes + (size_t)2 * QT * E2S * 8);
+    float* sE2 = reinterpret_cast<float*>(smraw + abytes + bbytes);
+    V4Sm& S = *reinterpret_cast<V4Sm*>(smraw + abytes + bbytes + WORK_BYTES);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int t0 = blockIdx.x * a.tiles_per_cta;
     const int t1 = min(a.ntiles, t0 + a.tiles_per_cta);
@@ -305,6 +355,7 @@ k_v4tc(V4Args a, Blk4 bk, const int4* __restrict__ tiles, const int4* __restrict
             tc::mbar_init(tc::smem_u32(&S.tfull[k]), 1);
             tc::mbar_init(tc::smem_u32(&S.tempty[k]), EPI_WARPS);
         }
+        for (int k = 0; k < 4; ++k) tc::mbar_init(tc::smem_u32(&S.e2[k]), NM / S3);
         tc::mbar_fence_init();
     }
     for (int i = tid; i < NM * 9; i += blockDim.x) (&S.rate[0][0])[i] = 0.0;
@@ -399,32 +450,45 @@ k_v4tc(V4Args a, Blk4 bk, const int4* __restrict__ tiles, const int4* __restrict
         __syncwarp();
     } else {
         // ------------------------------------------------------------ epilogue warps
-        // Thread (row r, half h): quartet r of the tile, s3 = 3h .. 3h+2.  It builds its half of the
-        // quartet's A row (blocks h and h + 2) and its own copy of E_q2, so that no thread reads what
-        // another wrote; the only synchronisation is through the mbarriers (every wait bounded).
-        const int wq = warp & 3, h = warp >> 2;      // TMEM lanes 32 wq .. +31; s3 = 3h .. 3h+2
-        const int r = wq * 32 + lane;                 // quartet row of the tile
+        // Thread (row r, third h): a quartet of the tile, s3 = 2h, 2h+1.  Quartet i is row 32 (i % 4) + i / 4, so
+        // that a short tile fills the warps evenly.  A thread builds a third of the quartet's A row (blocks 0, 3,
+        // or 1 and 2) and of its E_q2, which its three threads share; the only synchronisation is through the
+        // mbarriers (every wait bounded).
+        const int wq = warp & 3, h = warp >> 2;      // TMEM lanes 32 wq .. +31; s3 = 2h, 2h+1
+        const int r = wq * 32 + lane;                 // row of the tile
+        const int ri = lane * 4 + wq;                 // its quartet
         const int pol_lo0 = a.gq0 ? 3 : 0;
-        float2* myE2 = sE2 + (size_t)(h * QT + r) * E2S;
+        float* myE2 = sE2 + (size_t)r * E2S;  // [nu c][s2 / 2]: Re, Re, Im, Im of two s2
+        uint8_t* scr = reinterpret_cast<uint8_t*>(sE2) + E2_BYTES + (size_t)warp * (NM * S3 * 32 * 4 + HITS * 2);
+        float* sA2 = reinterpret_cast<float*>(scr);                          // [12][32] |Phi|^2 of (s2, s3), lane
+        unsigned short* hit = reinterpret_cast<unsigned short*>(scr + NM * S3 * 32 * 4);
+        auto give_up = [&]() {
+            if (lane == 0) {
+                atomicExch(err, 1);
+                *(volatile int*)&S.abort = 1;
+            }
+        };
+        // the warps of the rows are here (twice a tile: E_q2 no longer read, E_q2 written)
+        auto pair_sync = [&](uint32_t parity) {
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(tc::smem_u32(&S.e2[wq]));
+            return !__any_sync(0xffffffffu, !tc::mbar_wait(tc::smem_u32(&S.e2[wq]), parity, a.max_spins));
+        };
         for (int t = 0; t < nt; ++t) {
             // ---- tile set-up: wait until the MMAs of the previous tile no longer read A
             bool ok = t == 0 || tc::mbar_wait(tc::smem_u32(&S.afree), (uint32_t)((t - 1) & 1), a.max_spins);
-            if (__any_sync(0xffffffffu, !ok)) {
-                if (lane == 0) {
-                    atomicExch(err, 1);
-                    *(volatile int*)&S.abort = 1;
-                }
+            if (__any_sync(0xffffffffu, !ok) || !pair_sync(0u)) {
+                give_up();
                 break;
             }
             const int4 tr = tiles[t0 + t];
-            const bool valid = r < tr.z;
+            const bool valid = ri < tr.z;
             int4 qd = make_int4(tr.x, 0, 0, 0);
-            if (valid) qd = quart[tr.y + r];
+            if (valid) qd = quart[tr.y + ri];
             const int g1 = qd.x, g2 = qd.y, g3 = qd.z;
-            // A row: this thread's two blocks (h = 0: blocks 0, 2; h = 1: blocks 1, 3)
+            // A row: this thread's blocks
             if (valid) {
-                for (int bi = 0; bi < 2; ++bi) {
-                    const int b = h + 2 * bi;
+                for (int b = h == 0 ? 0 : h == 1 ? 3 : 1; b < (h == 0 ? 1 : h == 1 ? 4 : 3); ++b) {
                     const uint32_t sbo = (uint32_t)(bk.kpad[b] / 8) * 128u;
                     __nv_bfloat16* Ah = reinterpret_cast<__nv_bfloat16*>(sA) + QT * bk.koff[b];
                     __nv_bfloat16* Al = Ah + QT * bk.ktot;
@@ -447,25 +511,31 @@ k_v4tc(V4Args a, Blk4 bk, const int4* __restrict__ tiles, const int4* __restrict
                     }
                 }
 #pragma unroll 6
-                for (int j = 0; j < 36; ++j) myE2[j] = etab[(size_t)g2 * 36 + j];
+                for (int j = 6 * S3 * h; j < 6 * S3 * (h + 1); ++j) {
+                    const float2 e = etab[(size_t)g2 * 36 + j];
+                    float* o = myE2 + j / 2 * 4 + j % 2;
+                    o[0] = e.x;
+                    o[2] = e.y;
+                }
             }
             tc::fence_async_smem();
             tc::mbar_arrive(tc::smem_u32(&S.afull));
+            if (!pair_sync(1u)) {
+                give_up();
+                break;
+            }
             // per-quartet registers: E_q3 of this thread's s3, FP32 omegas, Gamma flags, term weights
-            float2 e3[6][3];
-            float w1f[NM], w2f[NM], w3f[3];
+            float2 e3[6][S3];
+            float w2f[NM], w3f[S3];
 #pragma unroll
             for (int x = 0; x < 6; ++x)
 #pragma unroll
-                for (int y = 0; y < 3; ++y)
-                    e3[x][y] = valid ? etab[(size_t)g3 * 36 + x * NM + 3 * h + y] : make_float2(0.f, 0.f);
+                for (int y = 0; y < S3; ++y)
+                    e3[x][y] = valid ? etab[(size_t)g3 * 36 + x * NM + S3 * h + y] : make_float2(0.f, 0.f);
 #pragma unroll
-            for (int s = 0; s < NM; ++s) {
-                w1f[s] = wf[(size_t)g1 * NM + s];
-                w2f[s] = valid ? wf[(size_t)g2 * NM + s] : 0.f;
-            }
+            for (int s = 0; s < NM; ++s) w2f[s] = valid ? wf[(size_t)g2 * NM + s] : 0.f;
 #pragma unroll
-            for (int y = 0; y < 3; ++y) w3f[y] = valid ? wf[(size_t)g3 * NM + 3 * h + y] : 0.f;
+            for (int y = 0; y < S3; ++y) w3f[y] = valid ? wf[(size_t)g3 * NM + S3 * h + y] : 0.f;
             // term weights in units of 1/6 (channel 1) and 1/2 (channels 2, 3): the distinct orderings
             // of (g1, g2, g3) by their first two points (every one of the six when they differ)
             int c1 = 0, c2[3] = {0, 0, 0}, c3[3] = {0, 0, 0};
@@ -485,193 +555,201 @@ k_v4tc(V4Args a, Blk4 bk, const int4* __restrict__ tiles, const int4* __restrict
                 }
             }
             const bool gam1 = g1 == 0, gam2 = g2 == 0, gam3 = g3 == 0;
+            // the seven terms' weights, four bits each, and the mask of the nonzero ones in the order of the
+            // screen's bits, without the acoustic modes of Gamma
+            const unsigned cw = c1 | c2[0] << 4 | c2[1] << 8 | c2[2] << 12 | c3[0] << 16 | c3[1] << 20 | c3[2] << 24;
+            unsigned allow = 0u;
+#pragma unroll
+            for (int m = 0; m < 7; ++m) allow |= ((cw >> (4 * m)) & 15u) != 0u ? 0x204081u << (6 - m) : 0u;
+#pragma unroll
+            for (int y = 0; y < S3; ++y)
+                if (gam3 && S3 * h + y < 3) allow &= y == 0 ? 0x1fc07fu : 0xfe03f80u;
+            const f2 w3p = pack2(w3f[0], w3f[1]), nrf2 = pack2(-a.rf * a.rf, -a.rf * a.rf);
             // ---- chunks
             for (int ch = 0; ch < a.nch; ++ch) {
                 const int k = t * a.nch + ch, buf = k & 1;
                 const int s0 = a.chunk[ch] >> 1, s1b = 3 * (a.chunk[ch] & 1);
                 ok = tc::mbar_wait(tc::smem_u32(&S.tfull[buf]), (uint32_t)((k >> 1) & 1), a.max_spins);
                 if (__any_sync(0xffffffffu, !ok)) {
-                    if (lane == 0) {
-                        atomicExch(err, 1);
-                        *(volatile int*)&S.abort = 1;
-                    }
+                    give_up();
                     t = nt;
                     break;
                 }
                 tc::fence_after_sync();
-                double acc[9];
+                double acc[NT];
 #pragma unroll
-                for (int T = 0; T < 9; ++T) acc[T] = 0.0;
+                for (int T = 0; T < NT; ++T) acc[T] = 0.0;
                 const uint32_t tb = tm + ((uint32_t)(wq * 32) << 16) + (uint32_t)(buf * 256);
 #pragma unroll 1
                 for (int j = 0; j < 3; ++j) {
                     const int s1 = s1b + j;
                     const bool act = valid && s0 >= pol_lo0 && !(gam1 && s1 < 3);
-                    float2 phi[NM][3];
+                    f2 phx[NM / 2][S3], phy[NM / 2][S3];  // Re and Im of Phi, two s2 each
 #pragma unroll
-                    for (int x = 0; x < NM; ++x)
+                    for (int x = 0; x < NM / 2; ++x)
 #pragma unroll
-                        for (int y = 0; y < 3; ++y) phi[x][y] = make_float2(0.f, 0.f);
+                        for (int y = 0; y < S3; ++y) phx[x][y] = phy[x][y] = 0ull;
 #pragma unroll
                     for (int nu2 = 0; nu2 < 2; ++nu2) {
-                        // blocks (nu2, 0) = 2 nu2 and (nu2, 1) = 2 nu2 + 1: the 18 values of slot j
-                        // (value i = c*6 + ri*3 + d at column brow(j, i))
-                        float xv[2][18];
-                        __syncwarp();
+                        // Z[c][s3] = sum_{nu3 d} X'[c d][nu2 nu3] E3[nu3 d][s3], block 2 nu2 + nu3 at a time: the 18
+                        // values of slot j (value i = c*6 + ri*3 + d at column brow(j, i))
+                        float2 z[3][S3];
+#pragma unroll
+                        for (int c = 0; c < 3; ++c)
+#pragma unroll
+                            for (int y = 0; y < S3; ++y) z[c][y] = make_float2(0.f, 0.f);
 #pragma unroll
                         for (int nu3 = 0; nu3 < 2; ++nu3) {
-                            const uint32_t cb = tb + (uint32_t)((2 * nu2 + nu3) * CROWS);
-                            tc::tmem_ld16(cb + (uint32_t)(16 * j), xv[nu3]);
-                            tc::tmem_ld2(cb + (uint32_t)(48 + 2 * j), xv[nu3] + 16);
-                        }
-                        tc::tmem_ld_wait();
-                        if (j == 2 && nu2 == 1) {  // this warp's reads of the buffer are done
-                            tc::fence_before_sync();
+                            float xv[18];
                             __syncwarp();
-                            if (lane == 0) tc::mbar_arrive(tc::smem_u32(&S.tempty[buf]));
+                            const uint32_t cb = tb + (uint32_t)((2 * nu2 + nu3) * CROWS);
+                            tc::tmem_ld16(cb + (uint32_t)(16 * j), xv);
+                            tc::tmem_ld2(cb + (uint32_t)(48 + 2 * j), xv + 16);
+                            tc::tmem_ld_wait();
+                            if (j == 2 && nu2 == 1 && nu3 == 1) {  // this warp's reads of the buffer are done
+                                tc::fence_before_sync();
+                                __syncwarp();
+                                if (lane == 0) tc::mbar_arrive(tc::smem_u32(&S.tempty[buf]));
+                            }
+#pragma unroll
+                            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                                for (int d = 0; d < 3; ++d) {
+                                    const float xr = xv[c * 6 + d], xi = xv[c * 6 + 3 + d];
+#pragma unroll
+                                    for (int y = 0; y < S3; ++y) {
+                                        const float2 e = e3[nu3 * 3 + d][y];
+                                        z[c][y].x = fmaf(xr, e.x, fmaf(-xi, e.y, z[c][y].x));
+                                        z[c][y].y = fmaf(xr, e.y, fmaf(xi, e.x, z[c][y].y));
+                                    }
+                                }
                         }
-                        if (act) {
+                        // Phi[s2][s3] += E2[nu2 c][s2] Z[c][s3]
 #pragma unroll
-                            for (int c = 0; c < 3; ++c) {
-                                // Z[s3] = sum_{nu3 d} X'[c d][nu2 nu3] E3[nu3 d][s3]; value c*6 + ri*3 + d
-                                float2 z[3];
+                        for (int c = 0; c < 3; ++c) {
+                            f2 zx[S3], zy[S3], nzy[S3];
 #pragma unroll
-                                for (int y = 0; y < 3; ++y) z[y] = make_float2(0.f, 0.f);
+                            for (int y = 0; y < S3; ++y) {
+                                zx[y] = pack2(z[c][y].x, z[c][y].x);
+                                zy[y] = pack2(z[c][y].y, z[c][y].y);
+                                nzy[y] = pack2(-z[c][y].y, -z[c][y].y);
+                            }
 #pragma unroll
-                                for (int nu3 = 0; nu3 < 2; ++nu3)
+                            for (int x = 0; x < NM / 2; ++x) {
+                                const float4 e = *reinterpret_cast<const float4*>(myE2 + (nu2 * 3 + c) * 2 * NM + 4 * x);
+                                const f2 ex = pack2(e.x, e.y), ey = pack2(e.z, e.w);
 #pragma unroll
-                                    for (int d = 0; d < 3; ++d) {
-                                        const float xr = xv[nu3][c * 6 + d], xi = xv[nu3][c * 6 + 3 + d];
-#pragma unroll
-                                        for (int y = 0; y < 3; ++y) {
-                                            const float2 e = e3[nu3 * 3 + d][y];
-                                            z[y].x = fmaf(xr, e.x, fmaf(-xi, e.y, z[y].x));
-                                            z[y].y = fmaf(xr, e.y, fmaf(xi, e.x, z[y].y));
-                                        }
-                                    }
-                                // Phi[s2][s3] += E2[nu2 c][s2] Z[s3]
-                                const float2* e2p = myE2 + (nu2 * 3 + c) * NM;
-#pragma unroll
-                                for (int s2 = 0; s2 < NM; ++s2) {
-                                    const float2 e = e2p[s2];
-#pragma unroll
-                                    for (int y = 0; y < 3; ++y) {
-                                        phi[s2][y].x = fmaf(e.x, z[y].x, fmaf(-e.y, z[y].y, phi[s2][y].x));
-                                        phi[s2][y].y = fmaf(e.x, z[y].y, fmaf(e.y, z[y].x, phi[s2][y].y));
-                                    }
+                                for (int y = 0; y < S3; ++y) {
+                                    phx[x][y] = fma2(ex, zx[y], fma2(ey, nzy[y], phx[x][y]));
+                                    phy[x][y] = fma2(ex, zy[y], fma2(ey, zx[y], phy[x][y]));
                                 }
                             }
                         }
                     }
-                    if (!act) continue;
-                    // ---- screen every (s2, s3) of this (s0, s1) against the seven windows:
-                    // with u = w0 - w1, v = w0 + w1, P = w2 + w3, M = w2 - w3 the terms are u - P, v - P,
-                    // u + P, u + M, u - M, v - M, v + M; min(|x - y|, |x + y|) = ||x| - |y||
+                    // ---- screen every term of every (s2, s3) of this (s0, s1) in FP32: with u = w0 - w1,
+                    // v = w0 + w1, P = w2 + w3, M = w2 - w3 the terms are u - P, v - P, u + M, u - M, u + P,
+                    // v - M, v + M; a term is bit 27 - (14 (s2 % 2) + 7 y + m) of word s2 / 2
                     const double* r1 = rec + ((size_t)g1 * NM + s1) * a.rs;
+                    const float w1f = wf[(size_t)g1 * NM + s1], u = S.w0f[s0] - w1f, v = S.w0f[s0] + w1f;
+                    const f2 u2 = pack2(u, u), v2 = pack2(v, v), neg = pack2(-1.f, -1.f);
+                    unsigned wm[NM / 2];
+                    int n = 0;
+#pragma unroll
+                    for (int w = 0; w < NM / 2; ++w) {
+                        unsigned mm = 0u;
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            const int s2 = 2 * w + k;
+#pragma unroll
+                            for (int y = 0; y < S3; ++y) {
+                                const float2 px = unpack2(phx[w][y]), py = unpack2(phy[w][y]);
+                                const float re = k ? px.y : px.x, im = k ? py.y : py.x;
+                                sA2[(S3 * s2 + y) * 32 + lane] = re * re + im * im;
+                            }
+                            const f2 W2 = pack2(w2f[s2], w2f[s2]), P = add2(W2, w3p), M = fma2(w3p, neg, W2);
+                            // d^2 - rf^2 of both s3
+                            const f2 d[7] = {fma2(P, neg, u2), fma2(P, neg, v2), add2(u2, M), fma2(M, neg, u2),
+                                             add2(u2, P), fma2(M, neg, v2), add2(v2, M)};
+                            float2 t[7];
+#pragma unroll
+                            for (int m = 0; m < 7; ++m) t[m] = unpack2(fma2(d[m], d[m], nrf2));
+#pragma unroll
+                            for (int m = 0; m < 7; ++m) mm = __funnelshift_l(__float_as_uint(t[m].x), mm, 1);
+#pragma unroll
+                            for (int m = 0; m < 7; ++m) mm = __funnelshift_l(__float_as_uint(t[m].y), mm, 1);
+                        }
+                        if (gam2) mm &= w == 0 ? 0u : w == 1 ? 0x3fffu : ~0u;
+                        wm[w] = act ? mm & allow : 0u;
+                        n += __popc(wm[w]);
+                    }
+                    int end = n;
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int x = __shfl_up_sync(0xffffffffu, end, o);
+                        if (lane >= o) end += x;
+                    }
+                    const int total = __shfl_sync(0xffffffffu, end, 31);
+                    if (total == 0) continue;
+                    // ---- FP64 terms, two per lane: listed first, so that the lanes are full whichever quads
+                    // they come from
                     const double2 m1 = *reinterpret_cast<const double2*>(r1);
-                    const float u = S.w0f[s0] - w1f[s1], v = S.w0f[s0] + w1f[s1];
-                    const float au = fabsf(u), av = fabsf(v);
-                    // FP32 screen of the 18 (s2, s3) of this thread (unrolled: registers only), then
-                    // one copy of the FP64 code for the quads inside a window (a rolled loop keeps the
-                    // kernel's code within the instruction cache)
-                    unsigned am = 0u;
-                    float a2s[NM * 3];
+                    const double W0 = S.w0[s0], k1 = S.ob0[s0] * m1.y * a.mfac * a.pre;
+                    for (int base = 0; base < total; base += HITS) {
+                        int pos = end - n - base;
 #pragma unroll
-                    for (int s2 = 0; s2 < NM; ++s2)
-#pragma unroll
-                        for (int y = 0; y < 3; ++y) {
-                            a2s[3 * s2 + y] = phi[s2][y].x * phi[s2][y].x + phi[s2][y].y * phi[s2][y].y;
-                            if ((gam2 && s2 < 3) || (gam3 && 3 * h + y < 3)) continue;
-                            const float P = w2f[s2] + w3f[y], M = w2f[s2] - w3f[y];
-                            const float aM = fabsf(M);
-                            const bool any = fabsf(au - fabsf(P)) < a.rf || fabsf(v - P) < a.rf ||
-                                             fabsf(au - aM) < a.rf || fabsf(av - aM) < a.rf;
-                            if (any) am |= 1u << (3 * s2 + y);
-                        }
+                        for (int w = 0; w < NM / 2; ++w)
+                            for (unsigned b = wm[w]; b != 0u; b &= b - 1u, ++pos)
+                                if ((unsigned)pos < (unsigned)HITS)
+                                    hit[pos] = (unsigned short)(w << 10 | (__ffs(b) - 1) << 5 | lane);
+                        __syncwarp();
+                        const int nh = min(HITS, total - base);
 #pragma unroll 1
-                    while (am != 0u) {
-                        const int bq = __ffs(am) - 1;
-                        am &= am - 1u;
-                        const int s2 = bq / 3, s3 = 3 * h + bq % 3;
-                        const float a2 = a2s[bq];
-                        // FP64: W and the seven terms, from the mode records (omega, 1/omega, n(T))
-                        // of q2 and q3, one load each; the q1 record was read for this s1
-                        const double* r2 = rec + ((size_t)g2 * NM + s2) * a.rs;
-                        const double* r3 = rec + ((size_t)g3 * NM + s3) * a.rs;
-                        const double2 m2 = *reinterpret_cast<const double2*>(r2);
-                        const double2 m3 = *reinterpret_cast<const double2*>(r3);
-                        // occupations of up to four temperatures, loaded with the records (rs >= 6)
-                        double2 n2a = make_double2(0.0, 0.0), n2b = n2a, n3a = n2a, n3b = n2a;
-                        if (a.nT <= 4) {
-                            n2a = *reinterpret_cast<const double2*>(r2 + 2);
-                            n3a = *reinterpret_cast<const double2*>(r3 + 2);
-                            if (a.nT > 2) {
-                                n2b = *reinterpret_cast<const double2*>(r2 + 4);
-                                n3b = *reinterpret_cast<const double2*>(r3 + 4);
+                        for (int i = 0; i < nh; i += 64) {
+                            double g[2];
+                            const double *r2[2], *r3[2];
+                            unsigned sg[2];
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                const int ix = i + 32 * e + lane;
+                                const unsigned code = hit[ix < nh ? ix : 0];
+                                const int L = code & 31, p = 27 - ((code >> 5) & 31);
+                                const int sy = (p * 37) >> 8, m = p - 7 * sy;  // p / 7, p % 7
+                                const int s2 = 2 * (code >> 10) + sy / S3, y = sy % S3;
+                                const int G2 = __shfl_sync(0xffffffffu, g2, L), G3 = __shfl_sync(0xffffffffu, g3, L);
+                                const unsigned c = (__shfl_sync(0xffffffffu, cw, L) >> (4 * m)) & 15u;
+                                r2[e] = rec + ((size_t)G2 * NM + s2) * a.rs;
+                                r3[e] = rec + ((size_t)G3 * NM + S3 * h + y) * a.rs;
+                                const double2 m2 = *reinterpret_cast<const double2*>(r2[e]);
+                                const double2 m3 = *reinterpret_cast<const double2*>(r3[e]);
+                                sg[e] = (0x3564210u >> (4 * m)) & 7u;  // the points whose omega enters with +
+                                double d = W0 + (sg[e] & 1u ? m1.x : -m1.x);
+                                d += sg[e] & 2u ? m2.x : -m2.x;
+                                d += sg[e] & 4u ? m3.x : -m3.x;
+                                const double x = a.half_os2 * (d * d);
+                                const double wt = c * (m == 0 ? ONEBYSIX : 0.5) * (m2.y * m3.y);
+                                const double q = exp_neg(fmin(x, EXP_CUT)) * ((double)sA2[(S3 * s2 + y) * 32 + L] * k1) * wt;
+                                g[e] = ix < nh && x < EXP_CUT ? q : 0.0;
                             }
-                        }
-                        const double W0 = S.w0[s0], W1 = m1.x, W2 = m2.x, W3 = m3.x;
-                        const double Wv = (double)a2 * S.ob0[s0] * m1.y * m2.y * m3.y * a.mfac;
-                        const double dd[7] = {W0 - W1 - W2 - W3, W0 + W1 - W2 - W3, W0 + W2 - W1 - W3,
-                                              W0 + W3 - W1 - W2, W0 + W2 + W3 - W1, W0 + W1 + W3 - W2,
-                                              W0 + W1 + W2 - W3};
-                        const int cw[7] = {c1, c2[0], c2[1], c2[2], c3[0], c3[1], c3[2]};
-                        double gm[7], xs[7];
-                        unsigned need = 0u;  // the terms of this quad inside the cut
+                            // occupations: 1 + n of the points with +, n of the others
 #pragma unroll
-                        for (int m = 0; m < 7; ++m) {
-                            gm[m] = 0.0;
-                            xs[m] = a.half_os2 * (dd[m] * dd[m]);
-                            if (cw[m] != 0 && xs[m] < EXP_CUT) need |= 1u << m;
-                        }
-                        if (need == 0u) continue;
-                        // one exp call site for whichever terms a lane needs (lanes needing different
-                        // terms run it together); the values are those of the term-by-term form
-                        while (need != 0u) {
-                            const int m = __ffs(need) - 1;
-                            need &= need - 1u;
-                            double x = xs[0];
-                            int c = cw[0];
+                            for (int T = 0; T < NT; ++T) {
+                                if (T >= a.nT) break;
+                                const double n1 = r1[2 + T], p1 = 1.0 + n1;
 #pragma unroll
-                            for (int k = 1; k < 7; ++k)
-                                if (m == k) {
-                                    x = xs[k];
-                                    c = cw[k];
+                                for (int e = 0; e < 2; ++e) {
+                                    const double n2 = r2[e][2 + T], n3 = r3[e][2 + T];
+                                    acc[T] += g[e] * ((sg[e] & 1u ? p1 : n1) * (sg[e] & 2u ? 1.0 + n2 : n2) *
+                                                      (sg[e] & 4u ? 1.0 + n3 : n3));
                                 }
-                            const double wt = m == 0 ? c * ONEBYSIX : c * 0.5;
-                            const double g = (a.pre * exp(-x)) * wt * Wv;
-#pragma unroll
-                            for (int k = 0; k < 7; ++k)
-                                if (m == k) gm[k] = g;
-                        }
-                        // occupation factors of the seven terms, per temperature:
-                        // n1 n2 n3, (1+n1) n2 n3, (1+n2) n1 n3, (1+n3) n1 n2, (1+n2)(1+n3) n1,
-                        // (1+n1)(1+n3) n2, (1+n1)(1+n2) n3, over n0
-#pragma unroll
-                        for (int T = 0; T < 9; ++T) {
-                            if (T >= a.nT) break;
-                            double n2, n3;
-                            if (a.nT <= 4 && T < 4) {
-                                n2 = T == 0 ? n2a.x : T == 1 ? n2a.y : T == 2 ? n2b.x : n2b.y;
-                                n3 = T == 0 ? n3a.x : T == 1 ? n3a.y : T == 2 ? n3b.x : n3b.y;
-                            } else {
-                                n2 = r2[2 + T];
-                                n3 = r3[2 + T];
                             }
-                            const double n1 = r1[2 + T];
-                            const double p1 = 1.0 + n1, p2 = 1.0 + n2, p3 = 1.0 + n3;
-                            const double f = gm[0] * (n1 * n2 * n3) + gm[1] * (p1 * n2 * n3) + gm[2] * (p2 * n1 * n3) +
-                                             gm[3] * (p3 * n1 * n2) + gm[4] * (p2 * p3 * n1) + gm[5] * (p1 * p3 * n2) +
-                                             gm[6] * (p1 * p2 * n3);
-                            acc[T] += f * S.n0inv[T][s0];
                         }
+                        __syncwarp();
                     }
                 }
                 // this chunk's sums of s0: warp reduction, one shared-memory add per warp
 #pragma unroll
-                for (int T = 0; T < 9; ++T) {
+                for (int T = 0; T < NT; ++T) {
                     if (T >= a.nT) break;
-                    double vv = acc[T];
+                    double vv = acc[T] * S.n0inv[T][s0];
                     for (int o = 16; o > 0; o >>= 1) vv += __shfl_down_sync(0xffffffffu, vv, o);
                     if (lane == 0 && vv != 0.0) atomicAdd(&S.rate[s0][T], vv);
                 }
@@ -734,7 +812,7 @@ int run_v4tc_gauss(spring_ctx* c, int q0_first, int n_q0, double sigma, const in
     std::vector<short> hmap;
     SPRING_CHECK(v4_blocks(c, bk, hmap));
     const size_t abytes = (size_t)H * QT * bk.ktot * 2, bbytes = (size_t)CROWS * bk.ktot * 2;
-    const size_t smem = abytes + bbytes + (size_t)2 * QT * E2S * 8 + sizeof(V4Sm);
+    const size_t smem = abytes + bbytes + WORK_BYTES + sizeof(V4Sm);
     if (smem > 227 * 1024) return fail(c, SPRING_ERR_UNSUPPORTED, "tensor-core V4 needs %zu bytes of shared memory", smem);
     const size_t bimg_smem = (size_t)2 * H * CROWS * bk.ktot * 2 + (size_t)2 * KA * NM * 8;
     if (bimg_smem > 227 * 1024) return fail(c, SPRING_ERR_UNSUPPORTED, "V4 operand images need %zu bytes", bimg_smem);
@@ -764,7 +842,8 @@ int run_v4tc_gauss(spring_ctx* c, int q0_first, int n_q0, double sigma, const in
     k4_modes<<<(int)std::min<long long>(((long long)nq * NM * rs + threads - 1) / threads, 148LL * 16), threads, 0,
                c->stream>>>(nq, c->nT, rs, c->ph_grid.omega.p, c->ph_grid.oneby.p, c->ph_grid.nbe.p, c->d_v4_rec.p);
     SPRING_CHECK(launch_check(c, "k4_modes"));
-    cudaFuncSetAttribute(k_v4tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto* kern = c->nT <= 1 ? k_v4tc<1> : c->nT <= 4 ? k_v4tc<4> : k_v4tc<9>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaFuncSetAttribute(k4_bimg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bimg_smem);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
@@ -832,7 +911,7 @@ int run_v4tc_gauss(spring_ctx* c, int q0_first, int n_q0, double sigma, const in
         const int grid = (ntiles + a.tiles_per_cta - 1) / a.tiles_per_cta;
         SPRING_CHECK(zero(c, c->d_v4_stat.p + 1, sizeof(int), "V4 status"));
         if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "v4tc: injected launch failure");
-        k_v4tc<<<grid, V4_THREADS, smem, c->stream>>>(
+        kern<<<grid, V4_THREADS, smem, c->stream>>>(
             a, bk, c->d_v4_tiles.p, d_quart, reinterpret_cast<const __nv_bfloat16*>(c->d_v4_img.p), c->d_v4_ph.p,
             c->d_v4_etab.p, c->d_v4_wf.p, c->ph_irr.omega.p + (size_t)q0 * NM, c->ph_irr.oneby.p + (size_t)q0 * NM,
             c->ph_irr.nbe.p + (size_t)q0 * NM, c->d_v4_rec.p, d_rate, c->d_v4_stat.p + 1);

@@ -114,3 +114,18 @@ def test_v4tc_branch_mask(runs):
     for it in range(len(TEMPS)):
         np.testing.assert_allclose(rate[it][sel], full[it][sel], rtol=1e-12, atol=1e-300)
         assert not rate[it][~sel].any()
+
+
+@pytest.mark.parametrize("nT,sigma", [(1, 0.05), (4, 20.0), (5, 2.0), (9, 20.0)])
+def test_v4tc_term_lists(cr4, nT, sigma):
+    """Windows from nearly empty to all (more terms than one list of a warp holds) and every temperature class."""
+    temps = list(np.linspace(200.0, 1000.0, nT))
+    ctx, info = from_crystal(cr4, (4, 3, 3), temps, W=np.eye(3, dtype=np.int32)[None], Rxyz=np.eye(3)[None],
+                             with_fc4=True)
+    out = {}
+    for prec in ("fp64", "bf16x3"):
+        ctx.set_precision(prec)
+        out[prec] = ctx.linewidth4(1, 6, delta="gauss", sigma=sigma)
+    ctx.close()
+    assert out["fp64"].max() > 0
+    assert _max_rel(out["bf16x3"], out["fp64"]) < TOL["bf16x3"]
