@@ -142,10 +142,18 @@ struct V4Smem {
     double wq[QB][3][N];           // omega of the quartet's three grid points
     double nq[QB][9][3][N];        // their occupations per temperature
     int g[QB][4];                  // g1 g2 g3 valid
+    unsigned short slot[NA_MAX * NA_MAX * NA_MAX];  // (n1 na + n2) na + n3 by block of basis atoms
 };
 
+// One CTA works off groups of QB quartets.  Most of the work is D4: FC4, 444 KB out of L2, against the triple
+// phase products.  The neighbour triples are put in the order of their (nu, eta, ro) blocks, so that a block is
+// one loop with its loads in flight ahead; four lanes share an entry's sum and each loaded value serves the QB
+// quartets.  5^3, ten q0 (26 700 quartets): 4.45 -> 3.27 ms against one thread per (quartet, entry) with a loop
+// nest over the blocks' neighbours (D4 61 000 -> 35 000 of a group's 82 000 -> 57 000 cycles per atom), where
+// the L2 reads are the bound (about 6 TB/s).
+constexpr int V4T = 352;  // 81 entries x 4 lanes, in whole warps
 template <int EPI>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(V4T, 2)
 k_v4(V4Args a, const int4* __restrict__ quart, const double* __restrict__ fc4, const double* __restrict__ posr,
      const int* __restrict__ btyp, const int* __restrict__ off, const double* __restrict__ mrs,
      const double* __restrict__ qpnt, const int* __restrict__ q0int, const double2* __restrict__ ev0,
@@ -180,6 +188,7 @@ k_v4(V4Args a, const int4* __restrict__ quart, const double* __restrict__ fc4, c
         }
         for (int i = tid; i < QB * 1296; i += nt) S.phi[i / 1296][i % 1296] = make_double2(0.0, 0.0);
         for (int mu = 0; mu < NB; ++mu) {
+            const int* o = off + mu * (NB + 1);
             for (int i = tid; i < QB * 3 * na; i += nt) {
                 const int p = i / (3 * na), k = (i / na) % 3, Nn = i % na;
                 const int gg = S.g[p][k];
@@ -198,44 +207,51 @@ k_v4(V4Args a, const int4* __restrict__ quart, const double* __restrict__ fc4, c
                 const double* y = S.ph[p][1][n2];
                 const double* z = S.ph[p][2][n3];
                 const double xr = x[0] * y[0] - x[1] * y[1], xi = x[0] * y[1] + x[1] * y[0];
-                S.ppp[p][(n1 * na + n2) * na + n3] = make_double2(xr * z[0] - xi * z[1], xr * z[1] + xi * z[0]);
+                // slots are sorted by basis atom: place among the (nu, eta, ro) blocks
+                const int h = o[1], c[2] = {h, na - h};
+                const int nu = n1 >= h, eta = n2 >= h, ro = n3 >= h;
+                const int m1 = n1 - nu * h, m2 = n2 - eta * h, m3 = n3 - ro * h;
+                const int k = nu * h * na * na + c[nu] * (eta * h * na + c[eta] * ro * h) + (m1 * c[eta] + m2) * c[ro] + m3;
+                S.ppp[p][k] = make_double2(xr * z[0] - xi * z[1], xr * z[1] + xi * z[0]);
+                if (p == 0) S.slot[k] = (unsigned short)((n1 * na + n2) * na + n3);
             }
             __syncthreads();
-            // D4: thread per (pair, abcd); all eight (nu, eta, ro) blocks in registers
-            const int* o = off + mu * (NB + 1);
-            for (int u = tid; u < QB * 81; u += nt) {
-                const int p = u / 81, r = u % 81;
-                double2 acc[NB][NB][NB];
-#pragma unroll
-                for (int x = 0; x < NB; ++x)
-#pragma unroll
-                    for (int y = 0; y < NB; ++y)
-#pragma unroll
-                        for (int z = 0; z < NB; ++z) acc[x][y][z] = make_double2(0.0, 0.0);
-                const double* f = fc4 + (size_t)mu * na * na * na * 81 + r;
-#pragma unroll
-                for (int nu = 0; nu < NB; ++nu)
-                    for (int n1 = o[nu]; n1 < o[nu + 1]; ++n1)
-#pragma unroll
-                        for (int eta = 0; eta < NB; ++eta)
-                            for (int n2 = o[eta]; n2 < o[eta + 1]; ++n2)
-#pragma unroll
-                                for (int ro = 0; ro < NB; ++ro)
-                                    for (int n3 = o[ro]; n3 < o[ro + 1]; ++n3) {
-                                        const int s = (n1 * na + n2) * na + n3;
-                                        const double fv = __ldg(f + (size_t)s * 81);
-                                        const double2 q = S.ppp[p][s];
-                                        acc[nu][eta][ro].x = fma(fv, q.x, acc[nu][eta][ro].x);
-                                        acc[nu][eta][ro].y = fma(fv, q.y, acc[nu][eta][ro].y);
-                                    }
+            // D4: four lanes per entry abcd, both quartets; the eight (nu, eta, ro) blocks in turn
+            for (int u = tid; u < V4T; u += nt) {
+                const int rr = u >> 2, j = u & 3, r = min(rr, 80);
                 const int al = r / 27, be = (r / 9) % 3, ga = (r / 3) % 3, de = r % 3;
+                const double* f = fc4 + (size_t)mu * na * na * na * 81 + r;
+                const int c[2] = {o[1], na - o[1]};
+                int k0 = 0;
+#pragma unroll 1
+                for (int b = 0; b < 8; ++b) {
+                    const int nu = b >> 2, eta = (b >> 1) & 1, ro = b & 1;
+                    const int k1 = k0 + (nu ? c[1] : c[0]) * (eta ? c[1] : c[0]) * (ro ? c[1] : c[0]);
+                    double2 acc[QB];
 #pragma unroll
-                for (int nu = 0; nu < NB; ++nu)
+                    for (int p = 0; p < QB; ++p) acc[p] = make_double2(0.0, 0.0);
+#pragma unroll 6
+                    for (int k = k0 + j; k < k1; k += 4) {
+                        const double fv = __ldg(f + (size_t)S.slot[k] * 81);
 #pragma unroll
-                    for (int eta = 0; eta < NB; ++eta)
+                        for (int p = 0; p < QB; ++p) {
+                            const double2 q = S.ppp[p][k];
+                            acc[p].x = fma(fv, q.x, acc[p].x);
+                            acc[p].y = fma(fv, q.y, acc[p].y);
+                        }
+                    }
+                    k0 = k1;
 #pragma unroll
-                        for (int ro = 0; ro < NB; ++ro)
-                            S.A[p][((al * 6 + nu * 3 + be) * 6 + eta * 3 + ga) * 6 + ro * 3 + de] = acc[nu][eta][ro];
+                    for (int p = 0; p < QB; ++p) {
+                        double2 v = acc[p];
+                        for (int w = 1; w < 4; w *= 2) {
+                            v.x += __shfl_xor_sync(0xffffffffu, v.x, w);
+                            v.y += __shfl_xor_sync(0xffffffffu, v.y, w);
+                        }
+                        if (j == p && rr < 81)
+                            S.A[p][((al * 6 + nu * 3 + be) * 6 + eta * 3 + ga) * 6 + ro * 3 + de] = v;
+                    }
+                }
             }
             __syncthreads();
             // T1[a nb ec][s3] = sum_rd D4[a nb ec][rd] e3(rd, s3)
@@ -807,7 +823,7 @@ int run_lw4(spring_ctx* c, int q0_first, int n_q0, int delta_mode, double sigma,
         const int* q0i = c->d_irr_int.p + 3 * q0;
         if (delta_mode == SPRING_DELTA_GAUSS) {
             if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "v4: injected launch failure"); break; }
-            k_v4<0><<<grid, 256, smem, c->stream>>>(a, b.quart.p, c->d_fc4.p, c->d_fc4_posr.p, c->d_fc4_btyp.p,
+            k_v4<0><<<grid, V4T, smem, c->stream>>>(a, b.quart.p, c->d_fc4.p, c->d_fc4_posr.p, c->d_fc4_btyp.p,
                                                     c->d_fc4_off.p, c->d_mass_rs.p, c->d_qpnt.p, q0i, ev0, om0, ob0,
                                                     nbe0, c->ph_grid.evec.p, c->ph_grid.omega.p, c->ph_grid.oneby.p,
                                                     c->ph_grid.nbe.p, d_rate, nullptr);
@@ -822,7 +838,7 @@ int run_lw4(spring_ctx* c, int q0_first, int n_q0, int delta_mode, double sigma,
             }
             if ((rc = dalloc(c, wq, (size_t)a.nquart * 1296, "quartet W")) != SPRING_OK) break;
             if (launch_injected(c)) { rc = fail(c, SPRING_ERR_INJECTED, "v4: injected launch failure"); break; }
-            k_v4<1><<<grid, 256, smem, c->stream>>>(a, b.quart.p, c->d_fc4.p, c->d_fc4_posr.p, c->d_fc4_btyp.p,
+            k_v4<1><<<grid, V4T, smem, c->stream>>>(a, b.quart.p, c->d_fc4.p, c->d_fc4_posr.p, c->d_fc4_btyp.p,
                                                     c->d_fc4_off.p, c->d_mass_rs.p, c->d_qpnt.p, q0i, ev0, om0, ob0,
                                                     nbe0, c->ph_grid.evec.p, c->ph_grid.omega.p, c->ph_grid.oneby.p,
                                                     c->ph_grid.nbe.p, nullptr, wq.p);
