@@ -347,9 +347,9 @@ const char* spring_batch_last_error(const spring_batch* batch);
 int spring_batch_add_linewidth3(spring_batch* batch, spring_ctx* ctx, int i0_first, int n_q0, double sigma,
                                 const int* pol3, int* index);
 /* Launch configuration of the persistent kernel (288 threads per CTA):
- * config[0] 1 = two-atom cells (7-atom FC3 clusters, <= 9 temperatures) run as
- * groups of 8 pairs in the specialised layout, 0 = every cell as (pair, s0
- * block) items of the any-cell layout; config[1] CTAs per SM (0 = as many as
+ * config[0] 1 = two-atom cells (7-atom FC3 clusters, <= 9 temperatures) run
+ * their own kernel after the graph, 0 = they too are (pair, s0 block) items of
+ * the any-cell layout; config[1] CTAs per SM (0 = as many as
  * fit); config[2] s0 block for cells with Ndof > 12 (0 = 6, or 6, 12, 24);
  * config[3] work items taken per scheduler step.  Default {1, 0, 0, 1}. */
 int spring_batch_set_config(spring_batch* batch, const int* config);

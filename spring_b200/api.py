@@ -507,7 +507,7 @@ class Batch:
         return lw, om
 
     def set_config(self, two_atom=1, ctas_per_sm=0, s0_block=0, chunk=1):
-        """two_atom: run two-atom cells in the specialised 8-pair layout; ctas_per_sm (0: as many as
+        """two_atom: two-atom cells by their own kernel after the graph; ctas_per_sm (0: as many as
         fit); s0_block for Ndof > 12 (0: 6); chunk: work items per scheduler step."""
         cfg = np.array([two_atom, ctas_per_sm, s0_block, chunk], dtype=np.int32)
         self._call("spring_batch_set_config", _ptr(cfg))

@@ -147,11 +147,11 @@ struct V4Smem {
 
 // One CTA works off groups of QB quartets.  Most of the work is D4: FC4, 444 KB out of L2, against the triple
 // phase products.  The neighbour triples are put in the order of their (nu, eta, ro) blocks, so that a block is
-// one loop with its loads in flight ahead; four lanes share an entry's sum and each loaded value serves the QB
-// quartets.  5^3, ten q0 (26 700 quartets): 4.45 -> 3.27 ms against one thread per (quartet, entry) with a loop
-// nest over the blocks' neighbours (D4 61 000 -> 35 000 of a group's 82 000 -> 57 000 cycles per atom), where
-// the L2 reads are the bound (about 6 TB/s).
-constexpr int V4T = 352;  // 81 entries x 4 lanes, in whole warps
+// one loop with its loads in flight ahead; a warp reads 32 consecutive entries abcd of a triple, each for QB
+// quartets, and two warps share their sums.  Bound by the L2 reads and their latency.  5^3, ten q0 (26 700
+// quartets): 4.45 -> 2.75 ms against one thread per (quartet, entry) with a loop nest over the blocks' neighbours
+// (3.27 with four lanes per entry: 64-byte pieces of unaligned rows).
+constexpr int V4T = 256;
 template <int EPI>
 __global__ void __launch_bounds__(V4T, 2)
 k_v4(V4Args a, const int4* __restrict__ quart, const double* __restrict__ fc4, const double* __restrict__ posr,
@@ -216,11 +216,11 @@ k_v4(V4Args a, const int4* __restrict__ quart, const double* __restrict__ fc4, c
                 if (p == 0) S.slot[k] = (unsigned short)((n1 * na + n2) * na + n3);
             }
             __syncthreads();
-            // D4: four lanes per entry abcd, both quartets; the eight (nu, eta, ro) blocks in turn
-            for (int u = tid; u < V4T; u += nt) {
-                const int rr = u >> 2, j = u & 3, r = min(rr, 80);
-                const int al = r / 27, be = (r / 9) % 3, ga = (r / 3) % 3, de = r % 3;
-                const double* f = fc4 + (size_t)mu * na * na * na * 81 + r;
+            // D4: the eight (nu, eta, ro) blocks in turn, both quartets; even triples into A, odd ones into B
+            if (tid < 6 * 32) {
+                const int j = tid / 96, r = tid % 96, rc = min(r, 80);
+                const int al = rc / 27, be = (rc / 9) % 3, ga = (rc / 3) % 3, de = rc % 3;
+                const double* f = fc4 + (size_t)mu * na * na * na * 81 + rc;
                 const int c[2] = {o[1], na - o[1]};
                 int k0 = 0;
 #pragma unroll 1
@@ -230,8 +230,8 @@ k_v4(V4Args a, const int4* __restrict__ quart, const double* __restrict__ fc4, c
                     double2 acc[QB];
 #pragma unroll
                     for (int p = 0; p < QB; ++p) acc[p] = make_double2(0.0, 0.0);
-#pragma unroll 6
-                    for (int k = k0 + j; k < k1; k += 4) {
+#pragma unroll 12
+                    for (int k = k0 + j; k < k1; k += 2) {
                         const double fv = __ldg(f + (size_t)S.slot[k] * 81);
 #pragma unroll
                         for (int p = 0; p < QB; ++p) {
@@ -241,17 +241,18 @@ k_v4(V4Args a, const int4* __restrict__ quart, const double* __restrict__ fc4, c
                         }
                     }
                     k0 = k1;
+                    if (r < 81)
 #pragma unroll
-                    for (int p = 0; p < QB; ++p) {
-                        double2 v = acc[p];
-                        for (int w = 1; w < 4; w *= 2) {
-                            v.x += __shfl_xor_sync(0xffffffffu, v.x, w);
-                            v.y += __shfl_xor_sync(0xffffffffu, v.y, w);
-                        }
-                        if (j == p && rr < 81)
-                            S.A[p][((al * 6 + nu * 3 + be) * 6 + eta * 3 + ga) * 6 + ro * 3 + de] = v;
-                    }
+                        for (int p = 0; p < QB; ++p)
+                            (j ? S.B : S.A)[p][((al * 6 + nu * 3 + be) * 6 + eta * 3 + ga) * 6 + ro * 3 + de] = acc[p];
                 }
+            }
+            __syncthreads();
+            for (int i = tid; i < QB * 648; i += nt) {
+                const double2 x = S.B[i / 648][i % 648];
+                double2& y = S.A[i / 648][i % 648];
+                y.x += x.x;
+                y.y += x.y;
             }
             __syncthreads();
             // T1[a nb ec][s3] = sum_rd D4[a nb ec][rd] e3(rd, s3)

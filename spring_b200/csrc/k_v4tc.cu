@@ -749,7 +749,7 @@ k_v4tc(V4Args a, Blk4 bk, const int4* __restrict__ tiles, const int4* __restrict
 #pragma unroll
                 for (int T = 0; T < NT; ++T) {
                     if (T >= a.nT) break;
-                    double vv = acc[T] * S.n0inv[T][s0];
+                    double vv = acc[T] != 0.0 ? acc[T] * S.n0inv[T][s0] : 0.0;  // n0 = 0 at Gamma's acoustic modes
                     for (int o = 16; o > 0; o >>= 1) vv += __shfl_down_sync(0xffffffffu, vv, o);
                     if (lane == 0 && vv != 0.0) atomicAdd(&S.rate[s0][T], vv);
                 }

@@ -129,3 +129,4 @@ def test_v4tc_term_lists(cr4, nT, sigma):
     ctx.close()
     assert out["fp64"].max() > 0
     assert _max_rel(out["bf16x3"], out["fp64"]) < TOL["bf16x3"]
+    assert np.isfinite(out["bf16x3"]).all() and not out["bf16x3"][out["fp64"] == 0].any()  # Gamma's acoustic modes
