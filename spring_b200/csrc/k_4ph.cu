@@ -830,10 +830,11 @@ int run_lw4(spring_ctx* c, int q0_first, int n_q0, int delta_mode, double sigma,
                                                     c->ph_grid.nbe.p, d_rate, nullptr);
             rc = launch_check(c, "k_v4<gauss>");
         } else {
-            size_t free_b = 0, total_b = 0;
-            cudaMemGetInfo(&free_b, &total_b);
+            // asking for the free memory takes up to milliseconds on a busy host: only to grow the buffer
             const size_t need = (size_t)a.nquart * 1296 * sizeof(double);
-            if (need > (free_b + wq.n * sizeof(double)) / 2) {
+            size_t free_b = 0, total_b = 0;
+            if (need > wq.n * sizeof(double)) cudaMemGetInfo(&free_b, &total_b);
+            if (need > wq.n * sizeof(double) && need > (free_b + wq.n * sizeof(double)) / 2) {
                 rc = fail(c, SPRING_ERR_UNSUPPORTED, "tetrahedron four-phonon W of one q0 needs %zu bytes", need);
                 break;
             }

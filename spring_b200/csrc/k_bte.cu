@@ -861,12 +861,12 @@ int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* 
             k_bte_wf<<<std::min((nq * n + 255) / 256, 148 * 8), 256, 0, c->stream>>>(nq, n, c->ph_grid.omega.p, w.wf.p);
             rc = launch_check(c, "k_bte_wf");
         }
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
+        // entries to store at most; the free memory is asked for only when the kept buffers are too small
         const long long per = sizeof(int2) + sizeof(double2);
         const long long held = (long long)std::min(c->d_bt_kk.n, c->d_bt_pq.n);
-        long long most = std::max<long long>(held, (long long)(std::min((size_t)40 << 30, free_b / 2) / per));
-        most = std::min<long long>(most, c->bte_max_entries < 0 ? 0x7fffffffLL : c->bte_max_entries);
+        const long long cap_entries = c->bte_max_entries < 0 ? 0x7fffffffLL : c->bte_max_entries;
+        long long most = std::min(held, cap_entries);
+        bool asked = false;
         long long total = 0;
         stored = true;
         for (int b = 0; rc == SPRING_OK && stored && b < ntr; b += batch) {
@@ -880,6 +880,13 @@ int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* 
             int here = 0;
             if ((rc = d2h(c, &here, w.boff.p + segs, sizeof here, "operator count")) != SPRING_OK) break;
             const long long need = total + here;
+            if (need > most && !asked) {
+                size_t free_b = 0, total_b = 0;
+                cudaMemGetInfo(&free_b, &total_b);
+                most = std::max<long long>(held, (long long)(std::min((size_t)40 << 30, free_b / 2) / per));
+                most = std::min(most, cap_entries);
+                asked = true;
+            }
             if (need > most) { stored = false; break; }
             if (need > (long long)std::min(c->d_bt_kk.n, c->d_bt_pq.n)) {
                 // room for the remaining rows at the fill seen so far
