@@ -546,7 +546,7 @@ PATH_NODES = np.array([[0.0, 0.0, 0.0, 0], [0.0, 0.5, 0.5, 50], [0.25, 0.625, 0.
 def batched_leg(torch, steps=3):
     """Batched uneven workload: the 2-atom cell at 12^3/16^3/20^3 and the 8-atom cubic cell at
     8^3/10^3, 9 temperatures (100-900 K), Gaussian three-phonon linewidths of every irreducible q0
-    of all five in one persistent, graph-captured launch with the autotuned configuration; then
+    of all five in one batch run with the autotuned configuration; then
     Gaussian linewidths at 200 path points (Gamma-X-W-K-Gamma-L) on the 2-atom 12^3 context.
     Compared with each context's own spring_linewidth3 call (FP64) one after the other."""
     from spring_b200 import synthetic as S
@@ -646,8 +646,8 @@ def batched_leg(torch, steps=3):
                              "items_per_step": cfg[3]},
             "tuning": {"configs_tried": tried, "best_trial_ms": tuned_ms},
             "path_points": int(len(q)), "path_ms": path_ms, "path_mesh": [12, 12, 12],
-            "what": "one persistent FP64 launch over all five workloads' (pair, s0-block) items, heaviest "
-                    "first, replayed from a CUDA graph; path points on the 12^3 context afterwards",
+            "what": "one FP64 batch run over all five workloads, each cell's own kernel after the graph; path points "
+                    "on the 12^3 context afterwards",
             "mixed": {"batch_ms": batch_mixed, "separate_calls_ms": sep_mixed,
                       "separate_over_batch": sep_mixed / batch_mixed,
                       "evals_per_s_batch": (evals + path_evals) / (batch_mixed * 1e-3),
@@ -655,7 +655,7 @@ def batched_leg(torch, steps=3):
                       "path_evals_per_T": path_evals,
                       "max_rel_diff_vs_separate": err_m, "path_max_rel_diff_vs_separate": err_p,
                       "what": "two-atom workloads on BF16x3 through the tensor-core pass (the kernel of "
-                              "spring_linewidth3), 8-atom workloads in the persistent FP64 kernel, the 200 "
+                              "spring_linewidth3), 8-atom workloads in their FP64 matrix kernel, the 200 "
                               "path points inside the batch's CUDA graph; against each context's own call "
                               "with the same precision plus the path call, one after the other"}}
 

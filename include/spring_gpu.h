@@ -324,7 +324,7 @@ int spring_kappa_iter(spring_ctx* ctx, double eps_k, int max_iter, double* kappa
 int spring_kappa_iter_gauss(spring_ctx* ctx, double sigma, double eps_k, int max_iter, double* kappa,
                             double* kappa_rta, int* iters, double* stats);
 
-/* ---- batched linewidths (several workloads, one persistent launch) ------ */
+/* ---- batched linewidths (several workloads, one run) ------------------- */
 /* A batch holds Gaussian three-phonon linewidth requests on several contexts
  * (different cells, meshes and temperature sets, on one device) and runs them
  * as one persistent FP64 kernel over all their (pair, s0-block) work items,
@@ -336,8 +336,8 @@ int spring_kappa_iter_gauss(spring_ctx* ctx, double sigma, double eps_k, int max
  * process.  Requests on one context must not overlap in q0.  A request on a
  * two-atom context set to SPRING_BF16 / SPRING_BF16X3 runs through the
  * tensor-core pass of spring_linewidth3 (same kernel, same results) right
- * after the graph, inside the same spring_batch_run, and a request on a cell of
- * four or more atoms through the FP64 matrix kernel there; path requests
+ * after the graph, inside the same spring_batch_run, and FP64 requests on
+ * two-atom cells and on cells of four or more atoms through their matrix kernels there; path requests
  * (spring_batch_add_path) are launched inside the graph. */
 typedef struct spring_batch spring_batch;
 int spring_batch_create(spring_batch** batch);

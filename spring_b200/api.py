@@ -459,7 +459,7 @@ def from_crystal(cr, mesh, temps, phonons="device", W=None, Rxyz=None, with_fc3=
 
 class Batch:
     """A ``spring_batch``: Gaussian three-phonon linewidth requests on several contexts (cells,
-    meshes, temperature sets) run as one persistent, graph-captured launch."""
+    meshes, temperature sets) run as one graph-captured launch and the kernels of the cells that have their own."""
 
     def __init__(self):
         self._lib = L.load()

@@ -17,6 +17,7 @@
 // 4*27*sum_mu Na3^2 + 3*8*Ndof^4 flops per pair (41.7 kflop for the 2-atom cell).
 // W = |Phi|^2 (1/w0)(1/w1)(1/w2) Sctr3THz2/Nq, zero for Gamma acoustic modes.
 //
+// Cells of 12 and more branches run k_v3m.cu, two-atom cells k_v3s.cu; this is the form for the others.
 // One CTA handles one (pair, block of s0) work item, so that every tensor fits
 // in shared memory up to Ndof = 24.  Two epilogues:
 //   GAUSS: the pair's contribution to Gamma(q0,s0) for every temperature, fused

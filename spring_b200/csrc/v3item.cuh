@@ -1,5 +1,5 @@
 // The any-cell V3 work item (one pair, one s0 block) shared by the per-call
-// kernel (k_v3.cu) and the batched persistent kernel (k_batch.cu).  Reference
+// kernel (k_v3.cu) and the batched persistent kernel (batch.cu).  Reference
 // citations and the regrouping are described in k_v3.cu.
 #pragma once
 #include "spring_internal.cuh"
