@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(PHT, 2) k_phonons(PhArgs a, PhSet SA, const in
     double2* A = sm;             // [n][ld]
     double2* V = A + n * ld;     // [n][ld]
     double2* dD = V + n * ld;    // [3][n][n]
-    double2* rotE2 = dD + 3 * n * n;                       // [2][m/2] e^{i phi}; this round's and the last one's
+    double2* rotE2 = dD + 3 * n * n;                       // [2][m/2] e^{i phi}; the current rotations and the ones before
     double* rotC2 = reinterpret_cast<double*>(rotE2 + m);  // [2][m/2]
     double* rotS2 = rotC2 + m;                             // [2][m/2]
     double* lam = rotS2 + m;                               // [m]
