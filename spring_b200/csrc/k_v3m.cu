@@ -106,8 +106,8 @@ __global__ void __launch_bounds__(32 * MW, 1) k_v3m(V3Args a_, V3mLayout L, V3Pt
                         sKo[tid * MAX_NDOF + k] = (mu * 3 + al) * L.TB + 3 * p * L.S2;
                         sKr[tid * MAX_NDOF + k] = 3 * mu + al;
                     }
-        for (; k & 3; ++k) {
-            sKo[tid * MAX_NDOF + k] = 0;
+        for (; k & 3; ++k) {  // times zero: any block of T1 that is written (the first is not where atom 0 has no slots)
+            sKo[tid * MAX_NDOF + k] = sKo[tid * MAX_NDOF + k - 1];
             sKr[tid * MAX_NDOF + k] = n;
         }
         sKh[tid] = k;

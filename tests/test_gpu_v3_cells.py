@@ -50,3 +50,30 @@ def test_v3_cells_match_oracle(name, nT, pol):
             np.testing.assert_allclose(lw[it, i0], g["lw"], rtol=1e-9, atol=1e-14 * np.abs(lw).max())
         np.testing.assert_allclose(p3[i0], g["p3_q0"], rtol=1e-9, atol=1e-14 * np.abs(p3).max())
     ctx.close()
+
+
+def test_first_atom_without_fc3_neighbours_matches_oracle():
+    """No FC3 on the first atom: its part of the intermediate sums is never formed, and what lies in its place in
+    shared memory (here NaN, left there by a run with undefined eigenvectors) must not reach W."""
+    cr = _cell("nb4")
+    mesh, temps = (7, 3, 2), [300.0]              # about 900 pairs: every SM takes part
+    ident = np.eye(3, dtype=np.int32)[None]
+    kw = dict(W=ident, Rxyz=np.eye(3)[None])
+    st = D.Setup(cr, mesh, temps, **kw)
+    bad = dict(st.ph, evec=np.full_like(st.ph["evec"], np.nan))
+    before, _ = from_crystal(cr, mesh, temps, phonons={"grid": bad, "irr": st.ph0}, **kw)
+    cr.fc3_atm_num[0] = 0
+    ctx, _ = from_crystal(cr, mesh, temps, phonons={"grid": st.ph, "irr": st.ph0}, **kw)
+    for c in (before, ctx):                       # both prepared: nothing else runs between the two calls below
+        c.linewidth3(1, st.nq0, "gauss", 1.5)
+    before.linewidth3(1, st.nq0, "gauss", 1.5)
+    lw, _ = ctx.linewidth3(1, st.nq0, "gauss", 1.5)
+    assert np.all(np.isfinite(lw))
+    for i0 in (0, 5, st.nq0 - 1):
+        r = D.linewidth3_q0(st, i0, "gauss", 1.5, with_w=True)
+        np.testing.assert_allclose(lw[0, i0], r["lw"], rtol=1e-9, atol=1e-14 * np.abs(lw).max())
+        before.linewidth3(1, st.nq0, "gauss", 1.5)
+        w = ctx.scatter_w3(i0 + 1)
+        np.testing.assert_allclose(w, r["sctr"], rtol=1e-9, atol=1e-12 * r["sctr"].max())
+    before.close()
+    ctx.close()
