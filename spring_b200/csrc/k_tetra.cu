@@ -14,7 +14,9 @@
 // records (n(T), w), both laid out [s][q] so that a warp's neighbouring tetrahedra share cache lines.
 // With the same branch window on both legs the sums use the partner map's symmetry: p maps the
 // tetrahedra onto themselves and swaps the legs, W with them, so channel 3 equals channel 2 (weight 2)
-// and channel 1 needs s1 <= s2 only (weight 2 off the diagonal).
+// and channel 1 needs s1 <= s2 only (weight 2 off the diagonal).  W is stored both ways round for a pair of
+// different points; where q1 = p(q1) (at most eight points) W(s1, s2) equals W(s2, s1) only for FC3 that is
+// symmetric in its two neighbours, so the fold takes their mean there.
 // Case bounds and formulas follow the reference; the summation order differs (per-lane sums, then
 // warp/CTA reduction).
 // Roofline: issue (the screen) and the FP64 pipe (the evaluation); W is read from the L2-resident grid.
@@ -148,7 +150,12 @@ __global__ void __launch_bounds__(32 * TW, 3) k_tetra3(TetArgs a, const int4* __
             const double sg = !SYM && ch == 2 ? -1.0 : f;
             const int col = (si * n + s1) * n + s2;
 #pragma unroll
-            for (int v = 0; v < 4; ++v) A[v] *= sg * W[(size_t)x1[v] * n3 + col];
+            for (int v = 0; v < 4; ++v) {
+                const double* w = W + (size_t)x1[v] * n3;
+                double wv = w[col];
+                if (SYM && x1[v] == x2[v]) wv = 0.5 * (wv + w[(si * n + s2) * n + s1]);  // see the note on the fold
+                A[v] *= sg * wv;
+            }
             double(*o)[32] = acc + si * (NT + 1);
             o[NT][lane] += f * gw;
 #pragma unroll

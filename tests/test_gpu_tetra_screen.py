@@ -94,3 +94,26 @@ def test_isotope_rate_matches_oracle(cell, N, nT, delta):
         for it in range(nT):
             np.testing.assert_allclose(rate[it, i0], ref, rtol=1e-9, atol=1e-14 * max(1.0, np.abs(rate).max()))
     ctx.close()
+
+
+def _uneven(cr, seed=5):
+    """The crystal with force constants that are not symmetric in their two legs."""
+    cr.fc3 = cr.fc3 + np.random.default_rng(seed).normal(0.0, 1.0, size=cr.fc3.shape)
+    return cr
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cell,mesh,nT", [("rocksalt2", (3, 3, 3), 2), ("rocksalt2", (4, 4, 2), 1), ("rocksalt8", (2, 2, 2), 1)])
+def test_tetrahedron_sums_of_unsymmetrised_fc3_match_oracle(cell, mesh, nT):
+    """W of a pair of equal points is not symmetric in its branches then (2^3: every q0 has such points)."""
+    cr = _uneven(S.build(cell))
+    temps = list(np.linspace(100.0, 900.0, nT))
+    st = D.Setup(cr, mesh, temps, W=np.eye(3, dtype=np.int32)[None], Rxyz=np.eye(3)[None])
+    ctx, _ = from_crystal(cr, mesh, temps, phonons={"grid": st.ph, "irr": st.ph0}, W=st.W, Rxyz=st.Rxyz)
+    lw, p3 = ctx.linewidth3(1, st.nq0, delta="tetra")
+    for i0 in range(0, st.nq0, 3):
+        for it in range(nT):
+            r = D.linewidth3_q0(st, i0, delta="tetra", it=it)
+            np.testing.assert_allclose(lw[it, i0], r["lw"], rtol=1e-9, atol=1e-14 * np.abs(lw).max())
+        np.testing.assert_allclose(p3[i0], r["p3_q0"], rtol=1e-9, atol=1e-14 * np.abs(p3).max())
+    ctx.close()
