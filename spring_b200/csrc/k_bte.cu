@@ -20,11 +20,12 @@
 //                             dF term 0.5 (F(u,s2) + F(v,s1));
 // with p(x) = grid(-q0 - x).  Because F(-q) = -F(q), both terms are -(F(x, s1) + F(p(x), s2)) times a
 // coefficient at the grid modes (x, s1), (p(x), s2) - x = -v for the minus channel - that depends on the
-// temperature only through n there.  So the tetrahedron weights are computed once: every (tetrahedron,
-// mode triple) whose energy range holds w0 adds its vertex weights to a dense (P, Q) grid of its q0, and
-// the non-zero entries, with 4 W folded in and the two orderings of a pair merged, go to HBM as rows of
-// the same operator the Gaussian form uses; an iteration is one pass over it.  When the operator does not
-// fit (half the free memory), the (P, Q) grids are rebuilt batch by batch on every pass instead.
+// temperature only through n there (points that are their own inverse: see bte_entry).  So the tetrahedron
+// weights are computed once: every (tetrahedron, mode triple) whose energy range holds w0 adds its vertex
+// weights to a dense (P, Q) grid of its q0, and the non-zero entries, with 4 W folded in and the two
+// orderings of a pair merged, go to HBM as rows of the same operator the Gaussian form uses; an iteration is
+// one pass over it.  When the operator does not fit (half the free memory), the (P, Q) grids are rebuilt batch
+// by batch on every pass instead.
 // Weights: FP32 screen and queued FP64 evaluation as in k_tetra3.  The former kernel evaluated the
 // weights of every tetrahedron again in every iteration.
 // Roofline: FP64 ALU for the weights, HBM / L2 (24 bytes and two gathers per entry) for the iterations.
@@ -181,36 +182,48 @@ __global__ void __launch_bounds__(32 * TW, 4) k_bte_weights(WgtArgs a, const int
     }
 }
 
-// The merged entry of grid modes (x, s1), (p(x), s2) of one row, element j = (s1 n + s2) nq + x of its
-// (P, Q) block: both orderings of the pair share W and F(x, s1) + F(p(x), s2).  False when another
-// element stands for it or it is zero.
-__device__ __forceinline__ bool bte_entry(int j, int n, int nq, int s0, const int* __restrict__ p,
-                                          const double2* __restrict__ pq, const double* __restrict__ W, int2& kk,
-                                          double2& e) {
-    const int x = j % nq, s12 = j / nq, s1 = s12 / n, s2 = s12 % n, px = p[x];
-    if (px < x || (px == x && s2 < s1)) return false;
-    const double2 u = pq[j];
-    if (px == x && s1 == s2) {
-        e = make_double2(0.0, u.y);
-    } else {
-        const double2 v = pq[(s2 * n + s1) * nq + px];
-        e = make_double2(u.x - v.x, u.y + v.y);
-    }
-    if (e.x == 0.0 && e.y == 0.0) return false;
-    const double w = 4.0 * W[(size_t)x * n * n * n + (s0 * n + s1) * n + s2];
-    if (w == 0.0) return false;
-    e.x *= w;
-    e.y *= w;
-    kk = make_int2(x * n + s1, px * n + s2);
-    return true;
-}
-
 struct RowArgs {
     int n, nq, q0_first;
     const int* partner;    // [ntr][nq]
+    const int* neg;        // [nq]
     const double2* pq;     // [slot][s0][s1][s2][x]
     const double* wgrid;   // [slot][x][s0][s1][s2]
 };
+
+// The merged entries of grid modes k1 = (x, s1), k2 = (p(x), s2) of one row, element j = (s1 n + s2) nq + x of its
+// (P, Q) block.  With c = (n1 - n2) P + (1 + n1 + n2) Q of e[0], both orderings of the pair add c to 1/tau and
+// -c (F(k1) + F(k2)) to dF.  W is stored both ways round for different points; at x = p(x) W(s1, s2) and
+// W(s2, s1) differ unless FC3 is symmetric in its two neighbours, and so do their terms.
+// The sum F(k1) + F(k2) comes of F(-q) = -F(q).  A point that is its own inverse has F(-q) = F(q) instead, and F
+// vanishes there only when W is the same for (q1, q2) and (-q1, -q2) - again with symmetric FC3 only.  e[1] and
+// e[2] (in the same form, n of their own mode first) are what is missing from F(k1) and F(k2) then, to be
+// subtracted from dF and not part of 1/tau.
+// Returns which of the three are not zero, bit by bit; none when another element stands for this one.
+__device__ __forceinline__ unsigned bte_entry(const RowArgs& a, int j, int s0, const int* __restrict__ p,
+                                              const double2* __restrict__ pq, const double* __restrict__ W, int2& kk,
+                                              double2* e) {
+    const int n = a.n, nq = a.nq, x = j % nq, s12 = j / nq, s1 = s12 / n, s2 = s12 % n, px = p[x];
+    if (px < x || (px == x && s2 < s1)) return 0;
+    double2 u = pq[j], v = make_double2(0.0, 0.0);
+    if (px != x || s1 != s2) v = pq[(s2 * n + s1) * nq + px];
+    else u.x = 0.0;
+    if (u.x == 0.0 && u.y == 0.0 && v.x == 0.0 && v.y == 0.0) return 0;
+    const double* w = W + (size_t)x * n * n * n + (size_t)s0 * n * n;
+    const double w1 = 4.0 * w[s1 * n + s2], w2 = px == x ? 4.0 * w[s2 * n + s1] : w1;
+    kk = make_int2(x * n + s1, px * n + s2);
+    e[0] = make_double2((u.x - v.x) * w1, (u.y + v.y) * w1);
+    if (w2 != w1) e[0] = make_double2(u.x * w1 - v.x * w2, u.y * w1 + v.y * w2);
+    unsigned m = e[0].x != 0.0 || e[0].y != 0.0 ? 1 : 0;
+    if (a.neg[x] == x) {
+        e[1] = make_double2(2.0 * v.x * w2, -2.0 * e[0].y);
+        if (e[1].x != 0.0 || e[1].y != 0.0) m |= 2;
+    }
+    if (a.neg[px] == px) {
+        e[2] = make_double2(2.0 * u.x * w1, -2.0 * e[0].y);
+        if (e[2].x != 0.0 || e[2].y != 0.0) m |= 4;
+    }
+    return m;
+}
 
 // One block per segment of a row: blockIdx.x = (slot n + s0) nseg + segment, [seg, seg + 1) / nseg of the
 // row's elements.  COUNT: its entries to cnt.  Otherwise they are written in element order from base + boff
@@ -240,14 +253,16 @@ __global__ void __launch_bounds__(256) k_bte_entries(RowArgs a, int nseg, int* _
     for (int j0 = seg * step; j0 < j1; j0 += 256) {
         const int j = j0 + (int)threadIdx.x;
         int2 k;
-        double2 e;
-        const bool on = j < j1 && bte_entry(j, n, nq, s0, p, pq, W, k, e);
+        double2 e[3];
+        const unsigned on = j < j1 ? bte_entry(a, j, s0, p, pq, W, k, e) : 0u;
         if (COUNT) {
-            total += on;
+            total += __popc(on);
             continue;
         }
-        const unsigned m = __ballot_sync(0xffffffffu, on);
-        if (lane == 0) wsum[warp] = __popc(m);
+        unsigned m[3];
+#pragma unroll
+        for (int h = 0; h < 3; ++h) m[h] = __ballot_sync(0xffffffffu, on >> h & 1);
+        if (lane == 0) wsum[warp] = __popc(m[0]) + __popc(m[1]) + __popc(m[2]);
         __syncthreads();
         int before = 0, all = 0;
 #pragma unroll
@@ -255,10 +270,15 @@ __global__ void __launch_bounds__(256) k_bte_entries(RowArgs a, int nseg, int* _
             before += w < warp ? wsum[w] : 0;
             all += wsum[w];
         }
-        if (on) {
-            const long long o = base + before + __popc(m & ((1u << lane) - 1));
-            kk[o] = k;
-            pqo[o] = e;
+        long long o = base + before;
+#pragma unroll
+        for (int h = 0; h < 3; ++h) {
+            if (on >> h & 1) {
+                const long long i = o + __popc(m[h] & ((1u << lane) - 1));
+                kk[i] = h == 0 ? k : (h == 1 ? make_int2(~k.x, k.y) : make_int2(~k.y, k.x));
+                pqo[i] = e[h];
+            }
+            o += __popc(m[h]);
         }
         base += all;
         __syncthreads();
@@ -309,14 +329,20 @@ __global__ void __launch_bounds__(256) k_bte_dense(RowArgs a, const double* __re
     double v[3] = {0.0, 0.0, 0.0};
     for (int j = threadIdx.x; j < len; j += 256) {
         int2 k;
-        double2 e;
-        if (!bte_entry(j, n, nq, s0, p, pq, W, k, e)) continue;
+        double2 e[3];
+        const unsigned on = bte_entry(a, j, s0, p, pq, W, k, e);
+        if (!on) continue;
         const double n1 = nbe[k.x], n2 = nbe[k.y];
-        const double c = (n1 - n2) * e.x + (1.0 + n1 + n2) * e.y;
+        const double c = (n1 - n2) * e[0].x + (1.0 + n1 + n2) * e[0].y;
         if (MODE == 0) {
             v[0] += c;
-        } else {
-            for (int d = 0; d < 3; ++d) v[d] -= c * (Fg[4 * (size_t)k.x + d] + Fg[4 * (size_t)k.y + d]);
+            continue;
+        }
+        const double c1 = on & 2 ? (n1 - n2) * e[1].x + (1.0 + n1 + n2) * e[1].y : 0.0;
+        const double c2 = on & 4 ? (n2 - n1) * e[2].x + (1.0 + n1 + n2) * e[2].y : 0.0;
+        for (int d = 0; d < 3; ++d) {
+            const double f1 = Fg[4 * (size_t)k.x + d], f2 = Fg[4 * (size_t)k.y + d];
+            v[d] -= c * (f1 + f2) + (c1 * f1 + c2 * f2);
         }
     }
     constexpr int NV = MODE == 0 ? 1 : 3;
@@ -499,8 +525,12 @@ __global__ void k_bteg_gather(long long cnt, int rows, int shift, const s3::BteE
     }
 }
 
-// Row r holds the entries off[r nseg] .. off[(r + 1) nseg].  One block per row: c = (n1 - n2) P + (1 + n1 + n2) Q of its entries at one temperature, and their sum,
-// 1/tau.
+// The modes whose F an entry adds up: k1 and k2, or twice k1 where k1 is stored as its complement (e[1] and e[2]
+// of bte_entry; their coefficients are halved).
+__device__ __forceinline__ int2 bte_legs(int2 k) { return k.x < 0 ? make_int2(~k.x, ~k.x) : k; }
+
+// Row r holds the entries off[r nseg] .. off[(r + 1) nseg].  One block per row: c = (n1 - n2) P + (1 + n1 + n2) Q of
+// its entries at one temperature, and their sum, 1/tau.
 __global__ void __launch_bounds__(256) k_bteg_coef(int nseg, const int* __restrict__ off, const int2* __restrict__ kk,
                                                   const double2* __restrict__ pq, const double* __restrict__ nbe,
                                                   double* __restrict__ cf, double* __restrict__ inv_tau) {
@@ -510,10 +540,10 @@ __global__ void __launch_bounds__(256) k_bteg_coef(int nseg, const int* __restri
     for (int i = off[(size_t)blockIdx.x * nseg] + threadIdx.x; i < end; i += 256) {
         const int2 k = kk[i];
         const double2 e = pq[i];
-        const double n1 = nbe[k.x], n2 = nbe[k.y];
+        const double n1 = nbe[k.x < 0 ? ~k.x : k.x], n2 = nbe[k.y];
         const double c = (n1 - n2) * e.x + (1.0 + n1 + n2) * e.y;
-        cf[i] = c;
-        v[0] += c;
+        cf[i] = k.x < 0 ? 0.5 * c : c;
+        if (k.x >= 0) v[0] += c;
     }
     const double t = block_sum<1>(v, red);
     if (threadIdx.x == 0) inv_tau[blockIdx.x] = t;
@@ -528,7 +558,7 @@ __global__ void __launch_bounds__(256) k_bteg_rows(int nseg, const int* __restri
     const int end = off[((size_t)blockIdx.x + 1) * nseg];
     for (int i = off[(size_t)blockIdx.x * nseg] + threadIdx.x; i < end; i += 256) {
         const double c = cf[i];
-        const int2 k = kk[i];
+        const int2 k = bte_legs(kk[i]);
         const double2* f1 = reinterpret_cast<const double2*>(Fg + 4 * (size_t)k.x);
         const double2* f2 = reinterpret_cast<const double2*>(Fg + 4 * (size_t)k.y);
         const double2 u1 = f1[0], v1 = f1[1], u2 = f2[0], v2 = f2[1];
@@ -545,7 +575,7 @@ __global__ void __launch_bounds__(256) k_bteg_rows(int nseg, const int* __restri
 __global__ void k_bteg_encode(long long cnt, int n, const int2* __restrict__ kk, const int* __restrict__ pos,
                               const int* __restrict__ sgn, unsigned* __restrict__ ke) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (long long)gridDim.x * blockDim.x) {
-        const int2 k = kk[i];
+        const int2 k = bte_legs(kk[i]);
         const int a = k.x / n, b = k.y / n;
         const unsigned x = (pos[a] * n + k.x % n) | (sgn[a] < 0 ? 0x8000 : 0), y = (pos[b] * n + k.y % n) | (sgn[b] < 0 ? 0x8000 : 0);
         ke[i] = x | y << 16;
@@ -843,7 +873,7 @@ int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* 
         k_bte_weights<<<grid, 32 * TW, 0, c->stream>>>(a, reinterpret_cast<const int4*>(c->d_tetra.p));
         return launch_check(c, "k_bte_weights");
     };
-    auto row_args = [&](int b) { return RowArgs{n, nq, b, c->ps_tr.partner.p, w.pq.p, c->d_w.p}; };
+    auto row_args = [&](int b) { return RowArgs{n, nq, b, c->ps_tr.partner.p, c->d_neg.p, w.pq.p, c->d_w.p}; };
     bool stored = c->bt_gen == c->ph_gen && c->bt_pairs == c->ps_tr.gen && c->bt_n >= 0;
     const int len = n * n * nq;
     const int nseg = std::max(1, std::min(16, len / 4096));

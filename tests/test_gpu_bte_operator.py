@@ -70,3 +70,19 @@ def test_kappa_iter_gauss_rebuilt_operator_gives_the_same_bits():
     assert a["entries"] == b["entries"] and a["iters"][0] == 4
     np.testing.assert_array_equal(b["kappa"], a["kappa"])
     ctx.close()
+
+
+def test_kappa_iter_of_unsymmetrised_fc3_matches_oracle():
+    """W of a pair of equal points is not symmetric in its branches then, and F does not vanish where q = -q."""
+    cr = S.build("rocksalt2")
+    cr.fc3 = cr.fc3 + np.random.default_rng(5).normal(0.0, 1.0, size=cr.fc3.shape)
+    st = D.Setup(cr, (3, 3, 2), [300.0])
+    ctx, _ = from_crystal(cr, (3, 3, 2), [300.0], phonons={"grid": st.ph, "irr": st.ph0})
+    ref = D.bte_iter(st, eps_k=1e-6)
+    for entries in (-1, 10):                                 # stored, and recomputed in every iteration
+        ctx.set_option(L.SPRING_OPT_BTE_ENTRIES, entries)
+        out = ctx.kappa_iter(eps_k=1e-6)
+        np.testing.assert_allclose(out["kappa_rta"][0], ref["kappa_rta"], rtol=1e-9,
+                                   atol=1e-9 * np.abs(ref["kappa_rta"]).max())
+        np.testing.assert_allclose(out["kappa"][0], ref["kappa"], rtol=1e-6, atol=1e-6 * np.abs(ref["kappa"]).max())
+    ctx.close()
