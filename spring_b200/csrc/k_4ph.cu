@@ -441,19 +441,22 @@ struct T4Args {
 // s1, s2, s3) that ran every formula any lane of its warp needed; 15.3 and 45 ms with each hit sorting its own
 // energies and taking its own reciprocals.  Bound by issue (IPC 1.75) and the latency of the W reads.
 constexpr int T4W = 4;  // warps per block
+// n1 / n0 overflows by itself for n0 near the smallest double, where n2 n3 makes up for it: a power of two moves
+// between the two factors, which changes no bit of their product elsewhere.
+constexpr double T4UP = 18446744073709551616.0;  // 2^64
 
 template <int NT>
 struct T4Smem {
     double acc[T4W][N * NT][32];        // per-lane sums [s0][T]
     double val[T4W][2][10][32];         // p, m sets: sorted energies; 1/(30), (10), (21), (32), (20), (31)
-    double nf[T4W][2][NT][4][32];       // n2 n3 and (1 + n2) n3 by vertex
+    double nf[T4W][2][NT][4][32];       // n2 n3 and (1 + n2) n3 by vertex, times T4UP
     int off[T4W][4][32];                // by vertex: W offset of (s2, s3) | stride of s1 << 8
     int pos[T4W][4][32], v2[T4W][4][32], v3[T4W][4][32];  // quartet and points of each vertex
     int rank[T4W][2][32];               // vertices by rank, two bits each; 256: well separated
     unsigned short queue[T4W][32 * 6 * 3 * N];  // lane | check << 5
     double w0m[N][N], w0p[N][N];        // w0 - w1, w0 + w1 [s1][s0]
     float f0m[N][8], f0p[N][8];         // the same in FP32 (two values of padding)
-    double fac[NT][2][N][N];            // n1 / n0 / 6, (1 + n1) / n0 / 2 [T][.][s1][s0]
+    double fac[NT][2][N][N];            // n1 / n0 / 6, (1 + n1) / n0 / 2 [T][.][s1][s0], over T4UP
     double w0[N];
 };
 
@@ -487,8 +490,8 @@ __global__ void __launch_bounds__(32 * T4W, 3) k_tetra4(T4Args a, int per2, int 
             S.f0p[s1][s0] = (float)(w0 + w1);
             for (int T = 0; T < a.nT; ++T) {
                 const double n1 = nbeg[((size_t)T * a.nq + q1) * N + s1], n0 = nbe0[(size_t)T * a.nq0 * N + s0];
-                S.fac[T][0][s1][s0] = ONEBYSIX * (n1 / n0);
-                S.fac[T][1][s1][s0] = 0.5 * ((1.0 + n1) / n0);
+                S.fac[T][0][s1][s0] = ONEBYSIX * (n1 / (n0 * T4UP));
+                S.fac[T][1][s1][s0] = 0.5 * ((1.0 + n1) / (n0 * T4UP));
             }
         }
         __syncthreads();
@@ -589,8 +592,9 @@ __global__ void __launch_bounds__(32 * T4W, 3) k_tetra4(T4Args a, int per2, int 
 #pragma unroll
                         for (int v = 0; v < 4; ++v) {
                             const double n2 = nb[(size_t)v2[v] * N + s2], n3 = nb[(size_t)v3[v] * N + s3];
-                            S.nf[warp][0][T][v][lane] = n2 * n3;
-                            S.nf[warp][1][T][v][lane] = (1.0 + n2) * n3;
+                            const double u3 = n3 * T4UP;
+                            S.nf[warp][0][T][v][lane] = n2 * u3;
+                            S.nf[warp][1][T][v][lane] = (1.0 + n2) * u3;
                         }
                     }
                     const int c = __popcll(hit[0]) + __popcll(hit[1]);

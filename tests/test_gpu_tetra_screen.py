@@ -117,3 +117,20 @@ def test_tetrahedron_sums_of_unsymmetrised_fc3_match_oracle(cell, mesh, nT):
             np.testing.assert_allclose(lw[it, i0], r["lw"], rtol=1e-9, atol=1e-14 * np.abs(lw).max())
         np.testing.assert_allclose(p3[i0], r["p3_q0"], rtol=1e-9, atol=1e-14 * np.abs(p3).max())
     ctx.close()
+
+
+@pytest.mark.gpu
+def test_four_phonon_sums_with_a_vanishing_occupation_match_oracle():
+    """n(q0) near the smallest double: (1 + n1) / n0 by itself is beyond the largest."""
+    cr = S.build("rocksalt2", fc4=True)
+    mesh, temps = (3, 3, 2), [30.0]
+    W = np.eye(3, dtype=np.int32)[None]
+    st = D.Setup(cr, mesh, temps, W=W, Rxyz=np.eye(3)[None])
+    st.ph0["nbe"][0][4] = 5e-309
+    ctx, _ = from_crystal(cr, mesh, temps, phonons={"grid": st.ph, "irr": st.ph0}, W=W, Rxyz=np.eye(3)[None],
+                          with_fc4=True)
+    rate = ctx.linewidth4(5, 1, delta="tetra")
+    ro, _ = D.lw4_tetra(st, 4)
+    assert np.all(np.isfinite(ro)) and ro.max() > 1e250
+    np.testing.assert_allclose(rate[0, 0], ro, rtol=1e-9, atol=1e-12 * np.abs(ro).max())
+    ctx.close()
