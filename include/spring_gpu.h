@@ -380,8 +380,9 @@ int spring_batch_add_path(spring_batch* batch, spring_ctx* ctx, int n_path, cons
 int spring_batch_path_result(spring_batch* batch, int index, double* lw, double* omega);
 
 /* ---- options ----------------------------------------------------------- */
-/* SPRING_OPT_GENERIC_V3 = 1: always use the any-cell V3 kernel (default 0 picks the
- * two-atom specialisation when the cell fits it; both give the same W). */
+/* SPRING_OPT_GENERIC_V3 = 1: always use the any-cell FP64 V3 kernel, in batches too (default 0
+ * picks the two-atom kernel, or the matrix kernel of 12 and more branches, when the cell fits one;
+ * all give the same W). */
 #define SPRING_OPT_GENERIC_V3 1
 /* SPRING_OPT_WAIT_POLLS = 2: poll limit of each wait of one warp on another inside the
  * tensor-core kernels (value >= 0; a negative value restores the default, 2^26).  When a wait

@@ -199,7 +199,8 @@ bool tc_request(const spring_ctx* c) { return c->precision != SPRING_FP64 && c->
 
 // Requests that run by themselves after the graph: the tensor-core ones, and cells whose V3 an FP64 matrix
 // kernel takes (one CTA per SM with most of its shared memory; an item of the persistent kernel costs 15 times
-// the work there for 24 branches, 5 times for a two-atom cell).
+// the work there for 24 branches, 5 times for a two-atom cell).  SPRING_OPT_GENERIC_V3 on a context keeps its FP64
+// requests in the persistent kernel.
 bool own_pass(const spring_batch* b, const spring_ctx* c) {
     return tc_request(c) || spring::v3m_takes(c) || (b->cfg[0] && !c->force_generic_v3 && spring::v3s_takes(c));
 }

@@ -426,9 +426,9 @@ V3mLayout v3m_layout(int nb, int n, int na, int types) {
 // Whether launch_v3m takes the context's cell.  Fewer branches leave the 8-wide tiles half empty and a step
 // too short for its barriers: at 3 to 9 branches the kernel in k_v3.cu takes 0.24 - 0.33 ms where this one
 // takes 0.50 - 1.3; from 12 on this one is ahead (12: 0.93 -> 0.50 ms, 15: 3.0 -> 0.36, 18: 2.2 -> 0.40,
-// 24: 10.1 -> 0.55; W grids of 16 q0).
+// 24: 10.1 -> 0.55; W grids of 16 q0).  SPRING_OPT_GENERIC_V3 leaves every cell to k_v3.cu.
 bool v3m_takes(const spring_ctx* c) {
-    return c->ndof >= 12 && v3m_layout(c->nb, c->ndof, c->na3, c->fc3_types).bytes <= 227 * 1024;
+    return !c->force_generic_v3 && c->ndof >= 12 && v3m_layout(c->nb, c->ndof, c->na3, c->fc3_types).bytes <= 227 * 1024;
 }
 
 // Launch for pair set ps, q0 block [q0_first, +n_q0); *handled is false when the layout does not fit.
