@@ -355,10 +355,12 @@ int spring_batch_add_linewidth3(spring_batch* batch, spring_ctx* ctx, int i0_fir
 int spring_batch_set_config(spring_batch* batch, const int* config);
 int spring_batch_get_config(const spring_batch* batch, int* config);
 /* Autotuner: time the batch under candidate configurations (coordinate search
- * over the four parameters, each run timed with CUDA events; LW_Allq0 is not
- * touched) and keep the fastest.  The result is cached for the process by the
- * batch's shape (cells, meshes, temperatures, pair counts), so a later batch
- * of the same shape starts tuned.  best_ms and n_tried may be NULL. */
+ * over the four parameters, each run timed with CUDA events, the kernels after the
+ * graph included; LW_Allq0 is not touched) and keep the fastest.  A parameter that no
+ * request is subject to keeps its value; its candidates are counted and not run.  The
+ * result is cached for the process by the batch's shape (cells, meshes, temperatures,
+ * pair counts, precision and V3 option), so a later batch of the same shape starts
+ * tuned.  best_ms and n_tried may be NULL. */
 int spring_batch_tune(spring_batch* batch, int* config, double* best_ms, int* n_tried);
 /* Run every request (accumulating into each context's LW_Allq0, as
  * spring_linewidth3 does); the first run captures the CUDA graph. */

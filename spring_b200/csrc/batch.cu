@@ -186,7 +186,8 @@ std::string shape_key(const spring_batch* b) {
     std::string k;
     char buf[160];
     for (const auto& w : b->work) {
-        snprintf(buf, sizeof buf, "%d:%d:%d:%d:%lld;", w.c->ndof, w.c->nq, w.c->nT, w.c->na3, w.pairs);
+        snprintf(buf, sizeof buf, "%d:%d:%d:%d:%lld:%d:%d;", w.c->ndof, w.c->nq, w.c->nT, w.c->na3, w.pairs,
+                 w.c->precision, (int)w.c->force_generic_v3);
         k += buf;
     }
     return k;
@@ -400,22 +401,22 @@ int enqueue_paths(spring_batch* b) {
 }
 
 // The requests with a pass of their own after the graph (which zeroed their scratch): the pass of
-// spring_linewidth3 on each context's stream, then its LW_Allq0 update; the batch stream waits for
-// them.
-int run_own_passes(spring_batch* b) {
+// spring_linewidth3 on each context's stream, then (fold) its LW_Allq0 update; the batch stream waits
+// for them.
+int run_own_passes(spring_batch* b, bool fold) {
     for (const auto& w : b->work) {
         if (!w.own) continue;
         spring_ctx* c = w.c;
         BCHECK(join_ctx_out(b, c));
         int rc = spring::run_v3_gauss(c, w.q0, w.n_q0, w.sigma, w.pol, c->d_lw_tmp.p, c->d_p3.p);
-        if (rc == SPRING_OK) rc = spring::run_axpy_lw(c, 1.0, c->d_lw_tmp.p, c->d_lw_all.p, w.q0, w.n_q0);
+        if (rc == SPRING_OK && fold) rc = spring::run_axpy_lw(c, 1.0, c->d_lw_tmp.p, c->d_lw_all.p, w.q0, w.n_q0);
         if (rc != SPRING_OK) return bfail(b, rc, "request: %s", c->err.c_str());
         BCHECK(join_ctx_in(b, c));
     }
     return SPRING_OK;
 }
 
-// One timed run without the LW_Allq0 update (for the tuner).
+// One timed run, own passes included, without the LW_Allq0 update (for the tuner).
 int timed_trial(spring_batch* b, double* ms) {
     std::vector<BatchDesc> D;
     std::vector<long long> off;
@@ -425,6 +426,7 @@ int timed_trial(spring_batch* b, double* ms) {
     BCHECK(upload(b, D, off, smem));
     BCHECK(bcuda(b, cudaEventRecord(b->ev0, b->stream), "batch timing"));
     BCHECK(enqueue(b, D, off, smem, fold_total, false));
+    BCHECK(run_own_passes(b, false));
     BCHECK(bcuda(b, cudaEventRecord(b->ev1, b->stream), "batch timing"));
     BCHECK(bcuda(b, cudaEventSynchronize(b->ev1), "batch timing"));
     float t = 0.0f;
@@ -575,9 +577,24 @@ int spring_batch_tune(spring_batch* b, int* config, double* best_ms, int* n_trie
     };
     BCHECK(trial(best, &bms));  // warm-up of the baseline
     BCHECK(trial(best, &bms));
+    // whether a request is subject to parameter k of the best configuration so far
+    auto matters = [&](int k) {
+        for (int i = 0; i < 4; ++i) b->cfg[i] = best[i];
+        for (const auto& w : b->work) {
+            if (k == 0 ? !tc_request(w.c) && !w.c->force_generic_v3 && spring::v3s_takes(w.c)
+                       : !own_pass(b, w.c) && (k != 2 || w.c->ndof > 12))
+                return true;
+        }
+        return false;
+    };
     auto sweep = [&](int k, const std::vector<int>& vals) -> int {
+        const bool run = matters(k);
         for (int v : vals) {
             if (v == best[k]) continue;
+            if (!run) {  // the same launches: nothing to time
+                ++tried;
+                continue;
+            }
             int cand[4] = {best[0], best[1], best[2], best[3]};
             cand[k] = v;
             double ms = 0.0;
@@ -665,7 +682,7 @@ int spring_batch_run(spring_batch* b) {
     BCHECK(bcuda(b, cudaEventRecord(b->ev0, b->stream), "batch timing"));
     BCHECK(bcuda(b, cudaGraphLaunch(b->exec, b->stream), "batch graph launch"));
     b->work[0].c->launches += 2;
-    BCHECK(run_own_passes(b));
+    BCHECK(run_own_passes(b, true));
     BCHECK(bcuda(b, cudaEventRecord(b->ev1, b->stream), "batch timing"));
     BCHECK(join_out(b));
     BCHECK(bcuda(b, cudaEventSynchronize(b->ev1), "batch run"));

@@ -187,3 +187,30 @@ def test_batch_path_request_errors():
         b.path_result(0)  # no such request
     b.close()
     ctx.close()
+
+
+def test_batch_autotuner_times_the_whole_run():
+    """Every request here has a kernel of its own after the graph: the tuner's best time is that of a run, not of the
+    empty graph, and choosing between a request's two routes counts both."""
+    ctx2, _ = from_crystal(S.build("rocksalt2"), (12, 12, 12), TEMPS9)
+    ctx8, _ = from_crystal(S.build("rocksalt8"), (5, 5, 5), [300.0])
+    b = Batch()
+    for ctx in (ctx2, ctx8):
+        b.add_linewidth3(ctx, 1, ctx.nq0, SIGMA)
+    b.run()
+    kept = [ctx.get_linewidths() for ctx in (ctx2, ctx8)]
+    cfg, best_ms, _ = b.tune()
+    for ctx, lw in zip((ctx2, ctx8), kept):
+        np.testing.assert_array_equal(ctx.get_linewidths(), lw)   # trials leave the accumulated linewidths alone
+    ms = []
+    for _ in range(5):
+        b.run()
+        ms.append(b.result(0)[2])
+    assert 0.5 * min(ms) < best_ms < 2.0 * max(ms)
+    b.set_config(1 - cfg[0], *cfg[1:])
+    b.run()
+    b.run()
+    assert b.result(0)[2] > 0.9 * min(ms)                        # the route not chosen is not the faster one
+    b.close()
+    ctx2.close()
+    ctx8.close()
