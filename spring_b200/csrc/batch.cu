@@ -449,7 +449,8 @@ int spring_batch_destroy(spring_batch* b) {
     if (!b) return SPRING_OK;
     if (b->device >= 0) {
         spring::Guard g(b->device);
-        if (b->stream) cudaStreamSynchronize(b->stream);
+        // the stream is its first context's, which may be gone: the batch's own event is waited for
+        if (b->ev1) cudaEventSynchronize(b->ev1);
         drop_graph(b);
         if (b->d_desc) cudaFree(b->d_desc);
         if (b->d_off) cudaFree(b->d_off);

@@ -214,3 +214,13 @@ def test_batch_autotuner_times_the_whole_run():
     b.close()
     ctx2.close()
     ctx8.close()
+
+
+def test_batch_outlives_its_contexts():
+    """Contexts closed first: destroying the batch (as garbage collection may order it) touches none of theirs."""
+    ctx, _ = from_crystal(S.build("rocksalt2"), (3, 3, 3), [300.0])
+    b = Batch()
+    b.add_linewidth3(ctx, 1, ctx.nq0, SIGMA)
+    b.run()
+    ctx.close()
+    b.close()
