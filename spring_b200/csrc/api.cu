@@ -647,7 +647,7 @@ int spring_set_fc3(spring_ctx* c, int na3, const int* num, const int* idx, const
     SPRING_CHECK(h2d(c, c->d_fc3_btyp.p, btyp.data(), sizeof(int) * btyp.size(), "FC3 basis"));
     // no stream wait: h2d staged every byte in the context's pinned ring before queuing its copy
     c->fc3_set = true;
-    c->bt_gen = -1;   // the BTE operators depend on FC3
+    bte_stale(c);   // the BTE operators depend on FC3
     c->bteg_n = 0;
     return SPRING_OK;
 }
@@ -814,6 +814,7 @@ int spring_compute_phonons(spring_ctx* c, const double* temps, double freq_cut) 
     SPRING_CHECK(run_phonons_mesh(c));
     c->ph_grid.set = c->ph_irr.set = true;
     c->ph_gen += 1;
+    bte_stale(c);
     return SPRING_OK;
 }
 
@@ -844,6 +845,7 @@ int spring_set_phonons(spring_ctx* c, int which, const double* temps, const doub
     SPRING_CHECK(h2d(c, p.vel.p, vel, sizeof(double) * n * nd * 3, "group velocity"));
     p.set = true;
     c->ph_gen += 1;
+    bte_stale(c);
     return SPRING_OK;
 }
 

@@ -837,6 +837,15 @@ int run_bte_gauss(spring_ctx* c, double sigma, double eps_k, int max_iter, doubl
                             h_kappa_rta, h_iters);
 }
 
+// The stored tetrahedron operator no longer holds.  A small one's memory serves the next; a large one goes back, so
+// that calls which size themselves by the free memory find it.
+void bte_stale(spring_ctx* c) {
+    c->bt_gen = -1;
+    if (c->d_bt_kk.n * sizeof(int2) + c->d_bt_pq.n * sizeof(double2) <= ((size_t)256 << 20)) return;
+    dfree(c->d_bt_kk);
+    dfree(c->d_bt_pq);
+}
+
 int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* h_kappa_rta, int* h_iters) {
     if (c->ntr == 0) SPRING_CHECK(build_tr_set(c));
     if (!c->ps_tr.done) SPRING_CHECK(run_enumerate3(c, c->ps_tr));
@@ -978,6 +987,10 @@ int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* 
         };
         rc = bte_iterate(c, eps_k, max_iter, 1, 1, [&](int T) { return pass(0, T); }, [&](int T) { return pass(1, T); },
                          h_kappa, h_kappa_rta, h_iters);
+    }
+    if (w.pq.n * sizeof(double2) > ((size_t)256 << 20)) {  // one q0 of a large cell
+        cudaStreamSynchronize(c->stream);
+        dfree(w.pq);
     }
     return rc;
 }

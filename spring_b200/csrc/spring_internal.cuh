@@ -434,6 +434,7 @@ int run_mlp_train(spring_ctx* c, int n, const float* hX, const float* hy, int ep
 int run_mlp_predict(spring_ctx* c, int n, const float* hX, float* hy, int bf16);
 void free_mlp(Mlp& m);
 // k_bte.cu
+void bte_stale(spring_ctx* c);  // FC3 or the phonons changed
 int run_bte(spring_ctx* c, double eps_k, int max_iter, double* h_kappa, double* h_kappa_rta, int* h_iters);
 // k_tetra.cu
 int alloc_tetra_tables(spring_ctx* c);

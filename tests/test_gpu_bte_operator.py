@@ -2,6 +2,7 @@
 the form that is not stored, and cells with more than one pass over s0."""
 import numpy as np
 import pytest
+import torch
 
 from oracle import driver as D
 from spring_b200 import _lib as L
@@ -85,4 +86,27 @@ def test_kappa_iter_of_unsymmetrised_fc3_matches_oracle():
         np.testing.assert_allclose(out["kappa_rta"][0], ref["kappa_rta"], rtol=1e-9,
                                    atol=1e-9 * np.abs(ref["kappa_rta"]).max())
         np.testing.assert_allclose(out["kappa"][0], ref["kappa"], rtol=1e-6, atol=1e-6 * np.abs(ref["kappa"]).max())
+    ctx.close()
+
+
+def _free():
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def test_kappa_iter_gives_a_large_operator_back_when_it_is_stale():
+    """New phonons or FC3 make the stored operator useless: a large one does not keep its memory from later calls."""
+    cr = S.build("rocksalt2")
+    ctx, _ = from_crystal(cr, (12, 12, 12), [300.0])
+    first = ctx.kappa_iter(eps_k=1e-3, max_iter=2)
+    ctx.compute_phonons([300.0])
+    base = _free()
+    for stale in (lambda: ctx.compute_phonons([300.0]),
+                  lambda: ctx.set_fc3(cr.fc3_atm_num, cr.fc3_atm_indx, cr.fc3)):
+        again = ctx.kappa_iter(eps_k=1e-3, max_iter=2)
+        held = base - _free()
+        assert held > 128 << 20                              # the case is one: the operator is large
+        stale()
+        assert base - _free() < 16 << 20
+        np.testing.assert_allclose(again["kappa"], first["kappa"], rtol=1e-10, atol=1e-10 * np.abs(first["kappa"]).max())
     ctx.close()
