@@ -377,7 +377,7 @@ int prepare_paths(spring_batch* b) {
     for (auto& p : b->paths) {
         if (p.ready) continue;
         spring::Guard g(p.c->device);
-        const int rc = spring::path_prepare(p.c, p.plan, p.n_path, p.q.data(), p.zc.data());
+        const int rc = spring::path_prepare(p.c, p.plan, p.n_path, p.q.data(), p.zc.data(), false);
         if (rc != SPRING_OK) return bfail(b, rc, "path request: %s", p.c->err.c_str());
         p.ready = true;
     }

@@ -425,15 +425,20 @@ void path_release(PathPlan& p) {
     p.slots = 0;
 }
 
-int path_prepare(spring_ctx* c, PathPlan& p, int n_path, const double* h_q0, const int* h_zc) {
+// W grid, q2 phonons and (tables) tetrahedron tables of one path point.
+static size_t path_slot_bytes(const spring_ctx* c, bool tables) {
+    const size_t n = c->ndof;
+    return (size_t)c->nq * (n * n * n * sizeof(double) + n * n * sizeof(double2) + n * sizeof(double) * (6 + c->nT) +
+                            8 * sizeof(double) + (tables ? tetra_table_doubles(c) * sizeof(double) : 0));
+}
+constexpr size_t PATH_BUDGET = (size_t)512 << 20;
+
+int path_prepare(spring_ctx* c, PathPlan& p, int n_path, const double* h_q0, const int* h_zc, bool tables) {
     const int n = c->ndof, nq = c->nq;
     const size_t n3 = (size_t)n * n * n;
-    // slots: path points per batch (W grid + q2 phonons of a slot)
-    const size_t per_slot = (size_t)nq * (n3 * sizeof(double) + (size_t)n * n * sizeof(double2) +
-                                          (size_t)n * sizeof(double) * (6 + c->nT) + 8 * sizeof(double));
-    const size_t budget = (size_t)512 << 20;
     p.n_path = n_path;
-    p.slots = (int)std::max<size_t>(1, std::min<size_t>((size_t)n_path, budget / per_slot));
+    // slots: path points per batch
+    p.slots = (int)std::max<size_t>(1, std::min<size_t>((size_t)n_path, PATH_BUDGET / path_slot_bytes(c, tables)));
     const long long rows_max = (long long)p.slots * nq;
     SPRING_CHECK(dalloc(c, p.q0v, (size_t)3 * n_path, "path q0"));
     SPRING_CHECK(dalloc(c, p.zc, (size_t)n_path, "path flags"));
@@ -520,16 +525,18 @@ int path_fetch(spring_ctx* c, PathPlan& p, double* h_lw, double* h_omega) {
 
 int run_path(spring_ctx* c, int n_path, const double* h_q0, const int* h_zc, int delta_mode, double sigma,
              double* h_lw, double* h_omega) {
-    // The buffers stay with the context (at most the 512 MB budget of path_prepare plus the path's own
-    // results): allocating and freeing them took 5 of the 7.5 ms of 24 points at 12^3.
+    // The buffers stay with the context where they keep to the budget (512 MB, the tetrahedron tables counted in
+    // both forms, plus the path's own results): allocating and freeing them took 5 of the 7.5 ms of 24 points
+    // at 12^3.  One point of a large cell can be above it (24 branches at 18^3: 680 MB); its buffers go back.
     if (!c->path_ws) c->path_ws = new PathPlan();
     PathPlan& p = *static_cast<PathPlan*>(c->path_ws);
-    int rc = path_prepare(c, p, n_path, h_q0, h_zc);
+    int rc = path_prepare(c, p, n_path, h_q0, h_zc, true);
     if (rc == SPRING_OK && delta_mode == SPRING_DELTA_TETRA)
         rc = dalloc(c, p.tab2, (size_t)p.slots * c->nq * tetra_table_doubles(c), "path tetrahedron tables");
     if (rc == SPRING_OK) rc = path_enqueue(c, p, delta_mode, sigma);
     if (rc == SPRING_OK) rc = path_fetch(c, p, h_lw, h_omega);
     cudaStreamSynchronize(c->stream);
+    if (path_slot_bytes(c, true) > PATH_BUDGET) path_release(p);
     return rc;
 }
 

@@ -418,7 +418,8 @@ struct PathPlan {
     DBuf<int> zc, ex;
     Phonons php, ph2;
 };
-int path_prepare(spring_ctx* c, PathPlan& p, int n_path, const double* h_q0, const int* h_zc);
+// tables: the tetrahedron tables count towards the workspace's size
+int path_prepare(spring_ctx* c, PathPlan& p, int n_path, const double* h_q0, const int* h_zc, bool tables);
 int path_enqueue(spring_ctx* c, PathPlan& p, int delta_mode, double sigma);
 int path_fetch(spring_ctx* c, PathPlan& p, double* h_lw, double* h_omega);
 void path_release(PathPlan& p);

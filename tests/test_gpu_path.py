@@ -1,6 +1,7 @@
 """LineWidth.x path mode on the GPU (through the C ABI) against the CPU oracle."""
 import numpy as np
 import pytest
+import torch
 
 from oracle import driver as D
 from spring_b200 import synthetic as S
@@ -75,4 +76,37 @@ def test_linewidth_path_errors():
     with pytest.raises(SpringError) as e:
         ctx.linewidth_path(np.zeros((1, 3)), [1])
     assert e.value.code == 2
+    ctx.close()
+
+
+def test_linewidth_path_buffers_serve_paths_of_other_lengths_and_forms():
+    """One context's kept buffers against a new context for every call."""
+    cr = S.build("rocksalt2")
+    q = np.random.default_rng(1).uniform(-0.5, 0.5, size=(9, 3)) @ cr.G.T
+    z = np.ones(9, np.int32)
+    kept, _ = from_crystal(cr, (4, 4, 4), TEMPS)
+    for n, delta in ((5, "gauss"), (9, "tetra"), (2, "tetra"), (7, "gauss"), (9, "tetra")):
+        new, _ = from_crystal(cr, (4, 4, 4), TEMPS)
+        a, b = kept.linewidth_path(q[:n], z[:n], delta, 0.8), new.linewidth_path(q[:n], z[:n], delta, 0.8)
+        new.close()
+        np.testing.assert_allclose(a[0], b[0], rtol=1e-11, atol=1e-13 * b[0].max())
+        np.testing.assert_array_equal(a[1], b[1])
+    kept.close()
+
+
+@pytest.mark.parametrize("cell,N,nT,points", [("rocksalt2", 12, 9, 120), ("rocksalt8", 18, 1, 1)])
+def test_linewidth_path_keeps_a_bounded_workspace(cell, N, nT, points):
+    """Many points (tables of the tetrahedron form counted with the rest), and one point above the bound by itself."""
+    cr = S.build(cell)
+    temps = list(np.linspace(100.0, 900.0, nT))
+    W = np.eye(3, dtype=np.int32)[None]
+    ctx, _ = from_crystal(cr, (N, N, N), temps, W=W, Rxyz=np.eye(3)[None])
+    q = np.random.default_rng(1).uniform(-0.5, 0.5, size=(points, 3)) @ cr.G.T
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    lw, _ = ctx.linewidth_path(q, np.ones(points, np.int32), "tetra")
+    kept = before - torch.cuda.mem_get_info()[0]
+    assert np.all(np.isfinite(lw)) and lw.max() > 0.0
+    # 512 MB, and the results and the grid's own tables, in pieces of 2 MB
+    assert kept <= (512 + 64) << 20
     ctx.close()
