@@ -748,6 +748,10 @@ int enumerate4(spring_ctx* c, int q0, Enum4Bufs& b, bool want_all, int* d_perm, 
     return SPRING_OK;
 }
 
+size_t bytes4(const Enum4Bufs& b) {
+    return sizeof(int) * (b.g3.n + b.rep.n + b.pos.n + b.all.n) + sizeof(int4) * b.quart.n;
+}
+
 void free4(Enum4Bufs& b) {
     dfree(b.g3); dfree(b.rep); dfree(b.pos); dfree(b.all); dfree(b.quart); dfree(b.total);
 }
@@ -808,7 +812,7 @@ int run_lw4(spring_ctx* c, int q0_first, int n_q0, int delta_mode, double sigma,
     const size_t smem = sizeof(V4Smem);
     cudaFuncSetAttribute(k_v4<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaFuncSetAttribute(k_v4<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    // quartet lists and (up to 512 MB) their W stay with the context
+    // quartet lists (up to 256 MB) and their W (up to 512 MB) stay with the context
     if (!c->e4) c->e4 = new Enum4Bufs();
     Enum4Bufs& b = *static_cast<Enum4Bufs*>(c->e4);
     DBuf<double>& wq = c->d_w4;
@@ -867,7 +871,7 @@ int run_lw4(spring_ctx* c, int q0_first, int n_q0, int delta_mode, double sigma,
     }
     cudaStreamSynchronize(c->stream);
     if (wq.n * sizeof(double) > ((size_t)512 << 20)) dfree(wq);
-    if ((size_t)c->nq * c->nq > ((size_t)64 << 20)) free4(b);
+    if (bytes4(b) > ((size_t)256 << 20)) free4(b);
     return rc;
 }
 

@@ -1,6 +1,7 @@
 """Four-phonon path on the GPU (through the C ABI) against the CPU oracle and the golden quartet lists."""
 import numpy as np
 import pytest
+import torch
 
 from oracle import driver as D
 from spring_b200 import synthetic as S
@@ -114,3 +115,27 @@ def test_linewidth4_errors(cr4):
         ctx.linewidth4(1, 1, delta="gauss", sigma=0.0)
     assert e.value.code == 1
     ctx.close()
+
+
+def test_linewidth4_gives_large_quartet_lists_back(cr4):
+    """18^3: 490 MB of lists for one q0.  What stays with the context is bounded."""
+    W = np.eye(3, dtype=np.int32)[None]
+    ctx, _ = from_crystal(cr4, (18, 18, 18), [300.0], W=W, Rxyz=np.eye(3)[None], with_fc3=False, with_fc4=True)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    rate = ctx.linewidth4(2, 1, delta="gauss", pol4=np.array([[4, 4], [1, 1], [1, 1], [1, 1]], np.int32))
+    torch.cuda.synchronize()
+    assert np.all(np.isfinite(rate))
+    assert before - torch.cuda.mem_get_info()[0] <= 256 << 20
+    ctx.close()
+
+
+def test_linewidth4_buffers_serve_calls_of_other_forms(cr4):
+    """One context's kept lists and W against a new context for every call, after calls with more quartets."""
+    kept, info = from_crystal(cr4, (3, 3, 4), TEMPS, with_fc4=True)
+    for i0, n, delta in ((1, kept.nq0, "tetra"), (2, 1, "gauss"), (2, 1, "tetra"), (kept.nq0, 1, "tetra"), (1, 1, "gauss")):
+        new, _ = from_crystal(cr4, (3, 3, 4), TEMPS, with_fc4=True)
+        a, b = kept.linewidth4(i0, n, delta, 0.8), new.linewidth4(i0, n, delta, 0.8)
+        new.close()
+        np.testing.assert_allclose(a, b, rtol=1e-11, atol=1e-13 * b.max())
+    kept.close()
