@@ -65,12 +65,14 @@ struct PhSet {
 };
 
 // Work item i < n_a: point list_a[i] (or i when list_a is null) of set SA; else point i - n_a of set SB.
-// NN: n at compile time, or 0.  Bound by the chain of rotation rounds (about 160 at 24 branches), and a round
+// NN: the branches.  Bound by the chain of rotation rounds (about 160 at 24 branches), and a round
 // by its rotation's dependent FP64 divisions and square roots (2460 cycles when one thread does them all
 // against 1900 for the two update passes).  So three warps share a rotation (angle, threshold, phase), and
 // one pass updates A on both sides by 2x2 blocks, each from and to registers; V follows one round behind,
 // in the warps that have no rotations.  Rows are padded to an odd length.  24 branches, 295 points: 741 -> 259 us against one
-// thread per rotation, passes of their own for columns, rows and V, and serial sums.
+// thread per rotation, passes of their own for columns, rows and V, and serial sums.  Every branch count has its
+// own instance: with n at run time the index arithmetic makes 3, 9, 12, 15, 18 and 21 branches 50, 169, 202, 294,
+// 489 and 664 us at 8^3, against 42, 138, 160, 231, 394 and 548 (the same bits).
 constexpr int PHT = 384;
 template <int NN>
 __global__ void __launch_bounds__(PHT, 2) k_phonons(PhArgs a, PhSet SA, const int* __restrict__ list_a, int n_a, PhSet SB,
@@ -78,7 +80,7 @@ __global__ void __launch_bounds__(PHT, 2) k_phonons(PhArgs a, PhSet SA, const in
                                                     const int* __restrict__ num, const double* __restrict__ mrs,
                                                     const double* __restrict__ temps) {
     extern __shared__ double2 sm[];
-    const int n = NN ? NN : a.n;
+    constexpr int n = NN;
     const int m = n + (n & 1), mh = m / 2;  // even size for round-robin pairing (index n is a dummy)
     const int ld = n | 1;        // row stride of A and V
     double2* A = sm;             // [n][ld]
@@ -624,10 +626,6 @@ int launch_phonons(spring_ctx* c, const PhSet& A, const int* list_a, int n_a, co
     SPRING_CHECK(launch_ewald(c, A.qpts, A.nq, list_a, n_a, B.qpts, B.nq, n_b, gamma_mode, &a.dd));
     const int n = c->ndof;
     const size_t smem = ph_smem(n);
-    if (smem > 48 * 1024) {
-        cudaFuncSetAttribute(k_phonons<24>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(k_phonons<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    }
     const int items = n_a + n_b;
     if (items == 0) return SPRING_OK;
     if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "phonons: injected launch failure");
@@ -646,12 +644,24 @@ int launch_phonons(spring_ctx* c, const PhSet& A, const int* list_a, int n_a, co
     const int blocks = items < 148 * 32 ? items : 148 * 32;
     // the rotations' three warps and a thread per V update
     const int threads = std::min(PHT, 96 + (n * ((n + 1) / 2) + 31) / 32 * 32);
-    if (n == 24)
-        k_phonons<24><<<blocks, threads, smem, c->stream>>>(a, A, list_a, n_a, B, n_b, c->d_fc2.p, c->d_fc2_idx.p,
-                                                            c->d_fc2_num.p, c->d_mass_rs.p, c->d_temps.p);
-    else
-        k_phonons<0><<<blocks, threads, smem, c->stream>>>(a, A, list_a, n_a, B, n_b, c->d_fc2.p, c->d_fc2_idx.p,
-                                                           c->d_fc2_num.p, c->d_mass_rs.p, c->d_temps.p);
+#define SPRING_PH(NN)                                                                                              \
+    case NN:                                                                                                       \
+        if (smem > 48 * 1024)                                                                                      \
+            cudaFuncSetAttribute(k_phonons<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);           \
+        k_phonons<NN><<<blocks, threads, smem, c->stream>>>(a, A, list_a, n_a, B, n_b, c->d_fc2.p, c->d_fc2_idx.p, \
+                                                            c->d_fc2_num.p, c->d_mass_rs.p, c->d_temps.p);         \
+        break
+    switch (n) {
+        SPRING_PH(3);
+        SPRING_PH(6);
+        SPRING_PH(9);
+        SPRING_PH(12);
+        SPRING_PH(15);
+        SPRING_PH(18);
+        SPRING_PH(21);
+        SPRING_PH(24);
+    }
+#undef SPRING_PH
     return launch_check(c, "k_phonons");
 }
 
