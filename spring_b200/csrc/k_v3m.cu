@@ -480,14 +480,12 @@ int launch_v3m(spring_ctx* c, const PairSet& ps, const Q0View& v, int q0_first, 
         k_v3m<NT, EPI><<<grid, 32 * MW, L.bytes, c->stream>>>(a, L, P, c->d_fc3_off.p, range, n_q0, ps.cap,    \
                                                               (int)npairs);                                    \
     } while (0)
-    const int nt = (c->ndof + 7) / 8;
+    const int nt = (c->ndof + 7) / 8;  // 2 or 3: at least 12 branches
     if (epi == 0) {
-        if (nt == 1) SPRING_V3M(1, 0);
-        else if (nt == 2) SPRING_V3M(2, 0);
+        if (nt == 2) SPRING_V3M(2, 0);
         else SPRING_V3M(3, 0);
     } else {
-        if (nt == 1) SPRING_V3M(1, 1);
-        else if (nt == 2) SPRING_V3M(2, 1);
+        if (nt == 2) SPRING_V3M(2, 1);
         else SPRING_V3M(3, 1);
     }
 #undef SPRING_V3M
