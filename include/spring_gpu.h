@@ -327,9 +327,10 @@ int spring_kappa_iter_gauss(spring_ctx* ctx, double sigma, double eps_k, int max
 /* ---- batched linewidths (several workloads, one run) ------------------- */
 /* A batch holds Gaussian three-phonon linewidth requests on several contexts
  * (different cells, meshes and temperature sets, on one device) and runs them
- * as one persistent FP64 kernel over all their (pair, s0-block) work items,
- * heaviest workloads first, captured with its zero-fills and the LW_Allq0
- * updates in one CUDA graph that later runs replay.  Each request has the
+ * in one call.  Requests that have a kernel of their own (below) run it; the
+ * (pair, s0-block) work items of the others go through one persistent FP64
+ * kernel, heaviest workloads first, captured with the zero-fills and its
+ * LW_Allq0 updates in one CUDA graph that later runs replay.  Each request has the
  * meaning of spring_linewidth3(ctx, i0_first, n_q0, SPRING_DELTA_GAUSS, sigma,
  * pol3, ...) on its context (the q0 loop body of main.f90:552-715 for many
  * inputs at once); no counterpart in the reference, which runs one input per
@@ -337,8 +338,9 @@ int spring_kappa_iter_gauss(spring_ctx* ctx, double sigma, double eps_k, int max
  * two-atom context set to SPRING_BF16 / SPRING_BF16X3 runs through the
  * tensor-core pass of spring_linewidth3 (same kernel, same results) right
  * after the graph, inside the same spring_batch_run, and FP64 requests on
- * two-atom cells and on cells of four or more atoms through their matrix kernels there; path requests
- * (spring_batch_add_path) are launched inside the graph. */
+ * two-atom cells and on cells of four or more atoms (where the layout holds
+ * the cell) through their matrix kernels there, one after the other; path
+ * requests (spring_batch_add_path) are launched inside the graph. */
 typedef struct spring_batch spring_batch;
 int spring_batch_create(spring_batch** batch);
 int spring_batch_destroy(spring_batch* batch);

@@ -1,21 +1,22 @@
 // Batched three-phonon linewidths: several workloads (cells, meshes,
-// temperature sets) in one persistent launch.
+// temperature sets) in one run.
 //
 // Each request is spring_linewidth3 with the Gaussian delta on its context
 // (q0 loop body of src/Kappa/Src/main.f90:552-715, ScatterMatEl /
-// ScatterProbability + CalculateLinewidth, ThirdOrder_m.f90:278-543).  The
-// requests' (pair, s0-block) work items are concatenated, heaviest workload
-// first, and one persistent CTA per slot takes items from a global counter
-// (`chunk` at a time), so uneven workloads (Ndof 6 and 24, 12^3 to 20^3 meshes,
-// 1 to 9 temperatures) share one launch without tail effects.  Each item runs
-// the any-cell FP64 V3 work item of k_v3.cu against its workload's
-// descriptor (staged in shared memory when the workload changes); requests that
-// the tensor-core pass or an FP64 matrix kernel takes (two-atom cells, k_v3s.cu;
-// 12 and more branches, k_v3m.cu) run it right after the graph.  The zero
-// fills, the kernel and the LW_Allq0 updates are captured in one CUDA graph.
+// ScatterProbability + CalculateLinewidth, ThirdOrder_m.f90:278-543).  Most
+// have a kernel of their own - two-atom cells (k_v3s.cu), 12 and more branches
+// (k_v3m.cu), BF16 and BF16x3 contexts (k_v3tc.cu) - and run it on their
+// context's stream, one after the other.  The (pair, s0-block) work items of
+// the rest (cells of one and three atoms, cells that the matrix kernel's layout
+// does not hold, contexts with the generic option, two-atom cells when the
+// configuration says so) are concatenated, heaviest workload first, and one
+// persistent CTA per slot takes items from a global counter (`chunk` at a time),
+// each against its workload's descriptor (staged in shared memory when the
+// workload changes).  The zero fills, that kernel and its LW_Allq0 updates are
+// captured in one CUDA graph; the kernels of the others follow it.
 //
-// Autotuner: threads per CTA, CTAs per SM, the s0 block of large cells and the
-// items per scheduler step are chosen by timing the batch itself (CUDA events),
+// Autotuner: the two-atom route, CTAs per SM, the s0 block of large cells and the
+// items per scheduler step are chosen by timing the whole run (CUDA events),
 // coordinate by coordinate; the choice is cached for the process by the batch
 // shape.
 // Roofline: FP64 FMA, as k_v3 (41.3 kflop per pair for Ndof 6; 8.0 Mflop for
