@@ -341,8 +341,7 @@ int upload(spring_batch* b, const std::vector<BatchDesc>& D, const std::vector<l
     }
     if (!b->d_ctr) BCHECK(bcuda(b, cudaMalloc(&b->d_ctr, sizeof(unsigned long long)), "batch counter"));
     if (smem > 227 * 1024) return bfail(b, SPRING_ERR_UNSUPPORTED, "batch work item needs %zu bytes of shared memory", smem);
-    BCHECK(bcuda(b, cudaFuncSetAttribute(spring::k_v3_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                 "batch shared memory"));
+    BCHECK(bcuda(b, spring::allow_smem(spring::k_v3_batch), "batch shared memory"));
     BCHECK(bcuda(b, cudaMemcpyAsync(b->d_desc, D.data(), sizeof(BatchDesc) * nw, cudaMemcpyHostToDevice, b->stream),
                  "batch descriptors"));
     BCHECK(bcuda(b, cudaMemcpyAsync(b->d_off, off.data(), sizeof(long long) * (nw + 1), cudaMemcpyHostToDevice,

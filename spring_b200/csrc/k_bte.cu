@@ -717,7 +717,7 @@ int bte_operator_run(spring_ctx* c, int rows, int nseg, const int* off, const in
     int sms = 148;
     if (in_smem) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-        cudaFuncSetAttribute(k_bteg_rows_sm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(k_bteg_rows_sm);
         SPRING_CHECK(dalloc(c, w.ke, cnt, "operator modes"));
         if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "bte: injected launch failure");
         k_bteg_encode<<<(int)std::min<long long>((cnt + 255) / 256, 148LL * 16), 256, 0, c->stream>>>(

@@ -405,7 +405,7 @@ int launch_ewald(spring_ctx* c, const double* qa, int nqa, const int* list_a, in
     a.z = D.z.p;
     a.mrs = c->d_mass_rs.p;
     const size_t smem = ew_smem_bytes(a.nb, a.J);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_ewald, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(k_ewald);
     if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "ewald: injected launch failure");
     const int threads = std::min(EW_THREADS, std::max(64, (std::max(6 * a.nb * a.nb * a.J, 2 * a.E) + 31) / 32 * 32));
     // Parts where one CTA's seven evaluations at Gamma would be the critical path (2 atoms, 286 points: 92 us

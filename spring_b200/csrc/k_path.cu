@@ -454,7 +454,7 @@ int path_prepare(spring_ctx* c, PathPlan& p, int n_path, const double* h_q0, con
     SPRING_CHECK(h2d(c, p.zc.p, h_zc, sizeof(int) * n_path, "path flags"));
     const size_t smem = v3p_smem(n, c->na3, n <= 12 ? n : 6);
     if (smem > 227 * 1024) return fail(c, SPRING_ERR_UNSUPPORTED, "path V3 tile needs %zu bytes of shared memory", smem);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_v3_path, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(k_v3_path);
     return SPRING_OK;
 }
 

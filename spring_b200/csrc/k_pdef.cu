@@ -524,7 +524,7 @@ int run_point_defect(spring_ctx* c, int i0_first, int n_q0, double* d_rate) {
         k_pd_green<<<items, gthreads, sizeof(double2) * gthreads, c->stream>>>(a, P.wgt.p, P.ph.evec.p, P.G.p);
         if ((rc = launch_check(c, "k_pd_green")) != SPRING_OK) break;
         const size_t sm = sizeof(double2) * 3 * E + sizeof(double) * E;
-        if (sm > 48 * 1024) cudaFuncSetAttribute(k_pd_tmatrix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (sm > 48 * 1024) allow_smem(k_pd_tmatrix);
         k_pd_tmatrix<<<items, 128, sm, c->stream>>>(a, P.G.p, P.vfc.p, P.vm.p, c->ph_irr.evec.p, c->ph_irr.omega.p,
                                                    P.gamma0.p, P.mat_inv_full ? 1 : 0, d_rate + (size_t)b * n, P.te0.p);
         if ((rc = launch_check(c, "k_pd_tmatrix")) != SPRING_OK) break;

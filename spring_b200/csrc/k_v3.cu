@@ -79,7 +79,7 @@ int launch_v3(spring_ctx* c, const PairSet& ps, const Q0View& v, int q0_first, i
     }
     const size_t smem = v3_smem(a.n, a.na, a.sb, a.nT);
     if (smem > 227 * 1024) return fail(c, SPRING_ERR_UNSUPPORTED, "V3 tile needs %zu bytes of shared memory", smem);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_v3<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(k_v3<EPI>);
     const long long items = npairs * a.nsb;
     if (items == 0) return SPRING_OK;
     if (items > 0x7fffffffLL) return fail(c, SPRING_ERR_UNSUPPORTED, "too many V3 work items");

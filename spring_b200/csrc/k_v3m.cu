@@ -476,7 +476,7 @@ int launch_v3m(spring_ctx* c, const PairSet& ps, const Q0View& v, int q0_first, 
     if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "v3: injected launch failure");
 #define SPRING_V3M(NT, EPI)                                                                                    \
     do {                                                                                                       \
-        cudaFuncSetAttribute(k_v3m<NT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, L.bytes);            \
+        allow_smem(k_v3m<NT, EPI>);                                                                            \
         k_v3m<NT, EPI><<<grid, 32 * MW, L.bytes, c->stream>>>(a, L, P, c->d_fc3_off.p, range, n_q0, ps.cap,    \
                                                               (int)npairs);                                    \
     } while (0)

@@ -1005,7 +1005,7 @@ int launch_tc(spring_ctx* c, TcArgs& a, const TcQ0& src, double* d_lw, double* d
     alignas(64) CUtensorMap tmA;
     SPRING_CHECK(make_tmap_a(c, &tmA));
     if (smem > 227 * 1024) return fail(c, SPRING_ERR_UNSUPPORTED, "tensor-core V3 needs %zu bytes of shared memory", smem);
-    cudaFuncSetAttribute(k_v3tc<SPLIT, FAST, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k_v3tc<SPLIT, FAST, MODE>);
     if (launch_injected(c)) return fail(c, SPRING_ERR_INJECTED, "v3tc: injected launch failure");
     k_v3tc<SPLIT, FAST, MODE><<<c->tc_grid, TC_THREADS, smem, c->stream>>>(
         a, tmA, c->d_tc_tiles.p, c->d_tc_rec.p, reinterpret_cast<const __nv_bfloat16*>(c->d_tc_b.p), src.om0,

@@ -829,8 +829,8 @@ int run_v4tc_gauss(spring_ctx* c, int q0_first, int n_q0, double sigma, const in
                c->stream>>>(nq, c->nT, rs, c->ph_grid.omega.p, c->ph_grid.oneby.p, c->ph_grid.nbe.p, c->d_v4_rec.p);
     SPRING_CHECK(launch_check(c, "k4_modes"));
     auto* kern = c->nT <= 1 ? k_v4tc<1> : c->nT <= 4 ? k_v4tc<4> : k_v4tc<9>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k4_bimg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bimg_smem);
+    allow_smem(kern);
+    allow_smem(k4_bimg);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
     const double os = 1.0 / sigma;

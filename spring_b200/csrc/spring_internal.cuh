@@ -341,6 +341,16 @@ int pin_wait(spring_ctx* c, const char* what);
 int launch_check(spring_ctx* c, const char* what);
 bool launch_injected(spring_ctx* c);
 
+// Lets a kernel whose dynamic shared memory differs from launch to launch take all that a CTA can have.  The limit
+// belongs to the kernel, not to the launch: set to one launch's size, another thread's larger launch fails.
+template <class K>
+cudaError_t allow_smem(K kern) {
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, kern);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       227 * 1024 - (int)a.sharedSizeBytes);
+}
+
 // ---- kernels (host launchers), each defined in its own .cu -------------------
 // k_mesh.cu
 int run_make_mesh(spring_ctx* c, const int shift[3], int zero_centered);
